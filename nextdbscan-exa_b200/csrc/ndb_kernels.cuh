@@ -79,7 +79,6 @@ __device__ __forceinline__ int job_of_point(const JobDev *__restrict__ jobs, int
 constexpr int kBlock = 256;
 constexpr int kMaxRowCells = 5;
 constexpr int kMaxListCap = 64;  // largest min_pts - 1 for which neighbour lists are kept
-constexpr int kSmemListCap = 16;  // lists up to this length are staged in shared memory  // cells per stencil row looked up together (2*xr+1 <= 5)
 constexpr int kWarpsPerBlock = kBlock / kWarp;
 // The count runs two warps per block: an item's candidate list can be thousands of
 // points long, and small blocks free their slot as soon as both items are done.
@@ -651,6 +650,64 @@ __host__ __device__ constexpr float gram_gamma() {
 }
 constexpr float kGramSigma = 8.0f / 16777216.0f;
 
+// ---------------------------------------------------------------------------
+// Hit masks: lane l holds, per candidate it owns, one bit per owned point (bit k =
+// point k is in range of the candidate).  A pair's bit is the sign of a difference,
+// appended by one funnel shift, so the pair loop has no vote, no compare and no
+// branch; a 32x32 bit transpose per 32 candidates then hands lane k the candidates
+// that hit point k, and lane k counts them and writes point k's list entries.  Steps
+// without any hit skip the transpose.
+// Packing: points that reached min_pts leave the item.  The remaining ones move to the
+// first slots (coordinates in shared memory, count and index with their lane), so the
+// pair loop always runs over a dense range of slots.
+// Bound: instruction issue and the FMA pipe (8-D early exit: 28 thread instructions per
+// pair, FMA pipe 63 %).  The form before this one voted and updated counts and lists per
+// pair and step (58 instructions per pair).  Measured on B200, before and after: 8-D 2M
+// early exit 4.47 -> 2.69 ms, 2-D 100k full counts 0.565 -> 0.213 ms, 3-D 1M full
+// counts 1.63 -> 0.89 ms, 5-D 300k full counts 2.84 -> 1.56 ms.
+// ---------------------------------------------------------------------------
+// (acc << 1) | sign bit of x
+__device__ __forceinline__ unsigned push_sign(unsigned acc, float x) {
+    unsigned r;
+    asm("shf.l.wrap.b32 %0, %1, %2, 1;" : "=r"(r) : "r"(__float_as_uint(x)), "r"(acc));
+    return r;
+}
+
+// The reference's sum with b given negated: x + (-b) is the reference's difference (or
+// its negative), so every square is the same.  Two dimensions go through one packed
+// subtraction and one packed multiplication; the additions stay scalar and in order
+// (a packed addition after a packed multiplication would be contracted).
+template <int D>
+__device__ __forceinline__ float dist_negated(const float (&x)[D], const float (&nb)[D]) {
+    float len = 0.0f;
+#pragma unroll
+    for (int k = 0; k + 1 < D; k += 2) {
+        const float2 t = __fadd2_rn(make_float2(x[k], x[k + 1]), make_float2(nb[k], nb[k + 1]));
+        const float2 q = __fmul2_rn(t, t);
+        len = k ? __fadd_rn(len, q.x) : q.x;
+        len = __fadd_rn(len, q.y);
+    }
+    if constexpr (D & 1) {
+        const float t = __fadd_rn(x[D - 1], nb[D - 1]);
+        len = D > 1 ? __fadd_rn(len, __fmul_rn(t, t)) : __fmul_rn(t, t);
+    }
+    return len;
+}
+
+// 32x32 bit-matrix transpose across a warp: lane l holds row l (bit c = column
+// c) on entry and column l (bit r = row r) on return.
+__device__ __forceinline__ unsigned transpose32(unsigned x, int lane) {
+    const unsigned masks[5] = {0x0000FFFFu, 0x00FF00FFu, 0x0F0F0F0Fu, 0x33333333u, 0x55555555u};
+#pragma unroll
+    for (int s = 0; s < 5; ++s) {
+        const int j = 16 >> s;
+        const unsigned m = masks[s];
+        const unsigned y = __shfl_xor_sync(kFull, x, j);
+        x = (lane & j) ? ((x & ~m) | ((y >> j) & m)) : ((x & m) | ((y << j) & ~m));
+    }
+    return x;
+}
+
 template <int D, bool EARLY, bool GRAM = false>
 __global__ void __launch_bounds__(kCountWarps * kWarp) count_kernel(
     const int2 *__restrict__ items, int64_t n_items, const int32_t *__restrict__ cell_start,
@@ -669,7 +726,8 @@ __global__ void __launch_bounds__(kCountWarps * kWarp) count_kernel(
     __shared__ __align__(16) float s_a[kCountWarps][GRAM ? kTile * P : 4];  // centred points
     __shared__ float s_n[kCountWarps][GRAM ? kTile : 1];                     // their squared norms
     __shared__ RowTable s_rows[kCountWarps];
-    __shared__ int s_list[kCountWarps][kTile * kSmemListCap];
+    __shared__ int s_j[kCountWarps][CH * kWarp];  // the step's candidates
+    __shared__ int2 s_move[kCountWarps][kTile];   // (index, count) of the points a packing moves
     const int lane = threadIdx.x & 31, wib = threadIdx.x >> 5;
     if (n_items_dev) n_items = *n_items_dev;  // a list whose length the device wrote
     const int64_t item_id = (int64_t)blockIdx.x * kCountWarps + wib;
@@ -685,15 +743,14 @@ __global__ void __launch_bounds__(kCountWarps * kWarp) count_kernel(
         dense_skip = J.linked;
         list_cap = J.list_cap;
     }
-    // lists of up to kSmemListCap entries are gathered in shared memory and written
-    // out only for the points that end below min_pts; longer ones go straight out
-    const bool smem_list = list_stride <= kSmemListCap;
-    int *sl = s_list[wib];
     if (EARLY && dense_skip && ce - cs >= min_pts) {
         if (lane < cnt) nn_sorted[p0 + lane] = ce - cs;
         return;
     }
+    if (!nbr_list) list_cap = 0;
     float *si = s_i[wib];
+    float *sa = s_a[wib];
+    int *sj = s_j[wib];
     RowTable &rt = s_rows[wib];
     float o[GRAM ? D : 1];  // GRAM: the item's first point, the origin of the centring
     float nmax = 0.0f;      // GRAM: largest |a|^2 of the item
@@ -701,6 +758,10 @@ __global__ void __launch_bounds__(kCountWarps * kWarp) count_kernel(
     if (lane < cnt) {
         float x[D];
         load_point<D>(xs, p0 + lane, x);
+        if constexpr (!GRAM) {
+#pragma unroll
+            for (int k = 0; k < D; ++k) x[k] = -x[k];  // for dist_negated
+        }
         store_point_smem<D>(si + lane * P, x);
         if constexpr (GRAM) {
             float a[D];
@@ -710,7 +771,7 @@ __global__ void __launch_bounds__(kCountWarps * kWarp) count_kernel(
                 a[k] = __fsub_rn(x[k], o[k]);
                 n = __fmaf_rn(a[k], a[k], n);
             }
-            store_point_smem<D>(s_a[wib] + lane * P, a);
+            store_point_smem<D>(sa + lane * P, a);
             s_n[wib][lane] = n;
             nmax = n;
         }
@@ -721,123 +782,155 @@ __global__ void __launch_bounds__(kCountWarps * kWarp) count_kernel(
     }
     const int total = gather_rows<false>(nbr + (int64_t)cell * n_rows, n_rows, cell_start, 0, rt, lane);
     __syncwarp();
-    // running counts in registers: lane k holds the count of the item's point k
-    int mycnt = 0;
-    unsigned long long pairs = 0, band = 0;  // pairs tested; GRAM: pairs rechecked in the guard band
-    // points still counting (EARLY: below min_pts), and points whose neighbour list
-    // is still filling (count below list_cap): both warp-uniform, updated per chunk
-    unsigned act = __ballot_sync(kFull, lane < cnt);
-    unsigned lst = nbr_list && list_cap > 0 ? act : 0u;
-    int row = 0;  // this lane's stencil row: its candidate index only grows
+    // slot k < nk holds point p0 + pid of lane k, whose count is lane k's mycnt
+    int nk = cnt, pid = lane, mycnt = 0;
+    unsigned long long pairs = 0;
+    unsigned band = 0;  // GRAM: pairs rechecked in the guard band
+    int row = 0;        // this lane's stencil row: its candidate index only grows
     for (int tb = 0; tb < total; tb += kWarp * CH) {
         int j[CH];
-        float xj[CH][D];  // GRAM: the centred candidate b = x_j - o
+        float xj[CH][D];  // GRAM: -2 times the centred candidate b = x_j - o
         float tlo[CH], thi[CH];
+        unsigned miss[CH], over[CH];  // bit k: out of range; GRAM: above the hit bound, above the miss bound
 #pragma unroll
         for (int c = 0; c < CH; ++c) {
             const int t = tb + c * kWarp + lane;
             j[c] = t < total ? row_next(rt, row, t) : -1;
-            if (j[c] >= 0) load_point<D>(xs, j[c], xj[c]);
-            else fill_nan<D>(xj[c]);  // NaN fails the predicate
+            load_point<D>(xs, max(j[c], 0), xj[c]);  // lanes past the end read a valid point and are masked below
+            miss[c] = over[c] = 0;
             if constexpr (GRAM) {
                 float nb = 0.0f;
 #pragma unroll
                 for (int k = 0; k < D; ++k) {
-                    xj[c][k] = __fsub_rn(xj[c][k], o[k]);
-                    nb = __fmaf_rn(xj[c][k], xj[c][k], nb);
+                    const float b = __fsub_rn(xj[c][k], o[k]);
+                    nb = __fmaf_rn(b, b, nb);
+                    xj[c][k] = __fmul_rn(-2.0f, b);
                 }
                 // hit when v = |a|^2 - 2 a.b <= tlo, miss when v > thi (see the bound above)
                 const float slack = __fadd_rn(__fmul_rn(gram_kappa<D>(), __fadd_rn(nmax, nb)),
                                               __fmul_rn(kGramSigma, e2));
-                tlo[c] = j[c] >= 0 ? __fsub_rn(__fsub_rn(__fmul_rn(e2, 1.0f - gram_gamma<D>()), nb), slack) : -INFINITY;
-                thi[c] = j[c] >= 0 ? __fadd_rn(__fsub_rn(__fmul_rn(e2, 1.0f + gram_gamma<D>()), nb), slack) : -INFINITY;
+                tlo[c] = __fsub_rn(__fsub_rn(__fmul_rn(e2, 1.0f - gram_gamma<D>()), nb), slack);
+                thi[c] = __fadd_rn(__fsub_rn(__fmul_rn(e2, 1.0f + gram_gamma<D>()), nb), slack);
             }
         }
-        int active = 0;
-        for (unsigned it = act; it; it &= it - 1) {
-            const int k = __ffs(it) - 1;
-            bool hit[CH];
-            unsigned m[CH];
+#pragma unroll 2
+        for (int k = nk - 1; k >= 0; --k) {
             if constexpr (GRAM) {
                 float a[D];
-                load_point_smem<D>(s_a[wib] + k * P, a);
+                load_point_smem<D>(sa + k * P, a);
                 const float na = s_n[wib][k];
-                bool inband[CH];
 #pragma unroll
                 for (int c = 0; c < CH; ++c) {
-                    // four independent FMA chains (the bound holds for any order of
-                    // the sum), joined by three additions
-                    float g4[4] = {0.0f, 0.0f, 0.0f, 0.0f};
+                    // two FMA chains over the even and the odd dimensions, one starting
+                    // at |a|^2 (within the bound's share for forming v), joined by one addition
+                    float2 v2 = make_float2(na, 0.0f);
 #pragma unroll
-                    for (int q = 0; q < D; ++q) g4[q & 3] = __fmaf_rn(a[q], xj[c][q], g4[q & 3]);
-                    const float g = __fadd_rn(__fadd_rn(g4[0], g4[1]), __fadd_rn(g4[2], g4[3]));
-                    const float v = __fmaf_rn(-2.0f, g, na);
-                    hit[c] = v <= tlo[c];
-                    inband[c] = !hit[c] && v <= thi[c];
-                }
-                if (inband[0] || (CH > 1 && inband[CH - 1])) {
-                    // the guard band (rare): the reference's own sum decides
-                    float xi[D];
-                    load_point_smem<D>(si + k * P, xi);
-#pragma unroll
-                    for (int c = 0; c < CH; ++c) {
-                        if (!inband[c]) continue;
-                        float xr[D];
-                        load_point<D>(xs, j[c], xr);
-                        hit[c] = in_range<D>(xi, xr, e2);
-                        ++band;
-                    }
+                    for (int q = 0; q + 1 < D; q += 2)
+                        v2 = __ffma2_rn(make_float2(a[q], a[q + 1]), make_float2(xj[c][q], xj[c][q + 1]), v2);
+                    if constexpr (D & 1) v2.x = __fmaf_rn(a[D - 1], xj[c][D - 1], v2.x);
+                    const float v = __fadd_rn(v2.x, v2.y);
+                    miss[c] = push_sign(miss[c], __fsub_rn(tlo[c], v));
+                    over[c] = push_sign(over[c], __fsub_rn(thi[c], v));
                 }
             } else {
                 float xi[D];
                 load_point_smem<D>(si + k * P, xi);
-#pragma unroll
-                for (int c = 0; c < CH; ++c) hit[c] = in_range<D>(xi, xj[c], e2);
-            }
-#pragma unroll
-            for (int c = 0; c < CH; ++c) m[c] = __ballot_sync(kFull, hit[c]);
-            // the first list_cap neighbours of each point; complete for every point
-            // whose count stays below min_pts (list_cap = min_pts - 1)
-            if ((lst >> k) & 1u) {
-                int base = __shfl_sync(kFull, mycnt, k);
+                // the reference's sum; e2 - len is negative exactly when len > e2 (the
+                // difference of two different floats never rounds to zero, and
+                // coordinates in the grid are finite, so len is never NaN)
 #pragma unroll
                 for (int c = 0; c < CH; ++c) {
-                    const int slot = base + __popc(m[c] & lanemask_lt());
-                    if (hit[c] && slot < list_cap) {
-                        if (smem_list) sl[k * kSmemListCap + slot] = j[c];
-                        else nbr_list[(int64_t)(p0 + k) * list_stride + slot] = j[c];
-                    }
-                    base += __popc(m[c]);
+                    const float len = dist_negated<D>(xj[c], xi);
+                    miss[c] = push_sign(miss[c], __fsub_rn(e2, len));
                 }
             }
-            int got = 0;
+        }
+        pairs += (unsigned long long)nk * (unsigned long long)min(kWarp * CH, total - tb);
+        const unsigned slots = kFull >> (kWarp - nk);  // nk >= 1
+        unsigned hb[CH];
 #pragma unroll
-            for (int c = 0; c < CH; ++c) got += __popc(m[c]);
-            if (lane == k) mycnt += got;
-            ++active;
+        for (int c = 0; c < CH; ++c) {
+            hb[c] = j[c] >= 0 ? ~miss[c] & slots : 0u;
+            if constexpr (GRAM) {
+                // the guard band (rare): the reference's own sum decides
+                unsigned bb = j[c] >= 0 ? miss[c] & ~over[c] & slots : 0u;
+                if (bb) {
+                    band += __popc(bb);
+                    float xr[D];
+                    load_point<D>(xs, j[c], xr);
+                    for (; bb; bb &= bb - 1) {
+                        const int k = __ffs(bb) - 1;
+                        float xi[D];
+                        load_point_smem<D>(si + k * P, xi);
+                        if (in_range<D>(xi, xr, e2)) hb[c] |= 1u << k;
+                    }
+                }
+            }
         }
-        pairs += (unsigned long long)active * (unsigned long long)min(kWarp * CH, total - tb);
-        if (lst) lst &= __ballot_sync(kFull, mycnt < list_cap);
-        if (EARLY) {
-            act = __ballot_sync(kFull, lane < cnt && mycnt < min_pts);
-            if (!act) break;
+        if (!__any_sync(kFull, (hb[0] | hb[CH - 1]) != 0)) continue;
+        if (list_cap > 0) {
+#pragma unroll
+            for (int c = 0; c < CH; ++c) sj[c * kWarp + lane] = j[c];
+            __syncwarp();
         }
-    }
-    const int mine = lane < cnt ? mycnt : 0;
-    if (lane < cnt) nn_sorted[p0 + lane] = mine;
-    if (nbr_list && smem_list) {
+#pragma unroll
+        for (int c = 0; c < CH; ++c) {
+            unsigned m = transpose32(hb[c], lane);  // the candidates that hit this lane's point
+            int slot = mycnt;
+            mycnt += __popc(m);
+            // the first list_cap neighbours of each point; complete for every point
+            // whose count stays below min_pts (list_cap = min_pts - 1)
+            for (; m && slot < list_cap; m &= m - 1, ++slot)
+                nbr_list[(int64_t)(p0 + pid) * list_stride + slot] = sj[c * kWarp + __ffs(m) - 1];
+        }
         __syncwarp();
-        // every point's list: the border step reads the non-cores', the union
-        // starts from the cores' (for cell units, the items the count ran)
-        if (lane < cnt) {
-            const int len = min(mine, list_cap);
-            for (int q = 0; q < len; ++q) nbr_list[(int64_t)(p0 + lane) * list_stride + q] = sl[lane * kSmemListCap + q];
+        if (EARLY) {
+            const bool stay = lane < nk && mycnt < min_pts;
+            const unsigned act = __ballot_sync(kFull, stay);
+            const int left = __popc(act);
+            if (left == nk) continue;
+            if (lane < nk && !stay) nn_sorted[p0 + pid] = mycnt;
+            nk = left;
+            if (nk == 0) break;
+            const int dst = __popc(act & lanemask_lt());
+            float x[P], a[GRAM ? P : 1];
+            float n = 0.0f;
+            if (stay) {
+#pragma unroll
+                for (int q = 0; q < P; ++q) x[q] = si[lane * P + q];
+                if constexpr (GRAM) {
+#pragma unroll
+                    for (int q = 0; q < P; ++q) a[q] = sa[lane * P + q];
+                    n = s_n[wib][lane];
+                }
+            }
+            __syncwarp();
+            if (stay) {
+#pragma unroll
+                for (int q = 0; q < P; ++q) si[dst * P + q] = x[q];
+                if constexpr (GRAM) {
+#pragma unroll
+                    for (int q = 0; q < P; ++q) sa[dst * P + q] = a[q];
+                    s_n[wib][dst] = n;
+                }
+                s_move[wib][dst] = make_int2(pid, mycnt);
+            }
+            __syncwarp();
+            if (lane < nk) {
+                const int2 mv = s_move[wib][lane];
+                pid = mv.x;
+                mycnt = mv.y;
+            } else {
+                mycnt = 0;
+            }
+            __syncwarp();
         }
     }
+    if (lane < nk) nn_sorted[p0 + pid] = mycnt;
     if (lane == 0 && pairs) atomicAdd(pair_counter, pairs);
     if constexpr (GRAM) {
-        band = __reduce_add_sync(kFull, (unsigned)band);
-        if (lane == 0 && band) atomicAdd(band_counter, band);
+        band = __reduce_add_sync(kFull, band);
+        if (lane == 0 && band) atomicAdd(band_counter, (unsigned long long)band);
     }
 }
 

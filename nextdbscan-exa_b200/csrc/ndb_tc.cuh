@@ -182,14 +182,6 @@ __device__ __forceinline__ void tmem_ld16(uint32_t taddr, uint32_t (&v)[32]) {
         : "memory");
 }
 
-// (acc << 1) | sign bit of x: one funnel shift appends a sign bit to a mask built
-// from the last column down, so that column c ends at bit c
-__device__ __forceinline__ unsigned push_sign(unsigned acc, float x) {
-    unsigned r;
-    asm("shf.l.wrap.b32 %0, %1, %2, 1;" : "=r"(r) : "r"(__float_as_uint(x)), "r"(acc));
-    return r;
-}
-
 // Classification of the first NC accumulator columns of this thread's TMEM lane (one
 // candidate j) against its bounds tlo, thi of the comparison value v_c = n_c - 2 g_c.
 // v is formed negated, two columns per packed FMA: w_c = 2 g_c + (-n_c) is -v_c
@@ -223,20 +215,6 @@ __device__ __forceinline__ void classify(const uint32_t (&g)[32], const float *s
     }
     mlo = ml;
     mhi = mh;
-}
-
-// 32x32 bit-matrix transpose across a warp: lane l holds row l (bit c = column
-// c) on entry and column l (bit r = row r) on return.
-__device__ __forceinline__ unsigned transpose32(unsigned x, int lane) {
-    const unsigned masks[5] = {0x0000FFFFu, 0x00FF00FFu, 0x0F0F0F0Fu, 0x33333333u, 0x55555555u};
-#pragma unroll
-    for (int s = 0; s < 5; ++s) {
-        const int j = 16 >> s;
-        const unsigned m = masks[s];
-        const unsigned y = __shfl_xor_sync(kFull, x, j);
-        x = (lane & j) ? ((x & ~m) | ((y >> j) & m)) : ((x & m) | ((y << j) & ~m));
-    }
-    return x;
 }
 
 // Operand tile in shared memory: element (row r, k) of an R-row tile at

@@ -1,0 +1,45 @@
+"""The neighbour count where its work items change shape: cells of 1 to 70 points (items
+are 32 points of a cell), candidate lists that end inside a step, neighbour lists from
+one entry to past their cap, points of one item finishing at different steps.  Every
+count kernel against the oracle, bit for bit (integers: no tolerance)."""
+import numpy as np
+import pytest
+
+import oracle
+
+pytestmark = pytest.mark.gpu
+
+
+def clumps(d, sizes, seed):
+    """Clumps of the given sizes on a coarse lattice: inside a clump distances range from
+    0 to about 2 eps (eps = 1), and neighbouring clumps just touch."""
+    rng = np.random.default_rng(seed)
+    out = []
+    for q, m in enumerate(sizes):
+        c = np.zeros(d)
+        c[0], c[min(1, d - 1)] = 1.5 * (q % 5), c[min(1, d - 1)] + 1.5 * (q // 5)
+        out.append(c + rng.uniform(-0.9, 0.9, (m, d)) / np.sqrt(d))
+    x = np.concatenate(out)
+    return np.ascontiguousarray(x[rng.permutation(len(x))].astype(np.float32))
+
+
+SIZES = (1, 2, 5, 31, 32, 33, 63, 64, 65, 70, 7, 15, 16, 17, 96, 1, 40, 200, 3, 129)
+
+
+@pytest.mark.parametrize("d", [1, 2, 3, 4, 5, 7, 8, 9, 13, 16])
+@pytest.mark.parametrize("form", ["exact", "gram", "tensor"])
+def test_count_items_against_oracle(ctx, d, form):
+    if form != "exact" and d < 8:
+        pytest.skip("the filters are built for d >= 8")
+    x = clumps(d, SIZES, 100 + d)
+    kw = {"exact_count": form == "exact", "gram_filter": form == "gram", "tensor_filter": form == "tensor"}
+    for m in (1, 2, 17, 33, 66):
+        nn_o, ci_o, meta = oracle.grid(x, 1.0, m)
+        for full in (True, False):
+            nn, ci, r = ctx.run(x, 1.0, m, full_count=full, **kw)
+            if full:
+                np.testing.assert_array_equal(nn, nn_o)
+            else:
+                np.testing.assert_array_equal(np.minimum(nn, m), np.minimum(nn_o, m))
+            np.testing.assert_array_equal(ci, ci_o)
+            assert (r.clusters, r.noise, r.core_count) == (meta["clusters"], meta["noise"], meta["cores"])
