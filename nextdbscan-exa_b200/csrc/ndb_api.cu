@@ -143,7 +143,7 @@ constexpr size_t kSmallCountersOff = 512;    // u64[12]: 0 clusters 1 noise 2 co
                                              // 5 band pairs 6 work counter of the persistent count kernel
                                              // 8..11 filter audit (tc::audit_tile)
 constexpr int kCounters = 12;
-constexpr size_t kSmallScalarOff = 1024;     // u32[8]: 0 n_cells 1 n_items 2 n_cores
+constexpr size_t kSmallScalarOff = 1024;     // u32[8]: 0 n_cells 1 n_items 2 n_cores 4, 5 split items 6 union segments
 constexpr size_t kSmallErrOff = 1536;        // int
 constexpr size_t kSmallStencilOff = 2048;    // int4[kMaxRows]: stencil rows of the current job
 constexpr size_t kSmallBytes = 4096;
@@ -789,6 +789,35 @@ void classify_dispatch(ndb_ctx *ctx, const Plan &pl) {
 // ---------------------------------------------------------------------------
 // phase 2
 // ---------------------------------------------------------------------------
+// Point units: the unions beyond the neighbour lists.  comp_min holds the roots'
+// snapshot meanwhile, cell_cid the cells' roots, flags and pos the segment list (free
+// once the cells are built; n entries, at least one per item).
+template <int D>
+void union_points_phase(ndb_ctx *ctx, int64_t nv, int64_t n_cells, int64_t n_items, int n_rows, float e2,
+                        const JobDev *jobs, const int32_t *cell_job) {
+    cudaStream_t st = ctx->stream;
+    int *err = small_at<int>(ctx, kSmallErrOff);
+    uint32_t *n_seg = small_at<uint32_t>(ctx, kSmallScalarOff) + 6;
+    fill_bytes(ctx, ctx->cell_cid.ptr, 0xff, (size_t)n_cells * sizeof(int32_t), st);  // -1
+    fill_bytes(ctx, n_seg, 0, sizeof(uint32_t), st);
+    ++launch_counter(), flatten_points_kernel<<<blocks_for(nv), kBlock, 0, st>>>(
+        ctx->parent.as<int32_t>(), nv, err, ctx->pcell.as<int32_t>(), ctx->core_sorted.as<uint8_t>(),
+        ctx->comp_min.as<int32_t>(), ctx->cell_cid.as<int32_t>());
+    cudaEventRecord(ctx->kev[4], st);
+    const uint32_t seg_cap = (uint32_t)(std::min(ctx->flags.bytes, ctx->pos.bytes) / sizeof(uint32_t));
+    uint32_t *seg_item = ctx->flags.as<uint32_t>(), *seg_part = ctx->pos.as<uint32_t>();
+    ++launch_counter(), union_select_kernel<<<blocks_for(n_items * kWarp), kBlock, 0, st>>>(
+        ctx->items.as<int2>(), n_items, ctx->cell_start.as<int32_t>(), ctx->nbr.as<int2>(), n_rows,
+        ctx->cell_cid.as<int32_t>(), ctx->comp_min.as<int32_t>(), seg_item, seg_part,
+        seg_cap, n_seg);
+    ++launch_counter(), union_scan_kernel<D><<<(unsigned)ctx->sm_count * 16, kCountWarps * kWarp, 0, st>>>(
+        ctx->items.as<int2>(), n_items, ctx->cell_start.as<int32_t>(), ctx->nbr.as<int2>(), n_rows,
+        ctx->xs.as<float>(), e2, ctx->cell_cid.as<int32_t>(), ctx->comp_min.as<int32_t>(), ctx->parent.as<int32_t>(),
+        seg_item, seg_part, seg_cap, n_seg, small_at<unsigned long long>(ctx, kSmallCountersOff) + 3, err, jobs, cell_job);
+    ++launch_counter(), fill_kernel<<<blocks_for(nv), kBlock, 0, st>>>(ctx->comp_min.as<int32_t>(), nv, kNoCluster);
+    ck(ctx, cudaGetLastError());
+}
+
 // Border points: the minimum id over the cores in range, from the count's
 // neighbour lists when there are lists, else by a stencil scan.  Reads the core ids
 // in ci_sorted (point units) or cell_cid (cell units).
@@ -863,24 +892,12 @@ void labels_phase(ndb_ctx *ctx) {
                                                                                    kNoCluster);
         }
         else {
-            if (ctx->list_cap > 0) {
+            if (ctx->list_cap > 0)
                 ++launch_counter(), union_lists_kernel<<<blocks_for(nv), kBlock, 0, st>>>(
                     nv, ctx->nn_sorted.as<int32_t>(), ctx->nbr_list.as<int32_t>(), ctx->list_cap, ctx->list_cap,
                     ctx->core_sorted.as<uint8_t>(), ctx->parent.as<int32_t>(), err, nullptr, nullptr,
                     ctx->pcell.as<int32_t>(), 0, 0, ctx->cell_start.as<int32_t>(), ctx->min_pts);
-                ++launch_counter(), flatten_kernel<<<blocks_for(n_units), kBlock, 0, st>>>(ctx->parent.as<int32_t>(),
-                                                                                          n_units, err);
-            }
-            fill_bytes(ctx, ctx->cell_cid.ptr, 0xff, (size_t)n_cells * sizeof(int32_t), st);  // -1
-            ++launch_counter(), cell_root_kernel<<<blocks_for(nv), kBlock, 0, st>>>(
-                nv, ctx->pcell.as<int32_t>(), ctx->core_sorted.as<uint8_t>(), ctx->parent.as<int32_t>(),
-                ctx->cell_cid.as<int32_t>());
-            cudaEventRecord(ctx->kev[4], st);
-            const unsigned pgrid = (unsigned)((ctx->n_items + kCountWarps - 1) / kCountWarps);
-            ++launch_counter(), union_points_kernel<D><<<pgrid, kCountWarps * kWarp, 0, st>>>(
-                ctx->items.as<int2>(), ctx->n_items, ctx->cell_start.as<int32_t>(), ctx->nbr.as<int2>(), ctx->n_rows,
-                ctx->xs.as<float>(), ctx->e2, ctx->core_sorted.as<uint8_t>(), ctx->cell_has_core.as<uint8_t>(),
-                ctx->parent.as<int32_t>(), counters + 3, err, nullptr, nullptr, ctx->cell_cid.as<int32_t>());
+            union_points_phase<D>(ctx, nv, n_cells, ctx->n_items, ctx->n_rows, ctx->e2, nullptr, nullptr);
         }
         ck(ctx, cudaGetLastError());
     }
@@ -1791,23 +1808,12 @@ void run_group_keys(ndb_ctx *ctx, ndb_job *jobs, const std::vector<int> &members
             ++launch_counter(), fill_kernel<<<blocks_for(n_units), kBlock, 0, st>>>(ctx->comp_min.as<int32_t>(), n_units,
                                                                                    kNoCluster);
         } else {
-            if (bp.list_stride > 0) {
+            if (bp.list_stride > 0)
                 ++launch_counter(), union_lists_kernel<<<blocks_for(nv), kBlock, 0, st>>>(
                     nv, ctx->nn_sorted.as<int32_t>(), list, 0, bp.list_stride, ctx->core_sorted.as<uint8_t>(),
                     ctx->parent.as<int32_t>(), err, jobs_dev, cell_job, ctx->pcell.as<int32_t>(), 0, 0,
                     ctx->cell_start.as<int32_t>(), 0);
-                ++launch_counter(), flatten_kernel<<<blocks_for(n_units), kBlock, 0, st>>>(ctx->parent.as<int32_t>(),
-                                                                                          n_units, err);
-            }
-            fill_bytes(ctx, ctx->cell_cid.ptr, 0xff, (size_t)n_cells * sizeof(int32_t), st);  // -1
-            ++launch_counter(), cell_root_kernel<<<blocks_for(nv), kBlock, 0, st>>>(
-                nv, ctx->pcell.as<int32_t>(), ctx->core_sorted.as<uint8_t>(), ctx->parent.as<int32_t>(),
-                ctx->cell_cid.as<int32_t>());
-            const unsigned pgrid = (unsigned)((n_items + kCountWarps - 1) / kCountWarps);
-            ++launch_counter(), union_points_kernel<D><<<pgrid, kCountWarps * kWarp, 0, st>>>(
-                ctx->items.as<int2>(), n_items, ctx->cell_start.as<int32_t>(), ctx->nbr.as<int2>(), n_rows,
-                ctx->xs.as<float>(), 0.0f, ctx->core_sorted.as<uint8_t>(), ctx->cell_has_core.as<uint8_t>(),
-                ctx->parent.as<int32_t>(), counters + 3, err, jobs_dev, cell_job, ctx->cell_cid.as<int32_t>());
+            union_points_phase<D>(ctx, nv, n_cells, n_items, n_rows, 0.0f, jobs_dev, cell_job);
         }
         ck(ctx, cudaGetLastError());
     }

@@ -1280,17 +1280,116 @@ __global__ void __launch_bounds__(kBlock) union_cells_kernel(
 }
 
 // ---------------------------------------------------------------------------
-// Union-find over core points (general grids).  Pairs are visited once (j > i in
-// sorted order); a pair whose j already shares i's root is skipped before the
-// predicate.
+// Union-find over core points (general grids), after the list unions and a flatten
+// that left every core's root in a snapshot (snap: root, -1 for non-cores; cell_root:
+// the one root of each cell's cores, -1 without cores, -2 when they differ).  Pairs
+// are visited once (the candidate behind the item's point in sorted order).
+//
+// Two kernels.  union_select_kernel, one warp per item, finds the candidates that can
+// still matter: when the item's cores share one root, only the cells that are not
+// wholly under that root; else every stencil row.  It cuts them into segments of
+// kUnionSegment candidates and lists those; union_scan_kernel walks the listed
+// segments, one warp each.  Most items need nothing and a few need their whole
+// stencil, so one warp per item left the GPU idle behind the longest items
+// (5 % of warps resident at d = 16).  A stale snapshot root only makes a candidate
+// looked at, never skipped.
+//
+// Bound: latency of the snapshot loads; a step whose candidates all hang under the
+// item's root costs one coalesced load per lane.  Segment length: long enough that the
+// rebuilt row table (about a microsecond) does not show, short enough to fill the GPU.
+// Measured on B200 against one kernel with a warp per item, which read core flag,
+// parent and grandparent of every candidate: 16-D 200k 1.71 -> 0.28 ms, 8-D 2M 1.84 ->
+// 0.59 ms, 5-D 300k 0.36 -> 0.09 ms.
 // ---------------------------------------------------------------------------
+constexpr int kUnionSegment = 1024;
+
+// Candidate ranges of an item at and behind its first point p0; returns their total.
+// root: the snapshot root of this lane's point (-1 without one).  Depends on the
+// snapshot only, so both kernels build the same table.
+__device__ __forceinline__ int union_rows(int A, int p0, int root, const int32_t *__restrict__ cell_start,
+                                          const int2 *__restrict__ nbr, int n_rows,
+                                          const int32_t *__restrict__ cell_root, RowTable &rt, RowTable &rc,
+                                          int *need_cells, int lane) {
+    const int2 *nbr_row = nbr + (int64_t)A * n_rows;
+    const unsigned cores = __ballot_sync(kFull, root >= 0);
+    if (!cores) return 0;
+    const int root0 = __shfl_sync(kFull, root, __ffs(cores) - 1);
+    if (__all_sync(kFull, root < 0 || root == root0)) {
+        const int tcells = gather_rows<true>(nbr_row, n_rows, cell_start, A, rc, lane);
+        int n_need = 0;
+        for (int cb = 0; cb < tcells; cb += kWarp) {
+            const int t = cb + lane;
+            const int c = t < tcells ? row_lookup(rc, n_rows, t) : -1;
+            const int r = c >= 0 ? __ldg(cell_root + c) : -1;
+            const bool need = r != -1 && r != root0;
+            const unsigned m = __ballot_sync(kFull, need);
+            const int slot = n_need + __popc(m & lanemask_lt());
+            if (need && slot < kWarp) need_cells[slot] = c;
+            n_need += __popc(m);
+        }
+        __syncwarp();
+        if (n_need <= kWarp) {
+            int start = 0, len = 0;
+            if (lane < n_need) {
+                const int c = need_cells[lane];
+                start = max(cell_start[c], p0);
+                len = max(cell_start[c + 1] - start, 0);
+            }
+            return build_rows(start, len, n_need, rt, lane);
+        }
+    }
+    int start = 0, len = 0;
+    if (lane < n_rows) {
+        const int2 cr = nbr_row[lane];
+        if (cr.x < cr.y) {
+            start = max(cell_start[cr.x], p0);
+            len = max(cell_start[cr.y] - start, 0);
+        }
+    }
+    return build_rows(start, len, n_rows, rt, lane);
+}
+
+__global__ void __launch_bounds__(kBlock) union_select_kernel(
+    const int2 *__restrict__ items, int64_t n_items, const int32_t *__restrict__ cell_start,
+    const int2 *__restrict__ nbr, int n_rows, const int32_t *__restrict__ cell_root,
+    const int32_t *__restrict__ snap, uint32_t *__restrict__ seg_item, uint32_t *__restrict__ seg_part,
+    uint32_t seg_cap, uint32_t *__restrict__ n_seg) {
+    __shared__ RowTable s_rows[kWarpsPerBlock];
+    __shared__ RowTable s_cells[kWarpsPerBlock];
+    __shared__ int s_need[kWarpsPerBlock][kWarp];
+    const int lane = threadIdx.x & 31, wib = threadIdx.x >> 5;
+    const int64_t item_id = (int64_t)blockIdx.x * kWarpsPerBlock + wib;
+    if (item_id >= n_items) return;
+    const int2 item = items[item_id];
+    const int A = item.x, p0 = item.y;
+    if (__ldg(cell_root + A) == -1) return;
+    const int cnt = min(kTile, cell_start[A + 1] - p0);
+    const int root = lane < cnt ? __ldg(snap + p0 + lane) : -1;
+    const int total = union_rows(A, p0, root, cell_start, nbr, n_rows, cell_root, s_rows[wib], s_cells[wib],
+                                 s_need[wib], lane);
+    const int parts = (int)(((unsigned)total + kUnionSegment - 1) / kUnionSegment);
+    uint32_t base = 0;
+    if (lane == 0 && parts) base = atomicAdd(n_seg, (uint32_t)parts);
+    base = __shfl_sync(kFull, base, 0);
+    for (int q = lane; q < parts; q += kWarp) {
+        const uint64_t at = (uint64_t)base + (uint64_t)q;
+        if (at < seg_cap) {
+            seg_item[at] = (uint32_t)item_id;
+            seg_part[at] = (uint32_t)q;
+        }
+    }
+}
+
+// When the segments overran their list (possible only without neighbour lists, on
+// dense data), every item is walked whole instead.
 template <int D>
-__global__ void __launch_bounds__(kCountWarps * kWarp) union_points_kernel(
+__global__ void __launch_bounds__(kCountWarps * kWarp) union_scan_kernel(
     const int2 *__restrict__ items, int64_t n_items, const int32_t *__restrict__ cell_start,
     const int2 *__restrict__ nbr, int n_rows, const float *__restrict__ xs, float e2,
-    const uint8_t *__restrict__ core_sorted, const uint8_t *__restrict__ cell_has_core,
-    int32_t *parent, unsigned long long *__restrict__ pair_counter, int *err, const JobDev *__restrict__ jobs,
-    const int32_t *__restrict__ cell_job, const int32_t *__restrict__ cell_root) {
+    const int32_t *__restrict__ cell_root, const int32_t *__restrict__ snap, int32_t *parent,
+    const uint32_t *__restrict__ seg_item, const uint32_t *__restrict__ seg_part, uint32_t seg_cap,
+    const uint32_t *__restrict__ n_seg, unsigned long long *__restrict__ pair_counter, int *err, const JobDev *__restrict__ jobs,
+    const int32_t *__restrict__ cell_job) {
     constexpr int P = Stride<D>::P;
     __shared__ __align__(16) float s_i[kCountWarps][kTile * P];
     __shared__ int s_idx[kCountWarps][kTile];
@@ -1299,130 +1398,102 @@ __global__ void __launch_bounds__(kCountWarps * kWarp) union_points_kernel(
     __shared__ RowTable s_cells[kCountWarps];
     __shared__ int s_need[kCountWarps][kWarp];
     const int lane = threadIdx.x & 31, wib = threadIdx.x >> 5;
-    const int64_t item_id = (int64_t)blockIdx.x * kCountWarps + wib;
-    if (item_id >= n_items) return;
-    const int2 item = items[item_id];
-    const int A = item.x, p0 = item.y;
-    if (!cell_has_core[A]) return;
-    if (jobs) e2 = jobs[cell_job[A]].e2;
-    const int cnt = min(kTile, cell_start[A + 1] - p0);
     float *si = s_i[wib];
     int *sidx = s_idx[wib];
     int *sroot = s_root[wib];
     RowTable &rt = s_rows[wib];
-    const int nc = load_item_cores<D>(xs, core_sorted, p0, cnt, true, si, sidx, lane);
-    if (nc == 0) return;
-    // Cell-level pass (cell_root: the one root of each cell's cores, -2 when they
-    // differ, -1 without cores; taken after the list unions).  When the item's
-    // cores share root r, every candidate cell whose cores all hang under r is
-    // already joined to the item and is skipped whole; only the remaining cells'
-    // points are scanned.  A stale cell root (a root since hooked elsewhere) only
-    // makes a cell scanned, never skipped.
-    int total = -1, rows = n_rows;
-    if (cell_root) {
-        const int myroot = lane < nc ? uf_find(parent, sidx[lane], err) : -1;
-        const int root0 = __shfl_sync(kFull, myroot, 0);
-        if (__all_sync(kFull, lane >= nc || myroot == root0)) {
-            RowTable &rc = s_cells[wib];
-            const int tcells = gather_rows<true>(nbr + (int64_t)A * n_rows, n_rows, cell_start, A, rc, lane);
-            int n_need = 0;
-            bool overflow = false;
-            for (int cb = 0; cb < tcells; cb += kWarp) {
-                const int t = cb + lane;
-                const int c = t < tcells ? row_lookup(rc, n_rows, t) : -1;
-                const bool need = c >= 0 && cell_has_core[c] && __ldg(cell_root + c) != root0;
-                const unsigned m = __ballot_sync(kFull, need);
-                if (n_need + __popc(m) > kWarp) {
-                    overflow = true;
-                    break;
-                }
-                if (need) s_need[wib][n_need + __popc(m & lanemask_lt())] = c;
-                n_need += __popc(m);
-            }
-            __syncwarp();
-            if (!overflow) {
-                if (n_need == 0) return;
-                int start = 0, len = 0;
-                if (lane < n_need) {
-                    const int c = s_need[wib][lane];
-                    start = cell_start[c];
-                    len = cell_start[c + 1] - start;
-                }
-                total = build_rows(start, len, n_need, rt, lane);
-                rows = n_need;
-            }
-        }
-    }
-    if (total < 0) total = gather_rows<false>(nbr + (int64_t)A * n_rows, n_rows, cell_start, 0, rt, lane);
     unsigned long long pairs = 0;
-    int cur = 0;  // this lane's stencil row
-    // the next step's candidate, its core flag and its parent are loaded one step
-    // ahead (independent loads), so their latency overlaps this step's root refresh
-    // and tests; a parent read early is still an ancestor, so a stale one can only
-    // cost an extra predicate, never a missed union
-    int jn = lane < total ? row_next(rt, cur, lane) : -1;
-    bool cn = false;
-    int pn = -1;
-    if (jn >= 0) {
-        cn = core_sorted[jn] != 0;
-        pn = __ldcg(parent + jn);
-    }
-    for (int tb = 0; tb < total; tb += kWarp) {
-        const int j = jn;
-        bool valid = j > p0 && cn;
-        int pj = pn;
-        {
-            const int t = tb + kWarp + lane;
-            jn = t < total ? row_next(rt, cur, t) : -1;
-            cn = false;
-            pn = -1;
-            if (jn >= 0) {
-                cn = core_sorted[jn] != 0;
-                pn = __ldcg(parent + jn);
-            }
+    const bool listed = *n_seg <= seg_cap;
+    const uint32_t n_work = listed ? *n_seg : (uint32_t)n_items;
+    for (uint32_t w = blockIdx.x * kCountWarps + wib; w < n_work; w += gridDim.x * kCountWarps) {
+        const int2 item = items[listed ? seg_item[w] : w];
+        const int A = item.x, p0 = item.y;
+        if (jobs) e2 = jobs[cell_job[A]].e2;
+        const int cnt = min(kTile, cell_start[A + 1] - p0);
+        const int mine = lane < cnt ? __ldg(snap + p0 + lane) : -1;
+        const int total = union_rows(A, p0, mine, cell_start, nbr, n_rows, cell_root, rt, s_cells[wib], s_need[wib],
+                                     lane);
+        if (total == 0) continue;
+        const int first = listed ? (int)seg_part[w] * kUnionSegment : 0;
+        const int end = listed ? min(total - first, kUnionSegment) + first : total;
+        // the item's cores, compacted: slot k holds its coordinates, index and root
+        const unsigned cores = __ballot_sync(kFull, mine >= 0);
+        const int nc = __popc(cores);
+        if (mine >= 0) {
+            const int slot = __popc(cores & lanemask_lt());
+            float x[D];
+            load_point<D>(xs, p0 + lane, x);
+            store_point_smem<D>(si + slot * P, x);
+            sidx[slot] = p0 + lane;
+            sroot[slot] = mine;
         }
-        // roots of the item's cores, refreshed every chunk so that candidates already
-        // joined to them are skipped before the predicate
-        int myroot = lane < nc ? uf_find(parent, sidx[lane], err) : -1;
-        if (lane < nc) sroot[lane] = myroot;
-        // one root for all of the item's cores (the usual case once they are joined)
-        const int root0 = __shfl_sync(kFull, myroot, 0);
-        const bool uniform = __all_sync(kFull, lane >= nc || myroot == root0);
         __syncwarp();
-        float xj[D];
-        if (valid) {
-            pj = __ldcg(parent + pj);  // second hop: an ancestor of j, usually its root
-            if (uniform && pj == root0) valid = false;  // joined to every core of the item already
-        }
-        if (!__any_sync(kFull, valid)) continue;
-        if (valid) load_point<D>(xs, j, xj);
-        else fill_nan<D>(xj);
-        int tested = 0;
-        for (int k = 0; k < nc; ++k) {
-            const int ik = sidx[k];
-            if constexpr (D >= 8) {
-                // as in the count: the second half of the sum only when some lane's
-                // first half is still within e2 (exact: partial sums only grow)
-                const bool want = valid && j > ik && sroot[k] != pj;
+        // cur0: the current root of the largest group of the item's cores, whose
+        // snapshot root is snap0; diff: the slots under another root
+        const int r_first = lane < nc ? sroot[lane] : -1 - lane;
+        const unsigned peers = __match_any_sync(kFull, r_first);
+        const int most = __reduce_max_sync(kFull, lane < nc ? __popc(peers) * kWarp + lane : -1) & (kWarp - 1);
+        const int snap0 = __shfl_sync(kFull, r_first, most);
+        int cur0 = 0;
+        unsigned diff = 0;
+        bool refresh = true;
+        int row = 0;
+        int j = first + lane < end ? row_next(rt, row, first + lane) : -1;
+        int r = j >= 0 ? __ldg(snap + j) : -1;
+        for (int tb = first; tb < end; tb += kWarp) {
+            // the next step's candidate is loaded one step ahead
+            const int jc = j, rc = r;
+            const int t = tb + kWarp + lane;
+            j = t < end ? row_next(rt, row, t) : -1;
+            r = j >= 0 ? __ldg(snap + j) : -1;
+            if (refresh) {
+                const int now = lane < nc ? uf_find(parent, sroot[lane], err) : -1;
+                cur0 = __shfl_sync(kFull, now, most);
+                if (lane < nc) sroot[lane] = now;
+                diff = __ballot_sync(kFull, lane < nc && now != cur0);
+                refresh = false;
+                __syncwarp();
+            }
+            const bool valid = rc >= 0;
+            int rj = cur0;
+            if (valid && rc != snap0) rj = uf_find(parent, rc, err);
+            // candidates under another root meet every core, the others only the cores in diff
+            const unsigned other = __ballot_sync(kFull, valid && rj != cur0);
+            const unsigned test = other ? kFull >> (kWarp - nc) : diff;
+            if (!test) continue;
+            float xj[D];
+            if (valid) load_point<D>(xs, jc, xj);
+            else fill_nan<D>(xj);
+            int tested = 0;
+            bool joined = false;
+            for (unsigned it = test; it; it &= it - 1) {
+                const int k = __ffs(it) - 1;
+                const int rk = sroot[k];
+                const bool want = valid && jc > sidx[k] && rk != rj;
                 if (!__any_sync(kFull, want)) continue;
                 float xi[D];
                 load_point_smem<D>(si + k * P, xi);
-                constexpr int H = D / 2;
-                const float len = dist_part<D, 0, H>(xi, xj, 0.0f);
                 bool hit = false;
-                if (__any_sync(kFull, want && len <= e2)) hit = want && dist_part<D, H, D>(xi, xj, len) <= e2;
+                if constexpr (D >= 8) {
+                    // the second half of the sum only when some lane's first half is
+                    // still within e2 (exact: partial sums only grow)
+                    constexpr int H = D / 2;
+                    const float len = dist_part<D, 0, H>(xi, xj, 0.0f);
+                    if (__any_sync(kFull, want && len <= e2)) hit = want && dist_part<D, H, D>(xi, xj, len) <= e2;
+                } else {
+                    hit = want && in_range<D>(xi, xj, e2);
+                }
                 tested += want ? 1 : 0;
-                // finds from known ancestors: the core's root snapshot and pj; the
-                // shared root that comes back is again an ancestor of j
-                if (hit) pj = uf_union_root(parent, sroot[k], pj, err);
-            } else if (valid && j > ik && sroot[k] != pj) {
-                float xi[D];
-                load_point_smem<D>(si + k * P, xi);
-                ++tested;
-                if (in_range<D>(xi, xj, e2)) pj = uf_union_root(parent, sroot[k], pj, err);
+                // finds from known ancestors; the shared root that comes back is again
+                // an ancestor of the candidate
+                if (hit) {
+                    rj = uf_union_root(parent, rk, rj, err);
+                    joined = true;
+                }
             }
+            pairs += (unsigned long long)__reduce_add_sync(kFull, (unsigned)tested);
+            refresh = __any_sync(kFull, joined);
         }
-        pairs += (unsigned long long)__reduce_add_sync(kFull, (unsigned)tested);
         __syncwarp();
     }
     if (lane == 0 && pairs) atomicAdd(pair_counter, pairs);
@@ -1486,17 +1557,25 @@ __global__ void comp_min_cells_kernel(int64_t n_cells, const int32_t *__restrict
     }
 }
 
-// The one root of each cell's cores (parent flattened): -1 without cores, -2 when
-// they do not all share it.  One thread per point: the first core of a cell to
-// arrive installs its root, any core with another root marks the cell mixed; a
-// core whose root is already there skips the atomic.  cell_root starts at -1.
-__global__ void cell_root_kernel(int64_t nv, const int32_t *__restrict__ pcell,
-                                 const uint8_t *__restrict__ core_sorted, const int32_t *__restrict__ parent,
-                                 int32_t *cell_root) {
+// Point units, after the list unions: parent flattened (as flatten_kernel), every
+// core's root in snap (-1 for non-cores), and the one root of each cell's cores in
+// cell_root: -1 without cores, -2 when they do not all share it.  One thread per
+// point: the first core of a cell to arrive installs its root, any core with another
+// root marks the cell mixed; a core whose root is already there skips the atomic.
+// cell_root starts at -1.
+__global__ void flatten_points_kernel(int32_t *parent, int64_t nv, int *err, const int32_t *__restrict__ pcell,
+                                      const uint8_t *__restrict__ core_sorted, int32_t *__restrict__ snap,
+                                      int32_t *cell_root) {
     const int64_t s = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (s >= nv || !core_sorted[s]) return;
+    if (s >= nv) return;
+    if (!core_sorted[s]) {
+        snap[s] = -1;  // never an end of a union: parent[s] is s
+        return;
+    }
+    const int r = uf_find_ro(parent, (int)s, err);
+    parent[s] = r;
+    snap[s] = r;
     const int c = pcell[s];
-    const int r = parent[s];
     const int cur = __ldcg(cell_root + c);
     if (cur == r || cur == -2) return;
     const int old = cur == -1 ? atomicCAS(cell_root + c, -1, r) : cur;
