@@ -143,7 +143,7 @@ constexpr size_t kSmallCountersOff = 512;    // u64[12]: 0 clusters 1 noise 2 co
                                              // 5 band pairs 6 work counter of the persistent count kernel
                                              // 8..11 filter audit (tc::audit_tile)
 constexpr int kCounters = 12;
-constexpr size_t kSmallScalarOff = 1024;     // u32[8]: 0 n_cells 1 n_items 2 n_cores 4, 5 split items 6 union segments
+constexpr size_t kSmallScalarOff = 1024;     // u32[8]: 0 n_cells 1 n_items 2 n_cores 4 tensor items 5 exact items 6 union segments 7 tensor chunks
 constexpr size_t kSmallErrOff = 1536;        // int
 constexpr size_t kSmallStencilOff = 2048;    // int4[kMaxRows]: stencil rows of the current job
 constexpr size_t kSmallBytes = 4096;
@@ -636,69 +636,83 @@ inline int ctx_tc_min_item(const ndb_ctx *ctx) {
     return v <= 0 ? default_tc_min_item() : v;
 }
 
+// The tensor-core count of the chunks in chunks[0, *n_chunks).
 template <int D>
-void launch_count_tc(ndb_ctx *ctx, int64_t n_items, const int2 *items, const int32_t *cell_start, const int2 *nbr,
-                     int n_rows, const float *xs, float e2, int min_pts, bool early, int32_t *nn_sorted,
-                     int32_t *list, int list_cap, int list_stride, const JobDev *jobs, const int32_t *cell_job,
-                     const uint32_t *n_items_dev, bool audit) {
+void launch_count_tc(ndb_ctx *ctx, int64_t max_chunks, const int2 *chunks, const uint32_t *n_chunks, int chunk,
+                     const int32_t *cell_start, const int2 *nbr, int n_rows, const float *xs, float e2, int min_pts,
+                     bool early, int32_t *nn_sorted, int32_t *list, int list_cap, int list_stride,
+                     const JobDev *jobs, const int32_t *cell_job, bool audit) {
     if constexpr (D >= tc::kMinDim) {
         cudaStream_t st = ctx->stream;
         unsigned long long *counters = small_at<unsigned long long>(ctx, kSmallCountersOff);
         unsigned int *work = reinterpret_cast<unsigned int *>(counters + 6);
         fill_bytes(ctx, work, 0, sizeof(unsigned long long), st);
-        // the items' records (stencil rows as point ranges), which the kernel fetches
-        // one item ahead by bulk copies; without room for them (a memory cap, the
+        // the chunks' records (stencil rows as point ranges), which the kernel fetches
+        // one chunk ahead by bulk copies; without room for them (a memory cap, the
         // allocation-free entry point) the kernel gathers the rows itself
         int2 *rec = nullptr;
-        if (n_items_dev && grow(ctx, ctx->tc_rec, (size_t)n_items * tc::kRecBytes) == cudaSuccess) {
+        if (grow(ctx, ctx->tc_rec, (size_t)max_chunks * tc::kRecBytes) == cudaSuccess) {
             rec = ctx->tc_rec.as<int2>();
-            ++launch_counter(), tc::tc_records_kernel<<<blocks_for(n_items * kWarp), kBlock, 0, st>>>(
-                items, n_items_dev, cell_start, nbr, n_rows, cell_job, rec);
+            ++launch_counter(), tc::tc_records_kernel<<<blocks_for(max_chunks * kWarp), kBlock, 0, st>>>(
+                chunks, n_chunks, cell_start, nbr, n_rows, cell_job, chunk, rec);
             ck(ctx, cudaGetLastError());
         } else {
             cudaGetLastError();  // a refused or failed allocation leaves no error behind
         }
-        const unsigned grid = (unsigned)std::min<int64_t>(n_items, (int64_t)ctx->sm_count * tc::TcBlocks<D>::v);
-        if (audit)
-            ++launch_counter(), tc::count_tc_kernel<D, true><<<grid, tc::kThreads, 0, st>>>(
-                items, n_items, cell_start, nbr, n_rows, xs, e2, min_pts, early ? 1 : 0, nn_sorted, list, list_cap,
-                list_stride, counters + 2, counters + 5, work, small_at<int>(ctx, kSmallErrOff), jobs, cell_job,
-                n_items_dev, counters + 8, rec);
-        else
-            ++launch_counter(), tc::count_tc_kernel<D><<<grid, tc::kThreads, 0, st>>>(
-                items, n_items, cell_start, nbr, n_rows, xs, e2, min_pts, early ? 1 : 0, nn_sorted, list, list_cap,
-                list_stride, counters + 2, counters + 5, work, small_at<int>(ctx, kSmallErrOff), jobs, cell_job,
-                n_items_dev, nullptr, rec);
+        const unsigned grid = (unsigned)std::min<int64_t>(max_chunks, (int64_t)ctx->sm_count * tc::TcBlocks<D>::v);
+        auto launch = [&](auto audit_c) {
+            constexpr bool A = decltype(audit_c)::value;
+            ++launch_counter(), tc::count_tc_kernel<D, A><<<grid, tc::kThreads, 0, st>>>(
+                chunks, n_chunks, chunk, cell_start, nbr, n_rows, xs, e2, min_pts, early ? 1 : 0, nn_sorted, list,
+                list_cap, list_stride, counters + 2, counters + 5, work, small_at<int>(ctx, kSmallErrOff), jobs,
+                cell_job, counters + 8, rec);
+        };
+        if (audit) launch(std::true_type{});
+        else launch(std::false_type{});
         ck(ctx, cudaGetLastError());
     } else {
         throw Fail{NDB_ERR_INVALID_ARGUMENT};
     }
 }
 
+// Points per chunk of the tensor-core count.  Full counts: the 32 columns of one round,
+// since every point needs the whole round (8-D 2M: 8.5 ms; 256 points 10.2 ms, a longer
+// tail).  Early exit: enough to keep the columns filled (a chunk's last points run with
+// ever fewer), few enough that every resident CTA gets several chunks: 16-D 200k 64
+// points 1.40 ms, 256 points 2.23 ms; the 4,096-job batch's counts 32 points 143 ms, 64
+// 128 ms, 256 117 ms, 512 116 ms.
+inline int tc_chunk(const ndb_ctx *ctx, int64_t nv, bool early) {
+    if (!early) return tc::kN;
+    const int64_t per = nv / ((int64_t)ctx->sm_count * 5 * 4);
+    return (int)std::min<int64_t>(std::max<int64_t>(per / tc::kN * tc::kN, tc::kN), 256);
+}
+
 // The neighbour count of one pipeline.  tc: the tensor-core filter may run (input
-// eligible); then the items are split by size and each list goes to its kernel,
+// eligible); then the cells are split by size and each list goes to its kernel,
 // both launched at the upper bound and reading their list length on the device.
 template <int D>
 void count_items(ndb_ctx *ctx, bool tc, bool force_tc, bool gram, bool early, int64_t n_items, const int2 *items,
                  const int32_t *cell_start, const int2 *nbr, int n_rows, const float *xs, float e2, int min_pts,
                  int dense_skip, int32_t *nn_sorted, int32_t *list, int list_cap, int list_stride,
-                 const JobDev *jobs, const int32_t *cell_job, bool audit) {
+                 const JobDev *jobs, const int32_t *cell_job, bool audit, int64_t nv, int64_t n_cells) {
     if (n_items <= 0) return;
     cudaStream_t st = ctx->stream;
     unsigned long long *counters = small_at<unsigned long long>(ctx, kSmallCountersOff);
     const int2 *ex_items = items;
     const uint32_t *ex_n = nullptr;
     if (tc) {
+        // scalars: 4 32-point items in chunks, 5 items of the exact kernel, 7 chunks
         uint32_t *scal = small_at<uint32_t>(ctx, kSmallScalarOff);
         ensure(ctx, ctx->items_split, (size_t)(2 * n_items + 2) * sizeof(int2));
-        int2 *tc_items = ctx->items_split.as<int2>();
-        int2 *rest = tc_items + n_items + 1;
-        fill_bytes(ctx, scal + 4, 0, 2 * sizeof(uint32_t), st);
-        ++launch_counter(), split_items_kernel<<<blocks_for(n_items), kBlock, 0, st>>>(
-            items, n_items, cell_start, force_tc ? 1 : ctx_tc_min_item(ctx), tc_items, scal + 4, rest, scal + 5);
+        int2 *chunks = ctx->items_split.as<int2>();
+        int2 *rest = chunks + n_items + 1;
+        const int chunk = tc_chunk(ctx, nv, early);
+        fill_bytes(ctx, scal + 4, 0, 4 * sizeof(uint32_t), st);
+        ++launch_counter(), tc::split_cells_kernel<<<blocks_for(n_cells), kBlock, 0, st>>>(
+            cell_start, n_cells, force_tc ? 1 : ctx_tc_min_item(ctx), chunk, chunks, scal + 7, rest, scal + 5, scal + 4);
         ck(ctx, cudaGetLastError());
-        launch_count_tc<D>(ctx, n_items, tc_items, cell_start, nbr, n_rows, xs, e2, min_pts, early, nn_sorted, list,
-                           list_cap, list_stride, jobs, cell_job, scal + 4, audit);
+        launch_count_tc<D>(ctx, n_items, chunks, scal + 7, chunk, cell_start, nbr, n_rows, xs, e2, min_pts, early,
+                           nn_sorted, list, list_cap, list_stride, jobs, cell_job, audit);
         ex_items = rest;
         ex_n = scal + 5;
     }
@@ -744,7 +758,8 @@ void count_phase(ndb_ctx *ctx) {
                    ctx->n_items,
                    ctx->items.as<int2>(), ctx->cell_start.as<int32_t>(), ctx->nbr.as<int2>(), ctx->n_rows,
                    ctx->xs.as<float>(), ctx->e2, ctx->min_pts, ctx->cell_units, ctx->nn_sorted.as<int32_t>(), list,
-                   ctx->list_cap, ctx->list_cap, nullptr, nullptr, (ctx->flags_run & NDB_FLAG_FILTER_AUDIT) != 0);
+                   ctx->list_cap, ctx->list_cap, nullptr, nullptr, (ctx->flags_run & NDB_FLAG_FILTER_AUDIT) != 0,
+                   ctx->nv, ctx->n_cells);
     cudaEventRecord(ctx->kev[3], st);
 }
 
@@ -1756,7 +1771,7 @@ void run_group_keys(ndb_ctx *ctx, ndb_job *jobs, const std::vector<int> &members
                    ctx->items.as<int2>(),
                    ctx->cell_start.as<int32_t>(), ctx->nbr.as<int2>(), n_rows, ctx->xs.as<float>(), 0.0f, 0, 0,
                    ctx->nn_sorted.as<int32_t>(), list, 0, bp.list_stride, jobs_dev, cell_job,
-                   (flags & NDB_FLAG_FILTER_AUDIT) != 0);
+                   (flags & NDB_FLAG_FILTER_AUDIT) != 0, nv, n_cells);
     cudaEventRecord(ctx->kev[3], st);
     const int64_t n_words = (n + 31) / 32;
     ensure(ctx, ctx->core_sorted, n + 1);
