@@ -484,26 +484,23 @@ void classify_grid(ndb_ctx *ctx, const Plan &pl) {
     ensure(ctx, ctx->keys1, n * sizeof(K));
     ensure(ctx, ctx->ids0, n * sizeof(int32_t));
     ensure(ctx, ctx->ids1, n * sizeof(int32_t));
-    ensure(ctx, ctx->sort_hist, sort_hist_words(n) * sizeof(uint32_t));
-    const size_t scan_words = std::max(scan_scratch_words(n + 1), scan_scratch_words((int64_t)sort_hist_words(n)));
-    ensure(ctx, ctx->scan_scratch, (scan_words + 64) * sizeof(uint32_t));
+    ensure(ctx, ctx->sort_hist, sort_scratch_words<K>(n) * sizeof(uint32_t));
+    ensure(ctx, ctx->scan_scratch, (scan_scratch_words(n + 1) + 64) * sizeof(uint32_t));
 
     K invalid_key = (K)(pl.key_bits >= (int)(8 * sizeof(K)) ? ~(K)0 : (((K)1 << pl.key_bits) - 1));
     ++launch_counter(), key_kernel<D, K><<<blocks_for(n), kBlock, 0, st>>>(ctx->coords_dev, n, pl.g, invalid_key,
-                                                        ctx->keys0.as<K>(), ctx->ids0.as<int32_t>());
+                                                        ctx->keys0.as<K>());
     ck(ctx, cudaGetLastError());
     bool in_first = true;
     cudaEventRecord(ctx->kev[0], st);
     if (sizeof(K) == 4)
         ck(ctx, radix_sort_pairs_u32(reinterpret_cast<uint32_t *>(ctx->keys0.ptr), ctx->ids0.as<int32_t>(),
                                      reinterpret_cast<uint32_t *>(ctx->keys1.ptr), ctx->ids1.as<int32_t>(), n,
-                                     pl.key_bits, ctx->sort_hist.as<uint32_t>(), ctx->scan_scratch.as<uint32_t>(),
-                                     &in_first, st));
+                                     pl.key_bits, ctx->sort_hist.as<uint32_t>(), &in_first, st));
     else
         ck(ctx, radix_sort_pairs_u64(reinterpret_cast<uint64_t *>(ctx->keys0.ptr), ctx->ids0.as<int32_t>(),
                                      reinterpret_cast<uint64_t *>(ctx->keys1.ptr), ctx->ids1.as<int32_t>(), n,
-                                     pl.key_bits, ctx->sort_hist.as<uint32_t>(), ctx->scan_scratch.as<uint32_t>(),
-                                     &in_first, st));
+                                     pl.key_bits, ctx->sort_hist.as<uint32_t>(), &in_first, st));
     cudaEventRecord(ctx->kev[1], st);
     ctx->stats.sort_passes = (pl.key_bits + 7) / 8;
     ctx->stats.key_bytes = (int32_t)sizeof(K);
@@ -1681,25 +1678,22 @@ void run_group_keys(ndb_ctx *ctx, ndb_job *jobs, const std::vector<int> &members
     ensure(ctx, ctx->keys1, n * sizeof(K));
     ensure(ctx, ctx->ids0, n * sizeof(int32_t));
     ensure(ctx, ctx->ids1, n * sizeof(int32_t));
-    ensure(ctx, ctx->sort_hist, sort_hist_words(n) * sizeof(uint32_t));
-    const size_t scan_words = std::max(scan_scratch_words(n + 1), scan_scratch_words((int64_t)sort_hist_words(n)));
-    ensure(ctx, ctx->scan_scratch, (scan_words + 64) * sizeof(uint32_t));
+    ensure(ctx, ctx->sort_hist, sort_scratch_words<K>(n) * sizeof(uint32_t));
+    ensure(ctx, ctx->scan_scratch, (scan_scratch_words(n + 1) + 64) * sizeof(uint32_t));
     const K invalid_key = (K)(bp.key_bits >= (int)(8 * sizeof(K)) ? ~(K)0 : (((K)1 << bp.key_bits) - 1));
     ++launch_counter(), key_batch_kernel<D, K><<<dim3(gx, nj), kBlock, 0, st>>>(
-        ctx->coords.as<float>(), jobs_dev, invalid_key, ctx->keys0.as<K>(), ctx->ids0.as<int32_t>());
+        ctx->coords.as<float>(), jobs_dev, invalid_key, ctx->keys0.as<K>());
     ck(ctx, cudaGetLastError());
     bool in_first = true;
     cudaEventRecord(ctx->kev[0], st);
     if (sizeof(K) == 4)
         ck(ctx, radix_sort_pairs_u32(reinterpret_cast<uint32_t *>(ctx->keys0.ptr), ctx->ids0.as<int32_t>(),
                                      reinterpret_cast<uint32_t *>(ctx->keys1.ptr), ctx->ids1.as<int32_t>(), n,
-                                     bp.key_bits, ctx->sort_hist.as<uint32_t>(), ctx->scan_scratch.as<uint32_t>(),
-                                     &in_first, st));
+                                     bp.key_bits, ctx->sort_hist.as<uint32_t>(), &in_first, st));
     else
         ck(ctx, radix_sort_pairs_u64(reinterpret_cast<uint64_t *>(ctx->keys0.ptr), ctx->ids0.as<int32_t>(),
                                      reinterpret_cast<uint64_t *>(ctx->keys1.ptr), ctx->ids1.as<int32_t>(), n,
-                                     bp.key_bits, ctx->sort_hist.as<uint32_t>(), ctx->scan_scratch.as<uint32_t>(),
-                                     &in_first, st));
+                                     bp.key_bits, ctx->sort_hist.as<uint32_t>(), &in_first, st));
     cudaEventRecord(ctx->kev[1], st);
     if (!in_first) {
         std::swap(ctx->keys0, ctx->keys1);
@@ -2491,7 +2485,7 @@ constexpr size_t na_cap(int b) {
          : b == NA_CELL_KEY || b == NA_ITEMS ? 8 * (kNaN + 1)
          : b == NA_NBR ? 8 * kWarp * kNaN + 8  // classify refuses stencils of more than kWarp rows
          : b == NA_CORE_SORTED || b == NA_CELL_HAS_CORE ? kNaN + 1
-         : b == NA_SORT_HIST ? 4 * 256 * ((kNaN + kSortTile - 1) / kSortTile)
+         : b == NA_SORT_HIST ? 4 * sort_scratch_words<uint64_t>(kNaN)
          : b == NA_SCAN ? 4 * 4096
          : b == NA_SMALL ? kSmallBytes
          : b == NA_HASH_KEYS ? 8 * 4 * kNaN

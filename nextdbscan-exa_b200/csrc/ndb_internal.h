@@ -43,16 +43,28 @@ size_t scan_scratch_words(int64_t n);
 cudaError_t scan_exclusive_u32(const uint32_t *in, uint32_t *out, int64_t n, uint32_t *total_dev,
                                uint32_t *scratch, cudaStream_t st);
 
-constexpr int kSortTile = 2048;
-size_t sort_hist_words(int64_t n);
-// Stable LSD radix sort of (key, value) pairs on the low `bits` bits of the keys.
-// Sorts between (k0, v0) and (k1, v1); returns via *result_in_first whether the
-// sorted data ended in (k0, v0).
+// Elements of one sort tile, by key size.
+template <typename K>
+struct SortTile {
+    static constexpr int v = sizeof(K) == 4 ? 4096 : 2048;
+};
+constexpr int kSortRadix = 256, kSortMaxPasses = 8;
+// Scratch (in uint32 words, 16-byte aligned) of a sort of n pairs: the digit
+// histograms of all passes, one ticket per pass (64-bit slots), and one 64-bit state
+// word per digit and tile.
+constexpr int kSortHistWords = kSortMaxPasses * kSortRadix;
+constexpr int kSortTicketWords = 2 * kSortMaxPasses;
+template <typename K>
+constexpr size_t sort_scratch_words(int64_t n) {
+    return kSortHistWords + kSortTicketWords +
+           2 * (size_t)kSortRadix * (size_t)((n + SortTile<K>::v - 1) / SortTile<K>::v + (n <= 0));
+}
+// Stable LSD radix sort of (key, element index) pairs on the low `bits` bits of the
+// keys in k0: sorts between (k0, v0) and (k1, v1) and returns via *result_in_first
+// whether the sorted keys and indices ended in (k0, v0).  v0 need not be set.
 cudaError_t radix_sort_pairs_u32(uint32_t *k0, int32_t *v0, uint32_t *k1, int32_t *v1, int64_t n,
-                                 int bits, uint32_t *hist, uint32_t *scan_scratch,
-                                 bool *result_in_first, cudaStream_t st);
+                                 int bits, uint32_t *scratch, bool *result_in_first, cudaStream_t st);
 cudaError_t radix_sort_pairs_u64(uint64_t *k0, int32_t *v0, uint64_t *k1, int32_t *v1, int64_t n,
-                                 int bits, uint32_t *hist, uint32_t *scan_scratch,
-                                 bool *result_in_first, cudaStream_t st);
+                                 int bits, uint32_t *scratch, bool *result_in_first, cudaStream_t st);
 
 }  // namespace ndb

@@ -185,8 +185,7 @@ __device__ __forceinline__ long long cell_coord(const GridDev &g, int a, float x
 
 template <int D, typename K>
 __global__ void __launch_bounds__(kBlock) key_kernel(const float *__restrict__ coords, int64_t n,
-                                                     GridDev g, K invalid_key, K *__restrict__ keys,
-                                                     int32_t *__restrict__ ids) {
+                                                     GridDev g, K invalid_key, K *__restrict__ keys) {
     const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n) return;
     const float *p = coords + i * D;
@@ -199,7 +198,6 @@ __global__ void __launch_bounds__(kBlock) key_kernel(const float *__restrict__ c
         key = (K)kk;
     }
     keys[i] = key;
-    ids[i] = (int32_t)i;
 }
 
 // pos = exclusive scan of "first point of a cell" flags
@@ -2067,7 +2065,7 @@ __global__ void __launch_bounds__(kBlock) bbox_batch_kernel(const float *__restr
 template <int D, typename K>
 __global__ void __launch_bounds__(kBlock) key_batch_kernel(const float *__restrict__ coords,
                                                            const JobDev *__restrict__ jobs, K invalid_key,
-                                                           K *__restrict__ keys, int32_t *__restrict__ ids) {
+                                                           K *__restrict__ keys) {
     const JobDev &J = jobs[blockIdx.y];
     const GridDev g = J.g;
     for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < J.n; i += (int64_t)gridDim.x * blockDim.x) {
@@ -2087,7 +2085,6 @@ __global__ void __launch_bounds__(kBlock) key_batch_kernel(const float *__restri
             key = (K)kk;
         }
         keys[o] = key;
-        ids[o] = (int32_t)o;
     }
 }
 
