@@ -466,6 +466,12 @@ CellIndex<K> build_cell_index(ndb_ctx *ctx, int64_t n_cells, double columns, con
     return L;
 }
 
+// Blocks of a bounding-box pass: up to four points per thread before more blocks are
+// added, at most eight blocks per SM (every block ends in 2 d atomics).
+inline unsigned bbox_blocks(const ndb_ctx *ctx, int64_t n) {
+    return std::min<unsigned>(blocks_for(n, kBlock * 4), (unsigned)ctx->sm_count * 8);
+}
+
 // The lookup built by build_cell_index, for kernels of the label phase.
 template <typename K>
 CellIndex<K> cell_index(ndb_ctx *ctx) {
@@ -488,8 +494,8 @@ void classify_grid(ndb_ctx *ctx, const Plan &pl) {
     ensure(ctx, ctx->scan_scratch, (scan_scratch_words(n + 1) + 64) * sizeof(uint32_t));
 
     K invalid_key = (K)(pl.key_bits >= (int)(8 * sizeof(K)) ? ~(K)0 : (((K)1 << pl.key_bits) - 1));
-    ++launch_counter(), key_kernel<D, K><<<blocks_for(n), kBlock, 0, st>>>(ctx->coords_dev, n, pl.g, invalid_key,
-                                                        ctx->keys0.as<K>());
+    ++launch_counter(), key_kernel<D, K><<<blocks_for(n), kBlock, 0, st>>>(ctx->coords_dev, n, rows_aligned<D>(ctx->coords_dev),
+                                                        pl.g, invalid_key, ctx->keys0.as<K>());
     ck(ctx, cudaGetLastError());
     bool in_first = true;
     cudaEventRecord(ctx->kev[0], st);
@@ -527,7 +533,8 @@ void classify_grid(ndb_ctx *ctx, const Plan &pl) {
                                                             ctx->pcell.as<int32_t>());
     ck(ctx, cudaGetLastError());
     ensure(ctx, ctx->xs, (nv + 1) * P * sizeof(float));
-    ++launch_counter(), gather_kernel<D><<<blocks_for(nv), kBlock, 0, st>>>(ctx->coords_dev, perm, nv, ctx->xs.as<float>());
+    ++launch_counter(), gather_kernel<D><<<blocks_for(nv), kBlock, 0, st>>>(ctx->coords_dev, perm, nv,
+                                                        rows_aligned<D>(ctx->coords_dev), ctx->xs.as<float>());
     ck(ctx, cudaGetLastError());
     uint32_t n_cells32 = 0;
     ck(ctx, cudaMemcpyAsync(&n_cells32, scal + 0, sizeof(uint32_t), cudaMemcpyDeviceToHost, st));
@@ -1044,8 +1051,8 @@ ndb_status classify_impl(ndb_ctx *ctx, const float *coords, int64_t n, float eps
     } else {
         ++launch_counter(), bbox_init_kernel<<<1, 32, 0, st>>>(lo_hi, D, n_invalid, small_at<int>(ctx, kSmallErrOff),
                                                                ctx->uf_max_steps);
-        ++launch_counter(), bbox_kernel<D><<<std::min<unsigned>(blocks_for(n), 148 * 8), kBlock, 0, st>>>(
-            ctx->coords_dev, n, lo_hi, n_invalid);
+        ++launch_counter(), bbox_kernel<D><<<bbox_blocks(ctx, n), kBlock, 0, st>>>(
+            ctx->coords_dev, n, rows_aligned<D>(ctx->coords_dev), lo_hi, n_invalid);
     }
     ck(ctx, cudaGetLastError());
     int h_lo_hi[2 * kMaxDim];
@@ -1204,8 +1211,8 @@ template <int D>
 void bbox_chunk(ndb_ctx *ctx, const float *p, int64_t cnt) {
     int *lo_hi = ctx->load_box.as<int>();
     auto *inval = reinterpret_cast<unsigned long long *>(ctx->load_box.as<char>() + kLoadBoxInvalidOff);
-    ++launch_counter(), bbox_kernel<D><<<std::min<unsigned>(blocks_for(cnt), 148 * 8), kBlock, 0, ctx->stream>>>(
-        p, cnt, lo_hi, inval);
+    ++launch_counter(), bbox_kernel<D><<<bbox_blocks(ctx, cnt), kBlock, 0, ctx->stream>>>(
+        p, cnt, rows_aligned<D>(p), lo_hi, inval);
     ck(ctx, cudaGetLastError());
 }
 
@@ -1716,7 +1723,7 @@ void run_group_keys(ndb_ctx *ctx, ndb_job *jobs, const std::vector<int> &members
         ctx->pcell.as<int32_t>());
     ensure(ctx, ctx->xs, (nv + 1) * P * sizeof(float));
     ++launch_counter(), gather_kernel<D><<<blocks_for(nv), kBlock, 0, st>>>(ctx->coords.as<float>(), perm, nv,
-                                                                           ctx->xs.as<float>());
+                                                                           true, ctx->xs.as<float>());
     ck(ctx, cudaGetLastError());
     const uint32_t *m_cells = mail_from_device(ctx, scal + 0, 1, st);
     ck(ctx, cudaStreamSynchronize(st));

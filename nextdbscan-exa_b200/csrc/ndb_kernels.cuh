@@ -92,15 +92,6 @@ constexpr int kCountWarps = 2;
 // (data_process.cpp:196, :440) whose distance to any other first coordinate
 // squares to inf.
 // ---------------------------------------------------------------------------
-template <int D>
-__device__ __forceinline__ bool point_valid(const float *p) {
-    if (p[0] == FLT_MAX) return false;
-#pragma unroll
-    for (int k = 0; k < D; ++k)
-        if (!isfinite(p[k])) return false;
-    return true;
-}
-
 __device__ __forceinline__ int ordered_int(float f) {
     const int i = __float_as_int(f);
     return i >= 0 ? i : i ^ 0x7fffffff;
@@ -121,10 +112,93 @@ __global__ void bbox_init_kernel(int *lo_hi, int d, unsigned long long *n_invali
 
 __global__ void set_int_kernel(int *p, int v) { *p = v; }
 
-// lo_hi[0..D) = ordered-int min, lo_hi[D..2D) = ordered-int max.
+// The block's bounds and invalid points, added to lo_hi (ordered-int min, then max, per
+// dimension) and n_invalid.
 template <int D>
-__global__ void __launch_bounds__(kBlock) bbox_kernel(const float *__restrict__ coords, int64_t n,
+__device__ __forceinline__ void bbox_reduce(int (&lo)[D], int (&hi)[D], unsigned bad, int (*s_lh)[2 * D],
+                                            unsigned *s_bad, int *lh, unsigned long long *n_invalid) {
+    constexpr int W = kBlock / kWarp;
+#pragma unroll
+    for (int k = 0; k < D; ++k) {
+        lo[k] = __reduce_min_sync(kFull, lo[k]);
+        hi[k] = __reduce_max_sync(kFull, hi[k]);
+    }
+    bad = __reduce_add_sync(kFull, bad);
+    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+    if (lane == 0) {
+#pragma unroll
+        for (int k = 0; k < D; ++k) {
+            s_lh[w][k] = lo[k];
+            s_lh[w][D + k] = hi[k];
+        }
+        s_bad[w] = bad;
+    }
+    __syncthreads();
+    if (threadIdx.x < 2 * D) {
+        const int t = threadIdx.x;
+        int v = s_lh[0][t];
+        for (int q = 1; q < W; ++q) v = t < D ? min(v, s_lh[q][t]) : max(v, s_lh[q][t]);
+        if (t < D) {
+            if (v != 0x7fffffff) atomicMin(lh + t, v);
+        } else {
+            if (v != (int)0x80000000) atomicMax(lh + t, v);
+        }
+    }
+    if (threadIdx.x == 0) {
+        unsigned b = 0;
+        for (int q = 0; q < W; ++q) b += s_bad[q];
+        if (b) atomicAdd(n_invalid, (unsigned long long)b);
+    }
+}
+
+// One point's coordinates: 16-byte vector loads when a point's row is a multiple of
+// 16 bytes (d % 4 == 0; rows then start 16-byte aligned), 8-byte ones at d = 2.
+template <int D>
+__device__ __forceinline__ void load_row(const float *__restrict__ p, float (&x)[D]) {
+    if constexpr (D % 4 == 0) {
+#pragma unroll
+        for (int q = 0; q < D / 4; ++q) {
+            const float4 v = __ldg(reinterpret_cast<const float4 *>(p) + q);
+            x[4 * q + 0] = v.x;
+            x[4 * q + 1] = v.y;
+            x[4 * q + 2] = v.z;
+            x[4 * q + 3] = v.w;
+        }
+    } else if constexpr (D == 2) {
+        const float2 v = __ldg(reinterpret_cast<const float2 *>(p));
+        x[0] = v.x;
+        x[1] = v.y;
+    } else {
+#pragma unroll
+        for (int k = 0; k < D; ++k) x[k] = __ldg(p + k);
+    }
+}
+
+// The same for a caller's array, which may be aligned to 4 bytes only: vec says whether
+// its rows take the vector loads (rows_aligned).
+template <int D>
+__device__ __forceinline__ void load_row(const float *__restrict__ p, float (&x)[D], bool vec) {
+    if ((D % 4 == 0 || D == 2) && vec) {
+        load_row<D>(p, x);
+    } else {
+#pragma unroll
+        for (int k = 0; k < D; ++k) x[k] = __ldg(p + k);
+    }
+}
+template <int D>
+inline bool rows_aligned(const float *p) {
+    return ((uintptr_t)p & (D % 4 == 0 ? 15 : 7)) == 0;
+}
+
+// lo_hi[0..D) = ordered-int min, lo_hi[D..2D) = ordered-int max.  Warps reduce by
+// shuffles, the block through shared memory, and one thread per dimension and bound
+// issues the block's atomic: with one atomic per warp the kernel's time was the queue of
+// atomics on 2 D addresses (16-D 200k 128 -> 8 us, 8-D 2M 110 -> 17 us).
+template <int D>
+__global__ void __launch_bounds__(kBlock) bbox_kernel(const float *__restrict__ coords, int64_t n, bool vec,
                                                       int *lo_hi, unsigned long long *n_invalid) {
+    __shared__ int s_lh[kBlock / kWarp][2 * D];
+    __shared__ unsigned s_bad[kBlock / kWarp];
     int lo[D], hi[D];
 #pragma unroll
     for (int k = 0; k < D; ++k) {
@@ -134,10 +208,8 @@ __global__ void __launch_bounds__(kBlock) bbox_kernel(const float *__restrict__ 
     unsigned bad = 0;
     for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n;
          i += (int64_t)gridDim.x * blockDim.x) {
-        const float *p = coords + i * D;
         float x[D];
-#pragma unroll
-        for (int k = 0; k < D; ++k) x[k] = p[k];
+        load_row<D>(coords + i * D, x, vec);
         bool ok = x[0] != FLT_MAX;
 #pragma unroll
         for (int k = 0; k < D; ++k) ok = ok && isfinite(x[k]);
@@ -152,24 +224,7 @@ __global__ void __launch_bounds__(kBlock) bbox_kernel(const float *__restrict__ 
             hi[k] = max(hi[k], v);
         }
     }
-#pragma unroll
-    for (int k = 0; k < D; ++k) {
-#pragma unroll
-        for (int o = 16; o > 0; o >>= 1) {
-            lo[k] = min(lo[k], __shfl_xor_sync(kFull, lo[k], o));
-            hi[k] = max(hi[k], __shfl_xor_sync(kFull, hi[k], o));
-        }
-    }
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) bad += __shfl_xor_sync(kFull, bad, o);
-    if ((threadIdx.x & 31) == 0) {
-#pragma unroll
-        for (int k = 0; k < D; ++k) {
-            if (lo[k] != 0x7fffffff) atomicMin(lo_hi + k, lo[k]);
-            if (hi[k] != (int)0x80000000) atomicMax(lo_hi + D + k, hi[k]);
-        }
-        if (bad) atomicAdd(n_invalid, (unsigned long long)bad);
-    }
+    bbox_reduce<D>(lo, hi, bad, s_lh, s_bad, lo_hi, n_invalid);
 }
 
 // Cell coordinate along gridded dimension a.  Computed in double: with at most
@@ -184,13 +239,18 @@ __device__ __forceinline__ long long cell_coord(const GridDev &g, int a, float x
 }
 
 template <int D, typename K>
-__global__ void __launch_bounds__(kBlock) key_kernel(const float *__restrict__ coords, int64_t n,
+__global__ void __launch_bounds__(kBlock) key_kernel(const float *__restrict__ coords, int64_t n, bool vec,
                                                      GridDev g, K invalid_key, K *__restrict__ keys) {
     const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n) return;
     const float *p = coords + i * D;
     K key = invalid_key;
-    if (point_valid<D>(p)) {
+    float x[D];  // validity from one load of the row; the gridded coordinates are re-read (L1)
+    load_row<D>(p, x, vec);
+    bool ok = x[0] != FLT_MAX;
+#pragma unroll
+    for (int k = 0; k < D; ++k) ok = ok && isfinite(x[k]);
+    if (ok) {
         unsigned long long kk = 0;
 #pragma unroll
         for (int a = 0; a < kMaxGridDims; ++a)
@@ -226,15 +286,15 @@ __global__ void cell_write_kernel(const K *__restrict__ keys, int64_t nv, const 
 
 template <int D>
 __global__ void __launch_bounds__(kBlock) gather_kernel(const float *__restrict__ coords,
-                                                        const int32_t *__restrict__ perm, int64_t nv,
+                                                        const int32_t *__restrict__ perm, int64_t nv, bool vec,
                                                         float *__restrict__ xs) {
     constexpr int P = Stride<D>::P;
     const int64_t s = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (s >= nv) return;
-    const float *p = coords + (int64_t)perm[s] * D;
-    float v[P];
+    float x[D], v[P];
+    load_row<D>(coords + (int64_t)perm[s] * D, x, vec);
 #pragma unroll
-    for (int k = 0; k < P; ++k) v[k] = k < D ? p[k] : 0.0f;
+    for (int k = 0; k < P; ++k) v[k] = k < D ? x[k] : 0.0f;
     float *q = xs + s * P;
     if constexpr (P % 4 == 0) {
 #pragma unroll
@@ -1969,32 +2029,8 @@ __global__ void bbox_batch_init_kernel(int *lo_hi, int d, int n_jobs, unsigned l
     if (i < n_jobs) n_invalid[i] = 0ull;
 }
 
-// One point's coordinates: 16-byte vector loads when a point's row is a multiple of
-// 16 bytes (d % 4 == 0; rows then start 16-byte aligned), 8-byte ones at d = 2.
-template <int D>
-__device__ __forceinline__ void load_row(const float *__restrict__ p, float (&x)[D]) {
-    if constexpr (D % 4 == 0) {
-#pragma unroll
-        for (int q = 0; q < D / 4; ++q) {
-            const float4 v = __ldg(reinterpret_cast<const float4 *>(p) + q);
-            x[4 * q + 0] = v.x;
-            x[4 * q + 1] = v.y;
-            x[4 * q + 2] = v.z;
-            x[4 * q + 3] = v.w;
-        }
-    } else if constexpr (D == 2) {
-        const float2 v = __ldg(reinterpret_cast<const float2 *>(p));
-        x[0] = v.x;
-        x[1] = v.y;
-    } else {
-#pragma unroll
-        for (int k = 0; k < D; ++k) x[k] = __ldg(p + k);
-    }
-}
-
 // Per-job bounding boxes (ordered-int min/max per dimension) and invalid-point counts
-// of a batch: blocks (x, job).  Warps reduce by shuffles, the block through shared
-// memory, and one lane per dimension and bound issues the block's atomic.
+// of a batch: blocks (x, job).
 template <int D>
 __global__ void __launch_bounds__(kBlock) bbox_batch_kernel(const float *__restrict__ coords,
                                                             const JobDev *__restrict__ jobs, int *lo_hi,
@@ -2028,38 +2064,7 @@ __global__ void __launch_bounds__(kBlock) bbox_batch_kernel(const float *__restr
             hi[k] = max(hi[k], v);
         }
     }
-#pragma unroll
-    for (int k = 0; k < D; ++k) {
-        lo[k] = __reduce_min_sync(kFull, lo[k]);
-        hi[k] = __reduce_max_sync(kFull, hi[k]);
-    }
-    bad = __reduce_add_sync(kFull, bad);
-    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-    if (lane == 0) {
-#pragma unroll
-        for (int k = 0; k < D; ++k) {
-            s_lh[w][k] = lo[k];
-            s_lh[w][D + k] = hi[k];
-        }
-        s_bad[w] = bad;
-    }
-    __syncthreads();
-    if (threadIdx.x < 2 * D) {
-        const int t = threadIdx.x;
-        int v = s_lh[0][t];
-        for (int q = 1; q < W; ++q) v = t < D ? min(v, s_lh[q][t]) : max(v, s_lh[q][t]);
-        int *lh = lo_hi + (int64_t)j * 2 * D;
-        if (t < D) {
-            if (v != 0x7fffffff) atomicMin(lh + t, v);
-        } else {
-            if (v != (int)0x80000000) atomicMax(lh + t, v);
-        }
-    }
-    if (threadIdx.x == 0) {
-        unsigned b = 0;
-        for (int q = 0; q < W; ++q) b += s_bad[q];
-        if (b) atomicAdd(n_invalid + j, (unsigned long long)b);
-    }
+    bbox_reduce<D>(lo, hi, bad, s_lh, s_bad, lo_hi + (int64_t)j * 2 * D, n_invalid + j);
 }
 
 template <int D, typename K>
