@@ -41,7 +41,7 @@ struct ndb_ctx {
     DevBuf coords, keys0, keys1, ids0, ids1, flags, pos, pcell, xs;
     DevBuf nn_sorted, nn_orig, core_sorted, core_bits, core_prefix, ci_sorted, ci_orig, labels;
     // per-cell arrays
-    DevBuf cell_start, cell_key, nbr, item_cnt, items, cell_has_core, cell_cid, hash_keys, hash_vals;
+    DevBuf cell_start, cell_key, nbr, items, cell_has_core, cell_cid, hash_keys, hash_vals;
     // column table of the grid (CellIndex): one [first, end) cell range per column
     DevBuf col_range;
     size_t col_budget = size_t(1) << 27;  // largest column table (entries) a run may build, else the hash table
@@ -56,7 +56,7 @@ struct ndb_ctx {
     bool gram_count = false;          // CUDA-core count with the Gram filter (d >= 8)
     int sm_count = 148;
     // scratch
-    DevBuf sort_hist, scan_scratch, small;  // small: counters, bbox, scalars
+    DevBuf sort_hist, small;  // sort and chain-scan state; counters, bbox, scalars
     // batched runs: job table, per-job bounding boxes, cell -> job, per-job counters
     DevBuf jobs_dev, batch_bbox, cell_job, job_counters;
     // items split between the tensor-core count (full items) and the exact one, and
@@ -96,8 +96,8 @@ struct ndb_ctx {
         DevBuf *bufs[] = {&coords,      &keys0,       &keys1,       &ids0,        &ids1,        &flags,
                           &pos,         &pcell,       &xs,          &nn_sorted,   &nn_orig,     &core_sorted,
                           &core_bits,   &core_prefix, &ci_sorted,   &ci_orig,     &labels,      &cell_start,
-                          &cell_key,    &nbr,         &item_cnt,    &items,       &cell_has_core, &cell_cid,
-                          &parent,      &comp_min,    &sort_hist,   &scan_scratch, &small,      &hash_keys,
+                          &cell_key,    &nbr,         &items,       &cell_has_core, &cell_cid,
+                          &parent,      &comp_min,    &sort_hist,   &small,       &hash_keys,
                           &hash_vals,   &nbr_list,    &jobs_dev,    &batch_bbox,  &cell_job,    &job_counters,
                           &items_split, &col_range,   &ids_in,      &batch_in,    &batch_nn,    &batch_ci,
                           &load_box,    &tc_rec};
@@ -124,6 +124,7 @@ struct ndb_ctx {
     int cell_units = 0;
     int n_rows = 0;
     unsigned long long hash_mask = 0;
+    int32_t *nn_late = nullptr;  // ndb_b200_run on device buffers: the label phase writes the counts there
     int32_t *ci_user = nullptr;  // caller's cluster_index buffer of the current assign_labels call
     const float *coords_dev = nullptr;  // device coordinates of the current job
     GridDev grid{};
@@ -145,8 +146,7 @@ constexpr size_t kSmallCountersOff = 512;    // u64[12]: 0 clusters 1 noise 2 co
 constexpr int kCounters = 12;
 constexpr size_t kSmallScalarOff = 1024;     // u32[8]: 0 n_cells 1 n_items 2 n_cores 4 tensor items 5 exact items 6 union segments 7 tensor chunks
 constexpr size_t kSmallErrOff = 1536;        // int
-constexpr size_t kSmallStencilOff = 2048;    // int4[kMaxRows]: stencil rows of the current job
-constexpr size_t kSmallBytes = 4096;
+constexpr size_t kSmallBytes = 2048;
 
 // Destination window of the input-order output scatters: 24M int32 (96 MB) stays
 // within the 126 MB L2, so outputs larger than that are written in several passes.
@@ -215,11 +215,16 @@ inline void fill_bytes(ndb_ctx *ctx, void *p, int v, size_t bytes, cudaStream_t 
     ck(ctx, cudaGetLastError());
 }
 
+constexpr size_t kMailSingle = 16 * 1024;  // a single job's transfers: bounds, cell count, counters
+
 // The mailbox holds at least `bytes`; grown only between runs (nothing of the
 // context in flight).
 inline void ensure_mail(ndb_ctx *ctx, size_t bytes) {
     if (bytes <= ctx->mail_bytes) return;
-    bytes = (bytes + (size_t(1) << 20) - 1) & ~((size_t(1) << 20) - 1);
+    // small ones stay small: the driver serves them from a block it has already pinned
+    // (4 us against 1.5 ms for a megabyte of its own)
+    const size_t unit = bytes <= kMailSingle ? 4096 : size_t(1) << 20;
+    bytes = (bytes + unit - 1) / unit * unit;
     if (ctx->mail) {
         cudaFreeHost(ctx->mail);
         ctx->mail = ctx->mail_dev = nullptr;
@@ -439,6 +444,7 @@ template <typename K>
 CellIndex<K> build_cell_index(ndb_ctx *ctx, int64_t n_cells, double columns, const GridDev &g_one,
                               const JobDev *jobs, const int32_t *cell_job) {
     cudaStream_t st = ctx->stream;
+    const uint32_t *n_cells_dev = small_at<uint32_t>(ctx, kSmallScalarOff);
     CellIndex<K> L{nullptr, nullptr, nullptr, 0};
     ctx->use_cols = columns >= 1 && columns <= (double)ctx->col_budget;
     if (ctx->use_cols) {
@@ -446,7 +452,7 @@ CellIndex<K> build_cell_index(ndb_ctx *ctx, int64_t n_cells, double columns, con
         ensure(ctx, ctx->col_range, (cols + 1) * sizeof(int2));
         fill_bytes(ctx, ctx->col_range.ptr, 0, (size_t)(cols + 1) * sizeof(int2), st);
         ++launch_counter(), col_range_kernel<K><<<blocks_for(n_cells), kBlock, 0, st>>>(
-            ctx->cell_key.as<K>(), n_cells, g_one, jobs, cell_job, ctx->col_range.as<int2>());
+            ctx->cell_key.as<K>(), n_cells_dev, g_one, jobs, cell_job, ctx->col_range.as<int2>());
         ck(ctx, cudaGetLastError());
         L.col = ctx->col_range.as<int2>();
         return L;
@@ -458,7 +464,7 @@ CellIndex<K> build_cell_index(ndb_ctx *ctx, int64_t n_cells, double columns, con
     ensure(ctx, ctx->hash_vals, hsize * sizeof(int32_t));
     ++launch_counter(), hash_clear_kernel<K><<<blocks_for(hsize), kBlock, 0, st>>>(ctx->hash_keys.as<K>(), hsize);
     ++launch_counter(), hash_insert_kernel<K><<<blocks_for(n_cells), kBlock, 0, st>>>(
-        ctx->cell_key.as<K>(), n_cells, ctx->hash_keys.as<K>(), ctx->hash_vals.as<int32_t>(), ctx->hash_mask);
+        ctx->cell_key.as<K>(), n_cells_dev, ctx->hash_keys.as<K>(), ctx->hash_vals.as<int32_t>(), ctx->hash_mask);
     ck(ctx, cudaGetLastError());
     L.hkeys = ctx->hash_keys.as<K>();
     L.hvals = ctx->hash_vals.as<int32_t>();
@@ -479,99 +485,132 @@ CellIndex<K> cell_index(ndb_ctx *ctx) {
     return CellIndex<K>{nullptr, ctx->hash_keys.as<K>(), ctx->hash_vals.as<int32_t>(), ctx->hash_mask};
 }
 
-template <int D, typename K>
-void classify_grid(ndb_ctx *ctx, const Plan &pl) {
+// One pipeline: a single job, or the jobs of a batch (then e2, min_pts and list_cap come
+// from the job table).
+struct Pipe {
+    int64_t n = 0, nv = 0;  // points, points in the grid
+    int key_bits = 0;
+    GridDev g{};
+    const Stencil *stencil = nullptr;
+    double columns = 0;  // entries of the column table
+    bool linked = false, early = true;
+    float e2 = 0.0f;
+    int min_pts = 0;
+    const JobDev *jobs = nullptr;
+    int n_jobs = 0;
+    // neighbour lists: entries recorded and their stride (0: none)
+    int32_t *list = nullptr;
+    int list_cap = 0, list_stride = 0;
+    // set by grid_phase: upper bounds of the cells and items (exact counts on the
+    // device, scalars 0 and 1), and the batch's cell -> job map
+    int64_t cells = 0, items = 0;
+    const int32_t *cell_job = nullptr;
+};
+
+// Up to this many points a single job's cells are bounded by its points instead of
+// waiting for their count: the launches over the bound cost less than the round trip
+// (1,000 points 2-D: 15 us), and the row table stays under 18 MB.
+constexpr int64_t kNoCountPoints = int64_t(1) << 16;
+
+// State of the grid phase's chain scans, zeroed with the sort's scratch behind it: three
+// tickets, then the state words of the cells', items' and bitmap words' tiles.
+constexpr int kCellsPer = 8, kItemsPer = 4, kWordsPer = 8;  // elements per thread
+constexpr int64_t chain_tiles(int64_t n, int per) { return n / (kChainThreads * per) + 1; }
+constexpr size_t chain_words(int64_t n) {
+    return 4 + 2 * (size_t)(chain_tiles(n, kCellsPer) + chain_tiles(n, kItemsPer) + chain_tiles(n / 32 + 1, kWordsPer));
+}
+
+struct Chain {
+    uint32_t *ticket;
+    unsigned long long *state[3];
+};
+template <typename K>
+Chain chain_area(ndb_ctx *ctx, int64_t n) {
+    uint32_t *w = ctx->sort_hist.as<uint32_t>() + sort_scratch_words<K>(n);
+    auto *s = reinterpret_cast<unsigned long long *>(w + 4);
+    return Chain{w, {s, s + chain_tiles(n, kCellsPer), s + chain_tiles(n, kCellsPer) + chain_tiles(n, kItemsPer)}};
+}
+
+// Keys (written by launch_keys), sort, cells, cell index, stencil rows, work items.
+template <int D, typename K, typename F>
+void grid_phase(ndb_ctx *ctx, Pipe &p, const float *coords, F launch_keys) {
     cudaStream_t st = ctx->stream;
-    const int64_t n = ctx->n;
-    const int64_t nv = ctx->nv;
+    const int64_t n = p.n, nv = p.nv;
     constexpr int P = Stride<D>::P;
+    uint32_t *scal = small_at<uint32_t>(ctx, kSmallScalarOff);
 
     ensure(ctx, ctx->keys0, n * sizeof(K));
     ensure(ctx, ctx->keys1, n * sizeof(K));
     ensure(ctx, ctx->ids0, n * sizeof(int32_t));
     ensure(ctx, ctx->ids1, n * sizeof(int32_t));
-    ensure(ctx, ctx->sort_hist, sort_scratch_words<K>(n) * sizeof(uint32_t));
-    ensure(ctx, ctx->scan_scratch, (scan_scratch_words(n + 1) + 64) * sizeof(uint32_t));
+    const size_t zero_words = sort_scratch_words<K>(n) + chain_words(n);
+    ensure(ctx, ctx->sort_hist, (zero_words + 4) * sizeof(uint32_t));
+    ensure(ctx, ctx->core_bits, ((n + 31) / 32 + 1) * sizeof(uint32_t));
+    ensure(ctx, ctx->pcell, (n + 1) * sizeof(int32_t));
+    ensure(ctx, ctx->cell_start, (n + 2) * sizeof(int32_t));
+    ensure(ctx, ctx->cell_key, (n + 1) * sizeof(K));
+    ensure(ctx, ctx->xs, (nv + 1) * P * sizeof(float));
 
-    K invalid_key = (K)(pl.key_bits >= (int)(8 * sizeof(K)) ? ~(K)0 : (((K)1 << pl.key_bits) - 1));
-    ++launch_counter(), key_kernel<D, K><<<blocks_for(n), kBlock, 0, st>>>(ctx->coords_dev, n, rows_aligned<D>(ctx->coords_dev),
-                                                        pl.g, invalid_key, ctx->keys0.as<K>());
+    const K invalid_key = (K)(p.key_bits >= (int)(8 * sizeof(K)) ? ~(K)0 : (((K)1 << p.key_bits) - 1));
+    launch_keys(invalid_key, ctx->keys0.as<K>(), ctx->core_bits.as<uint32_t>());
     ck(ctx, cudaGetLastError());
     bool in_first = true;
     cudaEventRecord(ctx->kev[0], st);
     if (sizeof(K) == 4)
         ck(ctx, radix_sort_pairs_u32(reinterpret_cast<uint32_t *>(ctx->keys0.ptr), ctx->ids0.as<int32_t>(),
                                      reinterpret_cast<uint32_t *>(ctx->keys1.ptr), ctx->ids1.as<int32_t>(), n,
-                                     pl.key_bits, ctx->sort_hist.as<uint32_t>(), &in_first, st));
+                                     p.key_bits, ctx->sort_hist.as<uint32_t>(), zero_words, &in_first, st));
     else
         ck(ctx, radix_sort_pairs_u64(reinterpret_cast<uint64_t *>(ctx->keys0.ptr), ctx->ids0.as<int32_t>(),
                                      reinterpret_cast<uint64_t *>(ctx->keys1.ptr), ctx->ids1.as<int32_t>(), n,
-                                     pl.key_bits, ctx->sort_hist.as<uint32_t>(), &in_first, st));
+                                     p.key_bits, ctx->sort_hist.as<uint32_t>(), zero_words, &in_first, st));
     cudaEventRecord(ctx->kev[1], st);
-    ctx->stats.sort_passes = (pl.key_bits + 7) / 8;
-    ctx->stats.key_bytes = (int32_t)sizeof(K);
     if (!in_first) {
         std::swap(ctx->keys0, ctx->keys1);
         std::swap(ctx->ids0, ctx->ids1);
     }
-    const K *keys = ctx->keys0.as<K>();
-    const int32_t *perm = ctx->ids0.as<int32_t>();
+    const Chain chain = chain_area<K>(ctx, n);
 
     // cells
-    ensure(ctx, ctx->flags, (n + 1) * sizeof(uint32_t));
-    ensure(ctx, ctx->pos, (n + 1) * sizeof(uint32_t));
-    ensure(ctx, ctx->pcell, (n + 1) * sizeof(int32_t));
-    ensure(ctx, ctx->cell_start, (n + 2) * sizeof(int32_t));
-    ensure(ctx, ctx->cell_key, (n + 1) * sizeof(K));
-    uint32_t *scal = small_at<uint32_t>(ctx, kSmallScalarOff);
-    ++launch_counter(), cell_flag_kernel<K><<<blocks_for(nv), kBlock, 0, st>>>(keys, nv, ctx->flags.as<uint32_t>());
+    auto *m_cells = reinterpret_cast<volatile uint32_t *>(mail_slice(ctx, sizeof(uint32_t)));
+    auto *m_cells_dev = reinterpret_cast<volatile uint32_t *>(ctx->mail_dev + ((const char *)m_cells - ctx->mail));
+    ++launch_counter(), chain_scan_kernel<kCellsPer><<<(unsigned)chain_tiles(nv, kCellsPer), kChainThreads, 0, st>>>(
+        CellsOp<D, K>{ctx->keys0.as<K>(), ctx->ids0.as<int32_t>(), coords, rows_aligned<D>(coords), nv,
+                      ctx->xs.as<float>(), ctx->cell_start.as<int32_t>(), ctx->cell_key.as<K>(),
+                      ctx->pcell.as<int32_t>()},
+        nv, nullptr, chain.state[0], chain.ticket + 0, scal + 0, m_cells_dev);
     ck(ctx, cudaGetLastError());
-    ck(ctx, scan_exclusive_u32(ctx->flags.as<uint32_t>(), ctx->pos.as<uint32_t>(), nv, scal + 0,
-                               ctx->scan_scratch.as<uint32_t>(), st));
-    ++launch_counter(), cell_write_kernel<K><<<blocks_for(nv), kBlock, 0, st>>>(keys, nv, ctx->pos.as<uint32_t>(), scal + 0,
-                                                            ctx->cell_start.as<int32_t>(), ctx->cell_key.as<K>(),
-                                                            ctx->pcell.as<int32_t>());
-    ck(ctx, cudaGetLastError());
-    ensure(ctx, ctx->xs, (nv + 1) * P * sizeof(float));
-    ++launch_counter(), gather_kernel<D><<<blocks_for(nv), kBlock, 0, st>>>(ctx->coords_dev, perm, nv,
-                                                        rows_aligned<D>(ctx->coords_dev), ctx->xs.as<float>());
-    ck(ctx, cudaGetLastError());
-    uint32_t n_cells32 = 0;
-    ck(ctx, cudaMemcpyAsync(&n_cells32, scal + 0, sizeof(uint32_t), cudaMemcpyDeviceToHost, st));
-    ck(ctx, cudaStreamSynchronize(st));
-    const int64_t n_cells = n_cells32;
-    ctx->n_cells = n_cells;
+    if (!p.jobs && nv <= kNoCountPoints) {
+        p.cells = nv;
+    } else {
+        ck(ctx, cudaStreamSynchronize(st));
+        p.cells = nv > 0 ? *m_cells : 0;
+    }
+    if (p.jobs) {
+        ensure(ctx, ctx->cell_job, (p.cells + 1) * sizeof(int32_t));
+        ++launch_counter(), cell_job_kernel<K><<<blocks_for(p.cells), kBlock, 0, st>>>(
+            ctx->cell_key.as<K>(), p.cells, p.jobs, p.n_jobs, ctx->cell_job.as<int32_t>());
+        p.cell_job = ctx->cell_job.as<int32_t>();
+    }
 
     // neighbour rows, through the column table (or a hash table) of the cells
-    const int n_rows = pl.st.n_rows;
-    const CellIndex<K> L = build_cell_index<K>(ctx, n_cells, grid_columns(pl.g), pl.g, nullptr, nullptr);
-    ensure(ctx, ctx->nbr, (size_t)(n_cells * n_rows + 1) * sizeof(int2));
-    int4 *rows_dev = small_at<int4>(ctx, kSmallStencilOff);
-    ck(ctx, cudaMemcpyAsync(rows_dev, pl.st.rows, n_rows * sizeof(int4), cudaMemcpyHostToDevice, st));
+    const int n_rows = p.stencil->n_rows;
+    const CellIndex<K> L = build_cell_index<K>(ctx, p.cells, p.columns, p.g, p.jobs, p.cell_job);
+    ensure(ctx, ctx->nbr, (size_t)(p.cells * n_rows + 1) * sizeof(int2));
     const int rlog = row_group_log2(n_rows);
-    ++launch_counter(), rows_kernel<K><<<blocks_for(n_cells << rlog), kBlock, 0, st>>>(
-        ctx->cell_key.as<K>(), n_cells, pl.g, rows_dev, n_rows, rlog, L, ctx->nbr.as<int2>(), nullptr, nullptr);
+    ++launch_counter(), rows_kernel<K><<<blocks_for(p.cells << rlog), kBlock, 0, st>>>(
+        ctx->cell_key.as<K>(), scal + 0, p.g, *p.stencil, rlog, L, ctx->nbr.as<int2>(), p.jobs, p.cell_job);
     ck(ctx, cudaGetLastError());
 
-    // work items
-    ensure(ctx, ctx->item_cnt, (n_cells + 1) * sizeof(uint32_t));
-    ++launch_counter(), item_count_kernel<<<blocks_for(n_cells), kBlock, 0, st>>>(ctx->cell_start.as<int32_t>(), n_cells,
-                                                              ctx->item_cnt.as<uint32_t>());
-    ck(ctx, cudaGetLastError());
-    ck(ctx, scan_exclusive_u32(ctx->item_cnt.as<uint32_t>(), ctx->item_cnt.as<uint32_t>(), n_cells, scal + 1,
-                               ctx->scan_scratch.as<uint32_t>(), st));
-    uint32_t n_items32 = 0;
-    ck(ctx, cudaMemcpyAsync(&n_items32, scal + 1, sizeof(uint32_t), cudaMemcpyDeviceToHost, st));
-    ck(ctx, cudaStreamSynchronize(st));
-    ctx->n_items = n_items32;
-    ensure(ctx, ctx->items, (ctx->n_items + 1) * sizeof(int2));
-    ++launch_counter(), item_write_kernel<<<blocks_for(n_cells), kBlock, 0, st>>>(ctx->cell_start.as<int32_t>(), n_cells,
-                                                              ctx->item_cnt.as<uint32_t>(), ctx->items.as<int2>());
+    // work items: at most one per cell and one more per 32 points
+    p.items = std::min(nv, p.cells + nv / kTile);
+    ensure(ctx, ctx->items, (p.items + 1) * sizeof(int2));
+    ensure(ctx, ctx->cell_has_core, p.cells + 1);
+    ++launch_counter(), chain_scan_kernel<kItemsPer><<<(unsigned)chain_tiles(p.cells, kItemsPer), kChainThreads, 0, st>>>(
+        ItemsOp{ctx->cell_start.as<int32_t>(), ctx->items.as<int2>(), ctx->cell_has_core.as<uint8_t>()}, p.cells,
+        scal + 0, chain.state[1], chain.ticket + 1, scal + 1, nullptr);
     ck(ctx, cudaGetLastError());
 }
-
-template <int D>
-void count_phase(ndb_ctx *ctx);
 
 // The tensor-core filter's preconditions: d >= 8 (and, unless NDB_FLAG_TENSOR_FILTER
 // asks for it or counts are full, d at or above the automatic threshold: 12 by
@@ -699,21 +738,21 @@ void count_items(ndb_ctx *ctx, bool tc, bool force_tc, bool gram, bool early, in
                  const int32_t *cell_start, const int2 *nbr, int n_rows, const float *xs, float e2, int min_pts,
                  int dense_skip, int32_t *nn_sorted, int32_t *list, int list_cap, int list_stride,
                  const JobDev *jobs, const int32_t *cell_job, bool audit, int64_t nv, int64_t n_cells) {
-    if (n_items <= 0) return;
+    if (n_items <= 0) return;  // an upper bound; the count is scalar 1
     cudaStream_t st = ctx->stream;
     unsigned long long *counters = small_at<unsigned long long>(ctx, kSmallCountersOff);
+    uint32_t *scal = small_at<uint32_t>(ctx, kSmallScalarOff);
     const int2 *ex_items = items;
-    const uint32_t *ex_n = nullptr;
+    const uint32_t *ex_n = scal + 1;
     if (tc) {
         // scalars: 4 32-point items in chunks, 5 items of the exact kernel, 7 chunks
-        uint32_t *scal = small_at<uint32_t>(ctx, kSmallScalarOff);
         ensure(ctx, ctx->items_split, (size_t)(2 * n_items + 2) * sizeof(int2));
         int2 *chunks = ctx->items_split.as<int2>();
         int2 *rest = chunks + n_items + 1;
         const int chunk = tc_chunk(ctx, nv, early);
         fill_bytes(ctx, scal + 4, 0, 4 * sizeof(uint32_t), st);
         ++launch_counter(), tc::split_cells_kernel<<<blocks_for(n_cells), kBlock, 0, st>>>(
-            cell_start, n_cells, force_tc ? 1 : ctx_tc_min_item(ctx), chunk, chunks, scal + 7, rest, scal + 5, scal + 4);
+            cell_start, scal + 0, force_tc ? 1 : ctx_tc_min_item(ctx), chunk, chunks, scal + 7, rest, scal + 5, scal + 4);
         ck(ctx, cudaGetLastError());
         launch_count_tc<D>(ctx, n_items, chunks, scal + 7, chunk, cell_start, nbr, n_rows, xs, e2, min_pts, early,
                            nn_sorted, list, list_cap, list_stride, jobs, cell_job, audit);
@@ -725,8 +764,8 @@ void count_items(ndb_ctx *ctx, bool tc, bool force_tc, bool gram, bool early, in
     auto launch = [&](auto early_c, auto gram_c) {
         constexpr bool E = decltype(early_c)::value, G = decltype(gram_c)::value;
         ++launch_counter(), count_kernel<D, E, G><<<grid, kCountWarps * kWarp, 0, st>>>(
-            ex_items, n_items, cell_start, nbr, n_rows, xs, e2, min_pts, dense_skip, nn_sorted, list, list_cap,
-            list_stride, counters + 2, jobs, cell_job, ex_n, counters + 5);
+            ex_items, ex_n, cell_start, nbr, n_rows, xs, e2, min_pts, dense_skip, nn_sorted, list, list_cap,
+            list_stride, counters + 2, jobs, cell_job, counters + 5);
     };
     using T = std::true_type;
     using F = std::false_type;
@@ -743,97 +782,156 @@ void count_items(ndb_ctx *ctx, bool tc, bool force_tc, bool gram, bool early, in
     ck(ctx, cudaGetLastError());
 }
 
-template <int D>
-void count_phase(ndb_ctx *ctx) {
+// Neighbour counts and core flags of a pipeline.
+template <int D, typename K>
+void count_phase(ndb_ctx *ctx, const Pipe &p, bool tc, bool gram, uint32_t flags) {
     cudaStream_t st = ctx->stream;
-    unsigned long long *counters = small_at<unsigned long long>(ctx, kSmallCountersOff);
-    ensure(ctx, ctx->nn_sorted, (ctx->n + 1) * sizeof(int32_t));
-    const bool early = (ctx->flags_run & NDB_FLAG_FULL_COUNT) == 0;
-    // neighbour lists for the border step: min_pts - 1 entries per point
-    ctx->list_cap = 0;
-    const int64_t cap = (int64_t)ctx->min_pts - 1;
-    if (cap >= 1 && cap <= kMaxListCap && (size_t)(ctx->nv * cap) * sizeof(int32_t) <= ctx->list_budget) {
-        ensure(ctx, ctx->nbr_list, (size_t)(ctx->nv * cap + 1) * sizeof(int32_t));
-        ctx->list_cap = (int)cap;
-    }
-    int32_t *list = ctx->list_cap ? ctx->nbr_list.as<int32_t>() : nullptr;
+    const int64_t n = p.n, n_words = (n + 31) / 32;
+    uint32_t *scal = small_at<uint32_t>(ctx, kSmallScalarOff);
+    ensure(ctx, ctx->nn_sorted, (n + 1) * sizeof(int32_t));
     cudaEventRecord(ctx->kev[2], st);
-    count_items<D>(ctx, ctx->tc_count, (ctx->flags_run & NDB_FLAG_TENSOR_FILTER) != 0, ctx->gram_count, early,
-                   ctx->n_items,
-                   ctx->items.as<int2>(), ctx->cell_start.as<int32_t>(), ctx->nbr.as<int2>(), ctx->n_rows,
-                   ctx->xs.as<float>(), ctx->e2, ctx->min_pts, ctx->cell_units, ctx->nn_sorted.as<int32_t>(), list,
-                   ctx->list_cap, ctx->list_cap, nullptr, nullptr, (ctx->flags_run & NDB_FLAG_FILTER_AUDIT) != 0,
-                   ctx->nv, ctx->n_cells);
+    count_items<D>(ctx, tc, (flags & NDB_FLAG_TENSOR_FILTER) != 0, gram, p.early, p.items, ctx->items.as<int2>(),
+                   ctx->cell_start.as<int32_t>(), ctx->nbr.as<int2>(), p.stencil->n_rows, ctx->xs.as<float>(), p.e2,
+                   p.min_pts, p.linked, ctx->nn_sorted.as<int32_t>(), p.list, p.list_cap, p.list_stride, p.jobs,
+                   p.cell_job, (flags & NDB_FLAG_FILTER_AUDIT) != 0, p.nv, p.cells);
     cudaEventRecord(ctx->kev[3], st);
+    ensure(ctx, ctx->core_sorted, n + 1);
+    ensure(ctx, ctx->core_prefix, (n_words + 1) * sizeof(uint32_t));
+    ++launch_counter(), core_flags_kernel<<<blocks_for(n), kBlock, 0, st>>>(
+        ctx->nn_sorted.as<int32_t>(), p.nv, n, p.min_pts, ctx->ids0.as<int32_t>(), ctx->pcell.as<int32_t>(),
+        ctx->core_sorted.as<uint8_t>(), ctx->cell_has_core.as<uint8_t>(), ctx->core_bits.as<uint32_t>(), p.jobs,
+        p.cell_job, p.n_jobs);
+    // ranks among cores in input order (data_process.cpp:276-283, :153): per-word prefix of the bitmap
+    const Chain chain = chain_area<K>(ctx, n);
+    ++launch_counter(), chain_scan_kernel<kWordsPer><<<(unsigned)chain_tiles(n_words, kWordsPer), kChainThreads, 0, st>>>(
+        CorePrefixOp{ctx->core_bits.as<uint32_t>(), ctx->core_prefix.as<uint32_t>()}, n_words, nullptr, chain.state[2],
+        chain.ticket + 2, scal + 2, nullptr);
+    ck(ctx, cudaGetLastError());
 }
 
-void core_flags_phase(ndb_ctx *ctx) {
+template <int D, typename K>
+void classify_keys(ndb_ctx *ctx, Pipe &p) {
     cudaStream_t st = ctx->stream;
     const int64_t n = ctx->n;
-    const int64_t n_words = (n + 31) / 32;
-    uint32_t *scal = small_at<uint32_t>(ctx, kSmallScalarOff);
-    ensure(ctx, ctx->core_sorted, n + 1);
-    ensure(ctx, ctx->cell_has_core, ctx->n_cells + 1);
-    ensure(ctx, ctx->core_bits, (n_words + 1) * sizeof(uint32_t));
-    ensure(ctx, ctx->core_prefix, (n_words + 1) * sizeof(uint32_t));
-    fill_bytes(ctx, ctx->cell_has_core.ptr, 0, (size_t)ctx->n_cells + 1, st);
-    fill_bytes(ctx, ctx->core_bits.ptr, 0, (size_t)(n_words + 1) * sizeof(uint32_t), st);
-    ++launch_counter(), core_flags_kernel<<<blocks_for(n), kBlock, 0, st>>>(
-        ctx->nn_sorted.as<int32_t>(), ctx->nv, n, ctx->min_pts, ctx->ids0.as<int32_t>(), ctx->pcell.as<int32_t>(),
-        ctx->core_sorted.as<uint8_t>(), ctx->cell_has_core.as<uint8_t>(), ctx->core_bits.as<uint32_t>(), nullptr,
-        nullptr, 0);
-    // ranks among cores in input order (data_process.cpp:276-283, :153): per-word prefix of the bitmap
-    ++launch_counter(), popc_words_kernel<<<blocks_for(n_words), kBlock, 0, st>>>(
-        ctx->core_bits.as<uint32_t>(), n_words, ctx->core_prefix.as<uint32_t>());
-    ck(ctx, cudaGetLastError());
-    ck(ctx, scan_exclusive_u32(ctx->core_prefix.as<uint32_t>(), ctx->core_prefix.as<uint32_t>(), n_words, scal + 2,
-                               ctx->scan_scratch.as<uint32_t>(), st));
+    ctx->stats.sort_passes = (p.key_bits + 7) / 8;
+    ctx->stats.key_bytes = (int32_t)sizeof(K);
+    grid_phase<D, K>(ctx, p, ctx->coords_dev, [&](K invalid_key, K *keys, uint32_t *core_bits) {
+        ++launch_counter(), key_kernel<D, K><<<blocks_for(n), kBlock, 0, st>>>(
+            ctx->coords_dev, n, rows_aligned<D>(ctx->coords_dev), p.g, invalid_key, keys, core_bits);
+    });
+    ctx->n_cells = p.cells;
+    ctx->n_items = p.items;
+    // neighbour lists for the border step: min_pts - 1 entries per point
+    const int64_t cap = (int64_t)ctx->min_pts - 1;
+    if (cap >= 1 && cap <= kMaxListCap && (size_t)(p.nv * cap) * sizeof(int32_t) <= ctx->list_budget) {
+        ensure(ctx, ctx->nbr_list, (size_t)(p.nv * cap + 1) * sizeof(int32_t));
+        p.list = ctx->nbr_list.as<int32_t>();
+        p.list_cap = p.list_stride = (int)cap;
+    }
+    ctx->list_cap = p.list_cap;
+    cudaEventRecord(ctx->ev[1], st);
+    count_phase<D, K>(ctx, p, ctx->tc_count, ctx->gram_count, ctx->flags_run);
+    cudaEventRecord(ctx->ev[2], st);
+}
+
+// The context's current job as a pipeline, for the phases after the grid.
+Pipe ctx_pipe(ndb_ctx *ctx) {
+    Pipe p;
+    p.n = ctx->n;
+    p.nv = ctx->nv;
+    p.g = ctx->grid;
+    p.stencil = &ctx->stencil;
+    p.linked = ctx->cell_units != 0;
+    p.early = (ctx->flags_run & NDB_FLAG_FULL_COUNT) == 0;
+    p.e2 = ctx->e2;
+    p.min_pts = ctx->min_pts;
+    p.list = ctx->list_cap ? ctx->nbr_list.as<int32_t>() : nullptr;
+    p.list_cap = p.list_stride = ctx->list_cap;
+    p.cells = ctx->n_cells;
+    p.items = ctx->n_items;
+    return p;
 }
 
 template <int D>
 void classify_dispatch(ndb_ctx *ctx, const Plan &pl) {
-    if (pl.key_bits <= 32) {
-        ctx->key64 = false;
-        classify_grid<D, uint32_t>(ctx, pl);
-    } else {
-        ctx->key64 = true;
-        classify_grid<D, uint64_t>(ctx, pl);
-    }
-    cudaEventRecord(ctx->ev[1], ctx->stream);
-    count_phase<D>(ctx);
-    core_flags_phase(ctx);
-    cudaEventRecord(ctx->ev[2], ctx->stream);
+    Pipe p = ctx_pipe(ctx);
+    p.key_bits = pl.key_bits;
+    p.columns = grid_columns(pl.g);
+    p.list = nullptr;
+    p.list_cap = p.list_stride = 0;
+    ctx->key64 = pl.key_bits > 32;
+    if (ctx->key64) classify_keys<D, uint64_t>(ctx, p);
+    else classify_keys<D, uint32_t>(ctx, p);
 }
 
 // ---------------------------------------------------------------------------
 // phase 2
 // ---------------------------------------------------------------------------
-// Point units: the unions beyond the neighbour lists.  comp_min holds the roots'
-// snapshot meanwhile, cell_cid the cells' roots, flags and pos the segment list (free
-// once the cells are built; n entries, at least one per item).
-template <int D>
-void union_points_phase(ndb_ctx *ctx, int64_t nv, int64_t n_cells, int64_t n_items, int n_rows, float e2,
-                        const JobDev *jobs, const int32_t *cell_job) {
+// Union-find, component minima and core ids of a pipeline.  ci_sorted holds the roots'
+// snapshot until the ids are written, cell_cid (point units) the cells' roots.
+template <int D, typename K>
+void union_phase(ndb_ctx *ctx, const Pipe &p, unsigned long long *job_counters) {
     cudaStream_t st = ctx->stream;
-    int *err = small_at<int>(ctx, kSmallErrOff);
+    const int64_t n = p.n, nv = p.nv, units = p.linked ? p.cells : nv;
+    const uint32_t *n_cells = small_at<uint32_t>(ctx, kSmallScalarOff), *n_items = n_cells + 1;
     uint32_t *n_seg = small_at<uint32_t>(ctx, kSmallScalarOff) + 6;
-    fill_bytes(ctx, ctx->cell_cid.ptr, 0xff, (size_t)n_cells * sizeof(int32_t), st);  // -1
-    fill_bytes(ctx, n_seg, 0, sizeof(uint32_t), st);
-    ++launch_counter(), flatten_points_kernel<<<blocks_for(nv), kBlock, 0, st>>>(
-        ctx->parent.as<int32_t>(), nv, err, ctx->pcell.as<int32_t>(), ctx->core_sorted.as<uint8_t>(),
-        ctx->comp_min.as<int32_t>(), ctx->cell_cid.as<int32_t>());
-    cudaEventRecord(ctx->kev[4], st);
-    const uint32_t seg_cap = (uint32_t)(std::min(ctx->flags.bytes, ctx->pos.bytes) / sizeof(uint32_t));
-    uint32_t *seg_item = ctx->flags.as<uint32_t>(), *seg_part = ctx->pos.as<uint32_t>();
-    ++launch_counter(), union_select_kernel<<<blocks_for(n_items * kWarp), kBlock, 0, st>>>(
-        ctx->items.as<int2>(), n_items, ctx->cell_start.as<int32_t>(), ctx->nbr.as<int2>(), n_rows,
-        ctx->cell_cid.as<int32_t>(), ctx->comp_min.as<int32_t>(), seg_item, seg_part,
-        seg_cap, n_seg);
-    ++launch_counter(), union_scan_kernel<D><<<(unsigned)ctx->sm_count * 16, kCountWarps * kWarp, 0, st>>>(
-        ctx->items.as<int2>(), n_items, ctx->cell_start.as<int32_t>(), ctx->nbr.as<int2>(), n_rows,
-        ctx->xs.as<float>(), e2, ctx->cell_cid.as<int32_t>(), ctx->comp_min.as<int32_t>(), ctx->parent.as<int32_t>(),
-        seg_item, seg_part, seg_cap, n_seg, small_at<unsigned long long>(ctx, kSmallCountersOff) + 3, err, jobs, cell_job);
-    ++launch_counter(), fill_kernel<<<blocks_for(nv), kBlock, 0, st>>>(ctx->comp_min.as<int32_t>(), nv, kNoCluster);
+    unsigned long long *counters = small_at<unsigned long long>(ctx, kSmallCountersOff);
+    int *err = small_at<int>(ctx, kSmallErrOff);
+    ensure(ctx, ctx->parent, (units + 1) * sizeof(int32_t));
+    ensure(ctx, ctx->comp_min, (units + 1) * sizeof(int32_t));
+    ensure(ctx, ctx->ci_sorted, (n + 1) * sizeof(int32_t));
+    ensure(ctx, ctx->cell_cid, (p.cells + 1) * sizeof(int32_t));
+    int32_t *parent = ctx->parent.as<int32_t>(), *comp_min = ctx->comp_min.as<int32_t>();
+    int32_t *ci_sorted = ctx->ci_sorted.as<int32_t>(), *cell_cid = ctx->cell_cid.as<int32_t>();
+    const int32_t *cell_start = ctx->cell_start.as<int32_t>(), *pcell = ctx->pcell.as<int32_t>();
+    const int32_t *perm = ctx->ids0.as<int32_t>();
+    const uint8_t *core_sorted = ctx->core_sorted.as<uint8_t>(), *has_core = ctx->cell_has_core.as<uint8_t>();
+    const uint32_t *core_bits = ctx->core_bits.as<uint32_t>(), *core_prefix = ctx->core_prefix.as<uint32_t>();
+    const float *xs = ctx->xs.as<float>();
+    const int2 *nbr = ctx->nbr.as<int2>(), *items = ctx->items.as<int2>();
+    const int n_rows = p.stencil->n_rows;
+
+    ++launch_counter(), init_units_kernel<<<blocks_for(units), kBlock, 0, st>>>(
+        parent, comp_min, units, n_cells, p.linked ? nullptr : cell_cid, n_seg);
+    if (p.list_stride > 0)
+        ++launch_counter(), union_lists_kernel<<<blocks_for(nv), kBlock, 0, st>>>(
+            nv, ctx->nn_sorted.as<int32_t>(), p.list, p.list_cap, p.list_stride, core_sorted, parent, err, p.jobs,
+            p.cell_job, pcell, p.linked, p.linked && p.early, cell_start, p.min_pts);
+    if (p.linked) {
+        ++launch_counter(), union_near_kernel<D, K><<<blocks_for(p.cells), kBlock, 0, st>>>(
+            n_cells, p.g, ctx->cell_key.as<K>(), cell_start, cell_index<K>(ctx), xs, p.e2, core_sorted, has_core,
+            parent, counters + 3, err, p.jobs, p.cell_job);
+        ++launch_counter(), flatten_snap_kernel<<<blocks_for(p.cells), kBlock, 0, st>>>(parent, n_cells, err, has_core,
+                                                                                       ci_sorted);
+        cudaEventRecord(ctx->kev[4], st);
+        ++launch_counter(), union_cells_kernel<D><<<blocks_for(p.cells * kWarp), kBlock, 0, st>>>(
+            n_cells, cell_start, nbr, n_rows, xs, p.e2, core_sorted, has_core, parent, counters + 3, err, p.jobs,
+            p.cell_job, ci_sorted);
+        cudaEventRecord(ctx->kev[5], st);
+        ++launch_counter(), flatten_min_cells_kernel<<<blocks_for(p.cells), kBlock, 0, st>>>(
+            parent, n_cells, err, cell_start, has_core, core_sorted, perm, core_bits, core_prefix, comp_min);
+    } else {
+        // the segment list: n entries, at least one per item
+        ensure(ctx, ctx->flags, (n + 1) * sizeof(uint32_t));
+        ensure(ctx, ctx->pos, (n + 1) * sizeof(uint32_t));
+        const uint32_t seg_cap = (uint32_t)n;
+        uint32_t *seg_item = ctx->flags.as<uint32_t>(), *seg_part = ctx->pos.as<uint32_t>();
+        ++launch_counter(), flatten_points_kernel<<<blocks_for(nv), kBlock, 0, st>>>(parent, nv, err, pcell, core_sorted,
+                                                                                    ci_sorted, cell_cid);
+        cudaEventRecord(ctx->kev[4], st);
+        ++launch_counter(), union_select_kernel<<<blocks_for(p.items * kWarp), kBlock, 0, st>>>(
+            items, n_items, cell_start, nbr, n_rows, cell_cid, ci_sorted, seg_item, seg_part, seg_cap, n_seg);
+        const unsigned scan_blocks = (unsigned)std::min<int64_t>(p.items / kCountWarps + 1, (int64_t)ctx->sm_count * 16);
+        ++launch_counter(), union_scan_kernel<D><<<scan_blocks, kCountWarps * kWarp, 0, st>>>(
+            items, n_items, cell_start, nbr, n_rows, xs, p.e2, cell_cid, ci_sorted, parent, seg_item, seg_part, seg_cap,
+            n_seg, counters + 3, err, p.jobs, p.cell_job);
+        cudaEventRecord(ctx->kev[5], st);
+        ++launch_counter(), flatten_min_points_kernel<<<blocks_for(nv), kBlock, 0, st>>>(
+            parent, nv, err, core_sorted, perm, core_bits, core_prefix, comp_min);
+    }
+    ++launch_counter(), ids_kernel<<<blocks_for(std::max(nv, p.cells)), kBlock, 0, st>>>(
+        nv, n_cells, core_sorted, pcell, has_core, p.linked, parent, comp_min, ci_sorted, cell_cid, counters,
+        p.cell_job, job_counters);
     ck(ctx, cudaGetLastError());
 }
 
@@ -854,96 +952,27 @@ void border_phase(ndb_ctx *ctx) {
     } else if (ctx->n_items > 0) {
         const unsigned grid = (unsigned)((ctx->n_items + kWarpsPerBlock - 1) / kWarpsPerBlock);
         ++launch_counter(), border_kernel<D><<<grid, kBlock, 0, st>>>(
-            ctx->items.as<int2>(), ctx->n_items, ctx->cell_start.as<int32_t>(), ctx->nbr.as<int2>(), ctx->n_rows,
-            ctx->xs.as<float>(), ctx->e2, ctx->core_sorted.as<uint8_t>(), ctx->cell_has_core.as<uint8_t>(),
-            ctx->cell_units, ctx->cell_cid.as<int32_t>(), ctx->ci_sorted.as<int32_t>(), counters + 4);
+            ctx->items.as<int2>(), small_at<uint32_t>(ctx, kSmallScalarOff) + 1, ctx->cell_start.as<int32_t>(),
+            ctx->nbr.as<int2>(), ctx->n_rows, ctx->xs.as<float>(), ctx->e2, ctx->core_sorted.as<uint8_t>(),
+            ctx->cell_has_core.as<uint8_t>(), ctx->cell_units, ctx->cell_cid.as<int32_t>(),
+            ctx->ci_sorted.as<int32_t>(), counters + 4);
         ck(ctx, cudaGetLastError());
     }
 }
 
+// Input-order outputs below this size are written by one pass (finish_kernel).
+inline bool one_window(int64_t n) { return n <= kScatterWindow; }
+
 template <int D>
 void labels_phase(ndb_ctx *ctx) {
     cudaStream_t st = ctx->stream;
-    const int64_t n = ctx->n, nv = ctx->nv, n_cells = ctx->n_cells;
+    const int64_t n = ctx->n, nv = ctx->nv;
     unsigned long long *counters = small_at<unsigned long long>(ctx, kSmallCountersOff);
-    int *err = small_at<int>(ctx, kSmallErrOff);
-    uint32_t *scal = small_at<uint32_t>(ctx, kSmallScalarOff);
-
-    const int64_t n_units = ctx->cell_units ? n_cells : nv;
-    ensure(ctx, ctx->parent, (n_units + 1) * sizeof(int32_t));
-    ensure(ctx, ctx->comp_min, (n_units + 1) * sizeof(int32_t));
-    ensure(ctx, ctx->ci_sorted, (n + 1) * sizeof(int32_t));
-    ensure(ctx, ctx->cell_cid, (n_cells + 1) * sizeof(int32_t));
-    ++launch_counter(), iota_kernel<<<blocks_for(n_units), kBlock, 0, st>>>(ctx->parent.as<int32_t>(), n_units);
-    ++launch_counter(), fill_kernel<<<blocks_for(n_units), kBlock, 0, st>>>(ctx->comp_min.as<int32_t>(), n_units, kNoCluster);
-    ck(ctx, cudaGetLastError());
-
-    cudaEventRecord(ctx->kev[4], st);  // moved to the main union kernel below when there is one
-    if (ctx->n_items > 0) {
-        if (ctx->cell_units) {
-            if (ctx->list_cap > 0)
-                ++launch_counter(), union_lists_kernel<<<blocks_for(nv), kBlock, 0, st>>>(
-                    nv, ctx->nn_sorted.as<int32_t>(), ctx->nbr_list.as<int32_t>(), ctx->list_cap, ctx->list_cap,
-                    ctx->core_sorted.as<uint8_t>(), ctx->parent.as<int32_t>(), err, nullptr, nullptr,
-                    ctx->pcell.as<int32_t>(), 1, (ctx->flags_run & NDB_FLAG_FULL_COUNT) == 0,
-                    ctx->cell_start.as<int32_t>(), ctx->min_pts);
-            if (ctx->key64)
-                ++launch_counter(), union_near_kernel<D, uint64_t><<<blocks_for(n_cells), kBlock, 0, st>>>(
-                    n_cells, ctx->grid, ctx->cell_key.as<uint64_t>(), ctx->cell_start.as<int32_t>(),
-                    cell_index<uint64_t>(ctx), ctx->xs.as<float>(),
-                    ctx->e2, ctx->core_sorted.as<uint8_t>(), ctx->cell_has_core.as<uint8_t>(),
-                    ctx->parent.as<int32_t>(), counters + 3, err, nullptr, nullptr);
-            else
-                ++launch_counter(), union_near_kernel<D, uint32_t><<<blocks_for(n_cells), kBlock, 0, st>>>(
-                    n_cells, ctx->grid, ctx->cell_key.as<uint32_t>(), ctx->cell_start.as<int32_t>(),
-                    cell_index<uint32_t>(ctx), ctx->xs.as<float>(),
-                    ctx->e2, ctx->core_sorted.as<uint8_t>(), ctx->cell_has_core.as<uint8_t>(),
-                    ctx->parent.as<int32_t>(), counters + 3, err, nullptr, nullptr);
-            // comp_min holds the cells' root snapshot until the union is done
-            ++launch_counter(), flatten_snap_kernel<<<blocks_for(n_units), kBlock, 0, st>>>(
-                ctx->parent.as<int32_t>(), n_units, err, ctx->cell_has_core.as<uint8_t>(), ctx->comp_min.as<int32_t>());
-            cudaEventRecord(ctx->kev[4], st);
-            ++launch_counter(), union_cells_kernel<D><<<blocks_for(n_cells * kWarp), kBlock, 0, st>>>(
-                n_cells, ctx->cell_start.as<int32_t>(), ctx->nbr.as<int2>(), ctx->n_rows, ctx->xs.as<float>(),
-                ctx->e2, ctx->core_sorted.as<uint8_t>(), ctx->cell_has_core.as<uint8_t>(), ctx->parent.as<int32_t>(),
-                counters + 3, err, nullptr, nullptr, ctx->comp_min.as<int32_t>());
-            ++launch_counter(), fill_kernel<<<blocks_for(n_units), kBlock, 0, st>>>(ctx->comp_min.as<int32_t>(), n_units,
-                                                                                   kNoCluster);
-        }
-        else {
-            if (ctx->list_cap > 0)
-                ++launch_counter(), union_lists_kernel<<<blocks_for(nv), kBlock, 0, st>>>(
-                    nv, ctx->nn_sorted.as<int32_t>(), ctx->nbr_list.as<int32_t>(), ctx->list_cap, ctx->list_cap,
-                    ctx->core_sorted.as<uint8_t>(), ctx->parent.as<int32_t>(), err, nullptr, nullptr,
-                    ctx->pcell.as<int32_t>(), 0, 0, ctx->cell_start.as<int32_t>(), ctx->min_pts);
-            union_points_phase<D>(ctx, nv, n_cells, ctx->n_items, ctx->n_rows, ctx->e2, nullptr, nullptr);
-        }
-        ck(ctx, cudaGetLastError());
-    }
-    cudaEventRecord(ctx->kev[5], st);
-    ++launch_counter(), flatten_kernel<<<blocks_for(n_units), kBlock, 0, st>>>(ctx->parent.as<int32_t>(), n_units, err);
-    if (ctx->cell_units)
-        ++launch_counter(), comp_min_cells_kernel<<<blocks_for(n_cells), kBlock, 0, st>>>(
-            n_cells, ctx->cell_start.as<int32_t>(), ctx->cell_has_core.as<uint8_t>(), ctx->core_sorted.as<uint8_t>(),
-            ctx->ids0.as<int32_t>(), ctx->core_bits.as<uint32_t>(), ctx->core_prefix.as<uint32_t>(),
-            ctx->parent.as<int32_t>(), ctx->comp_min.as<int32_t>());
-    else
-        ++launch_counter(), comp_min_kernel<<<blocks_for(nv), kBlock, 0, st>>>(
-            nv, ctx->core_sorted.as<uint8_t>(), ctx->ids0.as<int32_t>(), ctx->pcell.as<int32_t>(), ctx->cell_units,
-            ctx->core_bits.as<uint32_t>(), ctx->core_prefix.as<uint32_t>(), ctx->parent.as<int32_t>(),
-            ctx->comp_min.as<int32_t>());
-    ++launch_counter(), core_ids_kernel<<<blocks_for(nv), kBlock, 0, st>>>(
-        nv, ctx->core_sorted.as<uint8_t>(), ctx->pcell.as<int32_t>(), ctx->cell_units, ctx->parent.as<int32_t>(),
-        ctx->comp_min.as<int32_t>(), ctx->ci_sorted.as<int32_t>(), counters, nullptr, nullptr);
-    if (ctx->cell_units)
-        ++launch_counter(), cell_ids_kernel<<<blocks_for(n_cells), kBlock, 0, st>>>(n_cells, ctx->cell_has_core.as<uint8_t>(),
-                                                                ctx->parent.as<int32_t>(), ctx->comp_min.as<int32_t>(),
-                                                                ctx->cell_cid.as<int32_t>(), counters, nullptr, nullptr);
-    ck(ctx, cudaGetLastError());
+    const Pipe p = ctx_pipe(ctx);
+    if (ctx->key64) union_phase<D, uint64_t>(ctx, p, nullptr);
+    else union_phase<D, uint32_t>(ctx, p, nullptr);
     cudaEventRecord(ctx->ev[3], st);
     cudaEventRecord(ctx->kev[6], st);
-    border_phase<D>(ctx);
-    cudaEventRecord(ctx->kev[7], st);
     // ids in input order, straight into the caller's device buffer when there is one
     int32_t *target = nullptr;
     if (ctx->ci_user && (ctx->flags_run & NDB_FLAG_DEVICE_PTRS)) {
@@ -952,12 +981,26 @@ void labels_phase(ndb_ctx *ctx) {
         ensure(ctx, ctx->ci_orig, (n + 1) * sizeof(int32_t));
         target = ctx->ci_orig.as<int32_t>();
     }
-    const int64_t wci = target ? kScatterWindow : n;  // no output: one pass counts
-    for (int64_t lo = 0; lo < n; lo += wci)
-        ++launch_counter(), output_ci_kernel<<<blocks_for(n), kBlock, 0, st>>>(
-            ctx->ci_sorted.as<int32_t>(), nv, n, ctx->ids0.as<int32_t>(), ctx->core_bits.as<uint32_t>(),
-            ctx->core_prefix.as<uint32_t>(), target, counters, nullptr, 0, nullptr, lo,
-            wci >= n ? INT64_MAX : lo + wci);
+    int32_t *nn_target = ctx->nn_late;  // ndb_b200_run: the counts not yet written
+    ctx->nn_late = nullptr;
+    if (one_window(n)) {
+        const bool lists = p.list_stride > 0;
+        if (!lists) border_phase<D>(ctx);
+        cudaEventRecord(ctx->kev[7], st);
+        ++launch_counter(), finish_kernel<<<blocks_for(n), kBlock, 0, st>>>(
+            nv, n, ctx->nn_sorted.as<int32_t>(), p.list, p.list_stride, lists, ctx->core_sorted.as<uint8_t>(),
+            ctx->cell_units, ctx->pcell.as<int32_t>(), ctx->cell_cid.as<int32_t>(), ctx->ci_sorted.as<int32_t>(),
+            ctx->ids0.as<int32_t>(), ctx->core_bits.as<uint32_t>(), ctx->core_prefix.as<uint32_t>(), nn_target, target,
+            counters, nullptr, 0, nullptr);
+    } else {
+        border_phase<D>(ctx);
+        cudaEventRecord(ctx->kev[7], st);
+        const int64_t wci = target ? kScatterWindow : n;  // no output: one pass counts
+        for (int64_t lo = 0; lo < n; lo += wci)
+            ++launch_counter(), output_ci_kernel<<<blocks_for(n), kBlock, 0, st>>>(
+                ctx->ci_sorted.as<int32_t>(), nv, n, ctx->ids0.as<int32_t>(), ctx->core_bits.as<uint32_t>(),
+                ctx->core_prefix.as<uint32_t>(), target, counters, lo, wci >= n ? INT64_MAX : lo + wci);
+    }
     ck(ctx, cudaGetLastError());
     cudaEventRecord(ctx->ev[4], st);
 }
@@ -988,27 +1031,44 @@ inline void audit_stats(ndb_stats &S, const unsigned long long *a) {
     S.filter_misclassified_pairs = (int64_t)a[3];
 }
 
-// Counters and times of phase 1, once its work on the context's stream is done.
+// The run's counters, scalars and error flag as the host reads them: one copy kernel
+// into the mailbox in stream order (valid once the stream is synchronized).
+struct Tally {
+    unsigned long long counters[kCounters];
+    uint32_t scal[8];
+    int err;
+};
+const char *mail_tally(ndb_ctx *ctx) {
+    constexpr size_t words = (kSmallErrOff + sizeof(int) - kSmallCountersOff) / sizeof(uint32_t);
+    return reinterpret_cast<const char *>(
+        mail_from_device(ctx, small_at<uint32_t>(ctx, kSmallCountersOff), words, ctx->stream));
+}
+Tally read_tally(const char *m) {
+    Tally t;
+    memcpy(t.counters, m, sizeof(t.counters));
+    memcpy(t.scal, m + (kSmallScalarOff - kSmallCountersOff), sizeof(t.scal));
+    memcpy(&t.err, m + (kSmallErrOff - kSmallCountersOff), sizeof(int));
+    return t;
+}
+
+// Counters and times of phase 1 (the label phase leaves counters 2, 5 and 8 to 11 and
+// scalars 0, 1 and 4 as phase 1 wrote them).
 template <int D>
-void classify_stats(ndb_ctx *ctx) {
-    unsigned long long h_counters[kCounters];
-    uint32_t h_tc_items = 0;
-    ck(ctx, cudaMemcpyAsync(h_counters, small_at<unsigned long long>(ctx, kSmallCountersOff), sizeof(h_counters),
-                            cudaMemcpyDeviceToHost, ctx->stream));
-    ck(ctx, cudaMemcpyAsync(&h_tc_items, small_at<uint32_t>(ctx, kSmallScalarOff) + 4, sizeof(uint32_t),
-                            cudaMemcpyDeviceToHost, ctx->stream));
-    ck(ctx, cudaStreamSynchronize(ctx->stream));
-    ctx->stats.tensor_items = ctx->tc_count ? h_tc_items : 0;
-    ctx->stats.count_pairs = (int64_t)h_counters[2];
-    ctx->stats.count_pair_dims = (int64_t)h_counters[2] * D;
-    ctx->stats.count_fp32_ops = (int64_t)h_counters[2] * (ctx->gram_count ? D + 3 : 3 * D);
-    ctx->stats.gram_filter = ctx->gram_count ? 1 : 0;
-    ctx->stats.band_pairs = (int64_t)h_counters[5];
-    audit_stats(ctx->stats, h_counters + 8);
-    ctx->stats.ms_grid = elapsed(ctx->ev[0], ctx->ev[1]);
-    ctx->stats.ms_count = elapsed(ctx->ev[1], ctx->ev[2]);
-    ctx->stats.ms_sort_kernels = elapsed(ctx->kev[0], ctx->kev[1]);
-    ctx->stats.ms_count_kernel = elapsed(ctx->kev[2], ctx->kev[3]);
+void classify_stats(ndb_ctx *ctx, const Tally &t) {
+    ndb_stats &S = ctx->stats;
+    S.n_cells = t.scal[0];
+    S.n_tiles = t.scal[1];
+    S.tensor_items = ctx->tc_count ? t.scal[4] : 0;
+    S.count_pairs = (int64_t)t.counters[2];
+    S.count_pair_dims = (int64_t)t.counters[2] * D;
+    S.count_fp32_ops = (int64_t)t.counters[2] * (ctx->gram_count ? D + 3 : 3 * D);
+    S.gram_filter = ctx->gram_count ? 1 : 0;
+    S.band_pairs = (int64_t)t.counters[5];
+    audit_stats(S, t.counters + 8);
+    S.ms_grid = elapsed(ctx->ev[0], ctx->ev[1]);
+    S.ms_count = elapsed(ctx->ev[1], ctx->ev[2]);
+    S.ms_sort_kernels = elapsed(ctx->kev[0], ctx->kev[1]);
+    S.ms_count_kernel = elapsed(ctx->kev[2], ctx->kev[3]);
 }
 
 template <int D>
@@ -1025,7 +1085,10 @@ ndb_status classify_impl(ndb_ctx *ctx, const float *coords, int64_t n, float eps
     ctx->stats = ndb_stats{};
     ctx->stats_pending = false;
     launch_counter() = 0;
+    ctx->nn_late = nullptr;
     ensure(ctx, ctx->small, kSmallBytes);
+    ensure_mail(ctx, kMailSingle);
+    ctx->mail_used = 0;  // every earlier call has waited for its transfers
     ck(ctx, cudaMemsetAsync(ctx->small.ptr, 0, kSmallBytes, st));
     cudaEventRecord(ctx->ev[0], st);
 
@@ -1055,11 +1118,14 @@ ndb_status classify_impl(ndb_ctx *ctx, const float *coords, int64_t n, float eps
             ctx->coords_dev, n, rows_aligned<D>(ctx->coords_dev), lo_hi, n_invalid);
     }
     ck(ctx, cudaGetLastError());
+    static_assert(kSmallInvalidOff >= kSmallBboxOff + 2 * kMaxDim * sizeof(int), "bounds, then the invalid points");
+    const char *m_box = reinterpret_cast<const char *>(mail_from_device(
+        ctx, small_at<uint32_t>(ctx, kSmallBboxOff), (kSmallInvalidOff + 8 - kSmallBboxOff) / sizeof(uint32_t), st));
+    ck(ctx, cudaStreamSynchronize(st));
     int h_lo_hi[2 * kMaxDim];
     unsigned long long h_invalid = 0;
-    ck(ctx, cudaMemcpyAsync(h_lo_hi, lo_hi, 2 * D * sizeof(int), cudaMemcpyDeviceToHost, st));
-    ck(ctx, cudaMemcpyAsync(&h_invalid, n_invalid, sizeof(h_invalid), cudaMemcpyDeviceToHost, st));
-    ck(ctx, cudaStreamSynchronize(st));
+    memcpy(h_lo_hi, m_box, sizeof(h_lo_hi));
+    memcpy(&h_invalid, m_box + (kSmallInvalidOff - kSmallBboxOff), sizeof(h_invalid));
     ctx->nv = n - (int64_t)h_invalid;
     double lo[kMaxDim], hi[kMaxDim];
     for (int a = 0; a < D; ++a) {
@@ -1083,7 +1149,9 @@ ndb_status classify_impl(ndb_ctx *ctx, const float *coords, int64_t n, float eps
 
     classify_dispatch<D>(ctx, pl);
 
-    if (nn_out) {
+    if (nn_out && ctx->in_run && (flags & NDB_FLAG_DEVICE_PTRS) && one_window(n)) {
+        ctx->nn_late = nn_out;  // written with the ids
+    } else if (nn_out) {
         // counts in input order, straight into the caller's device buffer when there is one
         int32_t *target = nn_out;
         if (!(flags & NDB_FLAG_DEVICE_PTRS)) {
@@ -1092,7 +1160,7 @@ ndb_status classify_impl(ndb_ctx *ctx, const float *coords, int64_t n, float eps
         }
         for (int64_t lo = 0; lo < n; lo += kScatterWindow)
             ++launch_counter(), scatter_nn_kernel<<<blocks_for(n), kBlock, 0, st>>>(
-                ctx->nn_sorted.as<int32_t>(), ctx->nv, n, ctx->ids0.as<int32_t>(), target, nullptr, 0, lo,
+                ctx->nn_sorted.as<int32_t>(), ctx->nv, n, ctx->ids0.as<int32_t>(), target, lo,
                 n <= kScatterWindow ? INT64_MAX : lo + kScatterWindow);
         ck(ctx, cudaGetLastError());
         if (!(flags & NDB_FLAG_DEVICE_PTRS)) {
@@ -1109,8 +1177,6 @@ ndb_status classify_impl(ndb_ctx *ctx, const float *coords, int64_t n, float eps
         }
     }
     ctx->stats.n_valid = ctx->nv;
-    ctx->stats.n_cells = ctx->n_cells;
-    ctx->stats.n_tiles = ctx->n_items;
     ctx->stats.grid_dims = pl.g.k;
     ctx->stats.stencil_rows = pl.st.n_rows;
     ctx->stats.same_cell_linked = ctx->cell_units;
@@ -1124,8 +1190,9 @@ ndb_status classify_impl(ndb_ctx *ctx, const float *coords, int64_t n, float eps
         ctx->stats_pending = true;
         return NDB_OK;
     }
+    const char *m_tally = mail_tally(ctx);
     ck(ctx, cudaStreamSynchronize(st));
-    classify_stats<D>(ctx);
+    classify_stats<D>(ctx, read_tally(m_tally));
     return NDB_OK;
 }
 
@@ -1138,41 +1205,24 @@ ndb_status labels_impl(ndb_ctx *ctx, int32_t *ci_out, ndb_result *result) {
     const int64_t n = ctx->n;
     if (ci_out && !(ctx->flags_run & NDB_FLAG_DEVICE_PTRS))
         ck(ctx, cudaMemcpyAsync(ci_out, ctx->ci_orig.ptr, n * sizeof(int32_t), cudaMemcpyDeviceToHost, st));
-    unsigned long long h_counters[kCounters];
-    uint32_t h_scal[8];
-    int h_err = 0;
-    ck(ctx, cudaMemcpyAsync(h_counters, small_at<unsigned long long>(ctx, kSmallCountersOff), sizeof(h_counters),
-                            cudaMemcpyDeviceToHost, st));
-    ck(ctx, cudaMemcpyAsync(h_scal, small_at<uint32_t>(ctx, kSmallScalarOff), sizeof(h_scal), cudaMemcpyDeviceToHost,
-                            st));
-    ck(ctx, cudaMemcpyAsync(&h_err, small_at<int>(ctx, kSmallErrOff), sizeof(int), cudaMemcpyDeviceToHost, st));
+    ctx->mail_used = 0;  // phase 1's transfers have been read
+    const char *m_tally = mail_tally(ctx);
     ck(ctx, cudaStreamSynchronize(st));
+    const Tally t = read_tally(m_tally);
     if (ctx->stats_pending) {
-        // classify_stats without its own copies: the label phase leaves counters 2 and 5
-        // and scalar 4 as phase 1 wrote them
         ctx->stats_pending = false;
-        ctx->stats.tensor_items = ctx->tc_count ? h_scal[4] : 0;
-        ctx->stats.count_pairs = (int64_t)h_counters[2];
-        ctx->stats.count_pair_dims = (int64_t)h_counters[2] * D;
-        ctx->stats.count_fp32_ops = (int64_t)h_counters[2] * (ctx->gram_count ? D + 3 : 3 * D);
-        ctx->stats.gram_filter = ctx->gram_count ? 1 : 0;
-        ctx->stats.band_pairs = (int64_t)h_counters[5];
-        audit_stats(ctx->stats, h_counters + 8);
-        ctx->stats.ms_grid = elapsed(ctx->ev[0], ctx->ev[1]);
-        ctx->stats.ms_count = elapsed(ctx->ev[1], ctx->ev[2]);
-        ctx->stats.ms_sort_kernels = elapsed(ctx->kev[0], ctx->kev[1]);
-        ctx->stats.ms_count_kernel = elapsed(ctx->kev[2], ctx->kev[3]);
+        classify_stats<D>(ctx, t);
     }
-    if (h_err) return NDB_ERR_DEVICE_LIMIT;
-    ctx->n_cores = h_scal[2];
-    ctx->result.clusters = (int32_t)h_counters[0];
-    ctx->result.noise = (int32_t)h_counters[1];
+    if (t.err) return NDB_ERR_DEVICE_LIMIT;
+    ctx->n_cores = t.scal[2];
+    ctx->result.clusters = (int32_t)t.counters[0];
+    ctx->result.noise = (int32_t)t.counters[1];
     ctx->result.core_count = (int32_t)ctx->n_cores;
     ctx->result.n = (int32_t)n;
-    ctx->stats.union_pairs = (int64_t)h_counters[3];
-    ctx->stats.border_pairs = (int64_t)h_counters[4];
-    ctx->stats.union_pair_dims = (int64_t)h_counters[3] * D;
-    ctx->stats.border_pair_dims = (int64_t)h_counters[4] * D;
+    ctx->stats.union_pairs = (int64_t)t.counters[3];
+    ctx->stats.border_pairs = (int64_t)t.counters[4];
+    ctx->stats.union_pair_dims = (int64_t)t.counters[3] * D;
+    ctx->stats.border_pair_dims = (int64_t)t.counters[4] * D;
     ctx->stats.ms_union = elapsed(ctx->ev[2], ctx->ev[3]);
     ctx->stats.ms_border = elapsed(ctx->ev[3], ctx->ev[4]);
     ctx->stats.ms_union_kernel = elapsed(ctx->kev[4], ctx->kev[5]);
@@ -1668,7 +1718,6 @@ struct BatchPlan {
 template <int D, typename K>
 void run_group_keys(ndb_ctx *ctx, ndb_job *jobs, const std::vector<int> &members, BatchPlan &bp, uint32_t flags) {
     cudaStream_t st = ctx->stream;
-    constexpr int P = Stride<D>::P;
     const int nj = (int)members.size();
     const int64_t n = bp.total_n, nv = bp.nv;
     const JobDev *jobs_dev = ctx->jobs_dev.as<JobDev>();
@@ -1679,194 +1728,46 @@ void run_group_keys(ndb_ctx *ctx, ndb_job *jobs, const std::vector<int> &members
     for (auto &j : bp.jd) max_n = std::max<int64_t>(max_n, j.n);
     const unsigned gx = (unsigned)std::min<int64_t>((max_n + kBlock - 1) / kBlock, 64);
 
+    Pipe p;
+    p.n = n;
+    p.nv = nv;
+    p.key_bits = bp.key_bits;
+    p.g = bp.jd[0].g;
+    p.stencil = &bp.st;
+    p.columns = (double)bp.columns;
+    p.linked = bp.linked != 0;
+    p.early = (flags & NDB_FLAG_FULL_COUNT) == 0;
+    p.jobs = jobs_dev;
+    p.n_jobs = nj;
     cudaEventRecord(ctx->ev[0], st);
-    // composite keys and the sort
-    ensure(ctx, ctx->keys0, n * sizeof(K));
-    ensure(ctx, ctx->keys1, n * sizeof(K));
-    ensure(ctx, ctx->ids0, n * sizeof(int32_t));
-    ensure(ctx, ctx->ids1, n * sizeof(int32_t));
-    ensure(ctx, ctx->sort_hist, sort_scratch_words<K>(n) * sizeof(uint32_t));
-    ensure(ctx, ctx->scan_scratch, (scan_scratch_words(n + 1) + 64) * sizeof(uint32_t));
-    const K invalid_key = (K)(bp.key_bits >= (int)(8 * sizeof(K)) ? ~(K)0 : (((K)1 << bp.key_bits) - 1));
-    ++launch_counter(), key_batch_kernel<D, K><<<dim3(gx, nj), kBlock, 0, st>>>(
-        ctx->coords.as<float>(), jobs_dev, invalid_key, ctx->keys0.as<K>());
-    ck(ctx, cudaGetLastError());
-    bool in_first = true;
-    cudaEventRecord(ctx->kev[0], st);
-    if (sizeof(K) == 4)
-        ck(ctx, radix_sort_pairs_u32(reinterpret_cast<uint32_t *>(ctx->keys0.ptr), ctx->ids0.as<int32_t>(),
-                                     reinterpret_cast<uint32_t *>(ctx->keys1.ptr), ctx->ids1.as<int32_t>(), n,
-                                     bp.key_bits, ctx->sort_hist.as<uint32_t>(), &in_first, st));
-    else
-        ck(ctx, radix_sort_pairs_u64(reinterpret_cast<uint64_t *>(ctx->keys0.ptr), ctx->ids0.as<int32_t>(),
-                                     reinterpret_cast<uint64_t *>(ctx->keys1.ptr), ctx->ids1.as<int32_t>(), n,
-                                     bp.key_bits, ctx->sort_hist.as<uint32_t>(), &in_first, st));
-    cudaEventRecord(ctx->kev[1], st);
-    if (!in_first) {
-        std::swap(ctx->keys0, ctx->keys1);
-        std::swap(ctx->ids0, ctx->ids1);
-    }
-    const K *keys = ctx->keys0.as<K>();
-    const int32_t *perm = ctx->ids0.as<int32_t>();
-
-    // cells
-    ensure(ctx, ctx->flags, (n + 1) * sizeof(uint32_t));
-    ensure(ctx, ctx->pos, (n + 1) * sizeof(uint32_t));
-    ensure(ctx, ctx->pcell, (n + 1) * sizeof(int32_t));
-    ensure(ctx, ctx->cell_start, (n + 2) * sizeof(int32_t));
-    ensure(ctx, ctx->cell_key, (n + 1) * sizeof(K));
-    ++launch_counter(), cell_flag_kernel<K><<<blocks_for(nv), kBlock, 0, st>>>(keys, nv, ctx->flags.as<uint32_t>());
-    ck(ctx, scan_exclusive_u32(ctx->flags.as<uint32_t>(), ctx->pos.as<uint32_t>(), nv, scal + 0,
-                               ctx->scan_scratch.as<uint32_t>(), st));
-    ++launch_counter(), cell_write_kernel<K><<<blocks_for(nv), kBlock, 0, st>>>(
-        keys, nv, ctx->pos.as<uint32_t>(), scal + 0, ctx->cell_start.as<int32_t>(), ctx->cell_key.as<K>(),
-        ctx->pcell.as<int32_t>());
-    ensure(ctx, ctx->xs, (nv + 1) * P * sizeof(float));
-    ++launch_counter(), gather_kernel<D><<<blocks_for(nv), kBlock, 0, st>>>(ctx->coords.as<float>(), perm, nv,
-                                                                           true, ctx->xs.as<float>());
-    ck(ctx, cudaGetLastError());
-    const uint32_t *m_cells = mail_from_device(ctx, scal + 0, 1, st);
-    ck(ctx, cudaStreamSynchronize(st));
-    const int64_t n_cells = nv > 0 ? *m_cells : 0;
-    ensure(ctx, ctx->cell_job, (n_cells + 1) * sizeof(int32_t));
-    ++launch_counter(), cell_job_kernel<K><<<blocks_for(n_cells), kBlock, 0, st>>>(
-        ctx->cell_key.as<K>(), n_cells, jobs_dev, nj, ctx->cell_job.as<int32_t>());
-    const int32_t *cell_job = ctx->cell_job.as<int32_t>();
-
-    // neighbour rows through the column table (or the hash table) of the cells
-    const int n_rows = bp.st.n_rows;
-    const CellIndex<K> L = build_cell_index<K>(ctx, n_cells, (double)bp.columns, bp.jd[0].g, jobs_dev, cell_job);
-    ensure(ctx, ctx->nbr, (size_t)(n_cells * n_rows + 1) * sizeof(int2));
-    int4 *rows_dev = small_at<int4>(ctx, kSmallStencilOff);
-    mail_to_device(ctx, rows_dev, bp.st.rows, (size_t)n_rows, st);
-    const int rlog = row_group_log2(n_rows);
-    ++launch_counter(), rows_kernel<K><<<blocks_for(n_cells << rlog), kBlock, 0, st>>>(
-        ctx->cell_key.as<K>(), n_cells, bp.jd[0].g, rows_dev, n_rows, rlog, L, ctx->nbr.as<int2>(), jobs_dev,
-        cell_job);
-    ck(ctx, cudaGetLastError());
-
-    // work items
-    ensure(ctx, ctx->item_cnt, (n_cells + 1) * sizeof(uint32_t));
-    ++launch_counter(), item_count_kernel<<<blocks_for(n_cells), kBlock, 0, st>>>(
-        ctx->cell_start.as<int32_t>(), n_cells, ctx->item_cnt.as<uint32_t>());
-    ck(ctx, scan_exclusive_u32(ctx->item_cnt.as<uint32_t>(), ctx->item_cnt.as<uint32_t>(), n_cells, scal + 1,
-                               ctx->scan_scratch.as<uint32_t>(), st));
-    const uint32_t *m_items = mail_from_device(ctx, scal + 1, 1, st);
-    ck(ctx, cudaStreamSynchronize(st));
-    const int64_t n_items = n_cells > 0 ? *m_items : 0;
-    ensure(ctx, ctx->items, (n_items + 1) * sizeof(int2));
-    ++launch_counter(), item_write_kernel<<<blocks_for(n_cells), kBlock, 0, st>>>(
-        ctx->cell_start.as<int32_t>(), n_cells, ctx->item_cnt.as<uint32_t>(), ctx->items.as<int2>());
-
-    // neighbour counts and core flags
-    ensure(ctx, ctx->nn_sorted, (n + 1) * sizeof(int32_t));
-    int32_t *list = nullptr;
+    grid_phase<D, K>(ctx, p, ctx->coords.as<float>(), [&](K invalid_key, K *keys, uint32_t *core_bits) {
+        ++launch_counter(), key_batch_kernel<D, K><<<dim3(gx, nj), kBlock, 0, st>>>(
+            ctx->coords.as<float>(), jobs_dev, invalid_key, keys, core_bits);
+    });
     if (bp.list_stride > 0) {
         ensure(ctx, ctx->nbr_list, (size_t)(nv * bp.list_stride + 1) * sizeof(int32_t));
-        list = ctx->nbr_list.as<int32_t>();
+        p.list = ctx->nbr_list.as<int32_t>();
+        p.list_stride = bp.list_stride;
     }
-    const bool early = (flags & NDB_FLAG_FULL_COUNT) == 0;
     cudaEventRecord(ctx->ev[1], st);
-    cudaEventRecord(ctx->kev[2], st);
-    count_items<D>(ctx, bp.tc, (flags & NDB_FLAG_TENSOR_FILTER) != 0, bp.gram, early, n_items,
-                   ctx->items.as<int2>(),
-                   ctx->cell_start.as<int32_t>(), ctx->nbr.as<int2>(), n_rows, ctx->xs.as<float>(), 0.0f, 0, 0,
-                   ctx->nn_sorted.as<int32_t>(), list, 0, bp.list_stride, jobs_dev, cell_job,
-                   (flags & NDB_FLAG_FILTER_AUDIT) != 0, nv, n_cells);
-    cudaEventRecord(ctx->kev[3], st);
-    const int64_t n_words = (n + 31) / 32;
-    ensure(ctx, ctx->core_sorted, n + 1);
-    ensure(ctx, ctx->cell_has_core, n_cells + 1);
-    ensure(ctx, ctx->core_bits, (n_words + 1) * sizeof(uint32_t));
-    ensure(ctx, ctx->core_prefix, (n_words + 1) * sizeof(uint32_t));
-    fill_bytes(ctx, ctx->cell_has_core.ptr, 0, (size_t)n_cells + 1, st);
-    fill_bytes(ctx, ctx->core_bits.ptr, 0, (size_t)(n_words + 1) * sizeof(uint32_t), st);
-    ++launch_counter(), core_flags_kernel<<<blocks_for(n), kBlock, 0, st>>>(
-        ctx->nn_sorted.as<int32_t>(), nv, n, 0, perm, ctx->pcell.as<int32_t>(), ctx->core_sorted.as<uint8_t>(),
-        ctx->cell_has_core.as<uint8_t>(), ctx->core_bits.as<uint32_t>(), jobs_dev, cell_job, nj);
-    ++launch_counter(), popc_words_kernel<<<blocks_for(n_words), kBlock, 0, st>>>(
-        ctx->core_bits.as<uint32_t>(), n_words, ctx->core_prefix.as<uint32_t>());
-    ck(ctx, cudaGetLastError());
-    ck(ctx, scan_exclusive_u32(ctx->core_prefix.as<uint32_t>(), ctx->core_prefix.as<uint32_t>(), n_words, scal + 2,
-                               ctx->scan_scratch.as<uint32_t>(), st));
+    count_phase<D, K>(ctx, p, bp.tc, bp.gram, flags);
     cudaEventRecord(ctx->ev[2], st);
 
     // union-find, canonical ids, border points
-    const int64_t n_units = bp.linked ? n_cells : nv;
-    ensure(ctx, ctx->parent, (n_units + 1) * sizeof(int32_t));
-    ensure(ctx, ctx->comp_min, (n_units + 1) * sizeof(int32_t));
-    ensure(ctx, ctx->ci_sorted, (n + 1) * sizeof(int32_t));
-    ensure(ctx, ctx->cell_cid, (n_cells + 1) * sizeof(int32_t));
     ensure(ctx, ctx->job_counters, (size_t)(4 * nj + 4) * sizeof(unsigned long long));
     unsigned long long *jc = ctx->job_counters.as<unsigned long long>();
     fill_bytes(ctx, jc, 0, (size_t)(4 * nj + 4) * sizeof(unsigned long long), st);
-    ++launch_counter(), iota_kernel<<<blocks_for(n_units), kBlock, 0, st>>>(ctx->parent.as<int32_t>(), n_units);
-    ++launch_counter(), fill_kernel<<<blocks_for(n_units), kBlock, 0, st>>>(ctx->comp_min.as<int32_t>(), n_units,
-                                                                           kNoCluster);
-    cudaEventRecord(ctx->kev[4], st);
-    if (n_items > 0) {
-        if (bp.linked) {
-            if (bp.list_stride > 0)
-                ++launch_counter(), union_lists_kernel<<<blocks_for(nv), kBlock, 0, st>>>(
-                    nv, ctx->nn_sorted.as<int32_t>(), list, 0, bp.list_stride, ctx->core_sorted.as<uint8_t>(),
-                    ctx->parent.as<int32_t>(), err, jobs_dev, cell_job, ctx->pcell.as<int32_t>(), 1,
-                    (flags & NDB_FLAG_FULL_COUNT) == 0, ctx->cell_start.as<int32_t>(), 0);
-            ++launch_counter(), union_near_kernel<D, K><<<blocks_for(n_cells), kBlock, 0, st>>>(
-                n_cells, bp.jd[0].g, ctx->cell_key.as<K>(), ctx->cell_start.as<int32_t>(), L,
-                ctx->xs.as<float>(), 0.0f, ctx->core_sorted.as<uint8_t>(),
-                ctx->cell_has_core.as<uint8_t>(), ctx->parent.as<int32_t>(), counters + 3, err, jobs_dev, cell_job);
-            ++launch_counter(), flatten_snap_kernel<<<blocks_for(n_units), kBlock, 0, st>>>(
-                ctx->parent.as<int32_t>(), n_units, err, ctx->cell_has_core.as<uint8_t>(), ctx->comp_min.as<int32_t>());
-            ++launch_counter(), union_cells_kernel<D><<<blocks_for(n_cells * kWarp), kBlock, 0, st>>>(
-                n_cells, ctx->cell_start.as<int32_t>(), ctx->nbr.as<int2>(), n_rows, ctx->xs.as<float>(), 0.0f,
-                ctx->core_sorted.as<uint8_t>(), ctx->cell_has_core.as<uint8_t>(), ctx->parent.as<int32_t>(),
-                counters + 3, err, jobs_dev, cell_job, ctx->comp_min.as<int32_t>());
-            ++launch_counter(), fill_kernel<<<blocks_for(n_units), kBlock, 0, st>>>(ctx->comp_min.as<int32_t>(), n_units,
-                                                                                   kNoCluster);
-        } else {
-            if (bp.list_stride > 0)
-                ++launch_counter(), union_lists_kernel<<<blocks_for(nv), kBlock, 0, st>>>(
-                    nv, ctx->nn_sorted.as<int32_t>(), list, 0, bp.list_stride, ctx->core_sorted.as<uint8_t>(),
-                    ctx->parent.as<int32_t>(), err, jobs_dev, cell_job, ctx->pcell.as<int32_t>(), 0, 0,
-                    ctx->cell_start.as<int32_t>(), 0);
-            union_points_phase<D>(ctx, nv, n_cells, n_items, n_rows, 0.0f, jobs_dev, cell_job);
-        }
-        ck(ctx, cudaGetLastError());
-    }
-    cudaEventRecord(ctx->kev[5], st);
-    ++launch_counter(), flatten_kernel<<<blocks_for(n_units), kBlock, 0, st>>>(ctx->parent.as<int32_t>(), n_units, err);
-    if (bp.linked)
-        ++launch_counter(), comp_min_cells_kernel<<<blocks_for(n_cells), kBlock, 0, st>>>(
-            n_cells, ctx->cell_start.as<int32_t>(), ctx->cell_has_core.as<uint8_t>(), ctx->core_sorted.as<uint8_t>(),
-            perm, ctx->core_bits.as<uint32_t>(), ctx->core_prefix.as<uint32_t>(), ctx->parent.as<int32_t>(),
-            ctx->comp_min.as<int32_t>());
-    else
-        ++launch_counter(), comp_min_kernel<<<blocks_for(nv), kBlock, 0, st>>>(
-            nv, ctx->core_sorted.as<uint8_t>(), perm, ctx->pcell.as<int32_t>(), bp.linked,
-            ctx->core_bits.as<uint32_t>(), ctx->core_prefix.as<uint32_t>(), ctx->parent.as<int32_t>(),
-            ctx->comp_min.as<int32_t>());
-    ++launch_counter(), core_ids_kernel<<<blocks_for(nv), kBlock, 0, st>>>(
-        nv, ctx->core_sorted.as<uint8_t>(), ctx->pcell.as<int32_t>(), bp.linked, ctx->parent.as<int32_t>(),
-        ctx->comp_min.as<int32_t>(), ctx->ci_sorted.as<int32_t>(), counters, cell_job, jc);
-    if (bp.linked)
-        ++launch_counter(), cell_ids_kernel<<<blocks_for(n_cells), kBlock, 0, st>>>(
-            n_cells, ctx->cell_has_core.as<uint8_t>(), ctx->parent.as<int32_t>(), ctx->comp_min.as<int32_t>(),
-            ctx->cell_cid.as<int32_t>(), counters, cell_job, jc);
+    union_phase<D, K>(ctx, p, jc);
     cudaEventRecord(ctx->ev[3], st);
-    cudaEventRecord(ctx->kev[6], st);
-    if (bp.list_stride > 0)
-        ++launch_counter(), border_list_kernel<<<blocks_for(nv), kBlock, 0, st>>>(
-            nv, ctx->nn_sorted.as<int32_t>(), list, bp.list_stride, ctx->core_sorted.as<uint8_t>(), bp.linked,
-            ctx->pcell.as<int32_t>(), ctx->cell_cid.as<int32_t>(), ctx->ci_sorted.as<int32_t>(), counters + 4);
-    ck(ctx, cudaGetLastError());
-    cudaEventRecord(ctx->kev[7], st);
 
-    // outputs straight into each job's buffers, per-job meta
-    ++launch_counter(), scatter_nn_kernel<<<blocks_for(n), kBlock, 0, st>>>(ctx->nn_sorted.as<int32_t>(), nv, n, perm,
-                                                                           nullptr, jobs_dev, nj);
-    ++launch_counter(), output_ci_kernel<<<blocks_for(n), kBlock, 0, st>>>(
-        ctx->ci_sorted.as<int32_t>(), nv, n, perm, ctx->core_bits.as<uint32_t>(), ctx->core_prefix.as<uint32_t>(),
-        nullptr, counters, jobs_dev, nj, jc);
+    // border ids and outputs straight into each job's buffers, per-job meta
+    cudaEventRecord(ctx->kev[6], st);
+    ++launch_counter(), finish_kernel<<<blocks_for(n), kBlock, 0, st>>>(
+        nv, n, ctx->nn_sorted.as<int32_t>(), p.list, p.list_stride, p.list_stride > 0, ctx->core_sorted.as<uint8_t>(),
+        bp.linked, ctx->pcell.as<int32_t>(), ctx->cell_cid.as<int32_t>(), ctx->ci_sorted.as<int32_t>(),
+        ctx->ids0.as<int32_t>(), ctx->core_bits.as<uint32_t>(), ctx->core_prefix.as<uint32_t>(), nullptr, nullptr,
+        counters, jobs_dev, nj, jc);
+    cudaEventRecord(ctx->kev[7], st);
     ++launch_counter(), job_cores_kernel<<<blocks_for(nj), kBlock, 0, st>>>(
         jobs_dev, nj, ctx->core_bits.as<uint32_t>(), ctx->core_prefix.as<uint32_t>(), n, jc);
     ck(ctx, cudaGetLastError());
@@ -1876,7 +1777,7 @@ void run_group_keys(ndb_ctx *ctx, ndb_job *jobs, const std::vector<int> &members
     const unsigned long long *m_pairs = mail_from_device(ctx, counters + 2, 4, st);
     const unsigned long long *m_audit = mail_from_device(ctx, counters + 8, 4, st);
     const unsigned long long *m_jc = mail_from_device(ctx, jc, (size_t)4 * nj, st);
-    const uint32_t *m_tc = mail_from_device(ctx, scal + 4, 1, st);
+    const uint32_t *m_scal = mail_from_device(ctx, scal, 8, st);
     const int *m_err = mail_from_device(ctx, err, 1, st);
     if (!(flags & NDB_FLAG_DEVICE_PTRS)) {
         for (int m = 0; m < nj; ++m) {
@@ -1895,7 +1796,8 @@ void run_group_keys(ndb_ctx *ctx, ndb_job *jobs, const std::vector<int> &members
     memcpy(h_pairs, m_pairs, sizeof(h_pairs));
     memcpy(h_audit, m_audit, sizeof(h_audit));
     const std::vector<unsigned long long> h_jc(m_jc, m_jc + (size_t)4 * nj);
-    const uint32_t h_tc_items = bp.tc ? *m_tc : 0;
+    const uint32_t h_tc_items = bp.tc ? m_scal[4] : 0;
+    const int n_rows = bp.st.n_rows;
     const int h_err = *m_err;
     // statistics summed over the pipelines of one batched call
     ndb_stats &S = ctx->stats;
@@ -1916,8 +1818,8 @@ void run_group_keys(ndb_ctx *ctx, ndb_job *jobs, const std::vector<int> &members
     S.union_pair_dims += du * D;
     S.border_pair_dims += db * D;
     S.n_valid += nv;
-    S.n_cells += n_cells;
-    S.n_tiles += n_items;
+    S.n_cells += m_scal[0];
+    S.n_tiles += m_scal[1];
     S.grid_dims = std::max(S.grid_dims, bp.jd[0].g.k);
     S.stencil_rows = std::max(S.stencil_rows, n_rows);
     S.same_cell_linked |= bp.linked;
@@ -2480,8 +2382,8 @@ constexpr size_t kNaN = NDB_NOALLOC_MAX_POINTS;
 enum NaBuf {
     NA_KEYS0, NA_KEYS1, NA_IDS0, NA_IDS1, NA_FLAGS, NA_POS, NA_PCELL, NA_XS, NA_NN_SORTED, NA_NN_ORIG,
     NA_CORE_SORTED, NA_CORE_BITS, NA_CORE_PREFIX, NA_CI_SORTED, NA_CI_ORIG, NA_LABELS, NA_CELL_START, NA_CELL_KEY,
-    NA_NBR, NA_ITEM_CNT, NA_ITEMS, NA_CELL_HAS_CORE, NA_CELL_CID, NA_PARENT, NA_COMP_MIN, NA_SORT_HIST,
-    NA_SCAN, NA_SMALL, NA_HASH_KEYS, NA_HASH_VALS, NA_NBR_LIST, NA_ITEMS_SPLIT, NA_COUNT
+    NA_NBR, NA_ITEMS, NA_CELL_HAS_CORE, NA_CELL_CID, NA_PARENT, NA_COMP_MIN, NA_SORT_HIST,
+    NA_SMALL, NA_HASH_KEYS, NA_HASH_VALS, NA_NBR_LIST, NA_ITEMS_SPLIT, NA_COUNT
 };
 
 constexpr size_t na_cap(int b) {
@@ -2492,8 +2394,7 @@ constexpr size_t na_cap(int b) {
          : b == NA_CELL_KEY || b == NA_ITEMS ? 8 * (kNaN + 1)
          : b == NA_NBR ? 8 * kWarp * kNaN + 8  // classify refuses stencils of more than kWarp rows
          : b == NA_CORE_SORTED || b == NA_CELL_HAS_CORE ? kNaN + 1
-         : b == NA_SORT_HIST ? 4 * sort_scratch_words<uint64_t>(kNaN)
-         : b == NA_SCAN ? 4 * 4096
+         : b == NA_SORT_HIST ? 4 * (sort_scratch_words<uint64_t>(kNaN) + chain_words(kNaN) + 4)
          : b == NA_SMALL ? kSmallBytes
          : b == NA_HASH_KEYS ? 8 * 4 * kNaN
          : b == NA_HASH_VALS ? 4 * 4 * kNaN
@@ -2519,9 +2420,9 @@ DevBuf *na_buf(ndb_ctx &c, int b) {
     DevBuf *bufs[NA_COUNT] = {&c.keys0,       &c.keys1,     &c.ids0,      &c.ids1,         &c.flags,
                               &c.pos,         &c.pcell,     &c.xs,        &c.nn_sorted,    &c.nn_orig,
                               &c.core_sorted, &c.core_bits, &c.core_prefix, &c.ci_sorted,  &c.ci_orig,
-                              &c.labels,      &c.cell_start, &c.cell_key, &c.nbr,          &c.item_cnt,
+                              &c.labels,      &c.cell_start, &c.cell_key, &c.nbr,
                               &c.items,       &c.cell_has_core, &c.cell_cid, &c.parent,    &c.comp_min,
-                              &c.sort_hist,   &c.scan_scratch, &c.small,     &c.hash_keys, &c.hash_vals,
+                              &c.sort_hist,   &c.small,     &c.hash_keys, &c.hash_vals,
                               &c.nbr_list,    &c.items_split};
     return bufs[b];
 }

@@ -112,6 +112,118 @@ __device__ __forceinline__ unsigned lanemask_lt() {
 }
 
 // ---------------------------------------------------------------------------
+// Exclusive prefix over a sequence in one kernel.  Op gives value(e) (a small count),
+// early(e) (work that needs no prefix) and emit(e, value, prefix); tiles of 256 x ITEMS
+// elements follow each other through one state word per tile (decoupled look-back): the
+// tile's own sum first, then the sum including all tiles before it, so a separate
+// reduction, a scan of the partial sums and the intermediate arrays fall away.  Tiles
+// are taken in order from a ticket, so a tile's predecessors are running or done.
+// Every poll is bounded: past the limit the block sums the elements before its tile
+// itself, which needs no other block.  n comes from the device when n_dev is given (the
+// grid then covers an upper bound).  state and ticket start zeroed; the total goes to
+// *total and, when given, to *mail (mapped host memory).
+// ---------------------------------------------------------------------------
+constexpr int kChainThreads = 256;
+constexpr uint32_t kChainPolls = 1u << 16;
+
+template <int ITEMS, typename Op>
+__global__ void __launch_bounds__(kChainThreads) chain_scan_kernel(Op op, int64_t n, const uint32_t *__restrict__ n_dev,
+                                                                   unsigned long long *state, uint32_t *ticket,
+                                                                   uint32_t *total, volatile uint32_t *mail) {
+    constexpr int kTileLen = kChainThreads * ITEMS, kWarps = kChainThreads / kWarp;
+    constexpr unsigned long long kReady = 1ull << 63, kWhole = 1ull << 62;
+    __shared__ uint32_t s_w[kWarps];
+    __shared__ uint32_t s_tile, s_before, s_lost;
+    const int t = threadIdx.x, lane = t & 31, warp = t >> 5;
+    if (t == 0) {
+        s_tile = atomicAdd(ticket, 1u);
+        s_lost = 0;
+    }
+    if (n_dev) n = *n_dev;
+    __syncthreads();
+    const int64_t tile = s_tile, tile0 = tile * kTileLen;
+    if (tile > 0 && tile0 >= n) return;  // past the end: nobody waits for this tile
+    const int64_t first = tile0 + warp * (ITEMS * kWarp) + lane;  // this thread's elements: first + 32 j
+    uint32_t v[ITEMS], ex[ITEMS];
+    uint32_t run = 0;
+#pragma unroll
+    for (int j = 0; j < ITEMS; ++j) v[j] = first + j * kWarp < n ? op.value(first + j * kWarp) : 0u;
+#pragma unroll
+    for (int j = 0; j < ITEMS; ++j) {
+        uint32_t x = v[j];
+#pragma unroll
+        for (int o = 1; o < kWarp; o <<= 1) {
+            const uint32_t y = __shfl_up_sync(kFull, x, o);
+            if (lane >= o) x += y;
+        }
+        ex[j] = run + x - v[j];
+        run += __shfl_sync(kFull, x, kWarp - 1);
+    }
+    if (lane == 0) s_w[warp] = run;
+    __syncthreads();
+    uint32_t before_warp = 0, sum = 0;
+#pragma unroll
+    for (int w = 0; w < kWarps; ++w) {
+        if (w < warp) before_warp += s_w[w];
+        sum += s_w[w];
+    }
+    volatile unsigned long long *st = state;
+    if (t == 0) st[tile] = kReady | (tile == 0 ? kWhole : 0ull) | sum;
+#pragma unroll
+    for (int j = 0; j < ITEMS; ++j)
+        if (first + j * kWarp < n) op.early(first + j * kWarp);
+    if (warp == 0) {
+        uint32_t before = 0;
+        bool lost = false;
+        for (int64_t p = tile - 1; p >= 0 && !lost; p -= kWarp) {
+            const int64_t at = p - lane;
+            unsigned long long w = at >= 0 ? st[at] : kReady | kWhole;
+            unsigned whole = 0, upto = 0;
+            for (uint32_t it = 0;; ++it) {
+                const unsigned ready = __ballot_sync(kFull, (w & kReady) != 0);
+                whole = __ballot_sync(kFull, (w & kWhole) != 0);
+                upto = whole ? (whole & (0u - whole)) * 2u - 1u : kFull;  // lanes up to the nearest whole one
+                if ((ready & upto) == upto) break;
+                if (it >= kChainPolls) {
+                    lost = true;
+                    break;
+                }
+                if (!(w & kReady)) w = st[at];
+            }
+            before += __reduce_add_sync(kFull, (upto >> lane) & 1u ? (uint32_t)w : 0u);
+            if (whole) break;
+        }
+        if (lane == 0) {
+            s_before = before;
+            s_lost = lost;
+        }
+    }
+    __syncthreads();
+    if (s_lost) {
+        // a predecessor did not answer: sum the elements before this tile
+        uint32_t mine = 0;
+        for (int64_t e = t; e < tile0; e += kChainThreads) mine += op.value(e);
+        mine = __reduce_add_sync(kFull, mine);
+        __syncthreads();
+        if (t == 0) s_before = 0;
+        __syncthreads();
+        if (lane == 0) atomicAdd(&s_before, mine);
+        __syncthreads();
+    }
+    const uint32_t before = s_before;
+    if (t == 0) {
+        if (tile > 0) st[tile] = kReady | kWhole | (before + sum);
+        if (tile0 + kTileLen >= n) {
+            *total = before + sum;
+            if (mail) *mail = before + sum;
+        }
+    }
+#pragma unroll
+    for (int j = 0; j < ITEMS; ++j)
+        if (first + j * kWarp < n) op.emit(first + j * kWarp, v[j], before + before_warp + ex[j]);
+}
+
+// ---------------------------------------------------------------------------
 // Lock-free union-find over int32 ids.  parent[x] <= x always (the larger root
 // is hooked under the smaller), so every find terminates.  Reads go through L2
 // (ld.cg) because other SMs rewrite parents concurrently.

@@ -240,9 +240,11 @@ __device__ __forceinline__ long long cell_coord(const GridDev &g, int a, float x
 
 template <int D, typename K>
 __global__ void __launch_bounds__(kBlock) key_kernel(const float *__restrict__ coords, int64_t n, bool vec,
-                                                     GridDev g, K invalid_key, K *__restrict__ keys) {
+                                                     GridDev g, K invalid_key, K *__restrict__ keys,
+                                                     uint32_t *__restrict__ core_bits) {
     const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n) return;
+    if ((i & 31) == 0) core_bits[i >> 5] = 0;  // for core_flags_kernel
     const float *p = coords + i * D;
     K key = invalid_key;
     float x[D];  // validity from one load of the row; the gridded coordinates are re-read (L1)
@@ -260,52 +262,48 @@ __global__ void __launch_bounds__(kBlock) key_kernel(const float *__restrict__ c
     keys[i] = key;
 }
 
-// pos = exclusive scan of "first point of a cell" flags
-template <typename K>
-__global__ void cell_flag_kernel(const K *__restrict__ keys, int64_t nv, uint32_t *__restrict__ flags) {
-    const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= nv) return;
-    flags[i] = (i == 0 || keys[i] != keys[i - 1]) ? 1u : 0u;
-}
-
-template <typename K>
-__global__ void cell_write_kernel(const K *__restrict__ keys, int64_t nv, const uint32_t *__restrict__ pos,
-                                  const uint32_t *__restrict__ n_cells_dev, int32_t *__restrict__ cell_start,
-                                  K *__restrict__ cell_key, int32_t *__restrict__ pcell) {
-    const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= nv) return;
-    const bool first = (i == 0 || keys[i] != keys[i - 1]);
-    const uint32_t c = first ? pos[i] : pos[i] - 1;
-    if (first) {
-        cell_start[c] = (int32_t)i;
-        cell_key[c] = keys[i];
-    }
-    pcell[i] = (int32_t)c;
-    if (i == nv - 1) cell_start[*n_cells_dev] = (int32_t)nv;
-}
-
-template <int D>
-__global__ void __launch_bounds__(kBlock) gather_kernel(const float *__restrict__ coords,
-                                                        const int32_t *__restrict__ perm, int64_t nv, bool vec,
-                                                        float *__restrict__ xs) {
-    constexpr int P = Stride<D>::P;
-    const int64_t s = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (s >= nv) return;
-    float x[D], v[P];
-    load_row<D>(coords + (int64_t)perm[s] * D, x, vec);
+// Cells from the sorted keys (chain_scan_kernel): the prefix of the "first point of a
+// cell" flags numbers the cells; meanwhile every point's coordinates are gathered into
+// cell order.
+template <int D, typename K>
+struct CellsOp {
+    const K *keys;
+    const int32_t *perm;
+    const float *coords;
+    bool vec;
+    int64_t nv;
+    float *xs;
+    int32_t *cell_start;
+    K *cell_key;
+    int32_t *pcell;
+    __device__ uint32_t value(int64_t e) const { return e == 0 || keys[e] != keys[e - 1] ? 1u : 0u; }
+    __device__ void early(int64_t e) const {
+        constexpr int P = Stride<D>::P;
+        float x[D], v[P];
+        load_row<D>(coords + (int64_t)perm[e] * D, x, vec);
 #pragma unroll
-    for (int k = 0; k < P; ++k) v[k] = k < D ? x[k] : 0.0f;
-    float *q = xs + s * P;
-    if constexpr (P % 4 == 0) {
+        for (int k = 0; k < P; ++k) v[k] = k < D ? x[k] : 0.0f;
+        float *q = xs + e * P;
+        if constexpr (P % 4 == 0) {
 #pragma unroll
-        for (int k = 0; k < P / 4; ++k)
-            reinterpret_cast<float4 *>(q)[k] = make_float4(v[4 * k], v[4 * k + 1], v[4 * k + 2], v[4 * k + 3]);
-    } else if constexpr (P == 2) {
-        *reinterpret_cast<float2 *>(q) = make_float2(v[0], v[1]);
-    } else {
-        q[0] = v[0];
+            for (int k = 0; k < P / 4; ++k)
+                reinterpret_cast<float4 *>(q)[k] = make_float4(v[4 * k], v[4 * k + 1], v[4 * k + 2], v[4 * k + 3]);
+        } else if constexpr (P == 2) {
+            *reinterpret_cast<float2 *>(q) = make_float2(v[0], v[1]);
+        } else {
+            q[0] = v[0];
+        }
     }
-}
+    __device__ void emit(int64_t e, uint32_t first, uint32_t before) const {
+        const uint32_t c = before + first - 1;
+        if (first) {
+            cell_start[c] = (int32_t)e;
+            cell_key[c] = keys[e];
+        }
+        pcell[e] = (int32_t)c;
+        if (e == nv - 1) cell_start[c + 1] = (int32_t)nv;
+    }
+};
 
 // Open-addressing hash table of the non-empty cells: key -> cell index.  Empty
 // slots hold the all-ones key, which no cell has (it marks invalid points).
@@ -326,10 +324,10 @@ __device__ __forceinline__ uint64_t key_cas(uint64_t *a, uint64_t cmp, uint64_t 
 }
 
 template <typename K>
-__global__ void hash_insert_kernel(const K *__restrict__ cell_key, int64_t n_cells, K *hkeys,
+__global__ void hash_insert_kernel(const K *__restrict__ cell_key, const uint32_t *__restrict__ n_cells, K *hkeys,
                                    int32_t *__restrict__ hvals, unsigned long long mask) {
     const int64_t c = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (c >= n_cells) return;
+    if (c >= *n_cells) return;
     const K key = cell_key[c];
     unsigned long long h = hash_slot((unsigned long long)key, mask);
     for (unsigned long long probe = 0; probe <= mask; ++probe) {
@@ -393,10 +391,10 @@ __device__ __forceinline__ long long global_column(const K *__restrict__ cell_ke
 }
 
 template <typename K>
-__global__ void col_range_kernel(const K *__restrict__ cell_key, int64_t n_cells, GridDev g_one,
-                                 const JobDev *__restrict__ jobs, const int32_t *__restrict__ cell_job,
-                                 int2 *__restrict__ col) {
-    const int64_t c = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+__global__ void col_range_kernel(const K *__restrict__ cell_key, const uint32_t *__restrict__ n_cells_dev,
+                                 GridDev g_one, const JobDev *__restrict__ jobs,
+                                 const int32_t *__restrict__ cell_job, int2 *__restrict__ col) {
+    const int64_t c = (int64_t)blockIdx.x * blockDim.x + threadIdx.x, n_cells = *n_cells_dev;
     if (c >= n_cells) return;
     const long long mine = global_column(cell_key, c, g_one, jobs, cell_job);
     if (c == 0 || global_column(cell_key, c - 1, g_one, jobs, cell_job) != mine) col[mine].x = (int)c;
@@ -484,18 +482,19 @@ __device__ __forceinline__ void decode_key(K key, const GridDev &g, long long &x
 // One thread per cell (one key decode); the first hash probes of a row's cells
 // are issued together.
 template <typename K>
-__global__ void __launch_bounds__(kBlock) rows_kernel(const K *__restrict__ cell_key, int64_t n_cells,
-                                                      GridDev g_one, const int4 *__restrict__ rows, int n_rows,
-                                                      int group_log2, CellIndex<K> L, int2 *__restrict__ nbr,
+__global__ void __launch_bounds__(kBlock) rows_kernel(const K *__restrict__ cell_key,
+                                                      const uint32_t *__restrict__ n_cells_dev, GridDev g_one,
+                                                      Stencil stencil, int group_log2, CellIndex<K> L, int2 *__restrict__ nbr,
                                                       const JobDev *__restrict__ jobs,
                                                       const int32_t *__restrict__ cell_job) {
     // one lane per (cell, row): 2^group_log2 lanes (>= n_rows) per cell, so
     // a cell's rows are looked up in parallel and its row table is written at once
     __shared__ int4 s_rows[kMaxRows];
-    for (int r = threadIdx.x; r < n_rows; r += blockDim.x) s_rows[r] = rows[r];
+    const int n_rows = stencil.n_rows;
+    for (int r = threadIdx.x; r < n_rows; r += blockDim.x) s_rows[r] = stencil.rows[r];
     __syncthreads();
     const int64_t gid = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    const int64_t c = gid >> group_log2;
+    const int64_t c = gid >> group_log2, n_cells = *n_cells_dev;
     const int r = (int)(gid & ((1 << group_log2) - 1));
     if (c >= n_cells || r >= n_rows) return;
     unsigned long long key_base = 0;
@@ -559,22 +558,21 @@ __global__ void __launch_bounds__(kBlock) rows_kernel(const K *__restrict__ cell
     nbr[c * n_rows + r] = res;
 }
 
-__global__ void item_count_kernel(const int32_t *__restrict__ cell_start, int64_t n_cells,
-                                  uint32_t *__restrict__ cnt) {
-    const int64_t c = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (c >= n_cells) return;
-    const int32_t size = cell_start[c + 1] - cell_start[c];
-    cnt[c] = (uint32_t)((size + kTile - 1) / kTile);
-}
-
-__global__ void item_write_kernel(const int32_t *__restrict__ cell_start, int64_t n_cells,
-                                  const uint32_t *__restrict__ off, int2 *__restrict__ items) {
-    const int64_t c = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (c >= n_cells) return;
-    const int32_t s0 = cell_start[c], s1 = cell_start[c + 1];
-    uint32_t o = off[c];
-    for (int32_t p = s0; p < s1; p += kTile) items[o++] = make_int2((int)c, p);
-}
+// Work items (cell, first point), chunks of up to 32 points of a cell, in cell order
+// (chain_scan_kernel over the cells); also clears the cells' core flags.
+struct ItemsOp {
+    const int32_t *cell_start;
+    int2 *items;
+    uint8_t *cell_has_core;
+    __device__ uint32_t value(int64_t c) const {
+        return (uint32_t)((cell_start[c + 1] - cell_start[c] + kTile - 1) / kTile);
+    }
+    __device__ void early(int64_t c) const { cell_has_core[c] = 0; }
+    __device__ void emit(int64_t c, uint32_t cnt, uint32_t before) const {
+        const int32_t s0 = cell_start[c];
+        for (uint32_t q = 0; q < cnt; ++q) items[before + q] = make_int2((int)c, s0 + (int)q * kTile);
+    }
+};
 
 // ---------------------------------------------------------------------------
 // Row table: the candidate ranges of one cell's stencil rows, gathered by the
@@ -752,12 +750,11 @@ __device__ __forceinline__ unsigned transpose32(unsigned x, int lane) {
 
 template <int D, bool EARLY, bool GRAM = false>
 __global__ void __launch_bounds__(kCountWarps * kWarp) count_kernel(
-    const int2 *__restrict__ items, int64_t n_items, const int32_t *__restrict__ cell_start,
+    const int2 *__restrict__ items, const uint32_t *__restrict__ n_items, const int32_t *__restrict__ cell_start,
     const int2 *__restrict__ nbr, int n_rows, const float *__restrict__ xs, float e2, int min_pts,
     int dense_skip, int32_t *__restrict__ nn_sorted, int32_t *__restrict__ nbr_list, int list_cap,
     int list_stride, unsigned long long *__restrict__ pair_counter, const JobDev *__restrict__ jobs,
-    const int32_t *__restrict__ cell_job, const uint32_t *__restrict__ n_items_dev,
-    unsigned long long *__restrict__ band_counter) {
+    const int32_t *__restrict__ cell_job, unsigned long long *__restrict__ band_counter) {
     constexpr int P = Stride<D>::P;
     static_assert(!GRAM || D >= 8, "the Gram filter is built for d >= 8");
     // d >= 8: each lane holds two candidates per step (64 per warp), so an owned
@@ -771,9 +768,8 @@ __global__ void __launch_bounds__(kCountWarps * kWarp) count_kernel(
     __shared__ int s_j[kCountWarps][CH * kWarp];  // the step's candidates
     __shared__ int2 s_move[kCountWarps][kTile];   // (index, count) of the points a packing moves
     const int lane = threadIdx.x & 31, wib = threadIdx.x >> 5;
-    if (n_items_dev) n_items = *n_items_dev;  // a list whose length the device wrote
     const int64_t item_id = (int64_t)blockIdx.x * kCountWarps + wib;
-    if (item_id >= n_items) return;
+    if (item_id >= *n_items) return;
     const int2 item = items[item_id];
     const int cell = item.x, p0 = item.y;
     const int cs = cell_start[cell], ce = cell_start[cell + 1];
@@ -1002,10 +998,14 @@ __global__ void core_flags_kernel(const int32_t *__restrict__ nn_sorted, int64_t
     }
 }
 
-__global__ void popc_words_kernel(const uint32_t *__restrict__ bits, int64_t n_words, uint32_t *__restrict__ cnt) {
-    const int64_t w = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (w < n_words) cnt[w] = (uint32_t)__popc(bits[w]);
-}
+// Cores before each word of the bitmap (chain_scan_kernel over the words).
+struct CorePrefixOp {
+    const uint32_t *bits;
+    uint32_t *prefix;
+    __device__ uint32_t value(int64_t w) const { return (uint32_t)__popc(bits[w]); }
+    __device__ void early(int64_t) const {}
+    __device__ void emit(int64_t w, uint32_t, uint32_t before) const { prefix[w] = before; }
+};
 
 __device__ __forceinline__ bool is_core_o(const uint32_t *__restrict__ bits, int32_t o) {
     return (bits[o >> 5] >> (o & 31)) & 1u;
@@ -1023,30 +1023,27 @@ __device__ __forceinline__ int32_t core_rank(const uint32_t *__restrict__ bits, 
 // pass streams the sorted arrays (evict-first loads) and writes only the points
 // whose destination falls in its window, so the partial-sector writes stay in L2.
 __global__ void scatter_nn_kernel(const int32_t *__restrict__ nn_sorted, int64_t nv, int64_t n,
-                                  const int32_t *__restrict__ perm, int32_t *__restrict__ out,
-                                  const JobDev *__restrict__ jobs, int n_jobs, int64_t win_lo = 0,
-                                  int64_t win_hi = INT64_MAX) {
+                                  const int32_t *__restrict__ perm, int32_t *__restrict__ out, int64_t win_lo,
+                                  int64_t win_hi) {
     const int64_t s = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (s >= n) return;
     const int32_t o = __ldcs(perm + s);
     if (o < win_lo || o >= win_hi) return;
-    const int32_t v = s < nv ? __ldcs(nn_sorted + s) : 0;
-    if (jobs) {
-        const JobDev &J = jobs[job_of_point(jobs, n_jobs, o)];
-        if (J.nn_out) J.nn_out[o - J.off] = v;
-    } else {
-        out[o] = v;
+    out[o] = s < nv ? __ldcs(nn_sorted + s) : 0;
+}
+
+// Start of the label phase: every unit its own root, no component minimum yet; point
+// units: no cell root yet (cell_root, null for cell units) and no union segment.
+__global__ void init_units_kernel(int32_t *__restrict__ parent, int32_t *__restrict__ comp_min, int64_t bound,
+                                  const uint32_t *__restrict__ n_cells, int32_t *__restrict__ cell_root,
+                                  uint32_t *__restrict__ n_seg) {
+    const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+    if (i < bound) {
+        parent[i] = (int32_t)i;
+        comp_min[i] = kNoCluster;
+        if (cell_root && i < *n_cells) cell_root[i] = -1;
     }
-}
-
-__global__ void iota_kernel(int32_t *__restrict__ a, int64_t n) {
-    const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (i < n) a[i] = (int32_t)i;
-}
-
-__global__ void fill_kernel(int32_t *__restrict__ a, int64_t n, int32_t v) {
-    const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (i < n) a[i] = v;
+    if (i == 0 && cell_root) *n_seg = 0;
 }
 
 // bytes [0, bytes) of p set to v: n16 16-byte stores (p 16-byte aligned; 0 when it
@@ -1147,11 +1144,11 @@ __device__ __forceinline__ void load_first_cores(const float *__restrict__ xs, c
 
 template <int D, typename K>
 __global__ void __launch_bounds__(kBlock) union_near_kernel(
-    int64_t n_cells, GridDev g_one, const K *__restrict__ cell_key, const int32_t *__restrict__ cell_start,
+    const uint32_t *__restrict__ n_cells_dev, GridDev g_one, const K *__restrict__ cell_key, const int32_t *__restrict__ cell_start,
     CellIndex<K> L, const float *__restrict__ xs, float e2, const uint8_t *__restrict__ core_sorted,
     const uint8_t *__restrict__ cell_has_core, int32_t *parent, unsigned long long *__restrict__ pair_counter,
     int *err, const JobDev *__restrict__ jobs, const int32_t *__restrict__ cell_job) {
-    const int64_t idx = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+    const int64_t idx = (int64_t)blockIdx.x * blockDim.x + threadIdx.x, n_cells = *n_cells_dev;
     unsigned pairs = 0;
     if (idx < n_cells && cell_has_core[idx]) {
         const int A = (int)idx;
@@ -1223,7 +1220,7 @@ constexpr int kProbe = 4;  // points of a candidate cell tested by the probe
 // only costs a needless probe below, never a missed union.
 template <int D>
 __global__ void __launch_bounds__(kBlock) union_cells_kernel(
-    int64_t n_cells, const int32_t *__restrict__ cell_start, const int2 *__restrict__ nbr, int n_rows,
+    const uint32_t *__restrict__ n_cells, const int32_t *__restrict__ cell_start, const int2 *__restrict__ nbr, int n_rows,
     const float *__restrict__ xs, float e2, const uint8_t *__restrict__ core_sorted,
     const uint8_t *__restrict__ cell_has_core, int32_t *parent, unsigned long long *__restrict__ pair_counter,
     int *err, const JobDev *__restrict__ jobs, const int32_t *__restrict__ cell_job,
@@ -1234,7 +1231,7 @@ __global__ void __launch_bounds__(kBlock) union_cells_kernel(
     __shared__ int s_b[kWarpsPerBlock][kMaxCandCells];
     const int lane = threadIdx.x & 31, wib = threadIdx.x >> 5;
     const int64_t A64 = (int64_t)blockIdx.x * kWarpsPerBlock + wib;
-    if (A64 >= n_cells) return;
+    if (A64 >= *n_cells) return;
     const int A = (int)A64;
     if (!cell_has_core[A]) return;
     if (jobs) e2 = jobs[cell_job[A]].e2;
@@ -1392,7 +1389,7 @@ __device__ __forceinline__ int union_rows(int A, int p0, int root, const int32_t
 }
 
 __global__ void __launch_bounds__(kBlock) union_select_kernel(
-    const int2 *__restrict__ items, int64_t n_items, const int32_t *__restrict__ cell_start,
+    const int2 *__restrict__ items, const uint32_t *__restrict__ n_items, const int32_t *__restrict__ cell_start,
     const int2 *__restrict__ nbr, int n_rows, const int32_t *__restrict__ cell_root,
     const int32_t *__restrict__ snap, uint32_t *__restrict__ seg_item, uint32_t *__restrict__ seg_part,
     uint32_t seg_cap, uint32_t *__restrict__ n_seg) {
@@ -1401,7 +1398,7 @@ __global__ void __launch_bounds__(kBlock) union_select_kernel(
     __shared__ int s_need[kWarpsPerBlock][kWarp];
     const int lane = threadIdx.x & 31, wib = threadIdx.x >> 5;
     const int64_t item_id = (int64_t)blockIdx.x * kWarpsPerBlock + wib;
-    if (item_id >= n_items) return;
+    if (item_id >= *n_items) return;
     const int2 item = items[item_id];
     const int A = item.x, p0 = item.y;
     if (__ldg(cell_root + A) == -1) return;
@@ -1426,7 +1423,7 @@ __global__ void __launch_bounds__(kBlock) union_select_kernel(
 // dense data), every item is walked whole instead.
 template <int D>
 __global__ void __launch_bounds__(kCountWarps * kWarp) union_scan_kernel(
-    const int2 *__restrict__ items, int64_t n_items, const int32_t *__restrict__ cell_start,
+    const int2 *__restrict__ items, const uint32_t *__restrict__ n_items, const int32_t *__restrict__ cell_start,
     const int2 *__restrict__ nbr, int n_rows, const float *__restrict__ xs, float e2,
     const int32_t *__restrict__ cell_root, const int32_t *__restrict__ snap, int32_t *parent,
     const uint32_t *__restrict__ seg_item, const uint32_t *__restrict__ seg_part, uint32_t seg_cap,
@@ -1446,7 +1443,7 @@ __global__ void __launch_bounds__(kCountWarps * kWarp) union_scan_kernel(
     RowTable &rt = s_rows[wib];
     unsigned long long pairs = 0;
     const bool listed = *n_seg <= seg_cap;
-    const uint32_t n_work = listed ? *n_seg : (uint32_t)n_items;
+    const uint32_t n_work = listed ? *n_seg : *n_items;
     for (uint32_t w = blockIdx.x * kCountWarps + wib; w < n_work; w += gridDim.x * kCountWarps) {
         const int2 item = items[listed ? seg_item[w] : w];
         const int A = item.x, p0 = item.y;
@@ -1541,65 +1538,60 @@ __global__ void __launch_bounds__(kCountWarps * kWarp) union_scan_kernel(
     if (lane == 0 && pairs) atomicAdd(pair_counter, pairs);
 }
 
-// comp_min[root] = min core rank in the component.  Runs after flatten_kernel, so
-// parent[u] is the root; lanes that share a root combine their minimum first and
-// one lane per root issues the atomic (clusters have millions of cores).
-__global__ void comp_min_kernel(int64_t nv, const uint8_t *__restrict__ core_sorted,
-                                const int32_t *__restrict__ perm, const int32_t *__restrict__ pcell,
-                                int cell_units, const uint32_t *__restrict__ core_bits,
-                                const uint32_t *__restrict__ core_prefix, const int32_t *__restrict__ parent,
-                                int32_t *__restrict__ comp_min) {
+// Lanes that share a root combine their core rank r, and one lane per root adds it to
+// the component's minimum (clusters have millions of cores).
+__device__ __forceinline__ void add_comp_min(bool ok, int root, int r, int32_t *__restrict__ comp_min) {
+    unsigned pending = __ballot_sync(kFull, ok);
+    const int lane = threadIdx.x & 31;
+    while (pending) {
+        const int leader = __ffs(pending) - 1;
+        const int lroot = __shfl_sync(kFull, root, leader);
+        const bool mine = ok && root == lroot;
+        const int m = (int)__reduce_min_sync(kFull, mine ? (unsigned)r : (unsigned)kNoCluster);
+        if (lane == leader) atomicMin(comp_min + lroot, m);
+        pending &= ~__ballot_sync(kFull, mine);
+    }
+}
+
+// Point units: parent[s] = root of s for every core, comp_min[root] = smallest core rank
+// of the component.  Thread s is the only writer of parent[s] (read-only finds).
+__global__ void flatten_min_points_kernel(int32_t *parent, int64_t nv, int *err, const uint8_t *__restrict__ core_sorted,
+                                          const int32_t *__restrict__ perm, const uint32_t *__restrict__ core_bits,
+                                          const uint32_t *__restrict__ core_prefix, int32_t *__restrict__ comp_min) {
     const int64_t s = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     const bool ok = s < nv && core_sorted[s];
     int root = -1, r = kNoCluster;
     if (ok) {
-        root = parent[cell_units ? pcell[s] : (int)s];
+        root = uf_find_ro(parent, (int)s, err);
+        parent[s] = root;
         r = core_rank(core_bits, core_prefix, perm[s]);
     }
-    unsigned pending = __ballot_sync(kFull, ok);
-    const int lane = threadIdx.x & 31;
-    while (pending) {
-        const int leader = __ffs(pending) - 1;
-        const int lroot = __shfl_sync(kFull, root, leader);
-        const bool mine = ok && root == lroot;
-        const int m = (int)__reduce_min_sync(kFull, mine ? (unsigned)r : (unsigned)kNoCluster);
-        if (lane == leader) atomicMin(comp_min + lroot, m);
-        pending &= ~__ballot_sync(kFull, mine);
-    }
+    add_comp_min(ok, root, r, comp_min);
 }
 
-// Cell units: the smallest core rank of a cell is its first core's, because the
-// stable radix sort (started from the identity permutation) keeps the points of a
-// cell in input order.  One thread per cell instead of one per point: far fewer
-// atomics on the roots of large clusters.  Lanes sharing a root combine first.
-__global__ void comp_min_cells_kernel(int64_t n_cells, const int32_t *__restrict__ cell_start,
-                                      const uint8_t *__restrict__ cell_has_core,
-                                      const uint8_t *__restrict__ core_sorted, const int32_t *__restrict__ perm,
-                                      const uint32_t *__restrict__ core_bits,
-                                      const uint32_t *__restrict__ core_prefix, const int32_t *__restrict__ parent,
-                                      int32_t *__restrict__ comp_min) {
+// Cell units: the same per cell.  The smallest core rank of a cell is its first core's,
+// because the stable radix sort (of points in input order) keeps the points of a cell in
+// input order: one thread per cell instead of one per point.
+__global__ void flatten_min_cells_kernel(int32_t *parent, const uint32_t *__restrict__ n_cells, int *err,
+                                         const int32_t *__restrict__ cell_start,
+                                         const uint8_t *__restrict__ cell_has_core,
+                                         const uint8_t *__restrict__ core_sorted, const int32_t *__restrict__ perm,
+                                         const uint32_t *__restrict__ core_bits,
+                                         const uint32_t *__restrict__ core_prefix, int32_t *__restrict__ comp_min) {
     const int64_t c = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    const bool ok = c < n_cells && cell_has_core[c];
+    const bool ok = c < *n_cells && cell_has_core[c];
     int root = -1, r = kNoCluster;
     if (ok) {
+        root = uf_find_ro(parent, (int)c, err);
+        parent[c] = root;
         int p = cell_start[c];
         while (!core_sorted[p]) ++p;  // the cell has a core
-        root = parent[c];
         r = core_rank(core_bits, core_prefix, perm[p]);
     }
-    unsigned pending = __ballot_sync(kFull, ok);
-    const int lane = threadIdx.x & 31;
-    while (pending) {
-        const int leader = __ffs(pending) - 1;
-        const int lroot = __shfl_sync(kFull, root, leader);
-        const bool mine = ok && root == lroot;
-        const int m = (int)__reduce_min_sync(kFull, mine ? (unsigned)r : (unsigned)kNoCluster);
-        if (lane == leader) atomicMin(comp_min + lroot, m);
-        pending &= ~__ballot_sync(kFull, mine);
-    }
+    add_comp_min(ok, root, r, comp_min);
 }
 
-// Point units, after the list unions: parent flattened (as flatten_kernel), every
+// Point units, after the list unions: parent flattened, every
 // core's root in snap (-1 for non-cores), and the one root of each cell's cores in
 // cell_root: -1 without cores, -2 when they do not all share it.  One thread per
 // point: the first core of a cell to arrive installs its root, any core with another
@@ -1664,69 +1656,51 @@ __global__ void union_lists_kernel(int64_t nv, const int32_t *__restrict__ nn_so
     }
 }
 
-// parent[u] = root of u.  Thread u is the only writer of parent[u] here (read-only
-// finds), so after the kernel every parent is its root.
-__global__ void flatten_kernel(int32_t *parent, int64_t n_units, int *err) {
-    const int64_t u = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (u >= n_units) return;
-    const int r = uf_find_ro(parent, (int)u, err);
-    parent[u] = r;
-}
-
-// The same, also recording each cell's root in snap (-1 for a cell without cores)
-// for the candidate filter of union_cells_kernel.
-__global__ void flatten_snap_kernel(int32_t *parent, int64_t n_units, int *err,
+// After the list and near unions of cell units: parent[u] = root of u (thread u is its
+// only writer, with read-only finds), and each cell's root in snap (-1 for a cell
+// without cores) for the candidate filter of union_cells_kernel.
+__global__ void flatten_snap_kernel(int32_t *parent, const uint32_t *__restrict__ n_cells, int *err,
                                     const uint8_t *__restrict__ has_core, int32_t *__restrict__ snap) {
     const int64_t u = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (u >= n_units) return;
+    if (u >= *n_cells) return;
     const int r = uf_find_ro(parent, (int)u, err);
     parent[u] = r;
     snap[u] = has_core[u] ? r : -1;
 }
 
-// ids of the cores in sorted order; counters[0] += component roots (point units)
-__global__ void core_ids_kernel(int64_t nv, const uint8_t *__restrict__ core_sorted,
-                                const int32_t *__restrict__ pcell, int cell_units,
-                                const int32_t *__restrict__ parent, const int32_t *__restrict__ comp_min,
-                                int32_t *__restrict__ ci_sorted, unsigned long long *__restrict__ counters,
-                                const int32_t *__restrict__ cell_job, unsigned long long *__restrict__ job_counters) {
+// Ids of the cores in sorted order, and for cell units the id of every cell's component;
+// counters[0] += component roots.
+__global__ void ids_kernel(int64_t nv, const uint32_t *__restrict__ n_cells, const uint8_t *__restrict__ core_sorted,
+                           const int32_t *__restrict__ pcell, const uint8_t *__restrict__ cell_has_core,
+                           int cell_units, const int32_t *__restrict__ parent, const int32_t *__restrict__ comp_min,
+                           int32_t *__restrict__ ci_sorted, int32_t *__restrict__ cell_cid,
+                           unsigned long long *__restrict__ counters, const int32_t *__restrict__ cell_job,
+                           unsigned long long *__restrict__ job_counters) {
     const int64_t s = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     unsigned roots = 0;
     if (s < nv) {
+        int id = kNoCluster;
         if (core_sorted[s]) {
-            const int u = cell_units ? pcell[s] : (int)s;
-            const int root = parent[u];
-            ci_sorted[s] = comp_min[root];
+            const int cell = pcell[s], root = parent[cell_units ? cell : (int)s];
+            id = comp_min[root];
             if (!cell_units && root == (int)s) {
-                if (job_counters) atomicAdd(job_counters + 4 * cell_job[pcell[s]], 1ull);
+                if (job_counters) atomicAdd(job_counters + 4 * cell_job[cell], 1ull);
                 else roots = 1;
             }
-        } else {
-            ci_sorted[s] = kNoCluster;
         }
+        ci_sorted[s] = id;
     }
-    roots = __reduce_add_sync(kFull, roots);
-    if ((threadIdx.x & 31) == 0 && roots) atomicAdd(counters + 0, (unsigned long long)roots);
-}
-
-// clusters over cells + the id of every cell's component
-__global__ void cell_ids_kernel(int64_t n_cells, const uint8_t *__restrict__ cell_has_core,
-                                const int32_t *__restrict__ parent, const int32_t *__restrict__ comp_min,
-                                int32_t *__restrict__ cell_cid, unsigned long long *__restrict__ counters,
-                                const int32_t *__restrict__ cell_job, unsigned long long *__restrict__ job_counters) {
-    const int64_t c = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    unsigned roots = 0;
-    if (c < n_cells) {
-        if (cell_has_core[c]) {
-            const int root = parent[c];
-            cell_cid[c] = comp_min[root];
-            if (root == (int)c) {
-                if (job_counters) atomicAdd(job_counters + 4 * cell_job[c], 1ull);
+    if (cell_units && s < *n_cells) {
+        int id = kNoCluster;
+        if (cell_has_core[s]) {
+            const int root = parent[s];
+            id = comp_min[root];
+            if (root == (int)s) {
+                if (job_counters) atomicAdd(job_counters + 4 * cell_job[s], 1ull);
                 else roots = 1;
             }
-        } else {
-            cell_cid[c] = kNoCluster;
         }
+        cell_cid[s] = id;
     }
     roots = __reduce_add_sync(kFull, roots);
     if ((threadIdx.x & 31) == 0 && roots) atomicAdd(counters + 0, (unsigned long long)roots);
@@ -1744,7 +1718,7 @@ __global__ void cell_ids_kernel(int64_t n_cells, const uint8_t *__restrict__ cel
 // ---------------------------------------------------------------------------
 template <int D>
 __global__ void __launch_bounds__(kBlock) border_kernel(
-    const int2 *__restrict__ items, int64_t n_items, const int32_t *__restrict__ cell_start,
+    const int2 *__restrict__ items, const uint32_t *__restrict__ n_items, const int32_t *__restrict__ cell_start,
     const int2 *__restrict__ nbr, int n_rows, const float *__restrict__ xs, float e2,
     const uint8_t *__restrict__ core_sorted, const uint8_t *__restrict__ cell_has_core, int cell_units,
     const int32_t *__restrict__ cell_cid, int32_t *__restrict__ ci_sorted,
@@ -1756,7 +1730,7 @@ __global__ void __launch_bounds__(kBlock) border_kernel(
     __shared__ int2 s_cand[kWarpsPerBlock][kMaxCandCells];
     const int lane = threadIdx.x & 31, wib = threadIdx.x >> 5;
     const int64_t item_id = (int64_t)blockIdx.x * kWarpsPerBlock + wib;
-    if (item_id >= n_items) return;
+    if (item_id >= *n_items) return;
     const int2 item = items[item_id];
     const int A = item.x, p0 = item.y;
     const int cnt = min(kTile, cell_start[A + 1] - p0);
@@ -1914,18 +1888,65 @@ __global__ void border_list_kernel(int64_t nv, const int32_t *__restrict__ nn_so
 __global__ void output_ci_kernel(const int32_t *__restrict__ ci_sorted, int64_t nv, int64_t n,
                                  const int32_t *__restrict__ perm, const uint32_t *__restrict__ core_bits,
                                  const uint32_t *__restrict__ core_prefix, int32_t *__restrict__ out,
-                                 unsigned long long *__restrict__ counters, const JobDev *__restrict__ jobs,
-                                 int n_jobs, unsigned long long *__restrict__ job_counters, int64_t win_lo = 0,
-                                 int64_t win_hi = INT64_MAX) {
+                                 unsigned long long *__restrict__ counters, int64_t win_lo, int64_t win_hi) {
     // windows as in scatter_nn_kernel; every point is counted in its own window only
     const int64_t s = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     unsigned noise = 0, roots = 0;
-    int job = -1;  // batched runs: the point's job, whose counters take its noise and roots
     const int32_t o = s < n ? __ldcs(perm + s) : 0;
     if (s < n && o >= win_lo && o < win_hi) {
         int32_t v;
         if (s < nv) {
             v = __ldcs(ci_sorted + s);
+        } else if (is_core_o(core_bits, o)) {
+            v = core_rank(core_bits, core_prefix, o);
+            roots = 1;
+        } else {
+            v = kNoCluster;
+        }
+        noise = v == kNoCluster;
+        if (out) out[o] = v;
+    }
+    noise = __reduce_add_sync(kFull, noise);
+    roots = __reduce_add_sync(kFull, roots);
+    if ((threadIdx.x & 31) == 0) {
+        if (noise) atomicAdd(counters + 1, (unsigned long long)noise);
+        if (roots) atomicAdd(counters + 0, (unsigned long long)roots);
+    }
+}
+
+// The border step from the count's lists (border_list_kernel), the counts (scatter_nn_kernel)
+// and the ids (output_ci_kernel) in one pass over the points, for outputs that stay in
+// L2: the permutation is read once and nothing is launched in between.  nn_out may be
+// null; use_lists 0: a border kernel has run before.
+__global__ void finish_kernel(int64_t nv, int64_t n, const int32_t *__restrict__ nn_sorted,
+                              const int32_t *__restrict__ nbr_list, int list_stride, int use_lists,
+                              const uint8_t *__restrict__ core_sorted, int cell_units,
+                              const int32_t *__restrict__ pcell, const int32_t *__restrict__ cell_cid,
+                              int32_t *ci_sorted, const int32_t *__restrict__ perm,
+                              const uint32_t *__restrict__ core_bits, const uint32_t *__restrict__ core_prefix,
+                              int32_t *__restrict__ nn_out, int32_t *__restrict__ ci_out,
+                              unsigned long long *__restrict__ counters, const JobDev *__restrict__ jobs, int n_jobs,
+                              unsigned long long *__restrict__ job_counters) {
+    const int64_t s = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+    unsigned noise = 0, roots = 0, looked = 0;
+    int job = -1;  // batched runs: the point's job, whose counters take its noise and roots
+    if (s < n) {
+        const int32_t o = perm[s];
+        int32_t v, nn = 0;
+        if (s < nv) {
+            nn = nn_sorted[s];
+            if (use_lists && !core_sorted[s]) {
+                looked = (unsigned)min(nn, list_stride);
+                v = kNoCluster;
+                const int32_t *l = nbr_list + s * list_stride;
+                for (unsigned q = 0; q < looked; ++q) {
+                    const int j = l[q];
+                    if (core_sorted[j]) v = min(v, cell_units ? cell_cid[pcell[j]] : ci_sorted[j]);
+                }
+                ci_sorted[s] = v;
+            } else {
+                v = ci_sorted[s];
+            }
         } else if (is_core_o(core_bits, o)) {
             v = core_rank(core_bits, core_prefix, o);
             roots = 1;
@@ -1939,8 +1960,10 @@ __global__ void output_ci_kernel(const int32_t *__restrict__ ci_sorted, int64_t 
             const JobDev &J = jobs[job];
             if (v != kNoCluster) v -= core_rank(core_bits, core_prefix, (int32_t)J.off);
             if (J.ci_out) J.ci_out[o - J.off] = v;
-        } else if (out) {
-            out[o] = v;
+            if (J.nn_out) J.nn_out[o - J.off] = nn;
+        } else {
+            if (ci_out) ci_out[o] = v;
+            if (nn_out) nn_out[o] = nn;
         }
     }
     if (jobs) {
@@ -1957,9 +1980,11 @@ __global__ void output_ci_kernel(const int32_t *__restrict__ ci_sorted, int64_t 
     }
     noise = __reduce_add_sync(kFull, noise);
     roots = __reduce_add_sync(kFull, roots);
+    looked = __reduce_add_sync(kFull, looked);
     if ((threadIdx.x & 31) == 0) {
         if (noise) atomicAdd(counters + 1, (unsigned long long)noise);
         if (roots) atomicAdd(counters + 0, (unsigned long long)roots);
+        if (looked) atomicAdd(counters + 4, (unsigned long long)looked);
     }
 }
 
@@ -2070,11 +2095,12 @@ __global__ void __launch_bounds__(kBlock) bbox_batch_kernel(const float *__restr
 template <int D, typename K>
 __global__ void __launch_bounds__(kBlock) key_batch_kernel(const float *__restrict__ coords,
                                                            const JobDev *__restrict__ jobs, K invalid_key,
-                                                           K *__restrict__ keys) {
+                                                           K *__restrict__ keys, uint32_t *__restrict__ core_bits) {
     const JobDev &J = jobs[blockIdx.y];
     const GridDev g = J.g;
     for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < J.n; i += (int64_t)gridDim.x * blockDim.x) {
         const int64_t o = J.off + i;
+        if ((o & 31) == 0) core_bits[o >> 5] = 0;  // for core_flags_kernel
         const float *p = coords + o * D;
         K key = invalid_key;
         float x[D];  // validity from one vector load of the row; the gridded coordinates are re-read (L1)

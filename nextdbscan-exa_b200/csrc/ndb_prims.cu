@@ -1,103 +1,14 @@
-// ndb_prims.cu -- device-wide exclusive scan and stable LSD radix sort (key, value).
+// ndb_prims.cu -- stable LSD radix sort (key, value).
 //
-// These replace the reference's generic parallel primitives on the hot path
-// (exa::exclusive_scan magma_exa_omp.h:92-129, exa::copy_if :131-162, and the
-// sample sort :282-364 that the reference ships but never calls) with
-// purpose-built histogram / scan / scatter kernels.  Both are HBM-bound:
-// a scan moves 8 bytes per element (read + write) plus a 4-byte reduce pass, a
-// sort reads the keys once for the histograms of all its passes and moves
-// 2 x (key + value) bytes per element and pass.
+// With chain_scan_kernel (ndb_common.cuh) it replaces the reference's generic parallel
+// primitives on the hot path (exa::exclusive_scan magma_exa_omp.h:92-129, exa::copy_if
+// :131-162, and the sample sort :282-364 that the reference ships but never calls).
 #include "ndb_common.cuh"
 #include "ndb_internal.h"
 
 namespace ndb {
 
 namespace {
-
-constexpr int kScanThreads = 256;
-constexpr int kScanItems = kScanTile / kScanThreads;  // 8
-
-__device__ __forceinline__ int pad32(int e) { return e + (e >> 5); }
-
-__global__ void __launch_bounds__(kScanThreads) scan_reduce_kernel(const uint32_t *__restrict__ in,
-                                                                   int64_t n,
-                                                                   uint32_t *__restrict__ partials) {
-    const int t = threadIdx.x;
-    const int64_t base = (int64_t)blockIdx.x * kScanTile;
-    uint32_t s = 0;
-#pragma unroll
-    for (int i = 0; i < kScanItems; ++i) {
-        const int64_t e = base + i * kScanThreads + t;
-        if (e < n) s += in[e];
-    }
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(kFull, s, o);
-    __shared__ uint32_t s_w[kScanThreads / kWarp];
-    if ((t & 31) == 0) s_w[t >> 5] = s;
-    __syncthreads();
-    if (t == 0) {
-        uint32_t tot = 0;
-#pragma unroll
-        for (int w = 0; w < kScanThreads / kWarp; ++w) tot += s_w[w];
-        partials[blockIdx.x] = tot;
-    }
-}
-
-__global__ void __launch_bounds__(kScanThreads) scan_down_kernel(const uint32_t *in, uint32_t *out,
-                                                                 int64_t n,
-                                                                 const uint32_t *__restrict__ offsets,
-                                                                 uint32_t *__restrict__ total_dev) {
-    __shared__ uint32_t s[kScanTile + kScanTile / 32];
-    __shared__ uint32_t s_w[kScanThreads / kWarp];
-    const int t = threadIdx.x, lane = t & 31, warp = t >> 5;
-    const int64_t base = (int64_t)blockIdx.x * kScanTile;
-#pragma unroll
-    for (int i = 0; i < kScanItems; ++i) {
-        const int e = i * kScanThreads + t;
-        s[pad32(e)] = (base + e < n) ? in[base + e] : 0u;
-    }
-    __syncthreads();
-    uint32_t v[kScanItems];
-    uint32_t sum = 0;
-#pragma unroll
-    for (int i = 0; i < kScanItems; ++i) {
-        v[i] = s[pad32(t * kScanItems + i)];
-        sum += v[i];
-    }
-    uint32_t x = sum;
-#pragma unroll
-    for (int o = 1; o < 32; o <<= 1) {
-        const uint32_t y = __shfl_up_sync(kFull, x, o);
-        if (lane >= o) x += y;
-    }
-    if (lane == 31) s_w[warp] = x;
-    __syncthreads();
-    if (warp == 0) {
-        uint32_t w = lane < kScanThreads / kWarp ? s_w[lane] : 0u;
-#pragma unroll
-        for (int o = 1; o < kScanThreads / kWarp; o <<= 1) {
-            const uint32_t y = __shfl_up_sync(kFull, w, o);
-            if (lane >= o) w += y;
-        }
-        if (lane < kScanThreads / kWarp) s_w[lane] = w;
-    }
-    __syncthreads();
-    const uint32_t block_off = offsets ? offsets[blockIdx.x] : 0u;
-    uint32_t run = block_off + (warp > 0 ? s_w[warp - 1] : 0u) + x - sum;
-#pragma unroll
-    for (int i = 0; i < kScanItems; ++i) {
-        s[pad32(t * kScanItems + i)] = run;
-        run += v[i];
-    }
-    if (total_dev && blockIdx.x == gridDim.x - 1 && t == 0)
-        *total_dev = block_off + s_w[kScanThreads / kWarp - 1];
-    __syncthreads();
-#pragma unroll
-    for (int i = 0; i < kScanItems; ++i) {
-        const int e = i * kScanThreads + t;
-        if (base + e < n) out[base + e] = s[pad32(e)];
-    }
-}
 
 // ---------------------------------------------------------------------------
 // radix sort: 8-bit digits, least significant first, one kernel per pass.
@@ -315,14 +226,14 @@ __global__ void zero_words_kernel(uint4 *__restrict__ p, int64_t n) {
 
 template <typename K>
 cudaError_t radix_sort_pairs(K *k0, int32_t *v0, K *k1, int32_t *v1, int64_t n, int bits, uint32_t *scratch,
-                             bool *result_in_first, cudaStream_t st) {
+                             size_t zero_words, bool *result_in_first, cudaStream_t st) {
     *result_in_first = true;
     if (n <= 0) return cudaSuccess;
     const int64_t tiles = (n + SortTile<K>::v - 1) / SortTile<K>::v;
     const int passes = bits <= 0 ? 1 : (bits + 7) / 8;
     uint32_t *hist = scratch, *tickets = scratch + kSortHistWords;
     unsigned long long *state = reinterpret_cast<unsigned long long *>(tickets + kSortTicketWords);
-    const int64_t zero = (int64_t)sort_scratch_words<K>(n) / 4;
+    const int64_t zero = (int64_t)((zero_words + 3) / 4);
     ++launch_counter(), zero_words_kernel<<<(unsigned)((zero + kSortThreads * 4 - 1) / (kSortThreads * 4)), kSortThreads, 0, st>>>(
         reinterpret_cast<uint4 *>(scratch), zero);
     const int64_t hist_blocks = (n + kSortThreads * 8 - 1) / (kSortThreads * 8);
@@ -355,40 +266,16 @@ int &launch_counter() {
     return count;
 }
 
-size_t scan_scratch_words(int64_t n) {
-    const int64_t nb = (n + kScanTile - 1) / kScanTile;
-    if (nb <= 1) return 0;
-    return (size_t)((nb + 63) & ~int64_t(63)) + scan_scratch_words(nb);
-}
-
-cudaError_t scan_exclusive_u32(const uint32_t *in, uint32_t *out, int64_t n, uint32_t *total_dev,
-                               uint32_t *scratch, cudaStream_t st) {
-    if (n <= 0) {
-        if (total_dev) return cudaMemsetAsync(total_dev, 0, sizeof(uint32_t), st);
-        return cudaSuccess;
-    }
-    const int64_t nb = (n + kScanTile - 1) / kScanTile;
-    if (nb == 1) {
-        ++launch_counter(), scan_down_kernel<<<1, kScanThreads, 0, st>>>(in, out, n, nullptr, total_dev);
-        return cudaGetLastError();
-    }
-    uint32_t *partials = scratch;
-    uint32_t *rest = scratch + ((nb + 63) & ~int64_t(63));
-    ++launch_counter(), scan_reduce_kernel<<<(unsigned)nb, kScanThreads, 0, st>>>(in, n, partials);
-    cudaError_t e = scan_exclusive_u32(partials, partials, nb, nullptr, rest, st);
-    if (e != cudaSuccess) return e;
-    ++launch_counter(), scan_down_kernel<<<(unsigned)nb, kScanThreads, 0, st>>>(in, out, n, partials, total_dev);
-    return cudaGetLastError();
-}
-
 cudaError_t radix_sort_pairs_u32(uint32_t *k0, int32_t *v0, uint32_t *k1, int32_t *v1, int64_t n,
-                                 int bits, uint32_t *scratch, bool *result_in_first, cudaStream_t st) {
-    return radix_sort_pairs<uint32_t>(k0, v0, k1, v1, n, bits, scratch, result_in_first, st);
+                                 int bits, uint32_t *scratch, size_t zero_words, bool *result_in_first,
+                                 cudaStream_t st) {
+    return radix_sort_pairs<uint32_t>(k0, v0, k1, v1, n, bits, scratch, zero_words, result_in_first, st);
 }
 
 cudaError_t radix_sort_pairs_u64(uint64_t *k0, int32_t *v0, uint64_t *k1, int32_t *v1, int64_t n,
-                                 int bits, uint32_t *scratch, bool *result_in_first, cudaStream_t st) {
-    return radix_sort_pairs<uint64_t>(k0, v0, k1, v1, n, bits, scratch, result_in_first, st);
+                                 int bits, uint32_t *scratch, size_t zero_words, bool *result_in_first,
+                                 cudaStream_t st) {
+    return radix_sort_pairs<uint64_t>(k0, v0, k1, v1, n, bits, scratch, zero_words, result_in_first, st);
 }
 
 }  // namespace ndb

@@ -352,12 +352,13 @@ __device__ __forceinline__ int chunk_points(int cs, int ce, int p0, int chunk) {
 // first point); the others, and remainders of fewer than min_cnt points, into the exact
 // kernel's list, as items of 32 points.  Order within a list is free; the list lengths
 // land in device memory, n_items counts the 32-point items the chunks hold.
-__global__ void split_cells_kernel(const int32_t *__restrict__ cell_start, int64_t n_cells, int min_cnt, int chunk,
+__global__ void split_cells_kernel(const int32_t *__restrict__ cell_start,
+                                   const uint32_t *__restrict__ n_cells, int min_cnt, int chunk,
                                    int2 *__restrict__ chunks, uint32_t *__restrict__ n_chunks, int2 *__restrict__ rest,
                                    uint32_t *__restrict__ n_rest, uint32_t *__restrict__ n_items) {
     const int64_t c = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     int cs = 0, ce = 0;
-    if (c < n_cells) {
+    if (c < *n_cells) {
         cs = cell_start[c];
         ce = cell_start[c + 1];
     }
