@@ -550,6 +550,7 @@ void grid_phase(ndb_ctx *ctx, Pipe &p, const float *coords, F launch_keys) {
     ensure(ctx, ctx->cell_start, (n + 2) * sizeof(int32_t));
     ensure(ctx, ctx->cell_key, (n + 1) * sizeof(K));
     ensure(ctx, ctx->xs, (nv + 1) * P * sizeof(float));
+    ensure(ctx, ctx->nn_sorted, (n + 1) * sizeof(int32_t));
 
     const K invalid_key = (K)(p.key_bits >= (int)(8 * sizeof(K)) ? ~(K)0 : (((K)1 << p.key_bits) - 1));
     launch_keys(invalid_key, ctx->keys0.as<K>(), ctx->core_bits.as<uint32_t>());
@@ -577,7 +578,7 @@ void grid_phase(ndb_ctx *ctx, Pipe &p, const float *coords, F launch_keys) {
     ++launch_counter(), chain_scan_kernel<kCellsPer><<<(unsigned)chain_tiles(nv, kCellsPer), kChainThreads, 0, st>>>(
         CellsOp<D, K>{ctx->keys0.as<K>(), ctx->ids0.as<int32_t>(), coords, rows_aligned<D>(coords), nv,
                       ctx->xs.as<float>(), ctx->cell_start.as<int32_t>(), ctx->cell_key.as<K>(),
-                      ctx->pcell.as<int32_t>()},
+                      ctx->pcell.as<int32_t>(), p.early ? nullptr : ctx->nn_sorted.as<int32_t>()},
         nv, nullptr, chain.state[0], chain.ticket + 0, scal + 0, m_cells_dev);
     ck(ctx, cudaGetLastError());
     if (!p.jobs && nv <= kNoCountPoints) {
@@ -697,21 +698,23 @@ void launch_count_tc(ndb_ctx *ctx, int64_t max_chunks, const int2 *chunks, const
         if (grow(ctx, ctx->tc_rec, (size_t)max_chunks * tc::kRecBytes) == cudaSuccess) {
             rec = ctx->tc_rec.as<int2>();
             ++launch_counter(), tc::tc_records_kernel<<<blocks_for(max_chunks * kWarp), kBlock, 0, st>>>(
-                chunks, n_chunks, cell_start, nbr, n_rows, cell_job, chunk, rec);
+                chunks, n_chunks, cell_start, nbr, n_rows, cell_job, chunk, early ? 0 : 1, rec);
             ck(ctx, cudaGetLastError());
         } else {
             cudaGetLastError();  // a refused or failed allocation leaves no error behind
         }
         const unsigned grid = (unsigned)std::min<int64_t>(max_chunks, (int64_t)ctx->sm_count * tc::TcBlocks<D>::v);
-        auto launch = [&](auto audit_c) {
-            constexpr bool A = decltype(audit_c)::value;
-            ++launch_counter(), tc::count_tc_kernel<D, A><<<grid, tc::kThreads, 0, st>>>(
-                chunks, n_chunks, chunk, cell_start, nbr, n_rows, xs, e2, min_pts, early ? 1 : 0, nn_sorted, list,
-                list_cap, list_stride, counters + 2, counters + 5, work, small_at<int>(ctx, kSmallErrOff), jobs,
-                cell_job, counters + 8, rec);
+        auto launch = [&](auto full_c, auto audit_c) {
+            constexpr bool F = decltype(full_c)::value, A = decltype(audit_c)::value;
+            ++launch_counter(), tc::count_tc_kernel<D, F, A><<<grid, tc::kThreads, 0, st>>>(
+                chunks, n_chunks, chunk, cell_start, nbr, n_rows, xs, e2, min_pts, nn_sorted, list, list_cap,
+                list_stride, counters + 2, counters + 5, work, small_at<int>(ctx, kSmallErrOff), jobs, cell_job,
+                counters + 8, rec);
         };
-        if (audit) launch(std::true_type{});
-        else launch(std::false_type{});
+        using T = std::true_type;
+        using N = std::false_type;
+        if (early) audit ? launch(N{}, T{}) : launch(N{}, N{});
+        else audit ? launch(T{}, T{}) : launch(T{}, N{});
         ck(ctx, cudaGetLastError());
     } else {
         throw Fail{NDB_ERR_INVALID_ARGUMENT};
@@ -761,24 +764,25 @@ void count_items(ndb_ctx *ctx, bool tc, bool force_tc, bool gram, bool early, in
     }
     const unsigned grid = (unsigned)((n_items + kCountWarps - 1) / kCountWarps);
     // the counts on CUDA cores: the Gram-filtered kernel (d >= 8) or the exact one
-    auto launch = [&](auto early_c, auto gram_c) {
-        constexpr bool E = decltype(early_c)::value, G = decltype(gram_c)::value;
-        ++launch_counter(), count_kernel<D, E, G><<<grid, kCountWarps * kWarp, 0, st>>>(
-            ex_items, ex_n, cell_start, nbr, n_rows, xs, e2, min_pts, dense_skip, nn_sorted, list, list_cap,
-            list_stride, counters + 2, jobs, cell_job, counters + 5);
+    auto launch = [&](auto gram_c) {
+        constexpr bool G = decltype(gram_c)::value;
+        if (early)
+            ++launch_counter(), count_kernel<D, G><<<grid, kCountWarps * kWarp, 0, st>>>(
+                ex_items, ex_n, cell_start, nbr, n_rows, xs, e2, min_pts, dense_skip, nn_sorted, list, list_cap,
+                list_stride, counters + 2, jobs, cell_job, counters + 5);
+        else
+            ++launch_counter(), count_full_kernel<D, G><<<grid, kCountWarps * kWarp, 0, st>>>(
+                ex_items, ex_n, cell_start, nbr, n_rows, xs, e2, nn_sorted, list, list_cap, list_stride, counters + 2,
+                jobs, cell_job, counters + 5);
     };
-    using T = std::true_type;
-    using F = std::false_type;
     if constexpr (D >= 8) {
         if (gram) {
-            if (early) launch(T{}, T{});
-            else launch(F{}, T{});
+            launch(std::true_type{});
             ck(ctx, cudaGetLastError());
             return;
         }
     }
-    if (early) launch(T{}, F{});
-    else launch(F{}, F{});
+    launch(std::false_type{});
     ck(ctx, cudaGetLastError());
 }
 
@@ -788,7 +792,6 @@ void count_phase(ndb_ctx *ctx, const Pipe &p, bool tc, bool gram, uint32_t flags
     cudaStream_t st = ctx->stream;
     const int64_t n = p.n, n_words = (n + 31) / 32;
     uint32_t *scal = small_at<uint32_t>(ctx, kSmallScalarOff);
-    ensure(ctx, ctx->nn_sorted, (n + 1) * sizeof(int32_t));
     cudaEventRecord(ctx->kev[2], st);
     count_items<D>(ctx, tc, (flags & NDB_FLAG_TENSOR_FILTER) != 0, gram, p.early, p.items, ctx->items.as<int2>(),
                    ctx->cell_start.as<int32_t>(), ctx->nbr.as<int2>(), p.stencil->n_rows, ctx->xs.as<float>(), p.e2,
@@ -896,7 +899,7 @@ void union_phase(ndb_ctx *ctx, const Pipe &p, unsigned long long *job_counters) 
     if (p.list_stride > 0)
         ++launch_counter(), union_lists_kernel<<<blocks_for(nv), kBlock, 0, st>>>(
             nv, ctx->nn_sorted.as<int32_t>(), p.list, p.list_cap, p.list_stride, core_sorted, parent, err, p.jobs,
-            p.cell_job, pcell, p.linked, p.linked && p.early, cell_start, p.min_pts);
+            p.cell_job, pcell, p.linked, cell_start, p.min_pts);
     if (p.linked) {
         ++launch_counter(), union_near_kernel<D, K><<<blocks_for(p.cells), kBlock, 0, st>>>(
             n_cells, p.g, ctx->cell_key.as<K>(), cell_start, cell_index<K>(ctx), xs, p.e2, core_sorted, has_core,

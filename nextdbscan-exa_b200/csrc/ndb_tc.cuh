@@ -398,7 +398,7 @@ __global__ void split_cells_kernel(const int32_t *__restrict__ cell_start,
 // The records of the chunks in chunks[0, *n_chunks): one warp per chunk.
 __global__ void tc_records_kernel(const int2 *__restrict__ chunks, const uint32_t *__restrict__ n_chunks,
                                   const int32_t *__restrict__ cell_start, const int2 *__restrict__ nbr, int n_rows,
-                                  const int32_t *__restrict__ cell_job, int chunk, int2 *__restrict__ rec) {
+                                  const int32_t *__restrict__ cell_job, int chunk, int full, int2 *__restrict__ rec) {
     const int64_t w = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
     const int lane = threadIdx.x & 31;
     if (w >= (int64_t)*n_chunks) return;
@@ -408,8 +408,9 @@ __global__ void tc_records_kernel(const int2 *__restrict__ chunks, const uint32_
         const int2 cr = nbr[(int64_t)it.x * n_rows + lane];
         int2 v = make_int2(0, 0);
         if (cr.x < cr.y) {
-            const int a = cell_start[cr.x];
-            v = make_int2(a, cell_start[cr.y] - a);
+            // full counts: only the candidates at and behind the chunk's first point
+            const int a = full ? max(cell_start[cr.x], it.y) : cell_start[cr.x];
+            v = make_int2(a, max(cell_start[cr.y] - a, 0));
         }
         r[1 + lane] = v;
     }
@@ -420,12 +421,11 @@ __global__ void tc_records_kernel(const int2 *__restrict__ chunks, const uint32_
     }
 }
 
-template <int D, bool AUDIT = false>
+template <int D, bool FULL, bool AUDIT = false>
 __global__ void __launch_bounds__(kThreads, TcBlocks<D>::v) count_tc_kernel(
     const int2 *__restrict__ chunks, const uint32_t *__restrict__ n_chunks_dev, int chunk,
     const int32_t *__restrict__ cell_start, const int2 *__restrict__ nbr, int n_rows, const float *__restrict__ xs,
-    float e2, int min_pts, int early,
-    int32_t *__restrict__ nn_sorted, int32_t *__restrict__ nbr_list, int list_cap, int list_stride,
+    float e2, int min_pts, int32_t *nn_sorted, int32_t *__restrict__ nbr_list, int list_cap, int list_stride,
     unsigned long long *__restrict__ pair_counter, unsigned long long *__restrict__ band_counter,
     unsigned int *__restrict__ work, int *__restrict__ err, const JobDev *__restrict__ jobs,
     const int32_t *__restrict__ cell_job, unsigned long long *__restrict__ audit, const int2 *__restrict__ rec) {
@@ -566,7 +566,7 @@ __global__ void __launch_bounds__(kThreads, TcBlocks<D>::v) count_tc_kernel(
                 const int2 rw = lane < n_rows ? s_rec[slot][1 + lane] : make_int2(0, 0);
                 build_rows(rw.x, rw.y, n_rows, s_rt, lane);
             } else {
-                gather_rows<false>(nbr + (int64_t)cell * n_rows, n_rows, cell_start, 0, s_rt, lane);
+                gather_points_from(nbr + (int64_t)cell * n_rows, n_rows, cell_start, FULL ? p0 : 0, s_rt, lane);
             }
             s_listn[lane] = 0;
         } else if (warp == 1) {
@@ -578,6 +578,9 @@ __global__ void __launch_bounds__(kThreads, TcBlocks<D>::v) count_tc_kernel(
         const int n_tiles = (total + kM - 1) / kM;
         int run = 0, totals = 0;  // lane c: this warp's hits of column c; all warps' hits after the last tile
         int start = 0;            // lane c: the step at which column c's point joined
+        // FULL: this lane's column may still take list entries; the candidates' counts
+        bool open = nbr_list && lc > 0;
+        int had_cur = 0, had_nxt = 0;
         bool narrow = len <= kN / 2;  // the MMA computes 16 columns (N = 16)
 
         // One candidate row per thread.  fetch: the row's point index (a cursor over
@@ -585,7 +588,7 @@ __global__ void __launch_bounds__(kThreads, TcBlocks<D>::v) count_tc_kernel(
         // loaded into registers before the previous tile is processed so that the
         // load latency hides behind that work.  stage: centre, split, store.
         int row = 0;
-        auto fetch = [&](int t, int &jrow, float (&x)[D]) {
+        auto fetch = [&](int t, int &jrow, float (&x)[D], int &had) {
             const int v = t * kM + tid;
             if (t == 0) row = 0;
             jrow = -1;
@@ -593,6 +596,7 @@ __global__ void __launch_bounds__(kThreads, TcBlocks<D>::v) count_tc_kernel(
                 while (s_rt.off[row + 1] <= v) ++row;
                 jrow = s_rt.start[row] + (v - s_rt.off[row]);
                 load_point<D>(xs, jrow, x);
+                if constexpr (FULL) had = nbr_list ? __ldcg(nn_sorted + jrow) : lc;
             }
         };
         auto stage = [&](int buf, int jrow, const float (&x)[D], float &nj) {
@@ -628,7 +632,7 @@ __global__ void __launch_bounds__(kThreads, TcBlocks<D>::v) count_tc_kernel(
         int j_cur = -1, j_nxt = -1;
         float nj_cur = 0.0f, nj_nxt = 0.0f;
         float x_nxt[D];
-        fetch(0, j_cur, x_nxt);
+        fetch(0, j_cur, x_nxt, had_cur);
         stage(0, j_cur, x_nxt, nj_cur);
         fence_async_smem();
         tc_before_sync();
@@ -642,7 +646,7 @@ __global__ void __launch_bounds__(kThreads, TcBlocks<D>::v) count_tc_kernel(
         for (int step = 0, tile = 0;; ++step) {
             const int pb = step & 1;
             const int tile_nxt = tile + 1 == n_tiles ? 0 : tile + 1;
-            fetch(tile_nxt, j_nxt, x_nxt);
+            if (!FULL || tile_nxt > 0) fetch(tile_nxt, j_nxt, x_nxt, had_nxt);
             const bool ok = mbar_wait(&s_bar[pb], (phase >> pb) & 1u);
             if (ok) {
                 phase ^= 1u << pb;
@@ -685,107 +689,132 @@ __global__ void __launch_bounds__(kThreads, TcBlocks<D>::v) count_tc_kernel(
                 }
                 const unsigned cm = transpose32(hb, lane);  // rows of this warp that hit column `lane`
                 const int h = __popc(cm);
-                run += h;
-                if (nbr_list && h && totals < lc) {
-                    int slot = atomicAdd(&s_listn[lane], h);
-                    for (unsigned m = cm; m && slot < lc; m &= m - 1, ++slot)
-                        nbr_list[(int64_t)me * list_stride + slot] = s_j[pb][warp * 32 + __ffs(m) - 1];
+                if constexpr (FULL) {
+                    // a hit counts for both ends (see count_full_kernel); the columns hold
+                    // the points p0 .. p0 + len - 1 in order
+                    if (hb && j_cur >= p0 + len)
+                        add_hits(nn_sorted, nbr_list, lc, list_stride, j_cur, had_cur < lc, hb,
+                                 [&](int k) { return p0 + k; });
+                    if (h && open) {
+                        const int got = add_hits(nn_sorted, nbr_list, lc, list_stride, me, true, cm,
+                                                 [&](int k) { return s_j[pb][warp * 32 + k]; });
+                        open = got < lc;
+                    } else {
+                        run += h;
+                    }
+                } else {
+                    run += h;
+                    if (nbr_list && h && totals < lc) {
+                        int slot = atomicAdd(&s_listn[lane], h);
+                        for (unsigned m = cm; m && slot < lc; m &= m - 1, ++slot)
+                            nbr_list[(int64_t)me * list_stride + slot] = s_j[pb][warp * 32 + __ffs(m) - 1];
+                    }
+                    s_part[pb][warp][lane] = run;
                 }
-                s_part[pb][warp][lane] = run;
                 if (tid == 0) pairs += (unsigned long long)__popc(act) * (unsigned long long)min(kM, total - tile * kM);
             } else {
                 s_abort = 1;
                 atomicExch(err, 2);
             }
-            stage(pb ^ 1, j_nxt, x_nxt, nj_nxt);
+            if (!FULL || tile_nxt > 0) stage(pb ^ 1, j_nxt, x_nxt, nj_nxt);
             fence_async_smem();
             tc_before_sync();
             __syncthreads();
             tc_after_sync();
             if (s_abort) break;
-            totals = s_part[pb][0][lane] + s_part[pb][1][lane] + s_part[pb][2][lane] + s_part[pb][3][lane];
-            // columns whose point is done: at min_pts (early exit) or after a full round
-            const bool done = ((act >> lane) & 1u) && ((early && totals >= mp) || step - start + 1 >= n_tiles);
-            const unsigned fin = __ballot_sync(kFull, done);
-            if (fin) {
-                if (warp == 0 && done) nn_sorted[me] = totals;
-                const int rank = __popc(fin & lanemask_lt());
-                const bool refill = done && rank < len - next;
-                const unsigned which = __ballot_sync(kFull, refill);
-                act = (act & ~fin) | which;
-                if (!act) break;
-                if (refill) {
-                    me = p0 + next + rank;
-                    run = totals = 0;
-                    start = step + 1;
+            if constexpr (FULL) {
+                // every point needs the whole round: one tile after the other, then the
+                // hits still in registers
+                if (tile_nxt == 0) {
+                    if (run) atomicAdd(nn_sorted + me, run);
+                    break;
                 }
-                next += __popc(which);
-                // No MMA is in flight (the last one was waited for above), so the operand
-                // may be rewritten: warp 1 writes the new points' rows.
-                if (which) {
-                    if (warp == 0 && refill) s_listn[lane] = 0;
-                    if (warp == 1) fill_columns(which);
-                    __syncthreads();
-                }
-                // Packing (at most once per chunk, when the queue is empty): at most 16 columns
-                // are left, they move to the first 16 rows and the MMAs compute N = 16
-                // from then on, halving the classification.  Warp 1 moves the rows
-                // through the candidate buffer of the tile just processed (staged again
-                // only after the following barrier).
-                if (!narrow && __popc(act) <= kN / 2) {
-                    const int nk = __popc(act);
-                    const int src = lane < nk ? nth_set_bit(act, lane) : lane;
-                    run = __shfl_sync(kFull, run, src);
-                    totals = __shfl_sync(kFull, totals, src);
-                    me = __shfl_sync(kFull, me, src);
-                    start = __shfl_sync(kFull, start, src);
-                    if (warp == 0) {
-                        const int ln = s_listn[src];
-                        __syncwarp();
-                        s_listn[lane] = ln;
-                    } else if (warp == 1) {
-                        constexpr int TS = 2 * KC * 4 + P + 4;  // words per row in the buffer (16-byte multiple)
-                        uint32_t *tmp = &s_a[pb][0][0] + lane * TS;
-                        if (lane < nk) {
-#pragma unroll
-                            for (int h = 0; h < 2; ++h)
-#pragma unroll
-                                for (int q = 0; q < KC; ++q)
-                                    *reinterpret_cast<uint4 *>(tmp + (h * KC + q) * 4) =
-                                        *reinterpret_cast<const uint4 *>(&s_b[h][(q * kN + src) * 4]);
-#pragma unroll
-                            for (int q = 0; q < P / 4; ++q)
-                                *reinterpret_cast<float4 *>(tmp + 2 * KC * 4 + 4 * q) =
-                                    *reinterpret_cast<const float4 *>(&s_x[src * P + 4 * q]);
-                            tmp[2 * KC * 4 + P] = __float_as_uint(s_ni[src]);
-                            tmp[2 * KC * 4 + P + 1] = __float_as_uint(s_nneg[src]);
-                        }
-                        __syncwarp();
-                        if (lane < nk) {
-#pragma unroll
-                            for (int h = 0; h < 2; ++h)
-#pragma unroll
-                                for (int q = 0; q < KC; ++q)
-                                    *reinterpret_cast<uint4 *>(&s_b[h][(q * kN + lane) * 4]) =
-                                        *reinterpret_cast<const uint4 *>(tmp + (h * KC + q) * 4);
-#pragma unroll
-                            for (int q = 0; q < P / 4; ++q)
-                                *reinterpret_cast<float4 *>(&s_x[lane * P + 4 * q]) =
-                                    *reinterpret_cast<const float4 *>(tmp + 2 * KC * 4 + 4 * q);
-                            s_ni[lane] = __uint_as_float(tmp[2 * KC * 4 + P]);
-                            s_nneg[lane] = __uint_as_float(tmp[2 * KC * 4 + P + 1]);
-                            fence_async_smem();
-                        }
+            } else {
+                totals = s_part[pb][0][lane] + s_part[pb][1][lane] + s_part[pb][2][lane] + s_part[pb][3][lane];
+                // columns whose point is done: at min_pts or after a full round
+                const bool done = ((act >> lane) & 1u) && (totals >= mp || step - start + 1 >= n_tiles);
+                const unsigned fin = __ballot_sync(kFull, done);
+                if (fin) {
+                    if (warp == 0 && done) nn_sorted[me] = totals;
+                    const int rank = __popc(fin & lanemask_lt());
+                    const bool refill = done && rank < len - next;
+                    const unsigned which = __ballot_sync(kFull, refill);
+                    act = (act & ~fin) | which;
+                    if (!act) break;
+                    if (refill) {
+                        me = p0 + next + rank;
+                        run = totals = 0;
+                        start = step + 1;
                     }
-                    narrow = true;
-                    act = (1u << nk) - 1u;
-                    __syncthreads();
+                    next += __popc(which);
+                    // No MMA is in flight (the last one was waited for above), so the operand
+                    // may be rewritten: warp 1 writes the new points' rows.
+                    if (which) {
+                        if (warp == 0 && refill) s_listn[lane] = 0;
+                        if (warp == 1) fill_columns(which);
+                        __syncthreads();
+                    }
+                    // Packing (at most once per chunk, when the queue is empty): at most 16 columns
+                    // are left, they move to the first 16 rows and the MMAs compute N = 16
+                    // from then on, halving the classification.  Warp 1 moves the rows
+                    // through the candidate buffer of the tile just processed (staged again
+                    // only after the following barrier).
+                    if (!narrow && __popc(act) <= kN / 2) {
+                        const int nk = __popc(act);
+                        const int src = lane < nk ? nth_set_bit(act, lane) : lane;
+                        run = __shfl_sync(kFull, run, src);
+                        totals = __shfl_sync(kFull, totals, src);
+                        me = __shfl_sync(kFull, me, src);
+                        start = __shfl_sync(kFull, start, src);
+                        if (warp == 0) {
+                            const int ln = s_listn[src];
+                            __syncwarp();
+                            s_listn[lane] = ln;
+                        } else if (warp == 1) {
+                            constexpr int TS = 2 * KC * 4 + P + 4;  // words per row in the buffer (16-byte multiple)
+                            uint32_t *tmp = &s_a[pb][0][0] + lane * TS;
+                            if (lane < nk) {
+#pragma unroll
+                                for (int h = 0; h < 2; ++h)
+#pragma unroll
+                                    for (int q = 0; q < KC; ++q)
+                                        *reinterpret_cast<uint4 *>(tmp + (h * KC + q) * 4) =
+                                            *reinterpret_cast<const uint4 *>(&s_b[h][(q * kN + src) * 4]);
+#pragma unroll
+                                for (int q = 0; q < P / 4; ++q)
+                                    *reinterpret_cast<float4 *>(tmp + 2 * KC * 4 + 4 * q) =
+                                        *reinterpret_cast<const float4 *>(&s_x[src * P + 4 * q]);
+                                tmp[2 * KC * 4 + P] = __float_as_uint(s_ni[src]);
+                                tmp[2 * KC * 4 + P + 1] = __float_as_uint(s_nneg[src]);
+                            }
+                            __syncwarp();
+                            if (lane < nk) {
+#pragma unroll
+                                for (int h = 0; h < 2; ++h)
+#pragma unroll
+                                    for (int q = 0; q < KC; ++q)
+                                        *reinterpret_cast<uint4 *>(&s_b[h][(q * kN + lane) * 4]) =
+                                            *reinterpret_cast<const uint4 *>(tmp + (h * KC + q) * 4);
+#pragma unroll
+                                for (int q = 0; q < P / 4; ++q)
+                                    *reinterpret_cast<float4 *>(&s_x[lane * P + 4 * q]) =
+                                        *reinterpret_cast<const float4 *>(tmp + 2 * KC * 4 + 4 * q);
+                                s_ni[lane] = __uint_as_float(tmp[2 * KC * 4 + P]);
+                                s_nneg[lane] = __uint_as_float(tmp[2 * KC * 4 + P + 1]);
+                                fence_async_smem();
+                            }
+                        }
+                        narrow = true;
+                        act = (1u << nk) - 1u;
+                        __syncthreads();
+                    }
                 }
             }
             if (tid == 0) issue(pb ^ 1);
             pending |= 1u << (pb ^ 1);
             j_cur = j_nxt;
             nj_cur = nj_nxt;
+            had_cur = had_nxt;
             tile = tile_nxt;
         }
         if (s_abort) break;
