@@ -660,6 +660,12 @@ inline bool gram_eligible(const ndb_ctx *ctx, int d, float e2, const double *lo,
     return true;
 }
 
+// The FMA sum with the exact one near eps^2 (count_kernel, kDirect): not the plain form,
+// and eps^2 far enough from underflow for its error bound.
+inline bool direct_eligible(float e2, uint32_t flags) {
+    return !(flags & NDB_FLAG_EXACT_COUNT) && e2 >= 0x1p-100f;
+}
+
 // Which items the tensor kernel takes: it stages every candidate row once per item
 // and most of its per-tile epilogue is fixed, so it pays only for full items (many
 // points of one cell).  Measured on B200: with about 11 points per item the exact
@@ -737,7 +743,7 @@ inline int tc_chunk(const ndb_ctx *ctx, int64_t nv, bool early) {
 // eligible); then the cells are split by size and each list goes to its kernel,
 // both launched at the upper bound and reading their list length on the device.
 template <int D>
-void count_items(ndb_ctx *ctx, bool tc, bool force_tc, bool gram, bool early, int64_t n_items, const int2 *items,
+void count_items(ndb_ctx *ctx, bool tc, bool force_tc, bool gram, bool direct, bool early, int64_t n_items, const int2 *items,
                  const int32_t *cell_start, const int2 *nbr, int n_rows, const float *xs, float e2, int min_pts,
                  int dense_skip, int32_t *nn_sorted, int32_t *list, int list_cap, int list_stride,
                  const JobDev *jobs, const int32_t *cell_job, bool audit, int64_t nv, int64_t n_cells) {
@@ -763,37 +769,43 @@ void count_items(ndb_ctx *ctx, bool tc, bool force_tc, bool gram, bool early, in
         ex_n = scal + 5;
     }
     const unsigned grid = (unsigned)((n_items + kCountWarps - 1) / kCountWarps);
-    // the counts on CUDA cores: the Gram-filtered kernel (d >= 8) or the exact one
-    auto launch = [&](auto gram_c) {
-        constexpr bool G = decltype(gram_c)::value;
+    // the counts on CUDA cores: the Gram-filtered kernel (d >= 8), the FMA sum with the
+    // exact one near eps^2 (d >= 4, eps^2 far from underflow), or the exact sum alone
+    auto launch = [&](auto mode_c) {
+        constexpr int M = decltype(mode_c)::value;
         if (early)
-            ++launch_counter(), count_kernel<D, G><<<grid, kCountWarps * kWarp, 0, st>>>(
+            ++launch_counter(), count_kernel<D, M><<<grid, kCountWarps * kWarp, 0, st>>>(
                 ex_items, ex_n, cell_start, nbr, n_rows, xs, e2, min_pts, dense_skip, nn_sorted, list, list_cap,
                 list_stride, counters + 2, jobs, cell_job, counters + 5);
         else
-            ++launch_counter(), count_full_kernel<D, G><<<grid, kCountWarps * kWarp, 0, st>>>(
+            ++launch_counter(), count_full_kernel<D, M><<<grid, kCountWarps * kWarp, 0, st>>>(
                 ex_items, ex_n, cell_start, nbr, n_rows, xs, e2, nn_sorted, list, list_cap, list_stride, counters + 2,
                 jobs, cell_job, counters + 5);
     };
     if constexpr (D >= 8) {
         if (gram) {
-            launch(std::true_type{});
+            launch(std::integral_constant<int, kGram>{});
             ck(ctx, cudaGetLastError());
             return;
         }
     }
-    launch(std::false_type{});
+    if constexpr (D >= 4) {
+        if (direct) launch(std::integral_constant<int, kDirect>{});
+        else launch(std::integral_constant<int, kExact>{});
+    } else {
+        launch(std::integral_constant<int, kExact>{});
+    }
     ck(ctx, cudaGetLastError());
 }
 
 // Neighbour counts and core flags of a pipeline.
 template <int D, typename K>
-void count_phase(ndb_ctx *ctx, const Pipe &p, bool tc, bool gram, uint32_t flags) {
+void count_phase(ndb_ctx *ctx, const Pipe &p, bool tc, bool gram, bool direct, uint32_t flags) {
     cudaStream_t st = ctx->stream;
     const int64_t n = p.n, n_words = (n + 31) / 32;
     uint32_t *scal = small_at<uint32_t>(ctx, kSmallScalarOff);
     cudaEventRecord(ctx->kev[2], st);
-    count_items<D>(ctx, tc, (flags & NDB_FLAG_TENSOR_FILTER) != 0, gram, p.early, p.items, ctx->items.as<int2>(),
+    count_items<D>(ctx, tc, (flags & NDB_FLAG_TENSOR_FILTER) != 0, gram, direct, p.early, p.items, ctx->items.as<int2>(),
                    ctx->cell_start.as<int32_t>(), ctx->nbr.as<int2>(), p.stencil->n_rows, ctx->xs.as<float>(), p.e2,
                    p.min_pts, p.linked, ctx->nn_sorted.as<int32_t>(), p.list, p.list_cap, p.list_stride, p.jobs,
                    p.cell_job, (flags & NDB_FLAG_FILTER_AUDIT) != 0, p.nv, p.cells);
@@ -833,7 +845,7 @@ void classify_keys(ndb_ctx *ctx, Pipe &p) {
     }
     ctx->list_cap = p.list_cap;
     cudaEventRecord(ctx->ev[1], st);
-    count_phase<D, K>(ctx, p, ctx->tc_count, ctx->gram_count, ctx->flags_run);
+    count_phase<D, K>(ctx, p, ctx->tc_count, ctx->gram_count, direct_eligible(ctx->e2, ctx->flags_run), ctx->flags_run);
     cudaEventRecord(ctx->ev[2], st);
 }
 
@@ -1714,6 +1726,7 @@ struct BatchPlan {
     int list_stride = 0;
     bool tc = false;  // neighbour count on the tensor-core filter (every job eligible)
     bool gram = true; // CUDA-core count with the Gram filter (every job eligible)
+    bool direct = true;  // the FMA sum (every job eligible)
     int64_t total_n = 0, nv = 0;
     double columns = 0;  // entries of the pipeline's column table (sum over its jobs)
 };
@@ -1753,7 +1766,7 @@ void run_group_keys(ndb_ctx *ctx, ndb_job *jobs, const std::vector<int> &members
         p.list_stride = bp.list_stride;
     }
     cudaEventRecord(ctx->ev[1], st);
-    count_phase<D, K>(ctx, p, bp.tc, bp.gram, flags);
+    count_phase<D, K>(ctx, p, bp.tc, bp.gram, bp.direct, flags);
     cudaEventRecord(ctx->ev[2], st);
 
     // union-find, canonical ids, border points
@@ -1938,6 +1951,7 @@ void run_group(ndb_ctx *ctx, ndb_job *jobs, const std::vector<int> &members, uin
         }
         kept.push_back(members[m]);
         bp.gram = bp.gram && job_gram;
+        bp.direct = bp.direct && direct_eligible(jd.e2, flags);
         if (!have_stencil) {
             bp.st = pl.st;
             bp.tc = job_tc;

@@ -723,6 +723,28 @@ __device__ __forceinline__ float dist_negated(const float (&x)[D], const float (
     return len;
 }
 
+// The squared distance by FMAs (b negated), two chains joined by one addition: within
+// (D + 2) u of the real one, like the reference's sum, so the two decide a pair alike
+// unless |e2 - dist_fma| <= direct_gamma e2 (u = 2^-24; derivation at count_kernel).
+template <int D>
+__device__ __forceinline__ float dist_fma(const float (&x)[D], const float (&nb)[D]) {
+    float2 acc = make_float2(0.0f, 0.0f);
+#pragma unroll
+    for (int k = 0; k + 1 < D; k += 2) {
+        const float2 t = __fadd2_rn(make_float2(x[k], x[k + 1]), make_float2(nb[k], nb[k + 1]));
+        acc = k ? __ffma2_rn(t, t, acc) : __fmul2_rn(t, t);
+    }
+    if constexpr (D & 1) {
+        const float t = __fadd_rn(x[D - 1], nb[D - 1]);
+        acc.x = __fmaf_rn(t, t, acc.x);
+    }
+    return __fadd_rn(acc.x, acc.y);
+}
+template <int D>
+__host__ __device__ constexpr float direct_gamma() {
+    return 2.0f * (D + 8) * (1.0f / 16777216.0f);
+}
+
 // 32x32 bit-matrix transpose across a warp: lane l holds row l (bit c = column
 // c) on entry and column l (bit r = row r) on return.  Step j exchanges the
 // off-diagonal j x j blocks.  ROTATE: a lane takes its partner's word rotated by j
@@ -762,6 +784,20 @@ __device__ __forceinline__ float gram_value(const float (&a)[D], float na, const
     return __fadd_rn(v2.x, v2.y);
 }
 
+// kDirect: the out-of-range bits of a lane's candidates by the reference's sum (rare).
+template <int D, int CH>
+__device__ __forceinline__ void recheck_exact(const float *si, int nk, const float (&xj)[CH][D], float e2,
+                                           unsigned (&miss)[CH]) {
+    constexpr int P = Stride<D>::P;
+    for (int c = 0; c < CH; ++c) miss[c] = 0;
+    for (int k = nk - 1; k >= 0; --k) {
+        float xi[D];
+        load_point_smem<D>(si + k * P, xi);
+#pragma unroll
+        for (int c = 0; c < CH; ++c) miss[c] = push_sign(miss[c], __fsub_rn(e2, dist_negated<D>(xj[c], xi)));
+    }
+}
+
 // Full counts: adds the hits in m to point p's count; with `list`, the old count owns the
 // list slots from there on, and those below list_cap are written (other(bit): the point
 // at the other end).  Returns the count after the addition when it was asked for.
@@ -794,7 +830,21 @@ __device__ __forceinline__ int gather_points_from(const int2 *__restrict__ nbr_r
     return build_rows(start, len, n_rows, rt, lane);
 }
 
-template <int D, bool GRAM = false>
+// How a pair is decided (results never depend on it):
+//   kExact   the reference's sum
+//   kDirect  dist_fma against e2; when one of a lane's pairs of the step falls within
+//            direct_gamma e2 of e2, the lane decides the step's pairs by the reference's sum
+//   kGram    centred dot products with a guard band (d >= 8, see above)
+// kDirect: let S be the real squared distance of the FP32 points.  Both sums consist of
+// rounded differences, squares and at most D additions of non-negative terms, so both are
+// within (D + 2) u S of S (and of underflow, below 2^-140, which e2 >= 2^-100 hides).  If
+// the FMA sum is below e2 - w or above e2 + w with w >= 2 (D + 3) u e2 / (1 - 2 (D + 3) u),
+// the reference's sum lies on the same side; direct_gamma is 2 (D + 8) u.  It costs 2 d + 1
+// operations on the FMA pipe against 3 d (8-D 2M early exit 2.63 -> 2.29 ms, 16-D 200k 1.38
+// -> 1.28 ms).  Used for d >= 4; below, the sum is short.
+constexpr int kExact = 0, kDirect = 1, kGram = 2;
+
+template <int D, int MODE>
 __global__ void __launch_bounds__(kCountWarps * kWarp) count_kernel(
     const int2 *__restrict__ items, const uint32_t *__restrict__ n_items, const int32_t *__restrict__ cell_start,
     const int2 *__restrict__ nbr, int n_rows, const float *__restrict__ xs, float e2, int min_pts,
@@ -802,6 +852,7 @@ __global__ void __launch_bounds__(kCountWarps * kWarp) count_kernel(
     int list_stride, unsigned long long *__restrict__ pair_counter, const JobDev *__restrict__ jobs,
     const int32_t *__restrict__ cell_job, unsigned long long *__restrict__ band_counter) {
     constexpr int P = Stride<D>::P;
+    constexpr bool GRAM = MODE == kGram;
     static_assert(!GRAM || D >= 8, "the Gram filter is built for d >= 8");
     // d >= 8: each lane holds two candidates per step (64 per warp), so an owned
     // point is read from shared memory once per two pairs and the two distance sums
@@ -876,6 +927,7 @@ __global__ void __launch_bounds__(kCountWarps * kWarp) count_kernel(
         float xj[CH][D];  // GRAM: -2 times the centred candidate b = x_j - o
         float tlo[CH], thi[CH];
         unsigned miss[CH], over[CH];  // bit k: out of range; GRAM: above the hit bound, above the miss bound
+        float near = INFINITY;        // kDirect: smallest distance of a pair's sum from e2
 #pragma unroll
         for (int c = 0; c < CH; ++c) {
             const int t = tb + c * kWarp + lane;
@@ -917,10 +969,15 @@ __global__ void __launch_bounds__(kCountWarps * kWarp) count_kernel(
                 // coordinates in the grid are finite, so len is never NaN)
 #pragma unroll
                 for (int c = 0; c < CH; ++c) {
-                    const float len = dist_negated<D>(xj[c], xi);
-                    miss[c] = push_sign(miss[c], __fsub_rn(e2, len));
+                    const float len = MODE == kDirect ? dist_fma<D>(xj[c], xi) : dist_negated<D>(xj[c], xi);
+                    const float d = __fsub_rn(e2, len);
+                    miss[c] = push_sign(miss[c], d);
+                    if constexpr (MODE == kDirect) near = fminf(near, fabsf(d));
                 }
             }
+        }
+        if constexpr (MODE == kDirect) {
+            if (near <= __fmul_rn(e2, direct_gamma<D>())) recheck_exact<D, CH>(si, nk, xj, e2, miss);
         }
         pairs += (unsigned long long)nk * (unsigned long long)min(kWarp * CH, total - tb);
         const unsigned slots = kFull >> (kWarp - nk);  // nk >= 1
@@ -1024,7 +1081,7 @@ __global__ void __launch_bounds__(kCountWarps * kWarp) count_kernel(
 // ms, 3-D 1M 0.88 -> 0.51 ms, 2-D 100k 0.19 -> 0.11 ms; with the tensor-core count
 // (count_tc_kernel<D, true>, the same rule) 8-D 2M 9.1 -> 5.0 ms.
 // ---------------------------------------------------------------------------
-template <int D, bool GRAM = false>
+template <int D, int MODE>
 __global__ void __launch_bounds__(kCountWarps * kWarp) count_full_kernel(
     const int2 *__restrict__ items, const uint32_t *__restrict__ n_items, const int32_t *__restrict__ cell_start,
     const int2 *__restrict__ nbr, int n_rows, const float *__restrict__ xs, float e2, int32_t *nn_sorted,
@@ -1032,6 +1089,7 @@ __global__ void __launch_bounds__(kCountWarps * kWarp) count_full_kernel(
     const JobDev *__restrict__ jobs, const int32_t *__restrict__ cell_job,
     unsigned long long *__restrict__ band_counter) {
     constexpr int P = Stride<D>::P;
+    constexpr bool GRAM = MODE == kGram;
     static_assert(!GRAM || D >= 8, "the Gram filter is built for d >= 8");
     constexpr int CH = 2;  // candidates per lane and step: an owned point is read once per two pairs
     __shared__ __align__(16) float s_i[kCountWarps][kTile * P];
@@ -1097,6 +1155,7 @@ __global__ void __launch_bounds__(kCountWarps * kWarp) count_full_kernel(
         float xj[CH][D];  // GRAM: -2 times the centred candidate b = x_j - o
         float tlo[CH], thi[CH];
         unsigned miss[CH], over[CH];  // bit k: out of range; GRAM: above the hit bound, above the miss bound
+        float near = INFINITY;        // kDirect: smallest distance of a pair's sum from e2
 #pragma unroll
         for (int c = 0; c < CH; ++c) {
             const int t = tb + c * kWarp + lane;
@@ -1135,9 +1194,16 @@ __global__ void __launch_bounds__(kCountWarps * kWarp) count_full_kernel(
                 float xi[D];
                 load_point_smem<D>(si + k * P, xi);
 #pragma unroll
-                for (int c = 0; c < CH; ++c)
-                    miss[c] = push_sign(miss[c], __fsub_rn(e2, dist_negated<D>(xj[c], xi)));
+                for (int c = 0; c < CH; ++c) {
+                    const float len = MODE == kDirect ? dist_fma<D>(xj[c], xi) : dist_negated<D>(xj[c], xi);
+                    const float d = __fsub_rn(e2, len);
+                    miss[c] = push_sign(miss[c], d);
+                    if constexpr (MODE == kDirect) near = fminf(near, fabsf(d));
+                }
             }
+        }
+        if constexpr (MODE == kDirect) {
+            if (near <= __fmul_rn(e2, direct_gamma<D>())) recheck_exact<D, CH>(si, cnt, xj, e2, miss);
         }
         pairs += (unsigned long long)cnt * (unsigned long long)min(kWarp * CH, total - tb);
         unsigned hb[CH];

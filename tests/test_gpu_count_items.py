@@ -43,3 +43,20 @@ def test_count_items_against_oracle(ctx, d, form):
                 np.testing.assert_array_equal(np.minimum(nn, m), np.minimum(nn_o, m))
             np.testing.assert_array_equal(ci, ci_o)
             assert (r.clusters, r.noise, r.core_count) == (meta["clusters"], meta["noise"], meta["cores"])
+
+
+@pytest.mark.parametrize("d", [4, 5, 6, 7, 8, 11, 16])
+@pytest.mark.parametrize("eps", [1.0, 2.0])
+def test_pairs_exactly_at_eps(ctx, d, eps):
+    """Integer points: most pairs near eps are exactly at eps, where the FMA sum leaves the
+    decision to the reference's sum; half of them moved by a few ulp to either side."""
+    rng = np.random.default_rng(d)
+    x = rng.integers(0, 3, (3000, d)).astype(np.float32)
+    x[::2] += (rng.integers(-2, 3, x[::2].shape) * np.float32(2.0 ** -23)).astype(np.float32)
+    for m in (2, 9, 40):
+        nn_o, ci_o, meta = oracle.grid(x, eps, m)
+        for full in (True, False):
+            nn, ci, r = ctx.run(x, eps, m, full_count=full)
+            np.testing.assert_array_equal(nn if full else np.minimum(nn, m), nn_o if full else np.minimum(nn_o, m))
+            np.testing.assert_array_equal(ci, ci_o)
+            assert (r.clusters, r.noise, r.core_count) == (meta["clusters"], meta["noise"], meta["cores"])
