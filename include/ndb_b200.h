@@ -241,8 +241,9 @@ ndb_status ndb_b200_set_memory_limit(ndb_ctx *ctx, int64_t max_bytes);
  * library's default.  No counterpart in the reference, whose count has one form.
  *   tc_min_dim   smallest d at which the count may run on the tensor-core filter
  *                (clamped to >= 8).  Default: 8 with NDB_FLAG_FULL_COUNT, 12 with the
- *                early exit (or the NDB_TC_MIN_DIM environment variable); a value
- *                above 16 keeps every count on the exact kernel.
+ *                early exit (or the NDB_TC_MIN_DIM environment variable), there only
+ *                for runs of at least 2^24 points; a value above 16 keeps every count
+ *                off the tensor cores.
  *   tc_min_item  smallest item (points of one cell, up to 32) the tensor-core filter
  *                takes; smaller items go to the exact kernel.  Default 16 (or
  *                NDB_TC_MIN_ITEM); above 32 sends every item to the exact kernel.

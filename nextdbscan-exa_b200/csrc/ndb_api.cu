@@ -660,6 +660,18 @@ inline bool gram_eligible(const ndb_ctx *ctx, int d, float e2, const double *lo,
     return true;
 }
 
+// Whether an eligible pipeline of nv points takes the tensor-core filter.  Full counts do.
+// With early exit the CUDA-core count, whose cost follows the points still counting, is
+// faster until a pipeline has thousands of full chunks per CTA: 16-D 200k 1.05 against 1.28
+// ms, 16-D 1M 14.1 against 16.8 ms, 12-D 1M 6.7 against 9.5 ms, a 512-job batch (5M points
+// at d = 16) 13.9 against 14.5 ms; the 4,096-job batch (40M) 122 against 116 ms.  A caller's
+// flag or tuning decides alone.
+constexpr int64_t kTcEarlyPoints = int64_t(1) << 24;
+inline bool tc_pays(const ndb_ctx *ctx, int64_t nv, uint32_t flags) {
+    return (flags & (NDB_FLAG_FULL_COUNT | NDB_FLAG_TENSOR_FILTER)) || ctx->tuning.tc_min_dim > 0 ||
+           nv >= kTcEarlyPoints || getenv("NDB_TC_MIN_DIM") != nullptr;
+}
+
 // The FMA sum with the exact one near eps^2 (count_kernel, kDirect): not the plain form,
 // and eps^2 far enough from underflow for its error bound.
 inline bool direct_eligible(float e2, uint32_t flags) {
@@ -1159,7 +1171,8 @@ ndb_status classify_impl(ndb_ctx *ctx, const float *coords, int64_t n, float eps
     ctx->n_rows = pl.st.n_rows;
     ctx->cell_units = pl.cell_units ? 1 : 0;
     if (pl.st.n_rows > kWarp) return NDB_ERR_INVALID_ARGUMENT;  // row tables hold one row per lane
-    ctx->tc_count = tc_eligible(ctx, D, ctx->e2, lo, hi, pl.cell_units, pl.st.n_rows, flags);
+    ctx->tc_count = tc_eligible(ctx, D, ctx->e2, lo, hi, pl.cell_units, pl.st.n_rows, flags) &&
+                    tc_pays(ctx, ctx->nv, flags);
     ctx->gram_count = gram_eligible(ctx, D, ctx->e2, lo, hi, flags);
 
     classify_dispatch<D>(ctx, pl);
@@ -1972,6 +1985,7 @@ void run_group(ndb_ctx *ctx, ndb_job *jobs, const std::vector<int> &members, uin
         return;
     }
     bp.nv = nv;
+    bp.tc = bp.tc && tc_pays(ctx, nv, flags);
     // the all-ones key of invalid points must exceed every composite key
     int bits = 1;
     while (bits < 64 && ldexp(1.0, bits) - 1.0 < (double)key_base) ++bits;
