@@ -403,21 +403,24 @@ __global__ void col_range_kernel(const K *__restrict__ cell_key, const uint32_t 
     if (c == n_cells - 1 || global_column(cell_key, c + 1, g_one, jobs, cell_job) != mine) col[mine].y = (int)(c + 1);
 }
 
-// First cell of column range cr whose key is >= rowkey + x (cr.y when none); the
-// column's cells have keys rowkey + x' with strictly increasing x'.  A column
-// without gaps places it directly: position first + (x - x_first).
+// First cell of column range cr whose key is >= key (cr.y when none); the column's cells
+// have strictly increasing keys.  A column without gaps places it directly: first +
+// (key - first key).
 template <typename K>
-__device__ __forceinline__ int col_lower(const K *__restrict__ cell_key, int2 cr, unsigned long long rowkey,
-                                         long long x) {
+__device__ __forceinline__ int col_lower(const K *__restrict__ cell_key, int2 cr, K key) {
     if (cr.x >= cr.y) return cr.y;
-    const long long xf = (long long)((unsigned long long)__ldg(cell_key + cr.x) - rowkey);
-    if (x <= xf) return cr.x;
-    const long long p = cr.x + (x - xf);  // keys grow by >= 1 per cell: key[p] >= rowkey + x
-    if (p < cr.y && (unsigned long long)__ldg(cell_key + p) == rowkey + (unsigned long long)x) return (int)p;
-    int lo = cr.x + 1, hi = (int)(p < cr.y ? p : cr.y);
+    const K kf = __ldg(cell_key + cr.x);
+    if (key <= kf) return cr.x;
+    const K d = key - kf;  // keys grow by >= 1 per cell: cell_key[cr.x + d] >= key
+    int hi = cr.y;
+    if (d < (K)(cr.y - cr.x)) {
+        hi = cr.x + (int)d;
+        if (__ldg(cell_key + hi) == key) return hi;
+    }
+    int lo = cr.x + 1;
     while (lo < hi) {
         const int mid = (lo + hi) >> 1;
-        if ((unsigned long long)__ldg(cell_key + mid) < rowkey + (unsigned long long)x) lo = mid + 1;
+        if (__ldg(cell_key + mid) < key) lo = mid + 1;
         else hi = mid;
     }
     return lo;
@@ -430,8 +433,8 @@ __device__ __forceinline__ int find_cell(const CellIndex<K> &L, const K *__restr
     const unsigned long long key = rowkey + (unsigned long long)x;
     if (!L.col) return hash_find(L.hkeys, L.hvals, L.mask, key);
     const int2 cr = __ldg(L.col + ncol);
-    const int a = col_lower(cell_key, cr, rowkey, x);
-    return a < cr.y && (unsigned long long)__ldg(cell_key + a) == key ? a : -1;
+    const int a = col_lower(cell_key, cr, (K)key);
+    return a < cr.y && __ldg(cell_key + a) == (K)key ? a : -1;
 }
 
 // nbr[c * n_rows + r] = [first, last) cell index of row r around cell c: the cells
@@ -460,37 +463,18 @@ __device__ __forceinline__ void decode_key(K key, const GridDev &g, long long (&
 // nbr[c * n_rows + r] = [first, last) cell index of row r around cell c: the cells
 // of a row have consecutive keys, so the existing ones are consecutive in the
 // sorted cell list and the range runs from the smallest to the largest found.
-// Cell coordinates from a key (x fastest); 32-bit arithmetic for 32-bit keys.
-template <typename K>
-__device__ __forceinline__ void decode_key(K key, const GridDev &g, long long &x, long long &y, long long &z) {
-    if constexpr (sizeof(K) == 4) {
-        const uint32_t g0 = (uint32_t)g.g[0], g1 = (uint32_t)g.g[1];
-        const uint32_t rest = (uint32_t)key / g0;
-        x = (long long)((uint32_t)key - rest * g0);
-        y = g.k >= 3 ? (long long)(rest % g1) : (long long)rest;
-        z = g.k >= 3 ? (long long)(rest / g1) : 0;
-    } else {
-        const unsigned long long g0 = (unsigned long long)g.g[0], g1 = (unsigned long long)g.g[1];
-        const unsigned long long rest = (unsigned long long)key / g0;
-        x = (long long)((unsigned long long)key - rest * g0);
-        y = g.k >= 3 ? (long long)(rest % g1) : (long long)rest;
-        z = g.k >= 3 ? (long long)(rest / g1) : 0;
-    }
-}
-
-// nbr[c * n_rows + r] = [first, last) cell index of row r around cell c: the cells
-// of a row have consecutive keys, so the existing ones are consecutive in the
-// sorted cell list and the range runs from the smallest to the largest found.
-// One thread per cell (one key decode); the first hash probes of a row's cells
-// are issued together.
+// One lane per (cell, row): 2^group_log2 lanes (>= n_rows) per cell, so a cell's rows
+// are looked up in parallel and its row table is written at once.  Bound: instruction
+// issue, so keys, coordinates and columns are computed in the key's own width (a row's
+// key and column are the cell's plus the row's offsets; a coordinate below zero wraps
+// and fails the bound): against 64-bit arithmetic throughout the grid phase of 3-D 10M
+// takes 1.10 instead of 1.24 ms, of the 4,096-job batch 20.4 instead of 23.4 ms.
 template <typename K>
 __global__ void __launch_bounds__(kBlock) rows_kernel(const K *__restrict__ cell_key,
                                                       const uint32_t *__restrict__ n_cells_dev, GridDev g_one,
-                                                      Stencil stencil, int group_log2, CellIndex<K> L, int2 *__restrict__ nbr,
-                                                      const JobDev *__restrict__ jobs,
+                                                      Stencil stencil, int group_log2, CellIndex<K> L,
+                                                      int2 *__restrict__ nbr, const JobDev *__restrict__ jobs,
                                                       const int32_t *__restrict__ cell_job) {
-    // one lane per (cell, row): 2^group_log2 lanes (>= n_rows) per cell, so
-    // a cell's rows are looked up in parallel and its row table is written at once
     __shared__ int4 s_rows[kMaxRows];
     const int n_rows = stencil.n_rows;
     for (int r = threadIdx.x; r < n_rows; r += blockDim.x) s_rows[r] = stencil.rows[r];
@@ -499,61 +483,68 @@ __global__ void __launch_bounds__(kBlock) rows_kernel(const K *__restrict__ cell
     const int64_t c = gid >> group_log2, n_cells = *n_cells_dev;
     const int r = (int)(gid & ((1 << group_log2) - 1));
     if (c >= n_cells || r >= n_rows) return;
-    unsigned long long key_base = 0;
-    long long col_base = 0;
-    GridDev g = g_one;
-    if (jobs) {
-        const JobDev &J = jobs[cell_job[c]];
-        g = J.g;
-        key_base = J.key_base;
-        col_base = J.col_base;
-    }
-    long long cc[kMaxGridDims];
-    decode_key<K>((K)((unsigned long long)cell_key[c] - key_base), g, cc);
+    const JobDev *J = jobs ? jobs + cell_job[c] : nullptr;
+    const GridDev &g = J ? J->g : g_one;
+    const K key_base = J ? (K)J->key_base : (K)0;
+    const long long col_base = J ? J->col_base : 0;
     const int4 row = s_rows[r];
     const int off[kMaxGridDims] = {0, row.x, row.y, row.z};
+    const K local = cell_key[c] - key_base, g0 = (K)g.g[0];
+    K rest = local / g0;
+    const K x = local - rest * g0;
+    K base = cell_key[c] - x;  // key of x = 0 in the row's column
+    K col = rest, cstride = 1;
     bool in = true;
-    unsigned long long base = key_base;
-    long long ncol = 0, cstride = 1;  // the row's column: cells differing only in dimension 0
 #pragma unroll
     for (int a = 1; a < kMaxGridDims; ++a) {
         if (a < g.k) {
-            const long long v = cc[a] + off[a];
-            in = in && v >= 0 && v < g.g[a];
-            base += (unsigned long long)(v < 0 ? 0 : v) * g.stride[a];
-            ncol += (v < 0 ? 0 : v) * cstride;
-            cstride *= g.g[a];
+            const K ga = (K)g.g[a];
+            K q = 0, v = rest;
+            if (a < g.k - 1) {
+                q = rest / ga;
+                v = rest - q * ga;
+            }
+            rest = q;
+            const K o = (K)(long long)off[a];
+            in = in && (K)(v + o) < ga;
+            base += o * (K)g.stride[a];
+            col += o * cstride;
+            cstride *= ga;
         }
     }
     int2 res = make_int2(0, 0);
     if (in) {
-        const long long x0 = cc[0] - row.w < 0 ? 0 : cc[0] - row.w;
-        const long long x1 = cc[0] + row.w > g.g[0] - 1 ? g.g[0] - 1 : cc[0] + row.w;
+        const K w = (K)row.w;
+        const K x0 = x < w ? (K)0 : x - w, x1 = x + w > g0 - 1 ? g0 - 1 : x + w;
+        const K kmax = base + x1;
         // the row's existing cells are consecutive in the sorted cell list: find the
         // first one (a column-table search, or hashing from x0 on), then count the
         // keys that follow it within the row (independent loads, at most 2 row.w)
         int ca = -1;
         if (L.col) {
-            const int2 cr = __ldg(L.col + col_base + ncol);
-            const int a = col_lower(cell_key, cr, base, x0);
-            if (a < cr.y && (unsigned long long)__ldg(cell_key + a) <= base + (unsigned long long)x1) ca = a;
+            const int2 cr = __ldg(L.col + col_base + (long long)col);
+            const int a = col_lower(cell_key, cr, (K)(base + x0));
+            if (a < cr.y && __ldg(cell_key + a) <= kmax) ca = a;
         } else {
-            for (long long xx = x0; xx <= x1 && ca < 0; ++xx)
-                ca = hash_find(L.hkeys, L.hvals, L.mask, base + (unsigned long long)xx);
+            for (K xx = x0; xx <= x1 && ca < 0; ++xx)
+                ca = hash_find(L.hkeys, L.hvals, L.mask, (unsigned long long)(K)(base + xx));
         }
         if (ca >= 0) {
             // keys are sorted and unique: the row's cells after ca are a prefix of the
             // next keys; four independent loads cover rows of up to 5 cells
-            const unsigned long long kmax = base + (unsigned long long)x1;
+            const int n = (int)n_cells;
+            int cb = ca + 1;
+            bool more = true;
             K nk[4];
 #pragma unroll
-            for (int q = 0; q < 4; ++q) nk[q] = ca + 1 + q < n_cells ? __ldg(cell_key + ca + 1 + q) : ~(K)0;
-            int cb = ca + 1;
+            for (int q = 0; q < 4; ++q) nk[q] = ca + 1 + q < n ? __ldg(cell_key + ca + 1 + q) : (K)0;
 #pragma unroll
-            for (int q = 0; q < 4; ++q)
-                if (cb == ca + 1 + q && ca + 1 + q < n_cells && (unsigned long long)nk[q] <= kmax) ++cb;
-            if (cb == ca + 5)
-                while (cb < n_cells && (unsigned long long)__ldg(cell_key + cb) <= kmax) ++cb;
+            for (int q = 0; q < 4; ++q) {
+                more = more && ca + 1 + q < n && nk[q] <= kmax;
+                cb += more ? 1 : 0;
+            }
+            if (more)
+                while (cb < n && __ldg(cell_key + cb) <= kmax) ++cb;
             res = make_int2(ca, cb);
         }
     }
