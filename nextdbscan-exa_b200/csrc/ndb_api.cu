@@ -948,7 +948,7 @@ void union_phase(ndb_ctx *ctx, const Pipe &p, unsigned long long *job_counters) 
         cudaEventRecord(ctx->kev[4], st);
         ++launch_counter(), union_select_kernel<<<blocks_for(p.items * kWarp), kBlock, 0, st>>>(
             items, n_items, cell_start, nbr, n_rows, cell_cid, ci_sorted, seg_item, seg_part, seg_cap, n_seg);
-        const unsigned scan_blocks = (unsigned)std::min<int64_t>(p.items / kCountWarps + 1, (int64_t)ctx->sm_count * 16);
+        const unsigned scan_blocks = (unsigned)std::min<int64_t>(p.items / kCountWarps + 1, (int64_t)ctx->sm_count * 32);
         ++launch_counter(), union_scan_kernel<D><<<scan_blocks, kCountWarps * kWarp, 0, st>>>(
             items, n_items, cell_start, nbr, n_rows, xs, p.e2, cell_cid, ci_sorted, parent, seg_item, seg_part, seg_cap,
             n_seg, counters + 3, err, p.jobs, p.cell_job);

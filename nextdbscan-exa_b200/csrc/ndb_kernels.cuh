@@ -1613,10 +1613,11 @@ __global__ void __launch_bounds__(kBlock) union_cells_kernel(
 // item's root costs one coalesced load per lane.  Segment length: long enough that the
 // rebuilt row table (about a microsecond) does not show, short enough to fill the GPU.
 // Measured on B200 against one kernel with a warp per item, which read core flag,
-// parent and grandparent of every candidate: 16-D 200k 1.71 -> 0.28 ms, 8-D 2M 1.84 ->
-// 0.59 ms, 5-D 300k 0.36 -> 0.09 ms.
+// parent and grandparent of every candidate: 16-D 200k 1.71 -> 0.22 ms, 8-D 2M 1.84 ->
+// 0.36 ms, 5-D 300k 0.36 -> 0.10 ms.  Segments of 1,024 candidates: 0.28, 0.51 ms; of 512:
+// 0.18, 0.44 ms, but 5-D 2M (dense, many components at first) 9.8 instead of 8.1 ms.
 // ---------------------------------------------------------------------------
-constexpr int kUnionSegment = 1024;
+constexpr int kUnionSegment = 768;
 
 // Candidate ranges of an item at and behind its first point p0; returns their total.
 // root: the snapshot root of this lane's point (-1 without one).  Depends on the
