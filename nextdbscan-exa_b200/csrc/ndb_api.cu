@@ -146,6 +146,7 @@ constexpr size_t kSmallCountersOff = 512;    // u64[12]: 0 clusters 1 noise 2 co
 constexpr int kCounters = 12;
 constexpr size_t kSmallScalarOff = 1024;     // u32[8]: 0 n_cells 1 n_items 2 n_cores 4 tensor items 5 exact items 6 union segments 7 tensor chunks
 constexpr size_t kSmallErrOff = 1536;        // int
+constexpr size_t kSmallDoneOff = 1600;       // u32[2]: blocks done of bbox_kernel and finish_kernel (mail_last_block)
 constexpr size_t kSmallBytes = 2048;
 
 // Destination window of the input-order output scatters: 24M int32 (96 MB) stays
@@ -167,10 +168,9 @@ constexpr uint32_t kAllFlags = NDB_FLAG_APPROXIMATE | NDB_FLAG_FULL_COUNT | NDB_
 // internal: the job is the context's loaded copy (ndb_b200_run_loaded); never a caller's flag
 constexpr uint32_t kFlagLoaded = 0x80000000u;
 
-// load_box layout: lo_hi ints, then the invalid-point count, then two error words
+// load_box layout: encoded bounds, then the invalid-point count
 constexpr size_t kLoadBoxInvalidOff = 2 * kMaxDim * sizeof(int);
-constexpr size_t kLoadBoxErrOff = kLoadBoxInvalidOff + 8;
-constexpr size_t kLoadBoxBytes = kLoadBoxErrOff + 8;
+constexpr size_t kLoadBoxBytes = kLoadBoxInvalidOff + 8;
 constexpr size_t kPinChunk = size_t(32) << 20;  // bytes of one pinned staging chunk
 
 inline void ck(ndb_ctx *ctx, cudaError_t e) {
@@ -267,6 +267,11 @@ const T *mail_from_device(ndb_ctx *ctx, const T *src, size_t count, cudaStream_t
     char *h = mail_slice(ctx, count * sizeof(T));
     copy_words(ctx, src, ctx->mail_dev + (h - ctx->mail), count * sizeof(T), st);
     return reinterpret_cast<const T *>(h);
+}
+
+// Device address of a mailbox slice, for kernels that write it.
+inline volatile uint32_t *mail_device(ndb_ctx *ctx, const void *slice) {
+    return reinterpret_cast<volatile uint32_t *>(ctx->mail_dev + (static_cast<const char *>(slice) - ctx->mail));
 }
 
 // Host -> device through the mailbox: the data is copied into the mailbox now and
@@ -441,16 +446,13 @@ inline double grid_columns(const GridDev &g) {
 // its jobs fit the context's budget, else a hash table of the cell keys (load
 // factor <= 1/4, so most probes settle at the first slot).
 template <typename K>
-CellIndex<K> build_cell_index(ndb_ctx *ctx, int64_t n_cells, double columns, const GridDev &g_one,
+CellIndex<K> build_cell_index(ndb_ctx *ctx, int64_t n_cells, const GridDev &g_one,
                               const JobDev *jobs, const int32_t *cell_job) {
     cudaStream_t st = ctx->stream;
     const uint32_t *n_cells_dev = small_at<uint32_t>(ctx, kSmallScalarOff);
     CellIndex<K> L{nullptr, nullptr, nullptr, 0};
-    ctx->use_cols = columns >= 1 && columns <= (double)ctx->col_budget;
     if (ctx->use_cols) {
-        const size_t cols = (size_t)columns;
-        ensure(ctx, ctx->col_range, (cols + 1) * sizeof(int2));
-        fill_bytes(ctx, ctx->col_range.ptr, 0, (size_t)(cols + 1) * sizeof(int2), st);
+        // allocated and zeroed by the key phase
         ++launch_counter(), col_range_kernel<K><<<blocks_for(n_cells), kBlock, 0, st>>>(
             ctx->cell_key.as<K>(), n_cells_dev, g_one, jobs, cell_job, ctx->col_range.as<int2>());
         ck(ctx, cudaGetLastError());
@@ -543,8 +545,21 @@ void grid_phase(ndb_ctx *ctx, Pipe &p, const float *coords, F launch_keys) {
     ensure(ctx, ctx->keys1, n * sizeof(K));
     ensure(ctx, ctx->ids0, n * sizeof(int32_t));
     ensure(ctx, ctx->ids1, n * sizeof(int32_t));
-    const size_t zero_words = sort_scratch_words<K>(n) + chain_words(n);
-    ensure(ctx, ctx->sort_hist, (zero_words + 4) * sizeof(uint32_t));
+    // zeroed by the key kernel: the sort's and the chained scans' state, the column table
+    const size_t state_words = sort_scratch_words<K>(n) + chain_words(n);
+    ensure(ctx, ctx->sort_hist, (state_words + 4) * sizeof(uint32_t));
+    ZeroJob zero{ctx->sort_hist.as<uint4>(), nullptr, (int64_t)((state_words + 3) / 4), 0};
+    ctx->use_cols = p.columns >= 1 && p.columns <= (double)ctx->col_budget;
+    if (ctx->use_cols) {
+        const size_t cols = (size_t)p.columns;
+        ensure(ctx, ctx->col_range, (cols + 2) * sizeof(int2));
+        zero.b = ctx->col_range.as<uint4>();
+        zero.nb = (int64_t)(cols / 2 + 1);
+        if (zero.nb > 16 * n) {  // a wide grid of few points: more than the key kernel's threads should write
+            fill_bytes(ctx, zero.b, 0, (size_t)zero.nb * sizeof(uint4), st);
+            zero.nb = 0;
+        }
+    }
     ensure(ctx, ctx->core_bits, ((n + 31) / 32 + 1) * sizeof(uint32_t));
     ensure(ctx, ctx->pcell, (n + 1) * sizeof(int32_t));
     ensure(ctx, ctx->cell_start, (n + 2) * sizeof(int32_t));
@@ -553,18 +568,18 @@ void grid_phase(ndb_ctx *ctx, Pipe &p, const float *coords, F launch_keys) {
     ensure(ctx, ctx->nn_sorted, (n + 1) * sizeof(int32_t));
 
     const K invalid_key = (K)(p.key_bits >= (int)(8 * sizeof(K)) ? ~(K)0 : (((K)1 << p.key_bits) - 1));
-    launch_keys(invalid_key, ctx->keys0.as<K>(), ctx->core_bits.as<uint32_t>());
+    launch_keys(invalid_key, ctx->keys0.as<K>(), ctx->core_bits.as<uint32_t>(), zero);
     ck(ctx, cudaGetLastError());
     bool in_first = true;
     cudaEventRecord(ctx->kev[0], st);
     if (sizeof(K) == 4)
         ck(ctx, radix_sort_pairs_u32(reinterpret_cast<uint32_t *>(ctx->keys0.ptr), ctx->ids0.as<int32_t>(),
                                      reinterpret_cast<uint32_t *>(ctx->keys1.ptr), ctx->ids1.as<int32_t>(), n,
-                                     p.key_bits, ctx->sort_hist.as<uint32_t>(), zero_words, &in_first, st));
+                                     p.key_bits, ctx->sort_hist.as<uint32_t>(), &in_first, st));
     else
         ck(ctx, radix_sort_pairs_u64(reinterpret_cast<uint64_t *>(ctx->keys0.ptr), ctx->ids0.as<int32_t>(),
                                      reinterpret_cast<uint64_t *>(ctx->keys1.ptr), ctx->ids1.as<int32_t>(), n,
-                                     p.key_bits, ctx->sort_hist.as<uint32_t>(), zero_words, &in_first, st));
+                                     p.key_bits, ctx->sort_hist.as<uint32_t>(), &in_first, st));
     cudaEventRecord(ctx->kev[1], st);
     if (!in_first) {
         std::swap(ctx->keys0, ctx->keys1);
@@ -574,12 +589,11 @@ void grid_phase(ndb_ctx *ctx, Pipe &p, const float *coords, F launch_keys) {
 
     // cells
     auto *m_cells = reinterpret_cast<volatile uint32_t *>(mail_slice(ctx, sizeof(uint32_t)));
-    auto *m_cells_dev = reinterpret_cast<volatile uint32_t *>(ctx->mail_dev + ((const char *)m_cells - ctx->mail));
     ++launch_counter(), chain_scan_kernel<kCellsPer><<<(unsigned)chain_tiles(nv, kCellsPer), kChainThreads, 0, st>>>(
         CellsOp<D, K>{ctx->keys0.as<K>(), ctx->ids0.as<int32_t>(), coords, rows_aligned<D>(coords), nv,
                       ctx->xs.as<float>(), ctx->cell_start.as<int32_t>(), ctx->cell_key.as<K>(),
                       ctx->pcell.as<int32_t>(), p.early ? nullptr : ctx->nn_sorted.as<int32_t>()},
-        nv, nullptr, chain.state[0], chain.ticket + 0, scal + 0, m_cells_dev);
+        nv, nullptr, chain.state[0], chain.ticket + 0, scal + 0, mail_device(ctx, const_cast<const uint32_t *>(m_cells)));
     ck(ctx, cudaGetLastError());
     if (!p.jobs && nv <= kNoCountPoints) {
         p.cells = nv;
@@ -596,7 +610,7 @@ void grid_phase(ndb_ctx *ctx, Pipe &p, const float *coords, F launch_keys) {
 
     // neighbour rows, through the column table (or a hash table) of the cells
     const int n_rows = p.stencil->n_rows;
-    const CellIndex<K> L = build_cell_index<K>(ctx, p.cells, p.columns, p.g, p.jobs, p.cell_job);
+    const CellIndex<K> L = build_cell_index<K>(ctx, p.cells, p.g, p.jobs, p.cell_job);
     ensure(ctx, ctx->nbr, (size_t)(p.cells * n_rows + 1) * sizeof(int2));
     const int rlog = row_group_log2(n_rows);
     ++launch_counter(), rows_kernel<K><<<blocks_for(p.cells << rlog), kBlock, 0, st>>>(
@@ -842,9 +856,9 @@ void classify_keys(ndb_ctx *ctx, Pipe &p) {
     const int64_t n = ctx->n;
     ctx->stats.sort_passes = (p.key_bits + 7) / 8;
     ctx->stats.key_bytes = (int32_t)sizeof(K);
-    grid_phase<D, K>(ctx, p, ctx->coords_dev, [&](K invalid_key, K *keys, uint32_t *core_bits) {
+    grid_phase<D, K>(ctx, p, ctx->coords_dev, [&](K invalid_key, K *keys, uint32_t *core_bits, const ZeroJob &zero) {
         ++launch_counter(), key_kernel<D, K><<<blocks_for(n), kBlock, 0, st>>>(
-            ctx->coords_dev, n, rows_aligned<D>(ctx->coords_dev), p.g, invalid_key, keys, core_bits);
+            ctx->coords_dev, n, rows_aligned<D>(ctx->coords_dev), p.g, invalid_key, keys, core_bits, zero);
     });
     ctx->n_cells = p.cells;
     ctx->n_items = p.items;
@@ -987,13 +1001,40 @@ void border_phase(ndb_ctx *ctx) {
     }
 }
 
+constexpr int64_t kSelfTallyPoints = int64_t(1) << 18;
+constexpr size_t kTallyWords = (kSmallErrOff + sizeof(int) - kSmallCountersOff) / sizeof(uint32_t);
+
+// The run's counters, scalars and error flag as the host reads them: one copy kernel
+// into the mailbox in stream order, or finish_kernel itself (valid once the stream is
+// synchronized).
+struct Tally {
+    unsigned long long counters[kCounters];
+    uint32_t scal[8];
+    int err;
+};
+const char *mail_tally(ndb_ctx *ctx) {
+    return reinterpret_cast<const char *>(
+        mail_from_device(ctx, small_at<uint32_t>(ctx, kSmallCountersOff), kTallyWords, ctx->stream));
+}
+Tally read_tally(const char *m) {
+    Tally t;
+    memcpy(t.counters, m, sizeof(t.counters));
+    memcpy(t.scal, m + (kSmallScalarOff - kSmallCountersOff), sizeof(t.scal));
+    memcpy(&t.err, m + (kSmallErrOff - kSmallCountersOff), sizeof(int));
+    return t;
+}
+
 // Input-order outputs below this size are written by one pass (finish_kernel).
 inline bool one_window(int64_t n) { return n <= kScatterWindow; }
 
+// Returns the mailbox slice of the run's tally (read_tally), valid once the stream is
+// synchronized.
 template <int D>
-void labels_phase(ndb_ctx *ctx) {
+const char *labels_phase(ndb_ctx *ctx) {
     cudaStream_t st = ctx->stream;
     const int64_t n = ctx->n, nv = ctx->nv;
+    ctx->mail_used = 0;  // phase 1's transfers have been read
+    const char *m_tally = nullptr;
     unsigned long long *counters = small_at<unsigned long long>(ctx, kSmallCountersOff);
     const Pipe p = ctx_pipe(ctx);
     if (ctx->key64) union_phase<D, uint64_t>(ctx, p, nullptr);
@@ -1012,13 +1053,19 @@ void labels_phase(ndb_ctx *ctx) {
     ctx->nn_late = nullptr;
     if (one_window(n)) {
         const bool lists = p.list_stride > 0;
+        // small grids hand the tally over themselves; with many blocks their ticket costs more
+        // than the copy kernel it saves (3-D 10M: 0.29 against 0.24 ms)
+        const bool self = n <= kSelfTallyPoints;
+        if (self) m_tally = mail_slice(ctx, kTallyWords * sizeof(uint32_t));
         if (!lists) border_phase<D>(ctx);
         cudaEventRecord(ctx->kev[7], st);
         ++launch_counter(), finish_kernel<<<blocks_for(n), kBlock, 0, st>>>(
             nv, n, ctx->nn_sorted.as<int32_t>(), p.list, p.list_stride, lists, ctx->core_sorted.as<uint8_t>(),
             ctx->cell_units, ctx->pcell.as<int32_t>(), ctx->cell_cid.as<int32_t>(), ctx->ci_sorted.as<int32_t>(),
             ctx->ids0.as<int32_t>(), ctx->core_bits.as<uint32_t>(), ctx->core_prefix.as<uint32_t>(), nn_target, target,
-            counters, nullptr, 0, nullptr);
+            counters, nullptr, 0, nullptr, small_at<uint32_t>(ctx, kSmallDoneOff) + 1, (int)kTallyWords,
+            self ? mail_device(ctx, m_tally) : nullptr);
+        if (!self) m_tally = mail_tally(ctx);
     } else {
         border_phase<D>(ctx);
         cudaEventRecord(ctx->kev[7], st);
@@ -1027,9 +1074,11 @@ void labels_phase(ndb_ctx *ctx) {
             ++launch_counter(), output_ci_kernel<<<blocks_for(n), kBlock, 0, st>>>(
                 ctx->ci_sorted.as<int32_t>(), nv, n, ctx->ids0.as<int32_t>(), ctx->core_bits.as<uint32_t>(),
                 ctx->core_prefix.as<uint32_t>(), target, counters, lo, wci >= n ? INT64_MAX : lo + wci);
+        m_tally = mail_tally(ctx);
     }
     ck(ctx, cudaGetLastError());
     cudaEventRecord(ctx->ev[4], st);
+    return m_tally;
 }
 
 ndb_status check_ctx(ndb_ctx *ctx) {
@@ -1056,26 +1105,6 @@ inline void audit_stats(ndb_stats &S, const unsigned long long *a) {
     S.filter_max_err_over_bound = mr;
     S.filter_audited_pairs = (int64_t)a[2];
     S.filter_misclassified_pairs = (int64_t)a[3];
-}
-
-// The run's counters, scalars and error flag as the host reads them: one copy kernel
-// into the mailbox in stream order (valid once the stream is synchronized).
-struct Tally {
-    unsigned long long counters[kCounters];
-    uint32_t scal[8];
-    int err;
-};
-const char *mail_tally(ndb_ctx *ctx) {
-    constexpr size_t words = (kSmallErrOff + sizeof(int) - kSmallCountersOff) / sizeof(uint32_t);
-    return reinterpret_cast<const char *>(
-        mail_from_device(ctx, small_at<uint32_t>(ctx, kSmallCountersOff), words, ctx->stream));
-}
-Tally read_tally(const char *m) {
-    Tally t;
-    memcpy(t.counters, m, sizeof(t.counters));
-    memcpy(t.scal, m + (kSmallScalarOff - kSmallCountersOff), sizeof(t.scal));
-    memcpy(&t.err, m + (kSmallErrOff - kSmallCountersOff), sizeof(int));
-    return t;
 }
 
 // Counters and times of phase 1 (the label phase leaves counters 2, 5 and 8 to 11 and
@@ -1131,25 +1160,27 @@ ndb_status classify_impl(ndb_ctx *ctx, const float *coords, int64_t n, float eps
     }
 
     // bounding box of the grid-eligible points (a loaded job's was reduced while it arrived)
-    int *lo_hi = small_at<int>(ctx, kSmallBboxOff);
+    uint32_t *lo_hi = small_at<uint32_t>(ctx, kSmallBboxOff);
     unsigned long long *n_invalid = small_at<unsigned long long>(ctx, kSmallInvalidOff);
+    static_assert(kSmallInvalidOff >= kSmallBboxOff + 2 * kMaxDim * sizeof(int), "bounds, then the invalid points");
+    constexpr size_t box_words = (kSmallInvalidOff + 8 - kSmallBboxOff) / sizeof(uint32_t);
+    const char *m_box;
     if (flags & kFlagLoaded) {
         ck(ctx, cudaMemcpyAsync(lo_hi, ctx->load_box.ptr, 2 * D * sizeof(int), cudaMemcpyDeviceToDevice, st));
         ck(ctx, cudaMemcpyAsync(n_invalid, ctx->load_box.as<char>() + kLoadBoxInvalidOff, sizeof(unsigned long long),
                                 cudaMemcpyDeviceToDevice, st));
-        ++launch_counter(), set_int_kernel<<<1, 1, 0, st>>>(small_at<int>(ctx, kSmallErrOff) + 1, ctx->uf_max_steps);
+        m_box = reinterpret_cast<const char *>(mail_from_device(ctx, lo_hi, box_words, st));
     } else {
-        ++launch_counter(), bbox_init_kernel<<<1, 32, 0, st>>>(lo_hi, D, n_invalid, small_at<int>(ctx, kSmallErrOff),
-                                                               ctx->uf_max_steps);
+        m_box = mail_slice(ctx, box_words * sizeof(uint32_t));
         ++launch_counter(), bbox_kernel<D><<<bbox_blocks(ctx, n), kBlock, 0, st>>>(
-            ctx->coords_dev, n, rows_aligned<D>(ctx->coords_dev), lo_hi, n_invalid);
+            ctx->coords_dev, n, rows_aligned<D>(ctx->coords_dev), lo_hi, n_invalid,
+            small_at<uint32_t>(ctx, kSmallDoneOff), (int)box_words, mail_device(ctx, m_box));
     }
+    if (ctx->uf_max_steps)  // the union-find bound of the run (err[1], see uf_limit)
+        ++launch_counter(), set_int_kernel<<<1, 1, 0, st>>>(small_at<int>(ctx, kSmallErrOff) + 1, ctx->uf_max_steps);
     ck(ctx, cudaGetLastError());
-    static_assert(kSmallInvalidOff >= kSmallBboxOff + 2 * kMaxDim * sizeof(int), "bounds, then the invalid points");
-    const char *m_box = reinterpret_cast<const char *>(mail_from_device(
-        ctx, small_at<uint32_t>(ctx, kSmallBboxOff), (kSmallInvalidOff + 8 - kSmallBboxOff) / sizeof(uint32_t), st));
     ck(ctx, cudaStreamSynchronize(st));
-    int h_lo_hi[2 * kMaxDim];
+    uint32_t h_lo_hi[2 * kMaxDim];
     unsigned long long h_invalid = 0;
     memcpy(h_lo_hi, m_box, sizeof(h_lo_hi));
     memcpy(&h_invalid, m_box + (kSmallInvalidOff - kSmallBboxOff), sizeof(h_invalid));
@@ -1162,8 +1193,8 @@ ndb_status classify_impl(ndb_ctx *ctx, const float *coords, int64_t n, float eps
             memcpy(&f, &i, sizeof(f));
             return (double)f;
         };
-        lo[a] = ctx->nv > 0 ? dec(h_lo_hi[a]) : 0.0;
-        hi[a] = ctx->nv > 0 ? dec(h_lo_hi[D + a]) : 0.0;
+        lo[a] = ctx->nv > 0 ? dec(decode_lo(h_lo_hi[a])) : 0.0;
+        hi[a] = ctx->nv > 0 ? dec(decode_hi(h_lo_hi[D + a])) : 0.0;
     }
     const Plan pl = plan_grid(D, ctx->e2, lo, hi);
     ctx->grid = pl.g;
@@ -1228,13 +1259,11 @@ template <int D>
 ndb_status labels_impl(ndb_ctx *ctx, int32_t *ci_out, ndb_result *result) {
     cudaStream_t st = ctx->stream;
     ctx->ci_user = ci_out;
-    labels_phase<D>(ctx);
+    const char *m_tally = labels_phase<D>(ctx);
     ctx->ci_user = nullptr;
     const int64_t n = ctx->n;
     if (ci_out && !(ctx->flags_run & NDB_FLAG_DEVICE_PTRS))
         ck(ctx, cudaMemcpyAsync(ci_out, ctx->ci_orig.ptr, n * sizeof(int32_t), cudaMemcpyDeviceToHost, st));
-    ctx->mail_used = 0;  // phase 1's transfers have been read
-    const char *m_tally = mail_tally(ctx);
     ck(ctx, cudaStreamSynchronize(st));
     const Tally t = read_tally(m_tally);
     if (ctx->stats_pending) {
@@ -1287,10 +1316,10 @@ ndb_status labels_entry(ndb_ctx *ctx, int32_t *ci_out, ndb_result *result) {
 // bounding-box kernel reduces chunk k on the context's stream as soon as it landed.
 template <int D>
 void bbox_chunk(ndb_ctx *ctx, const float *p, int64_t cnt) {
-    int *lo_hi = ctx->load_box.as<int>();
+    uint32_t *lo_hi = ctx->load_box.as<uint32_t>();
     auto *inval = reinterpret_cast<unsigned long long *>(ctx->load_box.as<char>() + kLoadBoxInvalidOff);
     ++launch_counter(), bbox_kernel<D><<<bbox_blocks(ctx, cnt), kBlock, 0, ctx->stream>>>(
-        p, cnt, rows_aligned<D>(p), lo_hi, inval);
+        p, cnt, rows_aligned<D>(p), lo_hi, inval, nullptr, 0, nullptr);
     ck(ctx, cudaGetLastError());
 }
 
@@ -1317,10 +1346,7 @@ ndb_status load_bin_impl(ndb_ctx *ctx, FILE *f, int64_t *n_out, int32_t *d_out) 
         ctx->pin_bytes = kPinChunk;
     }
     for (int b = 0; b < 2; ++b) lazy_event(ctx, ctx->ev_pin[b]);
-    ++launch_counter(), bbox_init_kernel<<<1, 32, 0, st>>>(
-        ctx->load_box.as<int>(), d, reinterpret_cast<unsigned long long *>(ctx->load_box.as<char>() + kLoadBoxInvalidOff),
-        reinterpret_cast<int *>(ctx->load_box.as<char>() + kLoadBoxErrOff), 0);
-    ck(ctx, cudaGetLastError());
+    ck(ctx, cudaMemsetAsync(ctx->load_box.ptr, 0, kLoadBoxBytes, st));
     const int64_t per = (int64_t)(ctx->pin_bytes / (sizeof(float) * d));
     int k = 0;
     for (int64_t off = 0; off < n; off += per, ++k) {
@@ -1769,9 +1795,9 @@ void run_group_keys(ndb_ctx *ctx, ndb_job *jobs, const std::vector<int> &members
     p.jobs = jobs_dev;
     p.n_jobs = nj;
     cudaEventRecord(ctx->ev[0], st);
-    grid_phase<D, K>(ctx, p, ctx->coords.as<float>(), [&](K invalid_key, K *keys, uint32_t *core_bits) {
+    grid_phase<D, K>(ctx, p, ctx->coords.as<float>(), [&](K invalid_key, K *keys, uint32_t *core_bits, const ZeroJob &zero) {
         ++launch_counter(), key_batch_kernel<D, K><<<dim3(gx, nj), kBlock, 0, st>>>(
-            ctx->coords.as<float>(), jobs_dev, invalid_key, keys, core_bits);
+            ctx->coords.as<float>(), jobs_dev, invalid_key, keys, core_bits, zero);
     });
     if (bp.list_stride > 0) {
         ensure(ctx, ctx->nbr_list, (size_t)(nv * bp.list_stride + 1) * sizeof(int32_t));
@@ -1795,7 +1821,7 @@ void run_group_keys(ndb_ctx *ctx, ndb_job *jobs, const std::vector<int> &members
         nv, n, ctx->nn_sorted.as<int32_t>(), p.list, p.list_stride, p.list_stride > 0, ctx->core_sorted.as<uint8_t>(),
         bp.linked, ctx->pcell.as<int32_t>(), ctx->cell_cid.as<int32_t>(), ctx->ci_sorted.as<int32_t>(),
         ctx->ids0.as<int32_t>(), ctx->core_bits.as<uint32_t>(), ctx->core_prefix.as<uint32_t>(), nullptr, nullptr,
-        counters, jobs_dev, nj, jc);
+        counters, jobs_dev, nj, jc, nullptr, 0, nullptr);
     cudaEventRecord(ctx->kev[7], st);
     ++launch_counter(), job_cores_kernel<<<blocks_for(nj), kBlock, 0, st>>>(
         jobs_dev, nj, ctx->core_bits.as<uint32_t>(), ctx->core_prefix.as<uint32_t>(), n, jc);
@@ -1919,16 +1945,16 @@ void run_group(ndb_ctx *ctx, ndb_job *jobs, const std::vector<int> &members, uin
     // per-job bounding boxes, then every job's grid planned on the host (one sync)
     const size_t lh_bytes = ((size_t)nj * 2 * D * sizeof(int) + 15) & ~size_t(15);
     ensure(ctx, ctx->batch_bbox, lh_bytes + (size_t)nj * sizeof(unsigned long long) + 64);
-    int *lo_hi = ctx->batch_bbox.as<int>();
+    uint32_t *lo_hi = ctx->batch_bbox.as<uint32_t>();
     unsigned long long *inval = reinterpret_cast<unsigned long long *>(ctx->batch_bbox.as<char>() + lh_bytes);
-    ++launch_counter(), bbox_batch_init_kernel<<<blocks_for((int64_t)nj * D), kBlock, 0, st>>>(lo_hi, D, nj, inval);
+    fill_bytes(ctx, lo_hi, 0, lh_bytes + (size_t)nj * sizeof(unsigned long long), st);
     ++launch_counter(), bbox_batch_kernel<D><<<dim3(gx, nj), kBlock, 0, st>>>(ctx->coords.as<float>(),
                                                                              ctx->jobs_dev.as<JobDev>(), lo_hi, inval);
     ck(ctx, cudaGetLastError());
-    const int *m_lo_hi = mail_from_device(ctx, lo_hi, (size_t)nj * 2 * D, st);
+    const uint32_t *m_lo_hi = mail_from_device(ctx, lo_hi, (size_t)nj * 2 * D, st);
     const unsigned long long *m_inval = mail_from_device(ctx, inval, (size_t)nj, st);
     ck(ctx, cudaStreamSynchronize(st));
-    const std::vector<int> h_lo_hi(m_lo_hi, m_lo_hi + (size_t)nj * 2 * D);
+    const std::vector<uint32_t> h_lo_hi(m_lo_hi, m_lo_hi + (size_t)nj * 2 * D);
     const std::vector<unsigned long long> h_inval(m_inval, m_inval + nj);
 
     auto dec = [](int v) {
@@ -1947,8 +1973,8 @@ void run_group(ndb_ctx *ctx, ndb_job *jobs, const std::vector<int> &members, uin
         const int64_t jnv = jd.n - (int64_t)h_inval[m];
         double lo[kMaxDim], hi[kMaxDim];
         for (int a = 0; a < D; ++a) {
-            lo[a] = jnv > 0 ? dec(h_lo_hi[(size_t)m * 2 * D + a]) : 0.0;
-            hi[a] = jnv > 0 ? dec(h_lo_hi[(size_t)m * 2 * D + D + a]) : 0.0;
+            lo[a] = jnv > 0 ? dec(decode_lo(h_lo_hi[(size_t)m * 2 * D + a])) : 0.0;
+            hi[a] = jnv > 0 ? dec(decode_hi(h_lo_hi[(size_t)m * 2 * D + D + a])) : 0.0;
         }
         const Plan pl = plan_grid(D, jd.e2, lo, hi);
         const bool job_tc = tc_eligible(ctx, D, jd.e2, lo, hi, pl.cell_units, pl.st.n_rows, flags);

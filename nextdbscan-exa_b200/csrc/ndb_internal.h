@@ -54,14 +54,11 @@ constexpr size_t sort_scratch_words(int64_t n) {
 }
 // Stable LSD radix sort of (key, element index) pairs on the low `bits` bits of the
 // keys in k0: sorts between (k0, v0) and (k1, v1) and returns via *result_in_first
-// whether the sorted keys and indices ended in (k0, v0).  v0 need not be set.  The first
-// zero_words of the scratch are zeroed first (at least sort_scratch_words; a caller's
-// own zeroed words may follow the sort's).
+// whether the sorted keys and indices ended in (k0, v0).  v0 need not be set.  The
+// caller has zeroed the scratch.
 cudaError_t radix_sort_pairs_u32(uint32_t *k0, int32_t *v0, uint32_t *k1, int32_t *v1, int64_t n,
-                                 int bits, uint32_t *scratch, size_t zero_words, bool *result_in_first,
-                                 cudaStream_t st);
+                                 int bits, uint32_t *scratch, bool *result_in_first, cudaStream_t st);
 cudaError_t radix_sort_pairs_u64(uint64_t *k0, int32_t *v0, uint64_t *k1, int32_t *v1, int64_t n,
-                                 int bits, uint32_t *scratch, size_t zero_words, bool *result_in_first,
-                                 cudaStream_t st);
+                                 int bits, uint32_t *scratch, bool *result_in_first, cudaStream_t st);
 
 }  // namespace ndb

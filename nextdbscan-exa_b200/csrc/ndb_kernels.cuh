@@ -97,26 +97,36 @@ __device__ __forceinline__ int ordered_int(float f) {
     return i >= 0 ? i : i ^ 0x7fffffff;
 }
 
-// Also writes the union-find bound of the run (err[1], see uf_limit).
-__global__ void bbox_init_kernel(int *lo_hi, int d, unsigned long long *n_invalid, int *err, int uf_limit) {
-    const int t = threadIdx.x;
-    if (t < d) {
-        lo_hi[t] = 0x7fffffff;
-        lo_hi[d + t] = (int)0x80000000;
-    }
-    if (t == 0) {
-        *n_invalid = 0ull;
-        err[1] = uf_limit;
-    }
-}
-
 __global__ void set_int_kernel(int *p, int v) { *p = v; }
 
-// The block's bounds and invalid points, added to lo_hi (ordered-int min, then max, per
-// dimension) and n_invalid.
+// Bounds as unsigned words whose identity is 0, so that zeroed memory starts a reduction:
+// the maximum as its ordered unsigned value, the minimum as the complement of its own.
+__host__ __device__ __forceinline__ uint32_t encode_hi(int ordered) { return (uint32_t)ordered ^ 0x80000000u; }
+__host__ __device__ __forceinline__ uint32_t encode_lo(int ordered) { return ~encode_hi(ordered); }
+__host__ __device__ __forceinline__ int decode_hi(uint32_t v) { return (int)(v ^ 0x80000000u); }
+__host__ __device__ __forceinline__ int decode_lo(uint32_t v) { return decode_hi(~v); }
+
+// The last block of a grid to come here (its earlier atomics are visible to it) copies
+// `words` words from src to mail (mapped host memory): the host reads a kernel's result
+// without a copy behind it.  done starts at zero and is left so.
+__device__ __forceinline__ void mail_last_block(uint32_t *done, const uint32_t *src, int words,
+                                                volatile uint32_t *mail) {
+    __shared__ int s_last;
+    __threadfence();
+    __syncthreads();
+    if (threadIdx.x == 0) s_last = atomicAdd(done, 1u) == gridDim.x - 1;
+    __syncthreads();
+    if (!s_last) return;
+    __threadfence();
+    for (int i = threadIdx.x; i < words; i += blockDim.x) mail[i] = __ldcg(src + i);
+    if (threadIdx.x == 0) *done = 0;  // for the next launch
+}
+
+// The block's bounds and invalid points, added to lo_hi (encoded minima, then maxima)
+// and n_invalid.
 template <int D>
 __device__ __forceinline__ void bbox_reduce(int (&lo)[D], int (&hi)[D], unsigned bad, int (*s_lh)[2 * D],
-                                            unsigned *s_bad, int *lh, unsigned long long *n_invalid) {
+                                            unsigned *s_bad, uint32_t *lh, unsigned long long *n_invalid) {
     constexpr int W = kBlock / kWarp;
 #pragma unroll
     for (int k = 0; k < D; ++k) {
@@ -139,9 +149,9 @@ __device__ __forceinline__ void bbox_reduce(int (&lo)[D], int (&hi)[D], unsigned
         int v = s_lh[0][t];
         for (int q = 1; q < W; ++q) v = t < D ? min(v, s_lh[q][t]) : max(v, s_lh[q][t]);
         if (t < D) {
-            if (v != 0x7fffffff) atomicMin(lh + t, v);
+            if (v != 0x7fffffff) atomicMax(lh + t, encode_lo(v));
         } else {
-            if (v != (int)0x80000000) atomicMax(lh + t, v);
+            if (v != (int)0x80000000) atomicMax(lh + t, encode_hi(v));
         }
     }
     if (threadIdx.x == 0) {
@@ -190,13 +200,15 @@ inline bool rows_aligned(const float *p) {
     return ((uintptr_t)p & (D % 4 == 0 ? 15 : 7)) == 0;
 }
 
-// lo_hi[0..D) = ordered-int min, lo_hi[D..2D) = ordered-int max.  Warps reduce by
+// lo_hi[0..D) = encoded minima, lo_hi[D..2D) = encoded maxima.  Warps reduce by
 // shuffles, the block through shared memory, and one thread per dimension and bound
 // issues the block's atomic: with one atomic per warp the kernel's time was the queue of
-// atomics on 2 D addresses (16-D 200k 128 -> 8 us, 8-D 2M 110 -> 17 us).
+// atomics on 2 D addresses (16-D 200k 128 -> 7 us, 8-D 2M 110 -> 15 us).  With mail the
+// bounds and the invalid count (mail_words from lo_hi on) go to the host.
 template <int D>
 __global__ void __launch_bounds__(kBlock) bbox_kernel(const float *__restrict__ coords, int64_t n, bool vec,
-                                                      int *lo_hi, unsigned long long *n_invalid) {
+                                                      uint32_t *lo_hi, unsigned long long *n_invalid,
+                                                      uint32_t *done, int mail_words, volatile uint32_t *mail) {
     __shared__ int s_lh[kBlock / kWarp][2 * D];
     __shared__ unsigned s_bad[kBlock / kWarp];
     int lo[D], hi[D];
@@ -225,6 +237,7 @@ __global__ void __launch_bounds__(kBlock) bbox_kernel(const float *__restrict__ 
         }
     }
     bbox_reduce<D>(lo, hi, bad, s_lh, s_bad, lo_hi, n_invalid);
+    if (mail) mail_last_block(done, lo_hi, mail_words, mail);
 }
 
 // Cell coordinate along gridded dimension a.  Computed in double: with at most
@@ -238,11 +251,24 @@ __device__ __forceinline__ long long cell_coord(const GridDev &g, int a, float x
     return c;
 }
 
+// Memory the later grid kernels expect zeroed (the sort's and the chained scans' state,
+// the column table), zeroed by the key kernels' threads; t of `threads` takes its share.
+struct ZeroJob {
+    uint4 *a, *b;
+    int64_t na, nb;
+    __device__ void run(int64_t t, int64_t threads) const {
+        const uint4 z = make_uint4(0, 0, 0, 0);
+        for (int64_t i = t; i < na; i += threads) a[i] = z;
+        for (int64_t i = t; i < nb; i += threads) b[i] = z;
+    }
+};
+
 template <int D, typename K>
 __global__ void __launch_bounds__(kBlock) key_kernel(const float *__restrict__ coords, int64_t n, bool vec,
                                                      GridDev g, K invalid_key, K *__restrict__ keys,
-                                                     uint32_t *__restrict__ core_bits) {
+                                                     uint32_t *__restrict__ core_bits, ZeroJob zero) {
     const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+    zero.run(i, (int64_t)gridDim.x * blockDim.x);
     if (i >= n) return;
     if ((i & 31) == 0) core_bits[i >> 5] = 0;  // for core_flags_kernel
     const float *p = coords + i * D;
@@ -2188,7 +2214,8 @@ __global__ void output_ci_kernel(const int32_t *__restrict__ ci_sorted, int64_t 
 // The border step from the count's lists (border_list_kernel), the counts (scatter_nn_kernel)
 // and the ids (output_ci_kernel) in one pass over the points, for outputs that stay in
 // L2: the permutation is read once and nothing is launched in between.  nn_out may be
-// null; use_lists 0: a border kernel has run before.
+// null; use_lists 0: a border kernel has run before.  With mail the run's counters
+// (mail_words from counters on) go to the host.
 __global__ void finish_kernel(int64_t nv, int64_t n, const int32_t *__restrict__ nn_sorted,
                               const int32_t *__restrict__ nbr_list, int list_stride, int use_lists,
                               const uint8_t *__restrict__ core_sorted, int cell_units,
@@ -2197,7 +2224,8 @@ __global__ void finish_kernel(int64_t nv, int64_t n, const int32_t *__restrict__
                               const uint32_t *__restrict__ core_bits, const uint32_t *__restrict__ core_prefix,
                               int32_t *__restrict__ nn_out, int32_t *__restrict__ ci_out,
                               unsigned long long *__restrict__ counters, const JobDev *__restrict__ jobs, int n_jobs,
-                              unsigned long long *__restrict__ job_counters) {
+                              unsigned long long *__restrict__ job_counters, uint32_t *done, int mail_words,
+                              volatile uint32_t *mail) {
     const int64_t s = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     unsigned noise = 0, roots = 0, looked = 0;
     int job = -1;  // batched runs: the point's job, whose counters take its noise and roots
@@ -2257,6 +2285,7 @@ __global__ void finish_kernel(int64_t nv, int64_t n, const int32_t *__restrict__
         if (roots) atomicAdd(counters + 0, (unsigned long long)roots);
         if (looked) atomicAdd(counters + 4, (unsigned long long)looked);
     }
+    if (mail) mail_last_block(done, reinterpret_cast<const uint32_t *>(counters), mail_words, mail);
 }
 
 // ndb_b200_assign_border: the caller's id of every core (input order) into the
@@ -2315,21 +2344,11 @@ __global__ void __launch_bounds__(kBlock) gather_jobs_kernel(const JobDev *__res
         dst[i] = J.src[i];
 }
 
-__global__ void bbox_batch_init_kernel(int *lo_hi, int d, int n_jobs, unsigned long long *n_invalid) {
-    const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (i < (int64_t)n_jobs * d) {
-        const int64_t j = i / d, k = i - j * d;
-        lo_hi[j * 2 * d + k] = 0x7fffffff;
-        lo_hi[j * 2 * d + d + k] = (int)0x80000000;
-    }
-    if (i < n_jobs) n_invalid[i] = 0ull;
-}
-
-// Per-job bounding boxes (ordered-int min/max per dimension) and invalid-point counts
+// Per-job bounding boxes (encoded bounds) and invalid-point counts
 // of a batch: blocks (x, job).
 template <int D>
 __global__ void __launch_bounds__(kBlock) bbox_batch_kernel(const float *__restrict__ coords,
-                                                            const JobDev *__restrict__ jobs, int *lo_hi,
+                                                            const JobDev *__restrict__ jobs, uint32_t *lo_hi,
                                                             unsigned long long *n_invalid) {
     constexpr int W = kBlock / 32;
     __shared__ int s_lh[W][2 * D];
@@ -2366,7 +2385,10 @@ __global__ void __launch_bounds__(kBlock) bbox_batch_kernel(const float *__restr
 template <int D, typename K>
 __global__ void __launch_bounds__(kBlock) key_batch_kernel(const float *__restrict__ coords,
                                                            const JobDev *__restrict__ jobs, K invalid_key,
-                                                           K *__restrict__ keys, uint32_t *__restrict__ core_bits) {
+                                                           K *__restrict__ keys, uint32_t *__restrict__ core_bits,
+                                                           ZeroJob zero) {
+    zero.run(((int64_t)blockIdx.y * gridDim.x + blockIdx.x) * blockDim.x + threadIdx.x,
+             (int64_t)gridDim.y * gridDim.x * blockDim.x);
     const JobDev &J = jobs[blockIdx.y];
     const GridDev g = J.g;
     for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < J.n; i += (int64_t)gridDim.x * blockDim.x) {

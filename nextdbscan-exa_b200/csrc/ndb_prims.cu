@@ -219,23 +219,15 @@ __global__ void __launch_bounds__(kSortThreads, 4) sort_pass_kernel(const K *__r
     }
 }
 
-__global__ void zero_words_kernel(uint4 *__restrict__ p, int64_t n) {
-    const int64_t stride = (int64_t)gridDim.x * blockDim.x;
-    for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += stride) p[i] = make_uint4(0, 0, 0, 0);
-}
-
 template <typename K>
 cudaError_t radix_sort_pairs(K *k0, int32_t *v0, K *k1, int32_t *v1, int64_t n, int bits, uint32_t *scratch,
-                             size_t zero_words, bool *result_in_first, cudaStream_t st) {
+                             bool *result_in_first, cudaStream_t st) {
     *result_in_first = true;
     if (n <= 0) return cudaSuccess;
     const int64_t tiles = (n + SortTile<K>::v - 1) / SortTile<K>::v;
     const int passes = bits <= 0 ? 1 : (bits + 7) / 8;
     uint32_t *hist = scratch, *tickets = scratch + kSortHistWords;
     unsigned long long *state = reinterpret_cast<unsigned long long *>(tickets + kSortTicketWords);
-    const int64_t zero = (int64_t)((zero_words + 3) / 4);
-    ++launch_counter(), zero_words_kernel<<<(unsigned)((zero + kSortThreads * 4 - 1) / (kSortThreads * 4)), kSortThreads, 0, st>>>(
-        reinterpret_cast<uint4 *>(scratch), zero);
     const int64_t hist_blocks = (n + kSortThreads * 8 - 1) / (kSortThreads * 8);
     ++launch_counter(), sort_hist_kernel<K><<<(unsigned)(hist_blocks < 148 * 6 ? hist_blocks : 148 * 6), kSortThreads, 0, st>>>(
         k0, n, passes, hist);
@@ -267,15 +259,13 @@ int &launch_counter() {
 }
 
 cudaError_t radix_sort_pairs_u32(uint32_t *k0, int32_t *v0, uint32_t *k1, int32_t *v1, int64_t n,
-                                 int bits, uint32_t *scratch, size_t zero_words, bool *result_in_first,
-                                 cudaStream_t st) {
-    return radix_sort_pairs<uint32_t>(k0, v0, k1, v1, n, bits, scratch, zero_words, result_in_first, st);
+                                 int bits, uint32_t *scratch, bool *result_in_first, cudaStream_t st) {
+    return radix_sort_pairs<uint32_t>(k0, v0, k1, v1, n, bits, scratch, result_in_first, st);
 }
 
 cudaError_t radix_sort_pairs_u64(uint64_t *k0, int32_t *v0, uint64_t *k1, int32_t *v1, int64_t n,
-                                 int bits, uint32_t *scratch, size_t zero_words, bool *result_in_first,
-                                 cudaStream_t st) {
-    return radix_sort_pairs<uint64_t>(k0, v0, k1, v1, n, bits, scratch, zero_words, result_in_first, st);
+                                 int bits, uint32_t *scratch, bool *result_in_first, cudaStream_t st) {
+    return radix_sort_pairs<uint64_t>(k0, v0, k1, v1, n, bits, scratch, result_in_first, st);
 }
 
 }  // namespace ndb
