@@ -908,6 +908,12 @@ void classify_dispatch(ndb_ctx *ctx, const Plan &pl) {
 // ---------------------------------------------------------------------------
 // phase 2
 // ---------------------------------------------------------------------------
+// Up to these sizes the list unions of a point are shared by four threads, and the near
+// unions of a cell by one thread per face: there the unions are a chain of latencies
+// (3-D 10M, 0.9M cells: union phase 0.98 -> 0.94 ms by faces); beyond, the GPU is full
+// anyway (skewed 2-D 100M, 5.8M cells: 6.23 against 6.32 ms).
+constexpr int64_t kSplitListPoints = int64_t(1) << 17, kSplitFaceCells = int64_t(1) << 22;
+
 // Union-find, component minima and core ids of a pipeline.  ci_sorted holds the roots'
 // snapshot until the ids are written, cell_cid (point units) the cells' roots.
 template <int D, typename K>
@@ -934,12 +940,14 @@ void union_phase(ndb_ctx *ctx, const Pipe &p, unsigned long long *job_counters) 
 
     ++launch_counter(), init_units_kernel<<<blocks_for(units), kBlock, 0, st>>>(
         parent, comp_min, units, n_cells, p.linked ? nullptr : cell_cid, n_seg);
+    const int split_log2 = nv <= kSplitListPoints ? 2 : 0;
     if (p.list_stride > 0)
-        ++launch_counter(), union_lists_kernel<<<blocks_for(nv), kBlock, 0, st>>>(
+        ++launch_counter(), union_lists_kernel<<<blocks_for(nv << split_log2), kBlock, 0, st>>>(
             nv, ctx->nn_sorted.as<int32_t>(), p.list, p.list_cap, p.list_stride, core_sorted, parent, err, p.jobs,
-            p.cell_job, pcell, p.linked, cell_start, p.min_pts);
+            p.cell_job, pcell, p.linked, cell_start, p.min_pts, split_log2);
     if (p.linked) {
-        ++launch_counter(), union_near_kernel<D, K><<<blocks_for(p.cells), kBlock, 0, st>>>(
+        const unsigned faces = p.cells <= kSplitFaceCells ? (unsigned)std::min(D, 3) : 1u;
+        ++launch_counter(), union_near_kernel<D, K><<<dim3(blocks_for(p.cells), faces), kBlock, 0, st>>>(
             n_cells, p.g, ctx->cell_key.as<K>(), cell_start, cell_index<K>(ctx), xs, p.e2, core_sorted, has_core,
             parent, counters + 3, err, p.jobs, p.cell_job);
         ++launch_counter(), flatten_snap_kernel<<<blocks_for(p.cells), kBlock, 0, st>>>(parent, n_cells, err, has_core,

@@ -1423,11 +1423,11 @@ __device__ __forceinline__ bool cells_touch(int A, int B, const int32_t *__restr
 }
 
 // ---------------------------------------------------------------------------
-// First union pass over cells: one thread per cell A.  It looks at A's three
-// forward face neighbours (x+1, y+1, z+1; found through the key order and the cell
-// hash table), tests the first kNearProbe cores of A against the first
-// kNearProbe cores of each (independent loads, 16 predicates) and links A and B on
-// a hit.  Face adjacency already connects every cell of a dense region, so this
+// First union pass over cells: one thread per cell A and forward face (x+1, y+1, z+1;
+// the neighbour B is found through the key order and the cell index), or per cell with
+// the faces one after the other (gridDim.y).  It tests the first kNearProbe cores of A
+// against the first kNearProbe cores of B (independent loads, 16 predicates) and links A
+// and B on a hit.  Face adjacency already connects every cell of a dense region, so this
 // merges dense clusters with one cheap thread per cell; the full pass then sees
 // them as one root.
 // ---------------------------------------------------------------------------
@@ -1451,6 +1451,7 @@ __global__ void __launch_bounds__(kBlock) union_near_kernel(
     const uint8_t *__restrict__ cell_has_core, int32_t *parent, unsigned long long *__restrict__ pair_counter,
     int *err, const JobDev *__restrict__ jobs, const int32_t *__restrict__ cell_job) {
     const int64_t idx = (int64_t)blockIdx.x * blockDim.x + threadIdx.x, n_cells = *n_cells_dev;
+    const int only = gridDim.y > 1 ? (int)blockIdx.y : -1;  // this thread's face, -1: all of them
     unsigned pairs = 0;
     if (idx < n_cells && cell_has_core[idx]) {
         const int A = (int)idx;
@@ -1471,9 +1472,11 @@ __global__ void __launch_bounds__(kBlock) union_near_kernel(
         const long long col = col_base + cc[1] + (g.k >= 3 ? cc[2] * g.g[1] : 0);
         const unsigned long long row0 = key - (unsigned long long)cc[0];
         int nb[3] = {-1, -1, -1};
-        if (cc[0] + 1 < g.g[0] && A + 1 < n_cells && (unsigned long long)cell_key[A + 1] == key + 1ull) nb[0] = A + 1;
-        if (g.k >= 2 && cc[1] + 1 < g.g[1]) nb[1] = find_cell(L, cell_key, col + 1, row0 + g.stride[1], cc[0]);
-        if (g.k >= 3 && cc[2] + 1 < g.g[2])
+        if (only <= 0 && cc[0] + 1 < g.g[0] && A + 1 < n_cells && (unsigned long long)cell_key[A + 1] == key + 1ull)
+            nb[0] = A + 1;
+        if ((only < 0 || only == 1) && g.k >= 2 && cc[1] + 1 < g.g[1])
+            nb[1] = find_cell(L, cell_key, col + 1, row0 + g.stride[1], cc[0]);
+        if ((only < 0 || only == 2) && g.k >= 3 && cc[2] + 1 < g.g[2])
             nb[2] = find_cell(L, cell_key, col + g.g[1], row0 + g.stride[2], cc[0]);
         bool any = false;
 #pragma unroll
@@ -1919,7 +1922,10 @@ __global__ void flatten_points_kernel(int32_t *parent, int64_t nv, int *err, con
 // linked grid's cells of >= min_pts points take no part: with the early exit the count
 // records no list there, and with full counts their lists lead all over the stencil
 // (2-D 3M: 0.49 ms of unions against 1.08 with them); the near and cell passes join
-// those cells.
+// those cells.  2^split_log2 threads share a core's list: a thread's unions follow each
+// other, so few points are done sooner by more threads (100k points 2-D: 22 -> 9 us), many
+// points by fewer, whose finds start from the previous union's root (8-D 2M: one thread
+// 0.35 ms, two 0.53, four 1.0).
 #ifndef NDB_LIST_UNIONS
 #define NDB_LIST_UNIONS 16
 #endif
@@ -1929,8 +1935,9 @@ __global__ void union_lists_kernel(int64_t nv, const int32_t *__restrict__ nn_so
                                    const uint8_t *__restrict__ core_sorted, int32_t *parent, int *err,
                                    const JobDev *__restrict__ jobs, const int32_t *__restrict__ cell_job,
                                    const int32_t *__restrict__ pcell, int cell_units,
-                                   const int32_t *__restrict__ cell_start, int min_pts) {
-    const int64_t s = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+                                   const int32_t *__restrict__ cell_start, int min_pts, int split_log2) {
+    const int64_t gid = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+    const int64_t s = gid >> split_log2;
     if (s >= nv || !core_sorted[s]) return;
     int cap = list_cap;
     if (jobs) {
@@ -1945,7 +1952,7 @@ __global__ void union_lists_kernel(int64_t nv, const int32_t *__restrict__ nn_so
     // every union starts its find from the root the previous one left (an ancestor
     // of a), not from a itself
     int ra = a;
-    for (int q = 0; q < len; ++q) {
+    for (int q = (int)(gid & ((1 << split_log2) - 1)); q < len; q += 1 << split_log2) {
         const int j = l[q];
         if (j == (int)s || !core_sorted[j]) continue;
         const int b = cell_units ? pcell[j] : j;
