@@ -144,7 +144,7 @@ constexpr size_t kSmallCountersOff = 512;    // u64[12]: 0 clusters 1 noise 2 co
                                              // 5 band pairs 6 work counter of the persistent count kernel
                                              // 8..11 filter audit (tc::audit_tile)
 constexpr int kCounters = 12;
-constexpr size_t kSmallScalarOff = 1024;     // u32[8]: 0 n_cells 1 n_items 2 n_cores 4 tensor items 5 exact items 6 union segments 7 tensor chunks
+constexpr size_t kSmallScalarOff = 1024;     // u32[8]: 0 n_cells 1 n_items 2 n_cores 4 tensor items 5 exact items 6 and 7 union segments (u64); 7 tensor chunks before
 constexpr size_t kSmallErrOff = 1536;        // int
 constexpr size_t kSmallDoneOff = 1600;       // u32[2]: blocks done of bbox_kernel and finish_kernel (mail_last_block)
 constexpr size_t kSmallBytes = 2048;
@@ -630,9 +630,10 @@ void grid_phase(ndb_ctx *ctx, Pipe &p, const float *coords, F launch_keys) {
 // The tensor-core filter's preconditions: d >= 8 (and, unless NDB_FLAG_TENSOR_FILTER
 // asks for it or counts are full, d at or above the automatic threshold: 12 by
 // measurement on B200, where with early exit the filter beats the exact kernel on
-// full items at d = 16 but not at d = 8; NDB_TC_MIN_DIM overrides), the eps grid (row tables of <= 32 rows), eps^2 a
-// normal float far from under- and overflow, and coordinates within +-2^60 so that
-// no centred difference or squared norm overflows.  Results never depend on it.
+// full items of large pipelines at d = 16 but not at d = 8; NDB_TC_MIN_DIM overrides),
+// the eps grid (row tables of <= 32 rows), eps^2 a normal float far from under- and
+// overflow, and coordinates within +-2^60 so that no centred difference or squared norm
+// overflows.  Results never depend on it.
 inline int default_tc_min_dim() {
     static const int v = [] {
         const char *s = getenv("NDB_TC_MIN_DIM");
@@ -921,7 +922,7 @@ void union_phase(ndb_ctx *ctx, const Pipe &p, unsigned long long *job_counters) 
     cudaStream_t st = ctx->stream;
     const int64_t n = p.n, nv = p.nv, units = p.linked ? p.cells : nv;
     const uint32_t *n_cells = small_at<uint32_t>(ctx, kSmallScalarOff), *n_items = n_cells + 1;
-    uint32_t *n_seg = small_at<uint32_t>(ctx, kSmallScalarOff) + 6;
+    auto *n_seg = reinterpret_cast<unsigned long long *>(small_at<uint32_t>(ctx, kSmallScalarOff) + 6);
     unsigned long long *counters = small_at<unsigned long long>(ctx, kSmallCountersOff);
     int *err = small_at<int>(ctx, kSmallErrOff);
     ensure(ctx, ctx->parent, (units + 1) * sizeof(int32_t));

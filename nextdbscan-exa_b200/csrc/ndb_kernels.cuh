@@ -664,8 +664,8 @@ __device__ __forceinline__ int row_next(const RowTable &rt, int &row, int t) {
 // Neighbour count.  One warp per item (up to 32 points i of one cell).  The i
 // points sit in shared memory; lanes walk the flattened candidates of the
 // stencil rows 32 at a time (coalesced loads), every lane tests its candidate j
-// against each i (broadcast reads) and the warp adds popc(ballot) to that i's
-// count.  Rows are ordered nearest first.
+// against each i (broadcast reads), and transposed hit masks give that i's count.
+// Rows are ordered nearest first.
 // EARLY: stop once every i of the item has reached min_pts (exact counts below
 // min_pts, so exact core flags).  dense_skip: with same-cell-linked cells a cell
 // of >= min_pts points is all cores (every pair inside it is in range), so its
@@ -1338,7 +1338,7 @@ __global__ void scatter_nn_kernel(const int32_t *__restrict__ nn_sorted, int64_t
 // units: no cell root yet (cell_root, null for cell units) and no union segment.
 __global__ void init_units_kernel(int32_t *__restrict__ parent, int32_t *__restrict__ comp_min, int64_t bound,
                                   const uint32_t *__restrict__ n_cells, int32_t *__restrict__ cell_root,
-                                  uint32_t *__restrict__ n_seg) {
+                                  unsigned long long *__restrict__ n_seg) {
     const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (i < bound) {
         parent[i] = (int32_t)i;
@@ -1690,7 +1690,7 @@ __global__ void __launch_bounds__(kBlock) union_select_kernel(
     const int2 *__restrict__ items, const uint32_t *__restrict__ n_items, const int32_t *__restrict__ cell_start,
     const int2 *__restrict__ nbr, int n_rows, const int32_t *__restrict__ cell_root,
     const int32_t *__restrict__ snap, uint32_t *__restrict__ seg_item, uint32_t *__restrict__ seg_part,
-    uint32_t seg_cap, uint32_t *__restrict__ n_seg) {
+    uint32_t seg_cap, unsigned long long *__restrict__ n_seg) {
     __shared__ RowTable s_rows[kWarpsPerBlock];
     __shared__ RowTable s_cells[kWarpsPerBlock];
     __shared__ int s_need[kWarpsPerBlock][kWarp];
@@ -1705,11 +1705,11 @@ __global__ void __launch_bounds__(kBlock) union_select_kernel(
     const int total = union_rows(A, p0, root, cell_start, nbr, n_rows, cell_root, s_rows[wib], s_cells[wib],
                                  s_need[wib], lane);
     const int parts = (int)(((unsigned)total + kUnionSegment - 1) / kUnionSegment);
-    uint32_t base = 0;
-    if (lane == 0 && parts) base = atomicAdd(n_seg, (uint32_t)parts);
+    unsigned long long base = 0;  // 64 bits: the sum must not wrap where it overruns the list
+    if (lane == 0 && parts) base = atomicAdd(n_seg, (unsigned long long)parts);
     base = __shfl_sync(kFull, base, 0);
     for (int q = lane; q < parts; q += kWarp) {
-        const uint64_t at = (uint64_t)base + (uint64_t)q;
+        const unsigned long long at = base + (unsigned long long)q;
         if (at < seg_cap) {
             seg_item[at] = (uint32_t)item_id;
             seg_part[at] = (uint32_t)q;
@@ -1725,8 +1725,8 @@ __global__ void __launch_bounds__(kCountWarps * kWarp) union_scan_kernel(
     const int2 *__restrict__ nbr, int n_rows, const float *__restrict__ xs, float e2,
     const int32_t *__restrict__ cell_root, const int32_t *__restrict__ snap, int32_t *parent,
     const uint32_t *__restrict__ seg_item, const uint32_t *__restrict__ seg_part, uint32_t seg_cap,
-    const uint32_t *__restrict__ n_seg, unsigned long long *__restrict__ pair_counter, int *err, const JobDev *__restrict__ jobs,
-    const int32_t *__restrict__ cell_job) {
+    const unsigned long long *__restrict__ n_seg, unsigned long long *__restrict__ pair_counter, int *err,
+    const JobDev *__restrict__ jobs, const int32_t *__restrict__ cell_job) {
     constexpr int P = Stride<D>::P;
     __shared__ __align__(16) float s_i[kCountWarps][kTile * P];
     __shared__ int s_idx[kCountWarps][kTile];
@@ -1741,7 +1741,7 @@ __global__ void __launch_bounds__(kCountWarps * kWarp) union_scan_kernel(
     RowTable &rt = s_rows[wib];
     unsigned long long pairs = 0;
     const bool listed = *n_seg <= seg_cap;
-    const uint32_t n_work = listed ? *n_seg : *n_items;
+    const uint32_t n_work = listed ? (uint32_t)*n_seg : *n_items;
     for (uint32_t w = blockIdx.x * kCountWarps + wib; w < n_work; w += gridDim.x * kCountWarps) {
         const int2 item = items[listed ? seg_item[w] : w];
         const int A = item.x, p0 = item.y;
