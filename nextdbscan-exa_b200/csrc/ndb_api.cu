@@ -688,9 +688,10 @@ inline bool tc_pays(const ndb_ctx *ctx, int64_t nv, uint32_t flags) {
 }
 
 // The FMA sum with the exact one near eps^2 (count_kernel, kDirect): not the plain form,
-// and eps^2 far enough from underflow for its error bound.
+// and eps^2 far enough from underflow for its error bound, and from overflow for both sums
+// of a pair near eps^2 to be finite.
 inline bool direct_eligible(float e2, uint32_t flags) {
-    return !(flags & NDB_FLAG_EXACT_COUNT) && e2 >= 0x1p-100f;
+    return !(flags & NDB_FLAG_EXACT_COUNT) && e2 >= 0x1p-100f && e2 <= 0x1p100f;
 }
 
 // Which items the tensor kernel takes: it stages every candidate row once per item

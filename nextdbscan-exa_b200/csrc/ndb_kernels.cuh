@@ -854,8 +854,9 @@ __device__ __forceinline__ int gather_points_from(const int2 *__restrict__ nbr_r
 //   kGram    centred dot products with a guard band (d >= 8, see above)
 // kDirect: let S be the real squared distance of the FP32 points.  Both sums consist of
 // rounded differences, squares and at most D additions of non-negative terms, so both are
-// within (D + 2) u S of S (and of underflow, below 2^-140, which e2 >= 2^-100 hides).  If
-// the FMA sum is below e2 - w or above e2 + w with w >= 2 (D + 3) u e2 / (1 - 2 (D + 3) u),
+// within (D + 2) u S of S (and of underflow, below 2^-140, which e2 >= 2^-100 hides; a sum
+// that overflows belongs to a pair whose other sum is above e2 as well, since e2 <= 2^100).
+// If the FMA sum is below e2 - w or above e2 + w with w >= 2 (D + 3) u e2 / (1 - 2 (D + 3) u),
 // the reference's sum lies on the same side; direct_gamma is 2 (D + 8) u.  It costs 2 d + 1
 // operations on the FMA pipe against 3 d (8-D 2M early exit 2.63 -> 2.29 ms, 16-D 200k 1.38
 // -> 1.28 ms).  Used for d >= 4; below, the sum is short.
