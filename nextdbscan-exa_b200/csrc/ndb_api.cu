@@ -124,7 +124,8 @@ struct ndb_ctx {
     int cell_units = 0;
     int n_rows = 0;
     unsigned long long hash_mask = 0;
-    int32_t *nn_late = nullptr;  // ndb_b200_run on device buffers: the label phase writes the counts there
+    // ndb_b200_run on device buffers: the label phase writes the counts there (null outside the call)
+    int32_t *nn_late = nullptr;
     int32_t *ci_user = nullptr;  // caller's cluster_index buffer of the current assign_labels call
     const float *coords_dev = nullptr;  // device coordinates of the current job
     GridDev grid{};
@@ -1137,6 +1138,15 @@ void classify_stats(ndb_ctx *ctx, const Tally &t) {
     S.ms_count_kernel = elapsed(ctx->kev[2], ctx->kev[3]);
 }
 
+// The counts in input order.
+void scatter_counts(ndb_ctx *ctx, int32_t *target) {
+    const int64_t n = ctx->n;
+    for (int64_t lo = 0; lo < n; lo += kScatterWindow)
+        ++launch_counter(), scatter_nn_kernel<<<blocks_for(n), kBlock, 0, ctx->stream>>>(
+            ctx->nn_sorted.as<int32_t>(), ctx->nv, n, ctx->ids0.as<int32_t>(), target, lo,
+            n <= kScatterWindow ? INT64_MAX : lo + kScatterWindow);
+}
+
 template <int D>
 ndb_status classify_impl(ndb_ctx *ctx, const float *coords, int64_t n, float eps, int32_t min_pts, uint32_t flags,
                          int32_t *nn_out) {
@@ -1227,10 +1237,7 @@ ndb_status classify_impl(ndb_ctx *ctx, const float *coords, int64_t n, float eps
             ensure(ctx, ctx->nn_orig, (n + 1) * sizeof(int32_t));
             target = ctx->nn_orig.as<int32_t>();
         }
-        for (int64_t lo = 0; lo < n; lo += kScatterWindow)
-            ++launch_counter(), scatter_nn_kernel<<<blocks_for(n), kBlock, 0, st>>>(
-                ctx->nn_sorted.as<int32_t>(), ctx->nv, n, ctx->ids0.as<int32_t>(), target, lo,
-                n <= kScatterWindow ? INT64_MAX : lo + kScatterWindow);
+        scatter_counts(ctx, target);
         ck(ctx, cudaGetLastError());
         if (!(flags & NDB_FLAG_DEVICE_PTRS)) {
             if (ctx->in_run && ctx->copy_stream) {
@@ -1656,6 +1663,14 @@ static ndb_status run_checked(ndb_ctx *ctx, const float *coords, int64_t n, int3
     ndb_status s = classify_checked(ctx, coords, n, d, eps, min_pts, flags, nn_out);
     ctx->in_run = false;
     if (s == NDB_OK) s = ndb_b200_assign_labels(ctx, cluster_index_out, result);
+    if (ctx->nn_late) {
+        // the labels failed before they wrote the counts, which are whole: the caller gets
+        // them, and a later ndb_b200_assign_labels must not write to this call's buffer
+        scatter_counts(ctx, ctx->nn_late);
+        ctx->nn_late = nullptr;
+        if ((cudaGetLastError() != cudaSuccess || cudaStreamSynchronize(ctx->stream) != cudaSuccess) && s == NDB_OK)
+            s = NDB_ERR_CUDA;
+    }
     if (ctx->nn_pending) {
         // the counts are in the caller's buffer only once their copy is done
         ctx->nn_pending = false;
