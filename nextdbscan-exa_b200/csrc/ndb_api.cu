@@ -242,6 +242,15 @@ inline void ensure_mail(ndb_ctx *ctx, size_t bytes) {
     ctx->mail_bytes = bytes;
 }
 
+// Waits for what a failed call left on the stream.  A call that fails between its launches
+// (a refused allocation) must not return while a kernel may still read or write the
+// mailbox: the next call hands the same slices out again and fills them from the host at
+// once (mail_to_device), so a late write would land in its job table.
+inline void drain(ndb_ctx *ctx) {
+    cudaStreamSynchronize(ctx->stream);
+    cudaGetLastError();
+}
+
 // A 16-byte aligned slice of the mailbox; slices are handed out in order and
 // released together (mail_used = 0) once the stream has drained.
 inline char *mail_slice(ndb_ctx *ctx, size_t bytes) {
@@ -1313,6 +1322,7 @@ ndb_status classify_entry(ndb_ctx *ctx, const float *coords, int64_t n, float ep
     try {
         return classify_impl<D>(ctx, coords, n, eps, m, flags, nn_out);
     } catch (const Fail &f) {
+        drain(ctx);
         ctx->have_state = false;
         return f.st;
     }
@@ -1323,6 +1333,8 @@ ndb_status labels_entry(ndb_ctx *ctx, int32_t *ci_out, ndb_result *result) {
     try {
         return labels_impl<D>(ctx, ci_out, result);
     } catch (const Fail &f) {
+        drain(ctx);
+        ctx->ci_user = nullptr;
         return f.st;
     }
 }
@@ -1453,6 +1465,7 @@ ndb_status border_ids_entry(ndb_ctx *ctx, const int32_t *core_ids, int32_t *ci_o
     try {
         return border_ids_impl<D>(ctx, core_ids, ci_out);
     } catch (const Fail &f) {
+        drain(ctx);
         return f.st;
     }
 }
@@ -1662,15 +1675,15 @@ static ndb_status run_checked(ndb_ctx *ctx, const float *coords, int64_t n, int3
     ctx->in_run = true;
     ndb_status s = classify_checked(ctx, coords, n, d, eps, min_pts, flags, nn_out);
     ctx->in_run = false;
-    if (s == NDB_OK) s = ndb_b200_assign_labels(ctx, cluster_index_out, result);
+    const bool phase1 = s == NDB_OK;
+    if (phase1) s = ndb_b200_assign_labels(ctx, cluster_index_out, result);
     if (ctx->nn_late) {
         // the labels failed before they wrote the counts, which are whole: the caller gets
         // them, and a later ndb_b200_assign_labels must not write to this call's buffer
         scatter_counts(ctx, ctx->nn_late);
         ctx->nn_late = nullptr;
-        if ((cudaGetLastError() != cudaSuccess || cudaStreamSynchronize(ctx->stream) != cudaSuccess) && s == NDB_OK)
-            s = NDB_ERR_CUDA;
     }
+    if (phase1 && s != NDB_OK) drain(ctx);  // phase 1 may still run, and the counts' scatter
     if (ctx->nn_pending) {
         // the counts are in the caller's buffer only once their copy is done
         ctx->nn_pending = false;
@@ -2092,6 +2105,7 @@ ndb_status run_group_entry(ndb_ctx *ctx, ndb_job *jobs, const std::vector<int> &
         run_group<D>(ctx, jobs, members, flags, solo);
         return NDB_OK;
     } catch (const Fail &f) {
+        drain(ctx);
         for (int m : members)
             if (jobs[m].status == NDB_OK) jobs[m].status = f.st;
         return f.st;

@@ -72,3 +72,22 @@ def test_label_phase_past_the_memory_cap(pkg):
             c.run_device(x.data_ptr(), *x.shape, eps, m, nn.data_ptr(), ci.data_ptr(), full_count=True)
         c.set_memory_limit(0)
         check_after_the_failure(pkg, c, x, nn, ci, want)
+
+
+def test_batch_right_after_a_refused_run(pkg):
+    """The refused run's kernels are done when it returns, so the batch that follows at once
+    finds the transfer buffer they share idle."""
+    names = ("c1_n4000", "blobs_d8", "c2_n6000")
+    golden = [load_golden(k) for k in names]
+    problems = [(g["coords"], float(g["eps"]), int(g["min_pts"])) for g in golden]
+    x, eps, m, _, _ = device_job(repeat=10)  # 60,000 points
+    host = np.empty(len(x), dtype=np.int32)
+    with pkg.Context(0) as c:
+        c.run_batched(problems, full_count=True)  # the buffer at its size for the batch
+        for _ in range(10):
+            with pytest.raises(pkg.lib.NdbError, match="INVALID_ARGUMENT"):
+                c.run_device(x.data_ptr(), *x.shape, eps, m, None, host.ctypes.data, full_count=True)
+            for g, (nn, ci, r) in zip(golden, c.run_batched(problems, full_count=True)):
+                np.testing.assert_array_equal(nn, g["nn"])
+                np.testing.assert_array_equal(ci, g["cluster_index"])
+                assert list(r) == list(g["meta"])
