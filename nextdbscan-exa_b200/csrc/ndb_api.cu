@@ -38,7 +38,7 @@ struct ndb_ctx {
     std::string last_cuda_error;
 
     // inputs / per-point arrays
-    DevBuf coords, keys0, keys1, ids0, ids1, flags, pos, pcell, xs;
+    DevBuf coords, keys0, keys1, ids0, ids1, pcell, xs;
     DevBuf nn_sorted, nn_orig, core_sorted, core_bits, core_prefix, ci_sorted, ci_orig, labels;
     // per-cell arrays
     DevBuf cell_start, cell_key, nbr, items, cell_has_core, cell_cid, hash_keys, hash_vals;
@@ -86,6 +86,7 @@ struct ndb_ctx {
     int loaded_d = 0;
     // largest device footprint the context may hold (bytes); 0 = no cap
     size_t mem_limit = 0;
+    bool arena = false;  // the buffers are fixed slices sized for every upper bound (ndb_b200_run_noalloc)
     // count-kernel thresholds set by ndb_b200_set_tuning (0: the library's defaults)
     ndb_tuning tuning{0, 0, 0};
     // bound of the device-side union-find loops (ndb_b200_set_debug_limits; 0: kUfMaxSteps)
@@ -93,8 +94,8 @@ struct ndb_ctx {
 
     template <typename F>
     void for_each_buf(F f) {
-        DevBuf *bufs[] = {&coords,      &keys0,       &keys1,       &ids0,        &ids1,        &flags,
-                          &pos,         &pcell,       &xs,          &nn_sorted,   &nn_orig,     &core_sorted,
+        DevBuf *bufs[] = {&coords,      &keys0,       &keys1,       &ids0,        &ids1,
+                          &pcell,       &xs,          &nn_sorted,   &nn_orig,     &core_sorted,
                           &core_bits,   &core_prefix, &ci_sorted,   &ci_orig,     &labels,      &cell_start,
                           &cell_key,    &nbr,         &items,       &cell_has_core, &cell_cid,
                           &parent,      &comp_min,    &sort_hist,   &small,       &hash_keys,
@@ -521,8 +522,10 @@ struct Pipe {
 
 // Up to this many points a single job's cells are bounded by its points instead of
 // waiting for their count: the launches over the bound cost less than the round trip
-// (1,000 points 2-D: 15 us), and the row table stays under 18 MB.
+// (1,000 points 2-D: 15 us), and the row table stays under 18 MB.  Not under a memory cap
+// (sizes_counted): there every buffer takes the size that the job needs.
 constexpr int64_t kNoCountPoints = int64_t(1) << 16;
+inline bool sizes_counted(const ndb_ctx *ctx) { return ctx->mem_limit && !ctx->arena; }
 
 // State of the grid phase's chain scans, zeroed with the sort's scratch behind it: three
 // tickets, then the state words of the cells', items' and bitmap words' tiles.
@@ -605,7 +608,7 @@ void grid_phase(ndb_ctx *ctx, Pipe &p, const float *coords, F launch_keys) {
                       ctx->pcell.as<int32_t>(), p.early ? nullptr : ctx->nn_sorted.as<int32_t>()},
         nv, nullptr, chain.state[0], chain.ticket + 0, scal + 0, mail_device(ctx, const_cast<const uint32_t *>(m_cells)));
     ck(ctx, cudaGetLastError());
-    if (!p.jobs && nv <= kNoCountPoints) {
+    if (!p.jobs && nv <= kNoCountPoints && !sizes_counted(ctx)) {
         p.cells = nv;
     } else {
         ck(ctx, cudaStreamSynchronize(st));
@@ -631,10 +634,15 @@ void grid_phase(ndb_ctx *ctx, Pipe &p, const float *coords, F launch_keys) {
     p.items = std::min(nv, p.cells + nv / kTile);
     ensure(ctx, ctx->items, (p.items + 1) * sizeof(int2));
     ensure(ctx, ctx->cell_has_core, p.cells + 1);
+    const char *m_items = sizes_counted(ctx) ? mail_slice(ctx, sizeof(uint32_t)) : nullptr;
     ++launch_counter(), chain_scan_kernel<kItemsPer><<<(unsigned)chain_tiles(p.cells, kItemsPer), kChainThreads, 0, st>>>(
         ItemsOp{ctx->cell_start.as<int32_t>(), ctx->items.as<int2>(), ctx->cell_has_core.as<uint8_t>()}, p.cells,
-        scal + 0, chain.state[1], chain.ticket + 1, scal + 1, nullptr);
+        scal + 0, chain.state[1], chain.ticket + 1, scal + 1, m_items ? mail_device(ctx, m_items) : nullptr);
     ck(ctx, cudaGetLastError());
+    if (m_items) {  // for the item-sized buffers of the count
+        ck(ctx, cudaStreamSynchronize(st));
+        p.items = *reinterpret_cast<const volatile uint32_t *>(m_items);
+    }
 }
 
 // The tensor-core filter's preconditions: d >= 8 (and, unless NDB_FLAG_TENSOR_FILTER
@@ -972,11 +980,10 @@ void union_phase(ndb_ctx *ctx, const Pipe &p, unsigned long long *job_counters) 
         ++launch_counter(), flatten_min_cells_kernel<<<blocks_for(p.cells), kBlock, 0, st>>>(
             parent, n_cells, err, cell_start, has_core, core_sorted, perm, core_bits, core_prefix, comp_min);
     } else {
-        // the segment list: n entries, at least one per item
-        ensure(ctx, ctx->flags, (n + 1) * sizeof(uint32_t));
-        ensure(ctx, ctx->pos, (n + 1) * sizeof(uint32_t));
+        // the segment list: n entries, at least one per item, in the sort's other halves,
+        // which nothing reads after the sort
         const uint32_t seg_cap = (uint32_t)n;
-        uint32_t *seg_item = ctx->flags.as<uint32_t>(), *seg_part = ctx->pos.as<uint32_t>();
+        uint32_t *seg_item = ctx->keys1.as<uint32_t>(), *seg_part = ctx->ids1.as<uint32_t>();
         ++launch_counter(), flatten_points_kernel<<<blocks_for(nv), kBlock, 0, st>>>(parent, nv, err, pcell, core_sorted,
                                                                                     ci_sorted, cell_cid);
         cudaEventRecord(ctx->kev[4], st);
@@ -2476,7 +2483,7 @@ constexpr size_t kNaN = NDB_NOALLOC_MAX_POINTS;
 // Capacity of each buffer for jobs of up to kNaN points (upper bounds of the
 // requests the pipeline makes: keys may be 64-bit, coordinates padded to 16).
 enum NaBuf {
-    NA_KEYS0, NA_KEYS1, NA_IDS0, NA_IDS1, NA_FLAGS, NA_POS, NA_PCELL, NA_XS, NA_NN_SORTED, NA_NN_ORIG,
+    NA_KEYS0, NA_KEYS1, NA_IDS0, NA_IDS1, NA_PCELL, NA_XS, NA_NN_SORTED, NA_NN_ORIG,
     NA_CORE_SORTED, NA_CORE_BITS, NA_CORE_PREFIX, NA_CI_SORTED, NA_CI_ORIG, NA_LABELS, NA_CELL_START, NA_CELL_KEY,
     NA_NBR, NA_ITEMS, NA_CELL_HAS_CORE, NA_CELL_CID, NA_PARENT, NA_COMP_MIN, NA_SORT_HIST,
     NA_SMALL, NA_HASH_KEYS, NA_HASH_VALS, NA_NBR_LIST, NA_ITEMS_SPLIT, NA_COUNT
@@ -2513,8 +2520,8 @@ constexpr int kNaMaxDevices = 64;
 NoAllocState g_na_state[kNaMaxDevices];
 
 DevBuf *na_buf(ndb_ctx &c, int b) {
-    DevBuf *bufs[NA_COUNT] = {&c.keys0,       &c.keys1,     &c.ids0,      &c.ids1,         &c.flags,
-                              &c.pos,         &c.pcell,     &c.xs,        &c.nn_sorted,    &c.nn_orig,
+    DevBuf *bufs[NA_COUNT] = {&c.keys0,       &c.keys1,     &c.ids0,      &c.ids1,
+                              &c.pcell,     &c.xs,        &c.nn_sorted,    &c.nn_orig,
                               &c.core_sorted, &c.core_bits, &c.core_prefix, &c.ci_sorted,  &c.ci_orig,
                               &c.labels,      &c.cell_start, &c.cell_key, &c.nbr,
                               &c.items,       &c.cell_has_core, &c.cell_cid, &c.parent,    &c.comp_min,
@@ -2592,6 +2599,7 @@ extern "C" ndb_status ndb_b200_run_noalloc(const float *coords, int64_t n, int32
     // cap the footprint at the slices themselves: a request that would outgrow its
     // slice is refused before any cudaFree/cudaMalloc instead of reallocating
     s.ctx.mem_limit = s.ctx.held_bytes();
+    s.ctx.arena = true;
     s.ctx.list_budget = na_cap(NA_NBR_LIST) - 4;  // lists only where they fit the slice
     s.ctx.col_budget = 0;  // a column table's size follows the bounding box, not n: cells hashed instead
     s.ctx.own_stream = nullptr;
