@@ -302,9 +302,11 @@ const char *ndb_b200_version(void);
  * buffer request beyond its slice of the array returns NDB_ERR_OUT_OF_MEMORY (the
  * slices are sized for the largest request of any job within the limit).
  * The first call on a device does the set-up (it looks up the array's device
- * address and creates the shared state's timing events), so make it before any
- * stream capture.  Calls share the array: they are serialised per device, and GPU
- * work that overlaps a call and touches the same array would race. */
+ * address, pins 16 KiB of host memory for the calls' small transfers and creates the
+ * shared state's timing events), so make it before any stream capture and where an
+ * allocation may synchronise the device; n = 0 is enough.  Calls share the array:
+ * they are serialised per device, and GPU work that overlaps a call and touches the
+ * same array would race. */
 ndb_status ndb_b200_run_noalloc(const float *coords, int64_t n, int32_t d, float eps, int32_t min_pts,
                                 uint32_t flags, int32_t *nn_out, int32_t *cluster_index_out,
                                 ndb_result *result, void *cuda_stream);

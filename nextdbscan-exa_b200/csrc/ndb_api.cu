@@ -2466,7 +2466,9 @@ extern "C" ndb_status ndb_b200_run_batched(ndb_ctx *ctx, ndb_job *jobs, int64_t 
 // synchronise the device at the wrong moment, or a plugin host that hands out
 // only the buffers it owns.  For them this entry point runs the same pipeline as
 // ndb_b200_run with every scratch buffer carved out of one file-scope device
-// array of fixed size, so no call allocates.
+// array of fixed size.  The first call on a device sets up what the calls share (timing
+// events, and a transfer buffer of kMailSingle bytes of pinned host memory) whatever its
+// arguments are, n = 0 included; no later call allocates.
 //
 // The array lives in the library image: every GPU that loads the library holds
 // it until the process exits.  All calls share it and it keeps the last call's
@@ -2575,6 +2577,13 @@ extern "C" ndb_status ndb_b200_run_noalloc(const float *coords, int64_t n, int32
             s.ctx.last_cuda_error = cudaGetErrorString(e);
             cudaGetLastError();
             return NDB_ERR_CUDA;
+        }
+        // the transfer buffer (pinned host memory), kept by the state: a retry finds it
+        try {
+            ensure_mail(&s.ctx, kMailSingle);
+        } catch (const Fail &f) {
+            cudaGetLastError();
+            return f.st;
         }
         // the timing events, kept only once all of them exist (a failed attempt
         // leaves nothing behind, so a retry starts clean)
