@@ -520,12 +520,20 @@ struct Pipe {
     const int32_t *cell_job = nullptr;
 };
 
-// Up to this many points a single job's cells are bounded by its points instead of
-// waiting for their count: the launches over the bound cost less than the round trip
-// (1,000 points 2-D: 15 us), and the row table stays under 18 MB.  Not under a memory cap
-// (sizes_counted): there every buffer takes the size that the job needs.
+// A single job's cells may be bounded by its points instead of waiting for their count:
+// up to this many points the launches over the bound cost less than the round trip (1,000
+// points 2-D: 15 us).  The row table is then sized for as many cells as points, so only
+// where the context holds one of that size or it is small: allocating and freeing it costs
+// a context's first run about 60 us per megabyte (20,000 points 3-D: TIMES20; 60,000 points:
+// TIMES60).  Not under a memory cap (sizes_counted): there every buffer takes the size that the
+// job needs.
 constexpr int64_t kNoCountPoints = int64_t(1) << 16;
+constexpr size_t kNoCountTable = size_t(2) << 20;  // bytes
 inline bool sizes_counted(const ndb_ctx *ctx) { return ctx->mem_limit && !ctx->arena; }
+inline bool cells_bounded(const ndb_ctx *ctx, const Pipe &p) {
+    const size_t table = (size_t)(p.nv * p.stencil->n_rows + 1) * sizeof(int2);
+    return !p.jobs && p.nv <= kNoCountPoints && !sizes_counted(ctx) && table <= std::max(ctx->nbr.bytes, kNoCountTable);
+}
 
 // State of the grid phase's chain scans, zeroed with the sort's scratch behind it: three
 // tickets, then the state words of the cells', items' and bitmap words' tiles.
@@ -608,7 +616,7 @@ void grid_phase(ndb_ctx *ctx, Pipe &p, const float *coords, F launch_keys) {
                       ctx->pcell.as<int32_t>(), p.early ? nullptr : ctx->nn_sorted.as<int32_t>()},
         nv, nullptr, chain.state[0], chain.ticket + 0, scal + 0, mail_device(ctx, const_cast<const uint32_t *>(m_cells)));
     ck(ctx, cudaGetLastError());
-    if (!p.jobs && nv <= kNoCountPoints && !sizes_counted(ctx)) {
+    if (cells_bounded(ctx, p)) {
         p.cells = nv;
     } else {
         ck(ctx, cudaStreamSynchronize(st));
