@@ -110,7 +110,8 @@ typedef struct ndb_stats {
     float ms_sort_kernels;    /* device time of the radix sort (all passes) */
     float ms_count_kernel;    /* device time of the neighbour-count kernel */
     float ms_union_kernel;    /* device time of the main union kernel (cells, or points after the list unions) */
-    float ms_border_kernel;   /* device time of the border kernel */
+    float ms_border_kernel;   /* device time of the kernel that finds the border ids: with neighbour lists the one
+                               * that writes the outputs too (up to 24M points, and batched runs) */
     int32_t sort_passes;      /* radix passes (8 bits each) */
     int32_t key_bytes;        /* 4 or 8 */
     int32_t kernel_launches;  /* kernels launched by the last classify + assign_labels */

@@ -1092,14 +1092,17 @@ const char *labels_phase(ndb_ctx *ctx) {
         // than the copy kernel it saves (3-D 10M: 0.29 against 0.24 ms)
         const bool self = n <= kSelfTallyPoints;
         if (self) m_tally = mail_slice(ctx, kTallyWords * sizeof(uint32_t));
-        if (!lists) border_phase<D>(ctx);
-        cudaEventRecord(ctx->kev[7], st);
+        if (!lists) {
+            border_phase<D>(ctx);
+            cudaEventRecord(ctx->kev[7], st);
+        }
         ++launch_counter(), finish_kernel<<<blocks_for(n), kBlock, 0, st>>>(
             nv, n, ctx->nn_sorted.as<int32_t>(), p.list, p.list_stride, lists, ctx->core_sorted.as<uint8_t>(),
             ctx->cell_units, ctx->pcell.as<int32_t>(), ctx->cell_cid.as<int32_t>(), ctx->ci_sorted.as<int32_t>(),
             ctx->ids0.as<int32_t>(), ctx->core_bits.as<uint32_t>(), ctx->core_prefix.as<uint32_t>(), nn_target, target,
             counters, nullptr, 0, nullptr, small_at<uint32_t>(ctx, kSmallDoneOff) + 1, (int)kTallyWords,
             self ? mail_device(ctx, m_tally) : nullptr);
+        if (lists) cudaEventRecord(ctx->kev[7], st);
         if (!self) m_tally = mail_tally(ctx);
     } else {
         border_phase<D>(ctx);
