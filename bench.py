@@ -742,8 +742,10 @@ def roofline(kind, ms, s, n, hbm_peak, peak_src, clk):
              "border_kernel": s["border_pairs"]}[kind]
     pair_dims = {"count_kernel": s["count_pair_dims"], "union_kernel": s["union_pair_dims"],
                  "border_kernel": s["border_pair_dims"]}[kind]
-    # FP32 pipe operations: the exact sum takes a separately rounded sub, mul and add per
-    # dimension (no FMA credit); the Gram filter one FMA per dimension plus three
+    # FP32 pipe operations, as the library counts them for the form that ran: the exact sum
+    # takes a separately rounded sub, mul and add per dimension, the FMA sum a sub and an FMA
+    # and one addition, the Gram filter one FMA per dimension plus three, a pair on the tensor
+    # cores three (its classification)
     flops = s.get("count_fp32_ops") if kind == "count_kernel" and s.get("count_fp32_ops") else pair_dims * 3
     achieved = flops / (ms / 1000.0) / 1e12
     mhz = clk.get("sm_mhz") or 1965.0

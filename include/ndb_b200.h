@@ -129,8 +129,9 @@ typedef struct ndb_stats {
     double filter_max_err_over_bound; /* largest |D~ - d64| over the error bound the guard band is built from */
     int64_t filter_audited_pairs;     /* pairs measured */
     int64_t filter_misclassified_pairs; /* pairs decided outside the band that the exact predicate decides otherwise */
-    int64_t count_fp32_ops;           /* FP32 pipe operations of the CUDA-core count: 3d per pair for the exact
-                                       * sum, d + 3 per pair with the Gram filter (one FMA per dimension) */
+    int64_t count_fp32_ops;           /* FP32 pipe operations of the count.  Per pair on CUDA cores: 3d for the exact
+                                       * sum, 2d + 1 for the FMA sum (the default at d >= 4), d + 3 with the Gram
+                                       * filter; per pair on the tensor cores 3 (its classification) */
     int32_t gram_filter;              /* 1 when the CUDA-core count ran with the Gram filter (d >= 8) */
 } ndb_stats;
 

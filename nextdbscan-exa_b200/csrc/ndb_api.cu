@@ -135,6 +135,7 @@ struct ndb_ctx {
     ndb_result result{};
     bool have_labels = false;
     ndb_stats stats{};
+    int64_t tensor_pairs = 0;  // of a batched call so far: pairs counted on tensor cores
 };
 
 namespace {
@@ -142,9 +143,9 @@ namespace {
 // layout of ctx->small
 constexpr size_t kSmallBboxOff = 0;          // int[2*kMaxDim]
 constexpr size_t kSmallInvalidOff = 256;     // u64
-constexpr size_t kSmallCountersOff = 512;    // u64[12]: 0 clusters 1 noise 2 count pairs 3 union pairs 4 border pairs
-                                             // 5 band pairs 6 work counter of the persistent count kernel
-                                             // 8..11 filter audit (tc::audit_tile)
+constexpr size_t kSmallCountersOff = 512;    // u64[12]: 0 clusters 1 noise 2 count pairs on CUDA cores 3 union pairs
+                                             // 4 border pairs 5 band pairs 6 work counter of the persistent count
+                                             // kernel 7 count pairs on tensor cores 8..11 filter audit (tc::audit_tile)
 constexpr int kCounters = 12;
 constexpr size_t kSmallScalarOff = 1024;     // u32[8]: 0 n_cells 1 n_items 2 n_cores 4 tensor items 5 exact items 6 and 7 union segments (u64); 7 tensor chunks before
 constexpr size_t kSmallErrOff = 1536;        // int
@@ -768,7 +769,7 @@ void launch_count_tc(ndb_ctx *ctx, int64_t max_chunks, const int2 *chunks, const
             constexpr bool F = decltype(full_c)::value, A = decltype(audit_c)::value;
             ++launch_counter(), tc::count_tc_kernel<D, F, A><<<grid, tc::kThreads, 0, st>>>(
                 chunks, n_chunks, chunk, cell_start, nbr, n_rows, xs, e2, min_pts, nn_sorted, list, list_cap,
-                list_stride, counters + 2, counters + 5, work, small_at<int>(ctx, kSmallErrOff), jobs, cell_job,
+                list_stride, counters + 7, counters + 5, work, small_at<int>(ctx, kSmallErrOff), jobs, cell_job,
                 counters + 8, rec);
         };
         using T = std::true_type;
@@ -1145,7 +1146,16 @@ inline void audit_stats(ndb_stats &S, const unsigned long long *a) {
     S.filter_misclassified_pairs = (int64_t)a[3];
 }
 
-// Counters and times of phase 1 (the label phase leaves counters 2, 5 and 8 to 11 and
+// FP32 pipe operations of a count: `cuda` pairs on CUDA cores in the form that ran (the
+// exact sum's subtraction, multiplication and addition per dimension, the FMA sum's
+// subtraction and FMA per dimension and one addition, the Gram filter's FMA per dimension
+// and three), `tensor` pairs classified after their tensor-core products (an FMA and two
+// additions each).
+inline int64_t fp32_ops(int d, bool gram, bool direct, int64_t cuda, int64_t tensor) {
+    return cuda * (gram ? d + 3 : direct && d >= 4 ? 2 * d + 1 : 3 * d) + 3 * tensor;
+}
+
+// Counters and times of phase 1 (the label phase leaves counters 2, 5 and 7 to 11 and
 // scalars 0, 1 and 4 as phase 1 wrote them).
 template <int D>
 void classify_stats(ndb_ctx *ctx, const Tally &t) {
@@ -1153,9 +1163,10 @@ void classify_stats(ndb_ctx *ctx, const Tally &t) {
     S.n_cells = t.scal[0];
     S.n_tiles = t.scal[1];
     S.tensor_items = ctx->tc_count ? t.scal[4] : 0;
-    S.count_pairs = (int64_t)t.counters[2];
-    S.count_pair_dims = (int64_t)t.counters[2] * D;
-    S.count_fp32_ops = (int64_t)t.counters[2] * (ctx->gram_count ? D + 3 : 3 * D);
+    S.count_pairs = (int64_t)(t.counters[2] + t.counters[7]);
+    S.count_pair_dims = S.count_pairs * D;
+    S.count_fp32_ops = fp32_ops(D, ctx->gram_count, direct_eligible(ctx->e2, ctx->flags_run), (int64_t)t.counters[2],
+                                (int64_t)t.counters[7]);
     S.gram_filter = ctx->gram_count ? 1 : 0;
     S.band_pairs = (int64_t)t.counters[5];
     audit_stats(S, t.counters + 8);
@@ -1883,9 +1894,9 @@ void run_group_keys(ndb_ctx *ctx, ndb_job *jobs, const std::vector<int> &members
         jobs_dev, nj, ctx->core_bits.as<uint32_t>(), ctx->core_prefix.as<uint32_t>(), n, jc);
     ck(ctx, cudaGetLastError());
     cudaEventRecord(ctx->ev[4], st);
-    // count, union, border, band pairs (running totals), then the filter audit
-    // (running over the call's pipelines)
-    const unsigned long long *m_pairs = mail_from_device(ctx, counters + 2, 4, st);
+    // counters 2 to 7 (pairs: running totals over the call's pipelines), then the filter
+    // audit (running as well)
+    const unsigned long long *m_pairs = mail_from_device(ctx, counters + 2, 6, st);
     const unsigned long long *m_audit = mail_from_device(ctx, counters + 8, 4, st);
     const unsigned long long *m_jc = mail_from_device(ctx, jc, (size_t)4 * nj, st);
     const uint32_t *m_scal = mail_from_device(ctx, scal, 8, st);
@@ -1903,7 +1914,7 @@ void run_group_keys(ndb_ctx *ctx, ndb_job *jobs, const std::vector<int> &members
         }
     }
     ck(ctx, cudaStreamSynchronize(st));
-    unsigned long long h_pairs[4], h_audit[4];
+    unsigned long long h_pairs[6], h_audit[4];
     memcpy(h_pairs, m_pairs, sizeof(h_pairs));
     memcpy(h_audit, m_audit, sizeof(h_audit));
     const std::vector<unsigned long long> h_jc(m_jc, m_jc + (size_t)4 * nj);
@@ -1914,8 +1925,9 @@ void run_group_keys(ndb_ctx *ctx, ndb_job *jobs, const std::vector<int> &members
     ndb_stats &S = ctx->stats;
     S.pipelines += 1;
     // pair counters run on over the pipelines of a call: this pipeline's share
-    const int64_t dc = (int64_t)h_pairs[0] - S.count_pairs, du = (int64_t)h_pairs[1] - S.union_pairs,
-                  db = (int64_t)h_pairs[2] - S.border_pairs;
+    const int64_t dt = (int64_t)h_pairs[5] - ctx->tensor_pairs, du = (int64_t)h_pairs[1] - S.union_pairs,
+                  dc = (int64_t)(h_pairs[0] + h_pairs[5]) - S.count_pairs, db = (int64_t)h_pairs[2] - S.border_pairs;
+    ctx->tensor_pairs += dt;
     S.band_pairs = (int64_t)h_pairs[3];
     audit_stats(S, h_audit);
     S.tensor_items += h_tc_items;
@@ -1924,7 +1936,7 @@ void run_group_keys(ndb_ctx *ctx, ndb_job *jobs, const std::vector<int> &members
     S.union_pairs += du;
     S.border_pairs += db;
     S.count_pair_dims += dc * D;
-    S.count_fp32_ops += dc * (bp.gram ? D + 3 : 3 * D);
+    S.count_fp32_ops += fp32_ops(D, bp.gram, bp.direct, dc - dt, dt);
     S.gram_filter |= bp.gram ? 1 : 0;
     S.union_pair_dims += du * D;
     S.border_pair_dims += db * D;
@@ -2283,6 +2295,7 @@ extern "C" ndb_status ndb_b200_run_batched(ndb_ctx *ctx, ndb_job *jobs, int64_t 
     ctx->have_state = false;
     ctx->have_labels = false;
     ctx->stats = ndb_stats{};
+    ctx->tensor_pairs = 0;
     launch_counter() = 0;
     if (grow(ctx, ctx->small, kSmallBytes) != cudaSuccess) return NDB_ERR_OUT_OF_MEMORY;
     try {
