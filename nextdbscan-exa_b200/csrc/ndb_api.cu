@@ -524,10 +524,11 @@ struct Pipe {
 // A single job's cells may be bounded by its points instead of waiting for their count:
 // up to this many points the launches over the bound cost less than the round trip (1,000
 // points 2-D: 15 us).  The row table is then sized for as many cells as points, so only
-// where the context holds one of that size or it is small: allocating and freeing it costs
-// a context's first run about 60 us per megabyte (20,000 points 3-D: TIMES20; 60,000 points:
-// TIMES60).  Not under a memory cap (sizes_counted): there every buffer takes the size that the
-// job needs.
+// where the context holds one of that size or it is small: allocating and freeing the
+// larger one costs a context's first run more than the round trip (a new context, one run,
+// its release, counted against bounded cells: 20,000 points 3-D 1.34 against 1.94 ms, 60,000
+// points 2.61 against 3.69 ms).  Not under a memory cap (sizes_counted): there every buffer
+// takes the size that the job needs.
 constexpr int64_t kNoCountPoints = int64_t(1) << 16;
 constexpr size_t kNoCountTable = size_t(2) << 20;  // bytes
 inline bool sizes_counted(const ndb_ctx *ctx) { return ctx->mem_limit && !ctx->arena; }
