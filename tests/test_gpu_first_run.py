@@ -1,6 +1,7 @@
 """A context's first run allocates for the cells that the job has: a dense job of up to
 65,536 points does not get a row table for as many cells as points (12 MB here, where the
-job's buffers need 6), whose allocation would cost more than the rest of the run."""
+job's buffers need 6), whose allocation would cost more than the rest of the run.  Later
+runs may: the context is then one that comes back."""
 import numpy as np
 import pytest
 
@@ -15,9 +16,9 @@ def test_first_run_of_a_dense_job(pkg):
     x = (rng.integers(0, 3, (n, 3)) * 6 + rng.normal(0, 0.25, (n, 3))).astype(np.float32)
     nn_o, ci_o, meta = oracle.grid(x, 1.0, 5)
     with pkg.Context(0) as c:
-        for _ in range(2):
+        for first in (True, False):
             nn, ci, r = c.run(x, 1.0, 5, full_count=True)
             np.testing.assert_array_equal(nn, nn_o)
             np.testing.assert_array_equal(ci, ci_o)
             assert (r.clusters, r.noise, r.core_count) == (meta["clusters"], meta["noise"], meta["cores"])
-            assert c.device_bytes() < 12 << 20
+            assert c.device_bytes() < 12 << 20 or not first
