@@ -789,11 +789,18 @@ void launch_count_tc(ndb_ctx *ctx, int64_t max_chunks, const int2 *chunks, const
 // tail).  Early exit: enough to keep the columns filled (a chunk's last points run with
 // ever fewer), few enough that every resident CTA gets several chunks: 16-D 200k 64
 // points 1.40 ms, 256 points 2.23 ms; the 4,096-job batch's counts 32 points 143 ms, 64
-// 128 ms, 256 117 ms, 512 116 ms.
-inline int tc_chunk(const ndb_ctx *ctx, int64_t nv, bool early) {
+// 128 ms, 256 117 ms, 512 116 ms.  A larger minPts makes a chunk longer and its points more
+// alike, so from 32 on a CTA gets ten chunks instead of four where that leaves 64 points,
+// and from 512 on, where most points need the whole round, a chunk has no more than 64: at
+// 16-D 1M chunks of 64, 128 and 256 points take 18.6, 18.0 and 21.5 ms at minPts 32, 20.3,
+// 21.1 and 25.1 ms at 64, and 26.1, 26.8 and 32.6 ms at 1,024; 12-D 1M at minPts 24, where
+// points are done early, 8.7, 6.5 and 5.5 ms.
+inline int tc_chunk(const ndb_ctx *ctx, int64_t nv, int min_pts, bool early) {
     if (!early) return tc::kN;
-    const int64_t per = nv / ((int64_t)ctx->sm_count * 5 * 4);
-    return (int)std::min<int64_t>(std::max<int64_t>(per / tc::kN * tc::kN, tc::kN), 256);
+    const int64_t ctas = (int64_t)ctx->sm_count * 5, chunks = min_pts >= 32 ? 10 : 4;
+    const int64_t per = std::max(std::min<int64_t>(nv / (ctas * 4), 2 * tc::kN), nv / (ctas * chunks));
+    const int64_t most = min_pts >= 512 ? 2 * tc::kN : 8 * tc::kN;
+    return (int)std::min<int64_t>(std::max<int64_t>(per / tc::kN * tc::kN, tc::kN), most);
 }
 
 // The neighbour count of one pipeline.  tc: the tensor-core filter may run (input
@@ -815,7 +822,7 @@ void count_items(ndb_ctx *ctx, bool tc, bool force_tc, bool gram, bool direct, b
         ensure(ctx, ctx->items_split, (size_t)(2 * n_items + 2) * sizeof(int2));
         int2 *chunks = ctx->items_split.as<int2>();
         int2 *rest = chunks + n_items + 1;
-        const int chunk = tc_chunk(ctx, nv, early);
+        const int chunk = tc_chunk(ctx, nv, min_pts, early);
         fill_bytes(ctx, scal + 4, 0, 4 * sizeof(uint32_t), st);
         ++launch_counter(), tc::split_cells_kernel<<<blocks_for(n_cells), kBlock, 0, st>>>(
             cell_start, scal + 0, force_tc ? 1 : ctx_tc_min_item(ctx), chunk, chunks, scal + 7, rest, scal + 5, scal + 4);
