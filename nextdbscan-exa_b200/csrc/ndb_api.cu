@@ -950,7 +950,12 @@ void classify_dispatch(ndb_ctx *ctx, const Plan &pl) {
 // unions of a cell by one thread per face: there the unions are a chain of latencies
 // (3-D 10M, 0.9M cells: union phase 0.98 -> 0.94 ms by faces); beyond, the GPU is full
 // anyway (skewed 2-D 100M, 5.8M cells: 6.23 against 6.32 ms).
-constexpr int64_t kSplitListPoints = int64_t(1) << 17, kSplitFaceCells = int64_t(1) << 22;
+// Over points (grids that are not linked) the threads of a list meet at the same roots when
+// many points lie within eps of each other, so there only the smallest jobs split: 16-D 66,000
+// points, all near, 1.26 ms of unions by four threads, 0.66 by two, 0.34 by one; 8-D 66,000
+// clustered 0.19 by four and 0.17 by one, but 1,000 points 0.058 and 0.089.
+constexpr int64_t kSplitListPoints = int64_t(1) << 17, kSplitListPointUnits = int64_t(1) << 14;
+constexpr int64_t kSplitFaceCells = int64_t(1) << 22;
 
 // Union-find, component minima and core ids of a pipeline.  ci_sorted holds the roots'
 // snapshot until the ids are written, cell_cid (point units) the cells' roots.
@@ -978,7 +983,7 @@ void union_phase(ndb_ctx *ctx, const Pipe &p, unsigned long long *job_counters) 
 
     ++launch_counter(), init_units_kernel<<<blocks_for(units), kBlock, 0, st>>>(
         parent, comp_min, units, n_cells, p.linked ? nullptr : cell_cid, n_seg);
-    const int split_log2 = nv <= kSplitListPoints ? 2 : 0;
+    const int split_log2 = nv <= (p.linked ? kSplitListPoints : kSplitListPointUnits) ? 2 : 0;
     if (p.list_stride > 0)
         ++launch_counter(), union_lists_kernel<<<blocks_for(nv << split_log2), kBlock, 0, st>>>(
             nv, ctx->nn_sorted.as<int32_t>(), p.list, p.list_cap, p.list_stride, core_sorted, parent, err, p.jobs,
