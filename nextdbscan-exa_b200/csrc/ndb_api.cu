@@ -988,6 +988,9 @@ void union_phase(ndb_ctx *ctx, const Pipe &p, unsigned long long *job_counters) 
         ++launch_counter(), union_lists_kernel<<<blocks_for(nv << split_log2), kBlock, 0, st>>>(
             nv, ctx->nn_sorted.as<int32_t>(), p.list, p.list_cap, p.list_stride, core_sorted, parent, err, p.jobs,
             p.cell_job, pcell, p.linked, cell_start, p.min_pts, split_log2);
+    if (p.list_stride > 0 && !p.linked && !p.early)
+        ++launch_counter(), union_middle_kernel<D><<<blocks_for(nv), kBlock, 0, st>>>(
+            nv, pcell, cell_start, xs, p.e2, core_sorted, parent, err, p.jobs, p.cell_job);
     if (p.linked) {
         const unsigned faces = p.cells <= kSplitFaceCells ? (unsigned)std::min(D, 3) : 1u;
         ++launch_counter(), union_near_kernel<D, K><<<dim3(blocks_for(p.cells), faces), kBlock, 0, st>>>(

@@ -1970,6 +1970,30 @@ __global__ void union_lists_kernel(int64_t nv, const int32_t *__restrict__ nn_so
     }
 }
 
+// Exact counts over points, after the list unions: a core joins the middle core of its cell
+// when that is in range.  Such a count fills a list with hits around the item it came
+// from (every pair is met once, from the item that comes first), so on data that fill a cell
+// densely the lists leave one component per item, and every item then walks its whole
+// stencil: 9-D 66,000 uniform points, all near, union phase 1.47 -> 0.14 ms; 5-D 300k clustered
+// 0.18 -> 0.15 ms, 8-D 2M 1.47 -> 1.51 ms.  One distance per core that is not joined yet.
+template <int D>
+__global__ void union_middle_kernel(int64_t nv, const int32_t *__restrict__ pcell,
+                                    const int32_t *__restrict__ cell_start, const float *__restrict__ xs, float e2,
+                                    const uint8_t *__restrict__ core_sorted, int32_t *parent, int *err,
+                                    const JobDev *__restrict__ jobs, const int32_t *__restrict__ cell_job) {
+    const int64_t s = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+    if (s >= nv || !core_sorted[s]) return;
+    const int c = pcell[s], cs = cell_start[c], mid = cs + (cell_start[c + 1] - cs) / 2;
+    if (mid == (int)s || !core_sorted[mid]) return;
+    const int ra = uf_find(parent, (int)s, err), rm = uf_find(parent, mid, err);
+    if (ra == rm) return;
+    if (jobs) e2 = jobs[cell_job[c]].e2;
+    float xa[D], xm[D];
+    load_point<D>(xs, (int)s, xa);
+    load_point<D>(xs, mid, xm);
+    if (in_range<D>(xa, xm, e2)) uf_union_root(parent, ra, rm, err);
+}
+
 // After the list and near unions of cell units: parent[u] = root of u (thread u is its
 // only writer, with read-only finds), and each cell's root in snap (-1 for a cell
 // without cores) for the candidate filter of union_cells_kernel.

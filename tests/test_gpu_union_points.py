@@ -45,3 +45,20 @@ def test_more_segments_than_the_list_holds(ctx):
     assert tuple(r) == (2, 0, 200_000, 200_000)
     # the smallest point of the balls: 0 (the second ball) and 2 (the first)
     np.testing.assert_array_equal(ci, np.where(ball, 0, 2))
+
+
+@pytest.mark.parametrize("d,m", [(4, 2), (9, 32), (16, 28)])
+def test_exact_counts_on_points_all_near_leave_little_to_the_scan(ctx, d, m):
+    """20,000 points within eps of each other, 625 items: joined before the scan of
+    candidates, which would otherwise test every item against hundreds of others."""
+    x = np.random.default_rng(d).uniform(0, 1, (20_000, d)).astype(np.float32)
+    nn, ci, r = ctx.run(x, 1.01 * np.sqrt(d), m, full_count=True)
+    assert tuple(r) == (1, 0, 20_000, 20_000)
+    np.testing.assert_array_equal(nn, 20_000)
+    np.testing.assert_array_equal(ci, 0)
+    assert ctx.stats()["union_pairs"] < 20_000
+    (nn, ci, r), (nn2, ci2, r2) = ctx.run_batched([(x, 1.01 * np.sqrt(d), m), (x[:777], 1.01 * np.sqrt(d), m)],
+                                                  full_count=True)
+    assert tuple(r) == (1, 0, 20_000, 20_000) and tuple(r2) == (1, 0, 777, 777)
+    np.testing.assert_array_equal(ci, 0)
+    assert ctx.stats()["union_pairs"] < 20_777
