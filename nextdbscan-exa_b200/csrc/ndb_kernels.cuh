@@ -866,7 +866,7 @@ template <int D, int MODE>
 __global__ void __launch_bounds__(kCountWarps * kWarp) count_kernel(
     const int2 *__restrict__ items, const uint32_t *__restrict__ n_items, const int32_t *__restrict__ cell_start,
     const int2 *__restrict__ nbr, int n_rows, const float *__restrict__ xs, float e2, int min_pts,
-    int dense_skip, int32_t *__restrict__ nn_sorted, int32_t *__restrict__ nbr_list, int list_cap,
+    int dense_skip, int all, int32_t *__restrict__ nn_sorted, int32_t *__restrict__ nbr_list, int list_cap,
     int list_stride, unsigned long long *__restrict__ pair_counter, const JobDev *__restrict__ jobs,
     const int32_t *__restrict__ cell_job, unsigned long long *__restrict__ band_counter) {
     constexpr int P = Stride<D>::P;
@@ -895,6 +895,10 @@ __global__ void __launch_bounds__(kCountWarps * kWarp) count_kernel(
         min_pts = J.min_pts;
         dense_skip = J.linked;
         list_cap = J.list_cap;
+    }
+    if (all) {  // exact counts (sparse cells): no point leaves
+        min_pts = 0x7fffffff;
+        dense_skip = 0;
     }
     if (dense_skip && ce - cs >= min_pts) {
         if (lane < cnt) nn_sorted[p0 + lane] = ce - cs;

@@ -60,3 +60,51 @@ def test_pairs_exactly_at_eps(ctx, d, eps):
             np.testing.assert_array_equal(nn if full else np.minimum(nn, m), nn_o if full else np.minimum(nn_o, m))
             np.testing.assert_array_equal(ci, ci_o)
             assert (r.clusters, r.noise, r.core_count) == (meta["clusters"], meta["noise"], meta["cores"])
+
+
+@pytest.mark.parametrize("d", [4, 5, 7, 8, 9, 13, 16])
+def test_default_count_items_against_oracle(ctx, d):
+    """The same shapes by the FMA sum, the default at d >= 4."""
+    x = clumps(d, SIZES, 100 + d)
+    ctx.set_tuning(tc_min_dim=17)  # CUDA cores
+    try:
+        for m in (1, 2, 17, 33, 66):
+            nn_o, ci_o, meta = oracle.grid(x, 1.0, m)
+            for full in (True, False):
+                nn, ci, r = ctx.run(x, 1.0, m, full_count=full)
+                np.testing.assert_array_equal(nn if full else np.minimum(nn, m), nn_o if full else np.minimum(nn_o, m))
+                np.testing.assert_array_equal(ci, ci_o)
+                assert (r.clusters, r.noise, r.core_count) == (meta["clusters"], meta["noise"], meta["cores"])
+    finally:
+        ctx.reset_tuning()
+
+
+@pytest.mark.parametrize("d", [1, 2, 3, 4, 8, 16])
+@pytest.mark.parametrize("extra", [0, 499, 501, 1000, 3999, 4001])
+def test_cells_of_little_more_than_a_point(pkg, d, extra):
+    """1,000 places on a jittered line or lattice, some with more points: the exact counts of
+    grids with fewer than 3/2 points per cell (d <= 2: 5), and just above, have a form of
+    their own.  Every third place is within eps of the next."""
+    rng = np.random.default_rng(d + extra)
+    at = np.zeros((1000, d))
+    q = np.arange(1000)
+    for k, side in zip(range(min(d, 3)), {1: (1000,), 2: (40, 25), 3: (10, 10, 10)}[min(d, 3)]):
+        at[:, k] = 2.6 * (q % side)
+        q = q // side
+    at[::3, 0] += 1.75  # towards the next place
+    x = np.concatenate([at, at[np.arange(extra) % 1000]])
+    x = (x + rng.uniform(-0.02, 0.02, x.shape)).astype(np.float32)
+    x = np.ascontiguousarray(x[rng.permutation(len(x))])
+    for m in (1, 2, 3, 70):
+        nn_o, ci_o, meta = oracle.grid(x, 1.0, m)
+        for kw in ({}, {"exact_count": True}, {"gram_filter": True}) if d >= 8 else ({}, {"exact_count": True}):
+            for full in (True, False):
+                with pkg.Context(0) as c:  # a first run knows its cells' number, and so does a batch
+                    c.set_tuning(tc_min_dim=17)
+                    got = [c.run(x, 1.0, m, full_count=full, **kw)]
+                    got += c.run_batched([(x, 1.0, m), (x, 1.0, m)], full_count=full, **kw)
+                for nn, ci, r in got:
+                    np.testing.assert_array_equal(nn if full else np.minimum(nn, m),
+                                                  nn_o if full else np.minimum(nn_o, m))
+                    np.testing.assert_array_equal(ci, ci_o)
+                    assert (r.clusters, r.noise, r.core_count) == (meta["clusters"], meta["noise"], meta["cores"])
