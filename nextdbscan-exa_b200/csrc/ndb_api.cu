@@ -53,6 +53,7 @@ struct ndb_ctx {
     size_t list_budget = size_t(8) << 30;  // largest list buffer the context may use (else: scan border)
     int list_cap = 0;                 // entries per point, 0 when the lists are off
     bool tc_count = false;            // neighbour count on the tensor-core filter
+    bool sparse = false;              // few points per cell (Pipe::sparse)
     bool gram_count = false;          // CUDA-core count with the Gram filter (d >= 8)
     int sm_count = 148;
     // scratch
@@ -631,6 +632,7 @@ void grid_phase(ndb_ctx *ctx, Pipe &p, const float *coords, F launch_keys) {
     ck(ctx, cudaGetLastError());
     if (cells_bounded(ctx, p)) {
         p.cells = nv;
+        p.sparse = false;
     } else {
         ck(ctx, cudaStreamSynchronize(st));
         p.cells = nv > 0 ? *m_cells : 0;
@@ -910,6 +912,7 @@ void classify_keys(ndb_ctx *ctx, Pipe &p) {
             ctx->coords_dev, n, rows_aligned<D>(ctx->coords_dev), p.g, invalid_key, keys, core_bits, zero);
     });
     ctx->n_cells = p.cells;
+    ctx->sparse = p.sparse;
     ctx->n_items = p.items;
     // neighbour lists for the border step: min_pts - 1 entries per point
     const int64_t cap = (int64_t)ctx->min_pts - 1;
@@ -938,6 +941,7 @@ Pipe ctx_pipe(ndb_ctx *ctx) {
     p.list = ctx->list_cap ? ctx->nbr_list.as<int32_t>() : nullptr;
     p.list_cap = p.list_stride = ctx->list_cap;
     p.cells = ctx->n_cells;
+    p.sparse = ctx->sparse;
     p.items = ctx->n_items;
     return p;
 }
@@ -1021,11 +1025,15 @@ void union_phase(ndb_ctx *ctx, const Pipe &p, unsigned long long *job_counters) 
         // which nothing reads after the sort
         const uint32_t seg_cap = (uint32_t)n;
         uint32_t *seg_item = ctx->keys1.as<uint32_t>(), *seg_part = ctx->ids1.as<uint32_t>();
+        // without lists and with a point or two per cell hardly an item is settled beforehand
+        // and none is long: the scan takes the items themselves (no segment list)
+        if (p.list_stride == 0 && p.sparse) seg_item = nullptr;
         ++launch_counter(), flatten_points_kernel<<<blocks_for(nv), kBlock, 0, st>>>(parent, nv, err, pcell, core_sorted,
                                                                                     ci_sorted, cell_cid);
         cudaEventRecord(ctx->kev[4], st);
-        ++launch_counter(), union_select_kernel<<<blocks_for(p.items * kWarp), kBlock, 0, st>>>(
-            items, n_items, cell_start, nbr, n_rows, cell_cid, ci_sorted, seg_item, seg_part, seg_cap, n_seg);
+        if (seg_item)
+            ++launch_counter(), union_select_kernel<<<blocks_for(p.items * kWarp), kBlock, 0, st>>>(
+                items, n_items, cell_start, nbr, n_rows, cell_cid, ci_sorted, seg_item, seg_part, seg_cap, n_seg);
         const unsigned scan_blocks = (unsigned)std::min<int64_t>(p.items / kCountWarps + 1, (int64_t)ctx->sm_count * 32);
         ++launch_counter(), union_scan_kernel<D><<<scan_blocks, kCountWarps * kWarp, 0, st>>>(
             items, n_items, cell_start, nbr, n_rows, xs, p.e2, cell_cid, ci_sorted, parent, seg_item, seg_part, seg_cap,
