@@ -526,15 +526,16 @@ struct Pipe {
 
 // A single job's cells may be bounded by its points instead of waiting for their count:
 // up to this many points the launches over the bound cost less than the round trip (1,000
-// points 2-D: 15 us).  The row table is then sized for as many cells as points, whose
-// allocation and release cost a context that makes one run more than the round trip (a new
-// context, one run, its release, counted against bounded cells: 20,000 points 3-D 1.34
-// against 1.94 ms, 60,000 points 2.61 against 3.69 ms): so a context's first run counts,
-// unless the table is small, and its later ones, for which the table is there, are bounded.
-// Not under a memory cap (sizes_counted): there every buffer takes the size that the job
-// needs.
+// points 2-D: 15 us).  The row table and the other per-cell buffers are then sized for as
+// many cells as points, and every further 2 MB that the driver maps for them and releases
+// costs a context that makes one run about 0.6 ms (a new context, one run, its release,
+// counted against bounded cells: 52,000 points 2-D 1.24 against 2.45 ms, 7,000 points 16-D
+// with exact counts 1.33 against 2.05, 60,000 points 3-D 2.61 against 3.69 ms).  So a
+// context's first run counts, unless the table is tiny, and its later ones, for which the
+// table is there, are bounded.  Not under a memory cap (sizes_counted): there every buffer
+// takes the size that the job needs.
 constexpr int64_t kNoCountPoints = int64_t(1) << 16;
-constexpr size_t kNoCountTable = size_t(2) << 20;  // bytes
+constexpr size_t kNoCountTable = size_t(64) << 10;  // bytes
 inline bool sizes_counted(const ndb_ctx *ctx) { return ctx->mem_limit && !ctx->arena; }
 inline bool cells_bounded(const ndb_ctx *ctx, const Pipe &p) {
     const size_t table = (size_t)(p.nv * p.stencil->n_rows + 1) * sizeof(int2);

@@ -22,3 +22,17 @@ def test_first_run_of_a_dense_job(pkg):
             np.testing.assert_array_equal(ci, ci_o)
             assert (r.clusters, r.noise, r.core_count) == (meta["clusters"], meta["noise"], meta["cores"])
             assert c.device_bytes() < 12 << 20 or not first
+
+
+def test_first_run_of_a_small_job_sizes_its_row_table_by_its_cells(pkg):
+    """40,000 points in few cells, 2-D: five stencil rows of 8 bytes a cell.  The second run
+    bounds the cells by the points, 1.6 MB of rows; the first one has counted them."""
+    x = np.random.default_rng(2).uniform(0, 10, (40_000, 2)).astype(np.float32)
+    with pkg.Context(0) as c:
+        nn, ci, _ = c.run(x, 1.0, 5)
+        first = c.device_bytes()
+        assert c.stats()["n_cells"] < 400
+        nn2, ci2, _ = c.run(x, 1.0, 5)
+        assert first + 1_500_000 < c.device_bytes()
+    np.testing.assert_array_equal(ci, ci2)
+    np.testing.assert_array_equal(np.minimum(nn, 5), np.minimum(nn2, 5))
