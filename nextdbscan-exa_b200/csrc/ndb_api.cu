@@ -972,6 +972,7 @@ void classify_dispatch(ndb_ctx *ctx, const Plan &pl) {
 // clustered 0.19 by four and 0.17 by one, but 1,000 points 0.058 and 0.089.
 constexpr int64_t kSplitListPoints = int64_t(1) << 17, kSplitListPointUnits = int64_t(1) << 14;
 constexpr int64_t kSplitFaceCells = int64_t(1) << 22;
+constexpr int kShortLists = 4;  // entries per list below which union_middle_kernel runs with the early exit too
 
 // Union-find, component minima and core ids of a pipeline.  ci_sorted holds the roots'
 // snapshot until the ids are written, cell_cid (point units) the cells' roots.
@@ -1004,7 +1005,7 @@ void union_phase(ndb_ctx *ctx, const Pipe &p, unsigned long long *job_counters) 
         ++launch_counter(), union_lists_kernel<<<blocks_for(nv << split_log2), kBlock, 0, st>>>(
             nv, ctx->nn_sorted.as<int32_t>(), p.list, p.list_cap, p.list_stride, core_sorted, parent, err, p.jobs,
             p.cell_job, pcell, p.linked, cell_start, p.min_pts, split_log2);
-    if (p.list_stride > 0 && !p.linked && !p.early)
+    if (p.list_stride > 0 && !p.linked && (!p.early || p.list_stride < kShortLists))
         ++launch_counter(), union_middle_kernel<D><<<blocks_for(nv), kBlock, 0, st>>>(
             nv, pcell, cell_start, xs, p.e2, core_sorted, parent, err, p.jobs, p.cell_job);
     if (p.linked) {

@@ -1982,12 +1982,15 @@ __global__ void union_lists_kernel(int64_t nv, const int32_t *__restrict__ nn_so
     }
 }
 
-// Exact counts over points, after the list unions: a core joins the middle core of its cell
+// Exact counts over points (and short lists), after the list unions: a core joins the middle core of its cell
 // when that is in range.  Such a count fills a list with hits around the item it came
 // from (every pair is met once, from the item that comes first), so on data that fill a cell
 // densely the lists leave one component per item, and every item then walks its whole
 // stencil: 9-D 66,000 uniform points, all near, union phase 1.47 -> 0.14 ms; 5-D 300k clustered
 // 0.18 -> 0.15 ms, 8-D 2M 1.47 -> 1.51 ms.  One distance per core that is not joined yet.
+// With the early exit, whose lists begin with the first hits of the nearest row and so meet
+// in the same points, only lists of fewer than kShortLists entries need it: minPts 2, 13-D
+// 300k uniform points 47.6 -> 4.4 ms, 8-D 200k 9.8 -> 3.7 ms, 8-D 300k clustered 0.44 both ways.
 template <int D>
 __global__ void union_middle_kernel(int64_t nv, const int32_t *__restrict__ pcell,
                                     const int32_t *__restrict__ cell_start, const float *__restrict__ xs, float e2,
