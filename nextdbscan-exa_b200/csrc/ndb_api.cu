@@ -53,6 +53,7 @@ struct ndb_ctx {
     size_t list_budget = size_t(8) << 30;  // largest list buffer the context may use (else: scan border)
     int list_cap = 0;                 // entries per point, 0 when the lists are off
     bool tc_count = false;            // neighbour count on the tensor-core filter
+    bool tc_defer = false;            // the CUDA-core count may hand items on to the tensor-core one
     bool sparse = false;              // few points per cell (Pipe::sparse)
     bool gram_count = false;          // CUDA-core count with the Gram filter (d >= 8)
     int sm_count = 148;
@@ -521,6 +522,7 @@ struct Pipe {
     // point each (kSparse), and the batch's cell -> job map
     int64_t cells = 0, items = 0;
     bool sparse = false;
+    bool defer = false;  // the CUDA-core count may hand items on (kDeferDim)
     const int32_t *cell_job = nullptr;
 };
 
@@ -718,17 +720,24 @@ inline bool gram_eligible(const ndb_ctx *ctx, int d, float e2, const double *lo,
     return true;
 }
 
-// Whether an eligible pipeline of nv points takes the tensor-core filter.  Full counts do.
-// With early exit the CUDA-core count, whose cost follows the points still counting, is
-// faster until a pipeline has thousands of full chunks per CTA: 16-D 200k 1.05 against 1.28
-// ms, 16-D 1M 14.1 against 16.8 ms, 12-D 1M 6.7 against 9.5 ms, a 512-job batch (5M points
-// at d = 16) 13.9 against 14.5 ms; the 4,096-job batch (40M) 122 against 116 ms.  A caller's
-// flag or tuning decides alone.
+// Whether an eligible pipeline of nv points takes the tensor-core filter from the start.  Full
+// counts do.  With early exit the CUDA-core count, whose cost follows the points still
+// counting, is faster on clustered data until a pipeline has thousands of full chunks per
+// CTA: 16-D 200k 1.05 against 1.28 ms, 16-D 1M 14.1 against 16.8 ms, 12-D 1M 6.7 against 9.5
+// ms, a 512-job batch (5M points at d = 16) 13.9 against 14.5 ms; the 4,096-job batch (40M)
+// 122 against 116 ms.  Below that, items whose points are not done early go there all the
+// same (may_defer).  A caller's flag or tuning decides alone.
 constexpr int64_t kTcEarlyPoints = int64_t(1) << 24;
 inline bool tc_pays(const ndb_ctx *ctx, int64_t nv, uint32_t flags) {
     return (flags & (NDB_FLAG_FULL_COUNT | NDB_FLAG_TENSOR_FILTER)) || ctx->tuning.tc_min_dim > 0 ||
            nv >= kTcEarlyPoints || getenv("NDB_TC_MIN_DIM") != nullptr;
 }
+
+// Whether the CUDA-core count of an eligible pipeline that does not start on the tensor cores
+// may hand items on to them (kDeferDim).  Up to 65,536 points its launch waves are short
+// enough that nothing is gained (16-D 66,000 points of which none is done early 4.1 ms both
+// ways), and the extra launch would show.
+inline bool may_defer(int d, int64_t nv) { return d >= kDeferDim && nv > (int64_t(1) << 16); }
 
 // The FMA sum with the exact one near eps^2 (count_kernel, kDirect): not the plain form,
 // and eps^2 far enough from underflow for its error bound, and from overflow for both sums
@@ -762,17 +771,18 @@ template <int D>
 void launch_count_tc(ndb_ctx *ctx, int64_t max_chunks, const int2 *chunks, const uint32_t *n_chunks, int chunk,
                      const int32_t *cell_start, const int2 *nbr, int n_rows, const float *xs, float e2, int min_pts,
                      bool early, int32_t *nn_sorted, int32_t *list, int list_cap, int list_stride,
-                     const JobDev *jobs, const int32_t *cell_job, bool audit) {
+                     const JobDev *jobs, const int32_t *cell_job, bool audit, bool records = true) {
     if constexpr (D >= tc::kMinDim) {
         cudaStream_t st = ctx->stream;
         unsigned long long *counters = small_at<unsigned long long>(ctx, kSmallCountersOff);
         unsigned int *work = reinterpret_cast<unsigned int *>(counters + 6);
-        fill_bytes(ctx, work, 0, sizeof(unsigned long long), st);
+        if (jobs) fill_bytes(ctx, work, 0, sizeof(unsigned long long), st);  // a single job's is zero
         // the chunks' records (stencil rows as point ranges), which the kernel fetches
         // one chunk ahead by bulk copies; without room for them (a memory cap, the
-        // allocation-free entry point) the kernel gathers the rows itself
+        // allocation-free entry point) or for a list that is often empty (records false) the
+        // kernel gathers the rows itself
         int2 *rec = nullptr;
-        if (grow(ctx, ctx->tc_rec, (size_t)max_chunks * tc::kRecBytes) == cudaSuccess) {
+        if (records && grow(ctx, ctx->tc_rec, (size_t)max_chunks * tc::kRecBytes) == cudaSuccess) {
             rec = ctx->tc_rec.as<int2>();
             ++launch_counter(), tc::tc_records_kernel<<<blocks_for(max_chunks * kWarp), kBlock, 0, st>>>(
                 chunks, n_chunks, cell_start, nbr, n_rows, cell_job, chunk, early ? 0 : 1, rec);
@@ -824,7 +834,7 @@ template <int D>
 void count_items(ndb_ctx *ctx, bool tc, bool force_tc, bool gram, bool direct, bool early, int64_t n_items, const int2 *items,
                  const int32_t *cell_start, const int2 *nbr, int n_rows, const float *xs, float e2, int min_pts,
                  int dense_skip, int32_t *nn_sorted, int32_t *list, int list_cap, int list_stride,
-                 const JobDev *jobs, const int32_t *cell_job, bool audit, int64_t nv, int64_t n_cells, bool sparse) {
+                 const JobDev *jobs, const int32_t *cell_job, bool audit, int64_t nv, int64_t n_cells, bool sparse, bool defer) {
     if (n_items <= 0) return;  // an upper bound; the count is scalar 1
     cudaStream_t st = ctx->stream;
     unsigned long long *counters = small_at<unsigned long long>(ctx, kSmallCountersOff);
@@ -854,26 +864,30 @@ void count_items(ndb_ctx *ctx, bool tc, bool force_tc, bool gram, bool direct, b
         if (early || (sparse && !tc))  // not beside the tensor-core count, which counts for both ends
             ++launch_counter(), count_kernel<D, M><<<grid, kCountWarps * kWarp, 0, st>>>(
                 ex_items, ex_n, cell_start, nbr, n_rows, xs, e2, min_pts, dense_skip, early ? 0 : 1, nn_sorted, list,
-                list_cap, list_stride, counters + 2, jobs, cell_job, counters + 5);
+                list_cap, list_stride, counters + 2, jobs, cell_job, counters + 5,
+                defer ? ctx->keys1.as<int2>() : nullptr, scal + 4);
         else
             ++launch_counter(), count_full_kernel<D, M><<<grid, kCountWarps * kWarp, 0, st>>>(
                 ex_items, ex_n, cell_start, nbr, n_rows, xs, e2, nn_sorted, list, list_cap, list_stride, counters + 2,
                 jobs, cell_job, counters + 5);
     };
-    if constexpr (D >= 8) {
-        if (gram) {
-            launch(std::integral_constant<int, kGram>{});
-            ck(ctx, cudaGetLastError());
-            return;
-        }
-    }
-    if constexpr (D >= 4) {
-        if (direct) launch(std::integral_constant<int, kDirect>{});
-        else launch(std::integral_constant<int, kExact>{});
+    // the items that the CUDA-core count may hand on, and its votes (see kDeferDim); the list
+    // lies in the sort's spent keys: 8 bytes for at least 16 points
+    if (defer && jobs) fill_bytes(ctx, scal + 4, 0, 4 * sizeof(uint32_t), st);  // a single job's are zero
+    if (D >= 8 && gram) {
+        if constexpr (D >= 8) launch(std::integral_constant<int, kGram>{});
+    } else if (D >= 4 && direct) {
+        if constexpr (D >= 4) launch(std::integral_constant<int, kDirect>{});
     } else {
         launch(std::integral_constant<int, kExact>{});
     }
     ck(ctx, cudaGetLastError());
+    if constexpr (D >= kDeferDim) {
+        if (defer)
+            launch_count_tc<D>(ctx, nv / kDeferPoints + 1, ctx->keys1.as<int2>(), scal + 4, tc::kN, cell_start, nbr,
+                               n_rows, xs, e2, min_pts, true, nn_sorted, list, list_cap, list_stride, jobs, cell_job,
+                               false, false);
+    }
 }
 
 // Neighbour counts and core flags of a pipeline.
@@ -886,7 +900,7 @@ void count_phase(ndb_ctx *ctx, const Pipe &p, bool tc, bool gram, bool direct, u
     count_items<D>(ctx, tc, (flags & NDB_FLAG_TENSOR_FILTER) != 0, gram, direct, p.early, p.items, ctx->items.as<int2>(),
                    ctx->cell_start.as<int32_t>(), ctx->nbr.as<int2>(), p.stencil->n_rows, ctx->xs.as<float>(), p.e2,
                    p.min_pts, p.linked, ctx->nn_sorted.as<int32_t>(), p.list, p.list_cap, p.list_stride, p.jobs,
-                   p.cell_job, (flags & NDB_FLAG_FILTER_AUDIT) != 0, p.nv, p.cells, p.sparse);
+                   p.cell_job, (flags & NDB_FLAG_FILTER_AUDIT) != 0, p.nv, p.cells, p.sparse, p.defer);
     cudaEventRecord(ctx->kev[3], st);
     ensure(ctx, ctx->core_sorted, n + 1);
     ensure(ctx, ctx->core_prefix, (n_words + 1) * sizeof(uint32_t));
@@ -943,6 +957,7 @@ Pipe ctx_pipe(ndb_ctx *ctx) {
     p.list_cap = p.list_stride = ctx->list_cap;
     p.cells = ctx->n_cells;
     p.sparse = ctx->sparse;
+    p.defer = ctx->tc_defer;
     p.items = ctx->n_items;
     return p;
 }
@@ -1200,7 +1215,8 @@ void classify_stats(ndb_ctx *ctx, const Tally &t) {
     ndb_stats &S = ctx->stats;
     S.n_cells = t.scal[0];
     S.n_tiles = t.scal[1];
-    S.tensor_items = ctx->tc_count ? t.scal[4] : 0;
+    S.tensor_items = ctx->tc_count || ctx->tc_defer ? t.scal[4] : 0;
+    if (ctx->tc_defer) S.tensor_filter = t.scal[4] > 0 ? 1 : 0;
     S.count_pairs = (int64_t)(t.counters[2] + t.counters[7]);
     S.count_pair_dims = S.count_pairs * D;
     S.count_fp32_ops = fp32_ops(D, ctx->gram_count, direct_eligible(ctx->e2, ctx->flags_run), (int64_t)t.counters[2],
@@ -1298,8 +1314,9 @@ ndb_status classify_impl(ndb_ctx *ctx, const float *coords, int64_t n, float eps
     ctx->n_rows = pl.st.n_rows;
     ctx->cell_units = pl.cell_units ? 1 : 0;
     if (pl.st.n_rows > kWarp) return NDB_ERR_INVALID_ARGUMENT;  // row tables hold one row per lane
-    ctx->tc_count = tc_eligible(ctx, D, ctx->e2, lo, hi, pl.cell_units, pl.st.n_rows, flags) &&
-                    tc_pays(ctx, ctx->nv, flags);
+    const bool tc_ok = tc_eligible(ctx, D, ctx->e2, lo, hi, pl.cell_units, pl.st.n_rows, flags);
+    ctx->tc_count = tc_ok && tc_pays(ctx, ctx->nv, flags);
+    ctx->tc_defer = tc_ok && !ctx->tc_count && may_defer(D, ctx->nv);
     ctx->gram_count = gram_eligible(ctx, D, ctx->e2, lo, hi, flags);
 
     classify_dispatch<D>(ctx, pl);
@@ -1333,7 +1350,7 @@ ndb_status classify_impl(ndb_ctx *ctx, const float *coords, int64_t n, float eps
     ctx->stats.stencil_rows = pl.st.n_rows;
     ctx->stats.same_cell_linked = ctx->cell_units;
     ctx->stats.key_bits = pl.key_bits;
-    ctx->stats.tensor_filter = ctx->tc_count ? 1 : 0;
+    ctx->stats.tensor_filter = ctx->tc_count ? 1 : 0;  // with tc_defer: see classify_stats
     ctx->have_state = true;
     if (ctx->in_run) {
         // ndb_b200_run goes on with the label phase, which reads these counters with
@@ -1869,6 +1886,7 @@ struct BatchPlan {
     int linked = 0;
     int list_stride = 0;
     bool tc = false;  // neighbour count on the tensor-core filter (every job eligible)
+    bool defer = false;  // the CUDA-core count may hand items on to it
     bool gram = true; // CUDA-core count with the Gram filter (every job eligible)
     bool direct = true;  // the FMA sum (every job eligible)
     int64_t total_n = 0, nv = 0;
@@ -1897,6 +1915,7 @@ void run_group_keys(ndb_ctx *ctx, ndb_job *jobs, const std::vector<int> &members
     p.columns = (double)bp.columns;
     p.linked = bp.linked != 0;
     p.early = (flags & NDB_FLAG_FULL_COUNT) == 0;
+    p.defer = bp.defer;
     p.jobs = jobs_dev;
     p.n_jobs = nj;
     cudaEventRecord(ctx->ev[0], st);
@@ -1956,7 +1975,7 @@ void run_group_keys(ndb_ctx *ctx, ndb_job *jobs, const std::vector<int> &members
     memcpy(h_pairs, m_pairs, sizeof(h_pairs));
     memcpy(h_audit, m_audit, sizeof(h_audit));
     const std::vector<unsigned long long> h_jc(m_jc, m_jc + (size_t)4 * nj);
-    const uint32_t h_tc_items = bp.tc ? m_scal[4] : 0;
+    const uint32_t h_tc_items = bp.tc || bp.defer ? m_scal[4] : 0;
     const int n_rows = bp.st.n_rows;
     const int h_err = *m_err;
     // statistics summed over the pipelines of one batched call
@@ -1969,7 +1988,7 @@ void run_group_keys(ndb_ctx *ctx, ndb_job *jobs, const std::vector<int> &members
     S.band_pairs = (int64_t)h_pairs[3];
     audit_stats(S, h_audit);
     S.tensor_items += h_tc_items;
-    S.tensor_filter |= bp.tc ? 1 : 0;
+    S.tensor_filter |= bp.tc || h_tc_items ? 1 : 0;
     S.count_pairs += dc;
     S.union_pairs += du;
     S.border_pairs += db;
@@ -2117,7 +2136,9 @@ void run_group(ndb_ctx *ctx, ndb_job *jobs, const std::vector<int> &members, uin
         return;
     }
     bp.nv = nv;
-    bp.tc = bp.tc && tc_pays(ctx, nv, flags);
+    const bool tc_ok = bp.tc;
+    bp.tc = tc_ok && tc_pays(ctx, nv, flags);
+    bp.defer = tc_ok && !bp.tc && may_defer(D, nv);
     // the all-ones key of invalid points must exceed every composite key
     int bits = 1;
     while (bits < 64 && ldexp(1.0, bits) - 1.0 < (double)key_base) ++bits;

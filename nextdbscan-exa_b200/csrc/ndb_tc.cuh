@@ -448,6 +448,8 @@ __global__ void __launch_bounds__(kThreads, TcBlocks<D>::v) count_tc_kernel(
     __shared__ float s_nmax;
 
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const int64_t n_items = *n_chunks_dev;
+    if (n_items == 0) return;  // an empty list (often, when the CUDA-core count may hand items on)
     if (warp == 0) {
         tmem_alloc(&s_tmem, kTmemCols);
         tmem_relinquish();
@@ -464,7 +466,6 @@ __global__ void __launch_bounds__(kThreads, TcBlocks<D>::v) count_tc_kernel(
     __syncthreads();
     tc_after_sync();
     const uint32_t tmem = s_tmem;
-    const int64_t n_items = *n_chunks_dev;
     uint32_t phase = 0, pending = 0;  // per buffer: parity of its next completion; MMAs not yet waited for
     unsigned long long pairs = 0, band = 0;
     const float kap = kappa<KP>();
