@@ -726,10 +726,10 @@ inline bool gram_eligible(const ndb_ctx *ctx, int d, float e2, const double *lo,
 // CTA: 16-D 200k 1.05 against 1.28 ms, 16-D 1M 14.1 against 16.8 ms, 12-D 1M 6.7 against 9.5
 // ms, a 512-job batch (5M points at d = 16) 13.9 against 14.5 ms; the 4,096-job batch (40M)
 // 122 against 116 ms.  Below that, items whose points are not done early go there all the
-// same (may_defer).  A caller's flag or tuning decides alone.
+// same (may_defer).  A caller's flag (an audit needs the filter) or tuning decides alone.
 constexpr int64_t kTcEarlyPoints = int64_t(1) << 24;
 inline bool tc_pays(const ndb_ctx *ctx, int64_t nv, uint32_t flags) {
-    return (flags & (NDB_FLAG_FULL_COUNT | NDB_FLAG_TENSOR_FILTER)) || ctx->tuning.tc_min_dim > 0 ||
+    return (flags & (NDB_FLAG_FULL_COUNT | NDB_FLAG_TENSOR_FILTER | NDB_FLAG_FILTER_AUDIT)) || ctx->tuning.tc_min_dim > 0 ||
            nv >= kTcEarlyPoints || getenv("NDB_TC_MIN_DIM") != nullptr;
 }
 

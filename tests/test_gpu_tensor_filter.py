@@ -171,3 +171,17 @@ def test_filter_audit_every_pair_within_its_bound(ctx, pkg, full):
     if full:
         np.testing.assert_array_equal(nn_a, nn)
     assert res_a == res
+
+
+def test_an_audit_runs_the_filter_where_the_default_would_not(ctx):
+    """16-D with the early exit: the audit alone chooses the filter, as at sizes that take it
+    by default."""
+    rng = np.random.default_rng(7)
+    x = (rng.integers(0, 4, (6000, 1)) * 8 + rng.normal(0, 0.6, (6000, 16))).astype(np.float32)
+    nn, ci, res = ctx.run(x, 3.0, 12)
+    nn_a, ci_a, res_a = ctx.run(x, 3.0, 12, audit=True)
+    s = ctx.stats()
+    assert s["tensor_filter"] == 1 and s["filter_audited_pairs"] > 0 and s["filter_misclassified_pairs"] == 0
+    np.testing.assert_array_equal(ci_a, ci)
+    np.testing.assert_array_equal(np.minimum(nn_a, 12), np.minimum(nn, 12))
+    assert res_a == res
