@@ -810,19 +810,17 @@ void launch_count_tc(ndb_ctx *ctx, int64_t max_chunks, const int2 *chunks, const
 
 // Points per chunk of the tensor-core count.  Full counts: the 32 columns of one round,
 // since every point needs the whole round (8-D 2M: 8.5 ms; 256 points 10.2 ms, a longer
-// tail).  Early exit: enough to keep the columns filled (a chunk's last points run with
-// ever fewer), few enough that every resident CTA gets several chunks: 16-D 200k 64
-// points 1.40 ms, 256 points 2.23 ms; the 4,096-job batch's counts 32 points 143 ms, 64
-// 128 ms, 256 117 ms, 512 116 ms.  A larger minPts makes a chunk longer and its points more
-// alike, so from 32 on a CTA gets ten chunks instead of four where that leaves 64 points,
-// and from 512 on, where most points need the whole round, a chunk has no more than 64: at
-// 16-D 1M chunks of 64, 128 and 256 points take 18.6, 18.0 and 21.5 ms at minPts 32, 20.3,
-// 21.1 and 25.1 ms at 64, and 26.1, 26.8 and 32.6 ms at 1,024; 12-D 1M at minPts 24, where
-// points are done early, 8.7, 6.5 and 5.5 ms.
+// tail).  Early exit: up to 256, which keep the columns filled (a chunk's last points run with
+// ever fewer), but no more than leave every resident CTA forty chunks.  Where points are done
+// early long chunks gain (the 4,096-job batch's counts 32 points 143 ms, 64 128 ms, 256 117
+// ms, 512 116 ms; 16-D 1M at minPts 32, when asked for, 19.3 ms by 32 and 14.2 by 64); where
+// they are not, each takes 2 to 8 whole rounds and the last ones make a tail (12-D 1M without a
+// core 114 ms by 32, 119 by 64 and 153 by 256; 8-D 300k 3.5 by 32 and 4.3 by 64).  From minPts
+// 512 on, where most points need the whole round, a chunk has no more than 64 (16-D 1M at
+// 1,024: 64, 128 and 256 points 26.1, 26.8 and 32.6 ms).
 inline int tc_chunk(const ndb_ctx *ctx, int64_t nv, int min_pts, bool early) {
     if (!early) return tc::kN;
-    const int64_t ctas = (int64_t)ctx->sm_count * 5, chunks = min_pts >= 32 ? 10 : 4;
-    const int64_t per = std::max(std::min<int64_t>(nv / (ctas * 4), 2 * tc::kN), nv / (ctas * chunks));
+    const int64_t per = nv / ((int64_t)ctx->sm_count * 5 * 40);
     const int64_t most = min_pts >= 512 ? 2 * tc::kN : 8 * tc::kN;
     return (int)std::min<int64_t>(std::max<int64_t>(per / tc::kN * tc::kN, tc::kN), most);
 }

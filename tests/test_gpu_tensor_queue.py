@@ -1,6 +1,6 @@
 """The tensor-core count with the early exit where its chunks change length: chunks are
 equal shares of a cell of at most 32 to 256 points, by the points of the run and minPts, and
-a chunk's points wait for a column.  Runs of 100,000 to 800,000 points in cells of every
+a chunk's points wait for a column.  Runs of 100,000 to 8M points in cells of every
 ragged size against the plain count, exact integers."""
 import numpy as np
 import pytest
@@ -20,7 +20,7 @@ def ragged(n, d, seed):
     return np.ascontiguousarray(x[rng.permutation(n)].astype(np.float32))
 
 
-# chunks of 32 points; 64 (200,001); 128 and 64 (400,003); 256, 96 and 64 (800,011)
+# chunks of 32 points (or more, by the rule that lays them out)
 @pytest.mark.parametrize("d,n", [(8, 100_000), (8, 800_011), (12, 400_003), (16, 200_001), (16, 800_011)])
 @pytest.mark.parametrize("m", [5, 32, 60, 300, 600])
 def test_queue_against_the_plain_count(ctx, d, n, m):
@@ -31,3 +31,10 @@ def test_queue_against_the_plain_count(ctx, d, n, m):
     np.testing.assert_array_equal(np.minimum(nn, m), np.minimum(nn_e, m))
     np.testing.assert_array_equal(ci, ci_e)
     assert r == r_e
+
+
+# chunks of 64 points; 96 (64 from minPts 512 on); 256
+@pytest.mark.parametrize("d,n", [(9, 1_900_003), (16, 2_900_011), (8, 8_000_003)])
+@pytest.mark.parametrize("m", [5, 60, 600])
+def test_long_chunks_against_the_plain_count(ctx, d, n, m):
+    test_queue_against_the_plain_count(ctx, d, n, m)
