@@ -724,10 +724,14 @@ def roofline(kind, ms, s, n, hbm_peak, peak_src, clk):
     """Algorithmic work of one launch / its device time."""
     if kind == "radix_sort":
         kb = s["key_bytes"]
-        # per pass: upsweep reads keys; downsweep reads and writes (key, id)
+        # credited per pass: a read of the keys for the digit histogram, and (key, id) read and
+        # written.  The kernels read the keys once for the histograms of all passes and the
+        # first pass reads no ids, so what moves is up to a quarter less: "moved" below
         per_pass = s["n_valid"] * (kb + 2 * (kb + 4))
-        achieved = per_pass * s["sort_passes"] / max(s.get("pipelines") or 1, 1) / (ms / 1000.0) / 1e9
-        return {"kernel": "radix_sort (all passes)", "bound": "hbm", "achieved": achieved, "peak": hbm_peak,
+        passes = s["sort_passes"] / max(s.get("pipelines") or 1, 1)
+        achieved = per_pass * passes / (ms / 1000.0) / 1e9
+        moved = s["n_valid"] * (kb - 4 + passes * 2 * (kb + 4)) / (ms / 1000.0) / 1e9
+        return {"kernel": "radix_sort (all passes)", "moved": moved, "bound": "hbm", "achieved": achieved, "peak": hbm_peak,
                 "unit": "GB/s", "frac": achieved / hbm_peak, "traffic": None,
                 "peak_source": f"{peak_src} hbm_gbs"}
     if kind == "union_kernel":
