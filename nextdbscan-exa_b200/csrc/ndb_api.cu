@@ -149,7 +149,9 @@ constexpr size_t kSmallCountersOff = 512;    // u64[12]: 0 clusters 1 noise 2 co
                                              // 4 border pairs 5 band pairs 6 work counter of the persistent count
                                              // kernel 7 count pairs on tensor cores 8..11 filter audit (tc::audit_tile)
 constexpr int kCounters = 12;
-constexpr size_t kSmallScalarOff = 1024;     // u32[8]: 0 n_cells 1 n_items 2 n_cores 4 tensor items 5 exact items 6 and 7 union segments (u64); 7 tensor chunks before
+constexpr size_t kSmallScalarOff = 1024;     // u32[8]: 0 n_cells 1 n_items 2 n_cores 4 tensor items 5 exact items
+                                             // (or votes, and 6 votes no: kDeferDim) 7 tensor chunks; then 6 and 7
+                                             // union segments (u64)
 constexpr size_t kSmallErrOff = 1536;        // int
 constexpr size_t kSmallDoneOff = 1600;       // u32[2]: blocks done of bbox_kernel and finish_kernel (mail_last_block)
 constexpr size_t kSmallBytes = 2048;
@@ -705,7 +707,7 @@ inline bool tc_eligible(const ndb_ctx *ctx, int d, float e2, const double *lo, c
     return true;
 }
 
-// The Gram-filtered count on CUDA cores (count_kernel<D, E, true>), when asked for
+// The Gram-filtered count on CUDA cores (count_kernel<D, kGram>), when asked for
 // (NDB_FLAG_GRAM_FILTER or the context's tuning; measured on B200 it does not beat
 // the exact sum, whose cost there is latency rather than FP32 issue): d >= 8, not the
 // plain form (NDB_FLAG_EXACT_COUNT), eps^2 a normal float far from under- and

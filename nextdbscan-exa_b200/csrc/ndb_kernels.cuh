@@ -463,9 +463,6 @@ __device__ __forceinline__ int find_cell(const CellIndex<K> &L, const K *__restr
     return a < cr.y && __ldg(cell_key + a) == (K)key ? a : -1;
 }
 
-// nbr[c * n_rows + r] = [first, last) cell index of row r around cell c: the cells
-// of a row have consecutive keys, so the existing ones are consecutive in the
-// sorted cell list and the range runs from the smallest to the largest found.
 // Cell coordinates from a key (x fastest); 32-bit arithmetic for 32-bit keys.
 template <typename K>
 __device__ __forceinline__ void decode_key(K key, const GridDev &g, long long (&c)[kMaxGridDims]) {
@@ -666,8 +663,8 @@ __device__ __forceinline__ int row_next(const RowTable &rt, int &row, int t) {
 // stencil rows 32 at a time (coalesced loads), every lane tests its candidate j
 // against each i (broadcast reads), and transposed hit masks give that i's count.
 // Rows are ordered nearest first.
-// EARLY: stop once every i of the item has reached min_pts (exact counts below
-// min_pts, so exact core flags).  dense_skip: with same-cell-linked cells a cell
+// It stops once every i of the item has reached min_pts (exact counts below min_pts, so
+// exact core flags), or with `all` at the end of the candidates (exact counts).  dense_skip: with same-cell-linked cells a cell
 // of >= min_pts points is all cores (every pair inside it is in range), so its
 // points need no test at all; they report the cell size.
 // ---------------------------------------------------------------------------
