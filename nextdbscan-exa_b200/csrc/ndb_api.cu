@@ -661,9 +661,12 @@ void grid_phase(ndb_ctx *ctx, Pipe &p, const float *coords, F launch_keys) {
 
     // work items: at most one per cell and one more per 32 points
     p.items = std::min(nv, p.cells + nv / kTile);
+    // a context's first run, whose allocations cost more than a round trip (kNoCountTable),
+    // and one under a cap wait for their number: the tensor-core count's buffers follow it
+    const bool counted = sizes_counted(ctx) || (ctx->tc_count && !p.jobs && ctx->items.bytes == 0);
     ensure(ctx, ctx->items, (p.items + 1) * sizeof(int2));
     ensure(ctx, ctx->cell_has_core, p.cells + 1);
-    const char *m_items = sizes_counted(ctx) ? mail_slice(ctx, sizeof(uint32_t)) : nullptr;
+    const char *m_items = counted ? mail_slice(ctx, sizeof(uint32_t)) : nullptr;
     ++launch_counter(), chain_scan_kernel<kItemsPer><<<(unsigned)chain_tiles(p.cells, kItemsPer), kChainThreads, 0, st>>>(
         ItemsOp{ctx->cell_start.as<int32_t>(), ctx->items.as<int2>(), ctx->cell_has_core.as<uint8_t>()}, p.cells,
         scal + 0, chain.state[1], chain.ticket + 1, scal + 1, m_items ? mail_device(ctx, m_items) : nullptr);
