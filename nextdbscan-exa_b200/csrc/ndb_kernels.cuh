@@ -703,8 +703,8 @@ constexpr float kGramSigma = 8.0f / 16777216.0f;
 // Packing: points that reached min_pts leave the item.  The remaining ones move to the
 // first slots (coordinates in shared memory, count and index with their lane), so the
 // pair loop always runs over a dense range of slots.
-// Bound: instruction issue and the FMA pipe (8-D early exit: 28 thread instructions per
-// pair, FMA pipe 63 %).  The form before this one voted and updated counts and lists per
+// Bound: instruction issue and the FMA pipe (8-D early exit: 23 thread instructions per
+// pair, issue 60 %, FMA pipe 54 %).  The form before this one voted and updated counts and lists per
 // pair and step (58 instructions per pair).  Measured on B200, before and after: 8-D 2M
 // early exit 4.47 -> 2.69 ms, 2-D 100k full counts 0.565 -> 0.213 ms, 3-D 1M full
 // counts 1.63 -> 0.89 ms, 5-D 300k full counts 2.84 -> 1.56 ms.
@@ -864,16 +864,17 @@ constexpr int kExact = 0, kDirect = 1, kGram = 2;
 // defer provides; an item whose points are done soon costs less here.  Which it is depends
 // on the data, so items vote: after 1/64 of its candidates an item says whether its points
 // would reach min_pts at the rate of hits so far (n_defer: 0 items handed on, 1 votes, 2
-// votes for), and when at least half of kDeferVotes or more votes say no, every item hands
-// itself on at that look or at one of the next (1/32, 1/16, 1/8).  Only items of at least
+// votes against).  Once there are kDeferVotes votes, two per CTA of the tensor-core count, and
+// at least half of them are against, items hand themselves on at that look; an item that
+// looks before there are as many looks again at 1/32, 1/16 and 1/8.  Only items of at least
 // kDeferCandidates candidates and kDeferPoints unfinished points take part: below, a tile of
-// the tensor cores is not filled.  An item handed on is counted again from its first candidate.
-// Measured on B200 (count phase, never against always handed on against this): 16-D 1M of
-// which 9 % are core (minPts 64) 37.3, 30.9 and 30.2 ms, 16-D 200k without a core 26.4, 24.5
-// and 20.6 ms; where most points are done early 16-D 1M 12.5, 20.2 and 12.3 ms, 13-D 400k 9.3,
-// 17.8 and 9.3 ms.  By each item's own forecast instead of the vote the few that hand on make
-// a tail of their own (16-D 1M 13.9 ms).
-constexpr int kDeferDim = 12, kDeferPoints = 16, kDeferCandidates = 8192, kDeferVotes = 128;
+// the tensor cores is not filled.  An item handed on is counted again from its first
+// candidate.  Measured on B200 (count phase: always here, always handed on, this): 16-D 1M of
+// which 9 % are core (minPts 64) 37.4, 30.9 and 30.3 ms, 16-D 200k without a core 26.7, 25.2
+// and 20.7 ms; where most points are done early 16-D 1M 12.6, 20.2 and 12.3 ms, 13-D 400k 9.2,
+// 17.7 and 9.3 ms.  With fewer votes (128), or by each item's own forecast, the few that hand
+// on make a tail of their own (16-D 200k 1.57 against 1.24 ms, 1M 13.9 against 12.3).
+constexpr int kDeferDim = 12, kDeferPoints = 16, kDeferCandidates = 8192, kDeferVotes = 1480;
 
 template <int D, int MODE>
 __global__ void __launch_bounds__(kCountWarps * kWarp) count_kernel(
@@ -972,17 +973,18 @@ __global__ void __launch_bounds__(kCountWarps * kWarp) count_kernel(
                             atomicAdd(n_defer + 2, 1u);
                     }
                 }
-                look = look < (total >> 3) ? 2 * look : -1;
-                int go = 0;
+                int go = 0;  // 1: hand on, -1: too few votes yet
                 if (lane == 0 && nk >= kDeferPoints) {
                     const uint32_t votes = __ldcg(n_defer + 1), no = __ldcg(n_defer + 2);
-                    go = votes >= kDeferVotes && 2 * no >= votes;
-                    if (go) {
+                    go = votes < kDeferVotes ? -1 : 2 * no >= votes;
+                    if (go > 0) {
                         defer[atomicAdd(n_defer, 1u)] = item;
                         atomicAdd(pair_counter, pairs);
                     }
                 }
-                if (__shfl_sync(kFull, go, 0)) return;
+                go = __shfl_sync(kFull, go, 0);
+                if (go > 0) return;
+                look = go < 0 && look < (total >> 3) ? 2 * look : -1;
             }
         }
         int j[CH];
