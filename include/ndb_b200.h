@@ -304,7 +304,7 @@ const char *ndb_b200_version(void);
  * buffer request beyond its slice of the array returns NDB_ERR_OUT_OF_MEMORY (the
  * slices are sized for the largest request of any job within the limit).
  * The first call on a device does the set-up (it looks up the array's device
- * address, pins 16 KiB of host memory for the calls' small transfers and creates the
+ * address, pins 4 KiB of host memory for the calls' small transfers and creates the
  * shared state's timing events), so make it before any stream capture and where an
  * allocation may synchronise the device; n = 0 is enough.  Calls share the array:
  * they are serialised per device, and GPU work that overlaps a call and touches the

@@ -222,7 +222,10 @@ inline void fill_bytes(ndb_ctx *ctx, void *p, int v, size_t bytes, cudaStream_t 
     ck(ctx, cudaGetLastError());
 }
 
-constexpr size_t kMailSingle = 16 * 1024;  // a single job's transfers: bounds, cell count, counters
+// a single job's transfers: bounds, cell and item counts, counters (1.4 KB).  The driver hands
+// out small ones from a block it has pinned, and a new block costs milliseconds: with many
+// contexts alive 16 KB each met that several times as often.
+constexpr size_t kMailSingle = 4 * 1024;
 
 // The mailbox holds at least `bytes`; grown only between runs (nothing of the
 // context in flight).

@@ -983,7 +983,13 @@ __global__ void __launch_bounds__(kCountWarps * kWarp) count_kernel(
                     }
                 }
                 go = __shfl_sync(kFull, go, 0);
-                if (go > 0) return;
+                if (go > 0) {
+                    if constexpr (GRAM) {
+                        band = __reduce_add_sync(kFull, band);
+                        if (lane == 0 && band) atomicAdd(band_counter, (unsigned long long)band);
+                    }
+                    return;
+                }
                 look = go < 0 && look < (total >> 3) ? 2 * look : -1;
             }
         }
